@@ -220,293 +220,485 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
 }
 
 // =====================================================================================
-// Chunked form, stage 1 (fully parallel over chunks): per (b, hv, chunk) compute
+// Chunked form in fp32 on CUDA cores, for every geometry the tensor-core kernels do not take (fp32 inputs, K or V other
+// than 128).  Chunks are always 64 tokens (zero rows pad the last one): the mathematics does not depend on the chunk
+// length, and a longer chunk means fewer dependent steps in stage 2.  K is padded to KT = 64 or 128 channels.
+//
+// Stage 1, one CTA of 4*KT threads per (b, hv, chunk), all chunks in parallel:
 //   gamma = cumsum(g), A (strictly lower), Tm = (I+A)^-1 diag(beta),
 //   w = Tm (exp(gamma) k), u = Tm v, Aqk (lower incl. diagonal),
 //   qg = scale q exp(gamma), kg = k exp(gamma_last - gamma), dl = exp(gamma_last)
-// and store them in the workspace for the sequential stage.
+// into one record per chunk that stage 2 streams.  Bound: instruction issue.  What made it long was one exponential
+// per (i, j, channel): 262 K of them per chunk and a 64-deep serial substitution.  Now the exponent difference is
+// factored around a row between the two halves of a block (both factors <= 1 for a decay, so nothing overflows, and
+// what underflows is smaller still), halving the blocks from 32 to 4 rows: 8 K exponentials a level and plain products;
+// only the 4 x 4 diagonal blocks take the difference pair by pair.  The inverse is built from 8 x 8 blocks upwards.
+// 1024 tokens, 4 heads, K = V = 128, fp32: 202 -> 42 us.
+// A chunk whose gate is positive or not finite somewhere takes every pair directly (exponent clamped at 50).
 // =====================================================================================
-#define KDA_CMAX 64
+#define KC_C 64
+#define KC_AS 68                       // row stride of the 64 x 64 tiles (16-byte rows, 8 rows on 32 banks)
 
-struct KdaChunkWs {
-  float *w, *qg, *kg;   // [B,HV,Tp,K]
-  float *u;             // [B,HV,Tp,V]
-  float *aqk;           // [B,HV,NT,C,C]
-  float *dl;            // [B,HV,NT,K]
-};
+// one chunk record, in floats: w, qg, kg [64][KT+4]; Aqk [64][68]; dl [KT]; u [V/8][64][8]
+__host__ __device__ inline int64_t kc_record_floats(int KT, int V) {
+  return 3ll * KC_C * (KT + 4) + KC_C * KC_AS + KT + (int64_t)((V + 7) / 8) * 8 * KC_C;
+}
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int KT>
+__global__ void __launch_bounds__(4 * KT)
 kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                         const T* __restrict__ g, const T* __restrict__ beta, KdaChunkWs ws, int T_,
-                         int H, int HV, int K, int V, int C, int NT, float scale, float g_min,
+                         const T* __restrict__ g, const T* __restrict__ beta, float* __restrict__ ws, int T_,
+                         int H, int HV, int K, int V, int NT, float scale, float g_min,
                          int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b) {
-  extern __shared__ float smem[];
+  constexpr int NTH = 4 * KT, KS = KT + 4, NW = NTH / 32;
+  extern __shared__ __align__(16) float smem[];
+  float* sk = smem;                    // [64][KS] k
+  float* sq = sk + KC_C * KS;          // [64][KS] scale * q
+  float* sgam = sq + KC_C * KS;        // [64][KS] running sum of g from the start of the row's segment of 16
+  float* sx = sgam + KC_C * KS;        // [64][KS] k with one side of the factored exponent; later exp(gamma) k, then v
+  float* sy = sx + KC_C * KS;          // [32][KS] the same for q (rows on the i side)
+  float* sT = sy;                      // [64][68] (I + A)^-1, then Tm, once the factors are done with
+  float* sA = sy + (32 * KS > KC_C * KC_AS ? 32 * KS : KC_C * KC_AS);      // [64][68] A
+  float* sbeta = sA + KC_C * KC_AS;    // [64]
+  float* stot = sbeta + KC_C;          // [4][KT] sums over the segments
   const int n = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
-  const int G = HV / H, h = hv / G;
-  const int tid = threadIdx.x;
-  const int KS = K + 1;             // padded row stride
-  float* sk = smem;                 // [C][KS]   k
-  float* sq = sk + C * KS;          // [C][KS]   scale*q, later exp(gamma)*k
-  float* sgam = sq + C * KS;        // [C][KS]   gamma
-  float* sA = sgam + C * KS;        // [C][C+1]  A, then Tm
-  float* sbeta = sA + C * (C + 1);  // [C]
-  const int CS = C + 1;
-  const int t0 = n * C;
-  for (int idx = tid; idx < C * K; idx += 256) {
-    int i = idx / K, kk = idx % K;
-    int t = t0 + i;
+  const int h = hv / (HV / H);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t0 = n * KC_C;
+  float* rec = ws + (((int64_t)b * HV + hv) * NT + n) * kc_record_floats(KT, V);
+  float* o_w = rec;
+  float* o_qg = o_w + KC_C * KS;
+  float* o_kg = o_qg + KC_C * KS;
+  float* o_aqk = o_kg + KC_C * KS;
+  float* o_dl = o_aqk + KC_C * KC_AS;
+  float* o_u = o_dl + KT;
+
+  bool odd_gate = false;
+#pragma unroll 4
+  for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+    const int i = idx / KT, kk = idx % KT, t = t0 + i;
     float kv = 0.f, qv = 0.f, gv = 0.f;
-    if (t < T_) {
-      int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
-      int64_t goff = ((int64_t)b * T_ + t) * ld_g + (int64_t)hv * K + kk;
+    if (t < T_ && kk < K) {
+      const int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
       kv = ldf(k + qoff);
       qv = ldf(q + qoff) * scale;
-      gv = fmaxf(ldf(g + goff), g_min);
+      gv = fmaxf(ldf(g + ((int64_t)b * T_ + t) * ld_g + (int64_t)hv * K + kk), g_min);
+      odd_gate |= !(gv <= 0.f && gv > -1e30f);
     }
     sk[i * KS + kk] = kv;
     sq[i * KS + kk] = qv;
     sgam[i * KS + kk] = gv;
   }
-  for (int i = tid; i < C; i += 256) {
-    int t = t0 + i;
-    sbeta[i] = t < T_ ? ldf(beta + ((int64_t)b * T_ + t) * ld_b + hv) : 0.f;
+  if (tid < KC_C) sbeta[tid] = t0 + tid < T_ ? ldf(beta + ((int64_t)b * T_ + t0 + tid) * ld_b + hv) : 0.f;
+  for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) {
+    sA[idx] = 0.f;
+    if (idx % KC_AS > idx / KC_AS) o_aqk[idx] = 0.f;
   }
-  __syncthreads();
-  // running sum of g over the chunk, one channel per thread
-  for (int kk = tid; kk < K; kk += 256) {
-    float acc = 0.f;
-    for (int i = 0; i < C; ++i) {
-      acc += sgam[i * KS + kk];
-      sgam[i * KS + kk] = acc;
-    }
-  }
-  __syncthreads();
-  const int64_t bh = (int64_t)b * HV + hv;
-  const int64_t Tp = (int64_t)NT * C;
-  // A[i][j] (i>j) and Aqk[i][j] (i>=j): exact per-channel exponent differences
-  float* aqk_out = ws.aqk + (bh * NT + n) * C * C;
-  for (int idx = tid; idx < C * C; idx += 256) {
-    int i = idx / C, j = idx % C;
-    float a = 0.f, aq = 0.f;
-    if (j <= i) {
-      const float* ki = sk + i * KS;
-      const float* kj = sk + j * KS;
-      const float* qi = sq + i * KS;
-      const float* gi = sgam + i * KS;
-      const float* gj = sgam + j * KS;
-      for (int kk = 0; kk < K; ++kk) {
-        float e = expf(fminf(gi[kk] - gj[kk], 50.f)) * kj[kk];
-        a = fmaf(ki[kk], e, a);
-        aq = fmaf(qi[kk], e, aq);
-      }
-    }
-    sA[i * CS + j] = (j < i) ? a * sbeta[i] : 0.f;
-    aqk_out[idx] = aq;
-  }
-  __syncthreads();
-  // qg, kg, dl to the workspace; sq <- exp(gamma) * k for the w product
-  for (int idx = tid; idx < C * K; idx += 256) {
-    int i = idx / K, kk = idx % K;
-    float gm = sgam[i * KS + kk];
-    float gl = sgam[(C - 1) * KS + kk];
-    float eg = expf(gm);
-    int64_t off = (bh * Tp + t0 + i) * K + kk;
-    ws.qg[off] = sq[i * KS + kk] * eg;
-    ws.kg[off] = sk[i * KS + kk] * expf(gl - gm);
-    if (i == 0) ws.dl[(bh * NT + n) * K + kk] = expf(gl);
-  }
-  __syncthreads();
-  for (int idx = tid; idx < C * K; idx += 256) {
-    int i = idx / K, kk = idx % K;
-    sq[i * KS + kk] = expf(sgam[i * KS + kk]) * sk[i * KS + kk];
-  }
-  // (I + A)^-1 by forward substitution; column c is independent of the others
-  float* sT = sgam;  // reuse: [C][CS]  (C*CS <= C*KS needs C <= K; guarded on the host)
-  __syncthreads();
-  for (int c = tid; c < C; c += 256) {
-    for (int i = 0; i < C; ++i) {
-      float x = (i == c) ? 1.f : 0.f;
-      if (i > c) {
-        float acc = 0.f;
-        for (int j = c; j < i; ++j) acc = fmaf(sA[i * CS + j], sT[j * CS + c], acc);
-        x -= acc;
-      }
-      sT[i * CS + c] = (i >= c) ? x : 0.f;
-    }
-  }
-  __syncthreads();
-  for (int idx = tid; idx < C * C; idx += 256) {
-    int i = idx / C, j = idx % C;
-    sT[i * CS + j] *= sbeta[j];
-  }
-  __syncthreads();
-  // w = Tm (exp(gamma) k)
-  for (int idx = tid; idx < C * K; idx += 256) {
-    int i = idx / K, kk = idx % K;
-    float acc = 0.f;
-    for (int j = 0; j <= i; ++j) acc = fmaf(sT[i * CS + j], sq[j * KS + kk], acc);
-    ws.w[(bh * Tp + t0 + i) * K + kk] = acc;
-  }
-  // u = Tm v  (v read straight from global; each element is used by C-j rows)
-  for (int idx = tid; idx < C * V; idx += 256) {
-    int i = idx / V, vv = idx % V;
-    float acc = 0.f;
-    for (int j = 0; j <= i; ++j) {
-      int t = t0 + j;
-      float x = t < T_ ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + vv) : 0.f;
-      acc = fmaf(sT[i * CS + j], x, acc);
-    }
-    ws.u[(bh * Tp + t0 + i) * V + vv] = acc;
-  }
-}
-
-// =====================================================================================
-// Chunked form, stage 2 (sequential over chunks): one CTA owns 32 value columns of one
-// (batch, value head) and keeps that slice of the state in shared memory.
-//   vt = u - w S ; o = qg S + Aqk vt ; S <- diag(dl) S + kg^T vt
-// =====================================================================================
-template <typename T>
-__global__ void __launch_bounds__(256)
-kda_chunk_scan_kernel(KdaChunkWs ws, const float* __restrict__ S0, T* __restrict__ o,
-                      float* __restrict__ S_out, int T_, int HV, int K, int V, int C, int NT) {
-  extern __shared__ float smem[];
-  const int vb = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
-  const int tid = threadIdx.x;
-  const int VS = 32;
-  const int Kp = (K + 3) & ~3;
-  float* sw = smem;                  // [64][Kp]
-  float* sqg = sw + KDA_CMAX * Kp;   // [64][Kp]
-  float* skg = sqg + KDA_CMAX * Kp;  // [64][Kp]
-  float* saqk = skg + KDA_CMAX * Kp; // [64][64]
-  float* svt = saqk + KDA_CMAX * KDA_CMAX;  // [64][VS]  u, then vt
-  float* sS = svt + KDA_CMAX * VS;   // [Kp][VS]
-  float* sdl = sS + Kp * VS;         // [Kp]
-  const int64_t bh = (int64_t)b * HV + hv;
-  const int64_t Tp = (int64_t)NT * C;
-  const int v0 = vb * VS;
-  const int64_t sbase = bh * K * V;
-  for (int idx = tid; idx < Kp * VS; idx += 256) {
-    int kk = idx / VS, vv = idx % VS;
-    sS[idx] = (S0 && kk < K && v0 + vv < V) ? S0[sbase + (int64_t)kk * V + v0 + vv] : 0.f;
-  }
-  // rows >= C of the staging tiles stay zero for the whole kernel
-  for (int idx = tid; idx < KDA_CMAX * Kp; idx += 256) { sw[idx] = 0.f; sqg[idx] = 0.f; skg[idx] = 0.f; }
-  for (int idx = tid; idx < KDA_CMAX * KDA_CMAX; idx += 256) saqk[idx] = 0.f;
-  for (int idx = tid; idx < KDA_CMAX * VS; idx += 256) svt[idx] = 0.f;
-  const int ty = tid >> 3, tx = tid & 7;  // rows 2ty,2ty+1 ; cols 4tx..4tx+3
-  __syncthreads();
-  for (int n = 0; n < NT; ++n) {
-    const int64_t row0 = bh * Tp + (int64_t)n * C;
-    for (int idx = tid; idx < C * K; idx += 256) {
-      int i = idx / K, kk = idx % K;
-      int64_t off = (row0 + i) * K + kk;
-      sw[i * Kp + kk] = ws.w[off];
-      sqg[i * Kp + kk] = ws.qg[off];
-      skg[i * Kp + kk] = ws.kg[off];
-    }
-    for (int idx = tid; idx < C * C; idx += 256)
-      saqk[(idx / C) * KDA_CMAX + (idx % C)] = ws.aqk[(bh * NT + n) * C * C + idx];
-    for (int idx = tid; idx < C * VS; idx += 256) {
-      int i = idx / VS, vv = idx % VS;
-      svt[idx] = (v0 + vv < V) ? ws.u[(row0 + i) * V + v0 + vv] : 0.f;
-    }
-    for (int kk = tid; kk < Kp; kk += 256) sdl[kk] = kk < K ? ws.dl[(bh * NT + n) * K + kk] : 1.f;
-    __syncthreads();
-    // wS and qS for rows 2ty, 2ty+1
-    float aw[2][4] = {}, aq[2][4] = {};
-    const int r0 = 2 * ty;
-    for (int kk = 0; kk < Kp; ++kk) {
-      float4 sv = *reinterpret_cast<const float4*>(sS + kk * VS + 4 * tx);
-      float w0 = sw[r0 * Kp + kk], w1 = sw[(r0 + 1) * Kp + kk];
-      float q0 = sqg[r0 * Kp + kk], q1 = sqg[(r0 + 1) * Kp + kk];
-      aw[0][0] = fmaf(w0, sv.x, aw[0][0]); aw[0][1] = fmaf(w0, sv.y, aw[0][1]);
-      aw[0][2] = fmaf(w0, sv.z, aw[0][2]); aw[0][3] = fmaf(w0, sv.w, aw[0][3]);
-      aw[1][0] = fmaf(w1, sv.x, aw[1][0]); aw[1][1] = fmaf(w1, sv.y, aw[1][1]);
-      aw[1][2] = fmaf(w1, sv.z, aw[1][2]); aw[1][3] = fmaf(w1, sv.w, aw[1][3]);
-      aq[0][0] = fmaf(q0, sv.x, aq[0][0]); aq[0][1] = fmaf(q0, sv.y, aq[0][1]);
-      aq[0][2] = fmaf(q0, sv.z, aq[0][2]); aq[0][3] = fmaf(q0, sv.w, aq[0][3]);
-      aq[1][0] = fmaf(q1, sv.x, aq[1][0]); aq[1][1] = fmaf(q1, sv.y, aq[1][1]);
-      aq[1][2] = fmaf(q1, sv.z, aq[1][2]); aq[1][3] = fmaf(q1, sv.w, aq[1][3]);
-    }
-    // vt = u - wS (in place); every thread touches only its own 2x4 tile
+  const bool direct = __syncthreads_or(odd_gate);
+  // running sums: four threads per channel, 16 rows each.  They stay relative to their segment: a difference of two
+  // rows is then put together from short sums (gamma itself grows to tens, and its rounding with it)
+  {
+    const int kk = tid % KT, seg = tid / KT;
+    float r[16], acc = 0.f;
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int i = 0; i < 16; ++i) r[i] = sgam[(16 * seg + i) * KS + kk];
 #pragma unroll
-      for (int cidx = 0; cidx < 4; ++cidx)
-        svt[(r0 + r) * VS + 4 * tx + cidx] -= aw[r][cidx];
-    __syncthreads();
-    // o = qS + Aqk vt
-    for (int j = 0; j < C; ++j) {
-      float4 vv = *reinterpret_cast<const float4*>(svt + j * VS + 4 * tx);
-      float a0 = saqk[r0 * KDA_CMAX + j], a1 = saqk[(r0 + 1) * KDA_CMAX + j];
-      aq[0][0] = fmaf(a0, vv.x, aq[0][0]); aq[0][1] = fmaf(a0, vv.y, aq[0][1]);
-      aq[0][2] = fmaf(a0, vv.z, aq[0][2]); aq[0][3] = fmaf(a0, vv.w, aq[0][3]);
-      aq[1][0] = fmaf(a1, vv.x, aq[1][0]); aq[1][1] = fmaf(a1, vv.y, aq[1][1]);
-      aq[1][2] = fmaf(a1, vv.z, aq[1][2]); aq[1][3] = fmaf(a1, vv.w, aq[1][3]);
-    }
+    for (int i = 0; i < 16; ++i) { acc += r[i]; r[i] = acc; }
+    stot[seg * KT + kk] = acc;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      int i = r0 + r;
-      int t = n * C + i;
-      if (i < C && t < T_) {
-        T* orow = o + (((int64_t)b * T_ + t) * HV + hv) * V + v0 + 4 * tx;
+    for (int i = 0; i < 16; ++i) sgam[(16 * seg + i) * KS + kk] = r[i];
+  }
+  __syncthreads();
+  // A and Aqk below the diagonal blocks, half block size 32, 16, 8, 4
+  if (!direct) {
 #pragma unroll
-        for (int cidx = 0; cidx < 4; ++cidx)
-          if (v0 + 4 * tx + cidx < V) stf(orow + cidx, aq[r][cidx]);
-      }
-    }
-    // S <- diag(dl) S + kg^T vt : thread owns rows kk = 4*ty' .. for a strided set of rows
-    for (int kb = (tid >> 3) * 4; kb < Kp; kb += 128) {
-      float acc[4][4] = {};
-      for (int i = 0; i < C; ++i) {
-        float4 kv = *reinterpret_cast<const float4*>(skg + i * Kp + kb);
-        float4 vv = *reinterpret_cast<const float4*>(svt + i * VS + 4 * tx);
-        const float kr[4] = {kv.x, kv.y, kv.z, kv.w};
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          acc[r][0] = fmaf(kr[r], vv.x, acc[r][0]); acc[r][1] = fmaf(kr[r], vv.y, acc[r][1]);
-          acc[r][2] = fmaf(kr[r], vv.z, acc[r][2]); acc[r][3] = fmaf(kr[r], vv.w, acc[r][3]);
+    for (int s = 32; s >= 4; s >>= 1) {
+#pragma unroll 4
+      for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+        const int i = idx / KT, kk = idx % KT;
+        const float rl = sgam[i * KS + kk];
+        const int seg = i >> 4;
+        if (i & s) {                                      // gamma_i - gamma_ref, ref = the last row of the other half
+          const float d = s == 32 ? (seg == 3 ? rl + stot[2 * KT + kk] : rl)
+                        : s == 16 ? rl : rl - sgam[((i & ~(2 * s - 1)) + s - 1) * KS + kk];
+          const float e = expf(d);
+          sx[i * KS + kk] = sk[i * KS + kk] * e;
+          sy[((i / (2 * s)) * s + (i & (s - 1))) * KS + kk] = sq[i * KS + kk] * e;
+        } else {
+          float d;                                        // gamma_ref - gamma_i
+          if (s >= 16) {
+            d = stot[seg * KT + kk] - rl;
+            if (s == 32 && seg == 0) d += stot[KT + kk];
+          } else {
+            d = sgam[((i & ~(2 * s - 1)) + s - 1) * KS + kk] - rl;
+          }
+          sx[i * KS + kk] = sk[i * KS + kk] * expf(d);
         }
+      }
+      __syncthreads();
+      // 2 x 2 outputs per thread group, the channels of a group dealt out to `split` neighbouring lanes
+      const int split = NTH / (8 * s);
+      const int tile = tid / split, ks = tid % split;
+      const int per = (s / 2) * (s / 2);                  // tiles of one block
+      const int blk = tile / per, tb = tile % per;
+      int ti, tj;
+      if (s >= 8) {                                       // 4 x 4 tiles per 16: four rows each side per warp
+        const int t16 = tb % 16, hi = tb / 16, side = s / 8;
+        ti = 4 * (hi / side) + t16 / 4;
+        tj = 4 * (hi % side) + t16 % 4;
+      } else {
+        ti = tb / 2;
+        tj = tb % 2;
+      }
+      const int i0 = blk * 2 * s + s + 2 * ti, j0 = blk * 2 * s + 2 * tj, y0 = blk * s + 2 * ti;
+      float a[2][2] = {}, aq[2][2] = {};
+      for (int f = ks; f < KT / 4; f += split) {
+        float4 xi[2], yi[2], xj[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          xi[e] = *reinterpret_cast<const float4*>(sx + (i0 + e) * KS + 4 * f);
+          yi[e] = *reinterpret_cast<const float4*>(sy + (y0 + e) * KS + 4 * f);
+          xj[e] = *reinterpret_cast<const float4*>(sx + (j0 + e) * KS + 4 * f);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            a[e][c] = fmaf(xi[e].x, xj[c].x, a[e][c]); a[e][c] = fmaf(xi[e].y, xj[c].y, a[e][c]);
+            a[e][c] = fmaf(xi[e].z, xj[c].z, a[e][c]); a[e][c] = fmaf(xi[e].w, xj[c].w, a[e][c]);
+            aq[e][c] = fmaf(yi[e].x, xj[c].x, aq[e][c]); aq[e][c] = fmaf(yi[e].y, xj[c].y, aq[e][c]);
+            aq[e][c] = fmaf(yi[e].z, xj[c].z, aq[e][c]); aq[e][c] = fmaf(yi[e].w, xj[c].w, aq[e][c]);
+          }
+      }
+      for (int o = split >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            a[e][c] += __shfl_xor_sync(0xffffffffu, a[e][c], o);
+            aq[e][c] += __shfl_xor_sync(0xffffffffu, aq[e][c], o);
+          }
+      if (ks == 0) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            sA[(i0 + e) * KC_AS + j0 + c] = a[e][c] * sbeta[i0 + e];
+            o_aqk[(i0 + e) * KC_AS + j0 + c] = aq[e][c];
+          }
+      }
+      __syncthreads();
+    }
+  }
+  for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) sT[idx] = 0.f;
+  // the 4 x 4 diagonal blocks (every block of the triangle when `direct`): a warp per pair, its lanes over the channels
+  {
+    const int side = direct ? KC_C : 4, pairs = side * (side + 1) / 2, blocks = KC_C / side;
+    for (int p = warp; p < blocks * pairs; p += NW) {
+      const int blk = p / pairs;
+      int i = (int)((sqrtf(8.f * (p % pairs) + 1.f) - 1.f) * 0.5f);
+      if ((i + 1) * (i + 2) / 2 <= p % pairs) ++i;
+      if (i * (i + 1) / 2 > p % pairs) --i;
+      const int j = blk * side + p % pairs - i * (i + 1) / 2;
+      i += blk * side;
+      float a = 0.f, aq = 0.f;
+#pragma unroll
+      for (int c = 0; c < KT / 32; ++c) {
+        const int kk = lane + 32 * c;
+        const float kj = sk[j * KS + kk];
+        float e = kj;
+        if (i != j || direct) {
+          float d = sgam[i * KS + kk] - sgam[j * KS + kk];
+          for (int s = j >> 4; s < i >> 4; ++s) d += stot[s * KT + kk];
+          e = expf(fminf(d, 50.f)) * kj;
+        }
+        a = fmaf(sk[i * KS + kk], e, a);
+        aq = fmaf(sq[i * KS + kk], e, aq);
+      }
+      a = warp_sum(a);
+      aq = warp_sum(aq);
+      if (lane == 0) {
+        if (j < i) sA[i * KC_AS + j] = a * sbeta[i];
+        o_aqk[i * KC_AS + j] = aq;
+      }
+    }
+  }
+  __syncthreads();
+  // (I + A)^-1: the 8 x 8 diagonal blocks by substitution (a thread per column) ...
+  if (tid < KC_C) {
+    const int c = tid & 7, b0 = tid & ~7;
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float acc = i == c ? 1.f : 0.f;
+#pragma unroll
+      for (int j = 0; j < i; ++j) acc = fmaf(-sA[(b0 + i) * KC_AS + b0 + j], x[j], acc);
+      x[i] = i < c ? 0.f : acc;
+      sT[(b0 + i) * KC_AS + b0 + c] = x[i];
+    }
+  }
+  // ... meanwhile the element-wise outputs, and exp(gamma) k as the operand of w
+#pragma unroll 4
+  for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+    const int i = idx / KT, kk = idx % KT;
+    const int seg = i >> 4;
+    float gm = sgam[i * KS + kk], rest = stot[seg * KT + kk] - gm;     // gamma, gamma_last - gamma
+    for (int s = 0; s < seg; ++s) gm += stot[s * KT + kk];
+    for (int s = seg + 1; s < 4; ++s) rest += stot[s * KT + kk];
+    const float eg = expf(gm), kv = sk[i * KS + kk];
+    sx[i * KS + kk] = eg * kv;
+    o_qg[i * KS + kk] = sq[i * KS + kk] * eg;
+    o_kg[i * KS + kk] = kv * expf(rest);
+    if (i == KC_C - 1) o_dl[kk] = eg;
+  }
+  __syncthreads();
+  // ... then [[T00, 0], [-T11 A10 T00, T11]] for blocks of 8, 16 and 32
+#pragma unroll
+  for (int s = 8; s <= 32; s <<= 1) {
+    for (int idx = tid; idx < 32 * s; idx += NTH) {
+      const int blk = idx / (s * s), i = (idx / s) % s, c = idx % s, r0 = blk * 2 * s;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int j = 0; j < s; ++j) acc = fmaf(sA[(r0 + s + i) * KC_AS + r0 + j], sT[(r0 + j) * KC_AS + r0 + c], acc);
+      sgam[blk * s * s + i * s + c] = acc;
+    }
+    __syncthreads();
+    for (int idx = tid; idx < 32 * s; idx += NTH) {
+      const int blk = idx / (s * s), i = (idx / s) % s, c = idx % s, r0 = blk * 2 * s;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int j = 0; j < s; ++j) acc = fmaf(sT[(r0 + s + i) * KC_AS + r0 + s + j], sgam[blk * s * s + j * s + c], acc);
+      sT[(r0 + s + i) * KC_AS + r0 + c] = -acc;
+    }
+    __syncthreads();
+  }
+  for (int idx = tid; idx < KC_C * KC_C; idx += NTH) sT[(idx / KC_C) * KC_AS + idx % KC_C] *= sbeta[idx % KC_C];
+  __syncthreads();
+  // w = Tm (exp(gamma) k), then u = Tm v in tiles of KT columns: 4 rows x 4 columns per thread
+  const int ti = tid / (KT / 4), tc = 4 * (tid % (KT / 4));
+  auto product = [&](float (&acc)[4][4]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+    for (int j = 0; j < 4 * ti + 4; j += 4) {
+      float4 tr[4], xv[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        tr[r] = *reinterpret_cast<const float4*>(sT + (4 * ti + r) * KC_AS + j);
+        xv[r] = *reinterpret_cast<const float4*>(sx + (j + r) * KS + tc);
       }
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        float d = sdl[kb + r];
-        float4* sp = reinterpret_cast<float4*>(sS + (kb + r) * VS + 4 * tx);
-        float4 sv = *sp;
-        sv.x = fmaf(sv.x, d, acc[r][0]); sv.y = fmaf(sv.y, d, acc[r][1]);
-        sv.z = fmaf(sv.z, d, acc[r][2]); sv.w = fmaf(sv.w, d, acc[r][3]);
-        *sp = sv;
+        const float tj[4] = {tr[r].x, tr[r].y, tr[r].z, tr[r].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          acc[r][0] = fmaf(tj[e], xv[e].x, acc[r][0]); acc[r][1] = fmaf(tj[e], xv[e].y, acc[r][1]);
+          acc[r][2] = fmaf(tj[e], xv[e].z, acc[r][2]); acc[r][3] = fmaf(tj[e], xv[e].w, acc[r][3]);
+        }
+      }
+    }
+  };
+  float acc[4][4];
+  product(acc);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    *reinterpret_cast<float4*>(o_w + (4 * ti + r) * KS + tc) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+  for (int v0 = 0; v0 < V; v0 += KT) {
+    __syncthreads();
+#pragma unroll 4
+    for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+      const int i = idx / KT, c = idx % KT, t = t0 + i;
+      sx[i * KS + c] = t < T_ && v0 + c < V ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + v0 + c) : 0.f;
+    }
+    __syncthreads();
+    product(acc);
+    if (v0 + tc < V) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        *reinterpret_cast<float4*>(o_u + ((int64_t)((v0 + tc) / 8) * KC_C + 4 * ti + r) * 8 + (tc & 7)) =
+            make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    }
+  }
+}
+
+// =====================================================================================
+// Stage 2 (sequential over chunks): one CTA owns 8 value columns of one (batch, value head) and keeps that slice of
+// the state in shared memory.
+//   vt = u - w S ; o = qg S + Aqk vt ; S <- diag(dl) S + kg^T vt
+// Bound: shared-memory wavefronts (each operand row is read once per 8 columns) and the four barriers of a chunk.
+// 8 columns instead of 32: the chain of chunks cannot be shortened, so a chunk's step is, by spreading a head over
+// V / 8 CTAs (a single sequence of a few heads leaves the chip idle otherwise); the next chunk's operands are
+// bulk-copied into the buffers as each product releases them, so no step waits for memory.
+// 1024 tokens, 4 heads, K = V = 128, fp32: 257 -> 52 us (16 dependent chunks).
+// =====================================================================================
+#define KC_VS 8
+template <typename T, int KT>
+__global__ void __launch_bounds__(256)
+kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0, T* __restrict__ o,
+                      float* __restrict__ S_out, int T_, int HV, int K, int V, int NT, unsigned int* status) {
+  constexpr int KS = KT + 4, IG = 256 / KT, IR = KC_C / IG;
+  extern __shared__ __align__(16) float smem[];
+  float* sw = smem;                          // [64][KS], then qg [64][KS]
+  float* sqg = sw + KC_C * KS;
+  float* skg = sqg + KC_C * KS;              // [64][KS]
+  float* saqk = skg + KC_C * KS;             // [64][68], dl [KT] behind it as in the record
+  float* sdl = saqk + KC_C * KC_AS;
+  float* su = sdl + KT;                      // [64][8]
+  float* sS = su + KC_C * KC_VS;             // [KT][8]
+  float* svt = sS + KT * KC_VS;              // [64][8]
+  float4* red = reinterpret_cast<float4*>(svt + KC_C * KC_VS);      // [4][2][64]: partial sums of w S, then of o
+  float4* red3 = red + 4 * 2 * KC_C;                                // [IG][2][KT]: partial sums of kg^T vt
+  uint64_t* bars = reinterpret_cast<uint64_t*>(red3 + IG * 2 * KT); // w + qg + u | Aqk + dl | kg
+  const int vb = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
+  const int tid = threadIdx.x;
+  const int v0 = vb * KC_VS;
+  const int64_t bh = (int64_t)b * HV + hv, rf = kc_record_floats(KT, V), sbase = bh * K * V;
+  const float* rec = ws + bh * NT * rf;
+  auto load_w = [&](int n) {
+    mbarrier_expect_tx(&bars[0], (2 * KC_C * KS + KC_C * KC_VS) * 4);
+    bulk_copy_g2s(sw, rec + n * rf, 2 * KC_C * KS * 4, &bars[0]);
+    bulk_copy_g2s(su, rec + n * rf + 3 * KC_C * KS + KC_C * KC_AS + KT + (int64_t)vb * KC_C * KC_VS, KC_C * KC_VS * 4, &bars[0]);
+  };
+  auto load_a = [&](int n) {
+    mbarrier_expect_tx(&bars[1], (KC_C * KC_AS + KT) * 4);
+    bulk_copy_g2s(saqk, rec + n * rf + 3 * KC_C * KS, (KC_C * KC_AS + KT) * 4, &bars[1]);
+  };
+  auto load_k = [&](int n) {
+    mbarrier_expect_tx(&bars[2], KC_C * KS * 4);
+    bulk_copy_g2s(skg, rec + n * rf + 2 * KC_C * KS, KC_C * KS * 4, &bars[2]);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) mbarrier_init(&bars[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    load_w(0);
+    load_a(0);
+    load_k(0);
+  }
+  for (int idx = tid; idx < KT * KC_VS; idx += 256) {
+    const int kk = idx / KC_VS, c = idx % KC_VS;
+    sS[idx] = (S0 && kk < K && v0 + c < V) ? S0[sbase + (int64_t)kk * V + v0 + c] : 0.f;
+  }
+  __syncthreads();
+  const int r = tid & 63, ks = tid >> 6;
+  bool ok = true;
+  auto add4 = [](float4& a, float x, const float4& y) {
+    a.x = fmaf(x, y.x, a.x); a.y = fmaf(x, y.y, a.y); a.z = fmaf(x, y.z, a.z); a.w = fmaf(x, y.w, a.w);
+  };
+  const float4* S4 = reinterpret_cast<const float4*>(sS);
+  const float4* vt4 = reinterpret_cast<const float4*>(svt);
+  for (int n = 0; n < NT; ++n) {
+    ok = ok && mbarrier_wait_bounded(&bars[0], n & 1, KCH_STATUS_KDA_CHUNK, 1u << 24, status);
+    // partial sums of w S and qg S: row r, a quarter of the channels
+    float4 aw[2] = {}, aq[2] = {};
+#pragma unroll 4
+    for (int kk = ks * (KT / 4); kk < (ks + 1) * (KT / 4); kk += 4) {
+      const float4 w4 = *reinterpret_cast<const float4*>(sw + r * KS + kk);
+      const float4 q4 = *reinterpret_cast<const float4*>(sqg + r * KS + kk);
+      const float wv[4] = {w4.x, w4.y, w4.z, w4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 s0 = S4[2 * (kk + e)], s1 = S4[2 * (kk + e) + 1];
+        add4(aw[0], wv[e], s0); add4(aw[1], wv[e], s1);
+        add4(aq[0], qv[e], s0); add4(aq[1], qv[e], s1);
+      }
+    }
+    red[(ks * 2) * KC_C + r] = aw[0];
+    red[(ks * 2 + 1) * KC_C + r] = aw[1];
+    __syncthreads();
+    if (tid < 2 * KC_C) {
+      const int c4 = tid >> 6;
+      float4 x = reinterpret_cast<const float4*>(su)[2 * r + c4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const float4 y = red[(p * 2 + c4) * KC_C + r];
+        x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
+      }
+      reinterpret_cast<float4*>(svt)[2 * r + c4] = x;
+    }
+    __syncthreads();
+    if (tid == 0 && ok && n + 1 < NT) load_w(n + 1);
+    ok = ok && mbarrier_wait_bounded(&bars[1], n & 1, KCH_STATUS_KDA_CHUNK, 1u << 24, status);
+#pragma unroll
+    for (int j = ks * 16; j < ks * 16 + 16; j += 4) {
+      const float4 a4 = *reinterpret_cast<const float4*>(saqk + r * KC_AS + j);
+      const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        add4(aq[0], av[e], vt4[2 * (j + e)]);
+        add4(aq[1], av[e], vt4[2 * (j + e) + 1]);
+      }
+    }
+    red[(ks * 2) * KC_C + r] = aq[0];
+    red[(ks * 2 + 1) * KC_C + r] = aq[1];
+    ok = ok && mbarrier_wait_bounded(&bars[2], n & 1, KCH_STATUS_KDA_CHUNK, 1u << 24, status);
+    {
+      const int kk = tid % KT, ig = tid / KT;
+      float4 as[2] = {};
+#pragma unroll 8
+      for (int i = ig * IR; i < (ig + 1) * IR; ++i) {
+        const float kv = skg[i * KS + kk];
+        add4(as[0], kv, vt4[2 * i]);
+        add4(as[1], kv, vt4[2 * i + 1]);
+      }
+      red3[(ig * 2) * KT + kk] = as[0];
+      red3[(ig * 2 + 1) * KT + kk] = as[1];
+    }
+    __syncthreads();
+    if (tid == 0 && ok && n + 1 < NT) load_k(n + 1);
+    for (int idx = tid; idx < 2 * KT; idx += 256) {
+      const int kk = idx % KT, c4 = idx / KT;
+      float4 x = reinterpret_cast<float4*>(sS)[2 * kk + c4];
+      const float d = sdl[kk];
+      x.x *= d; x.y *= d; x.z *= d; x.w *= d;
+#pragma unroll
+      for (int p = 0; p < IG; ++p) {
+        const float4 y = red3[(p * 2 + c4) * KT + kk];
+        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+      }
+      reinterpret_cast<float4*>(sS)[2 * kk + c4] = x;
+    }
+    if (tid < 2 * KC_C) {
+      const int c4 = tid >> 6, t = n * KC_C + r;
+      float4 x = red[c4 * KC_C + r];
+#pragma unroll
+      for (int p = 1; p < 4; ++p) {
+        const float4 y = red[(p * 2 + c4) * KC_C + r];
+        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+      }
+      if (t < T_ && ok) {
+        T* orow = o + (((int64_t)b * T_ + t) * HV + hv) * V + v0 + 4 * c4;
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (v0 + 4 * c4 + c < V) stf(orow + c, xv[c]);
       }
     }
     __syncthreads();
+    if (tid == 0 && ok && n + 1 < NT) load_a(n + 1);
+  }
+  if (!ok) {            // give copies still in flight time to land before the shared memory goes
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    return;
   }
   if (S_out)
-    for (int idx = tid; idx < K * VS; idx += 256) {
-      int kk = idx / VS, vv = idx % VS;
-      if (v0 + vv < V) S_out[sbase + (int64_t)kk * V + v0 + vv] = sS[kk * VS + vv];
+    for (int idx = tid; idx < KT * KC_VS; idx += 256) {
+      const int kk = idx / KC_VS, c = idx % KC_VS;
+      if (kk < K && v0 + c < V) S_out[sbase + (int64_t)kk * V + v0 + c] = sS[idx];
     }
 }
 
-static size_t kda_ws_layout(KdaChunkWs* ws, char* base, int B, int HV, int K, int V, int C, int NT) {
-  size_t bh = (size_t)B * HV, Tp = (size_t)NT * C, off = 0;
-  auto take = [&](size_t n) { float* p = (float*)(base + off); off += ((n * 4 + 255) / 256) * 256; return p; };
-  float* w = take(bh * Tp * K);
-  float* qg = take(bh * Tp * K);
-  float* kg = take(bh * Tp * K);
-  float* u = take(bh * Tp * V);
-  float* aqk = take(bh * NT * C * C);
-  float* dl = take(bh * NT * K);
-  if (ws) { ws->w = w; ws->qg = qg; ws->kg = kg; ws->u = u; ws->aqk = aqk; ws->dl = dl; }
-  return off;
+static size_t kc_prepare_smem(int KT) {
+  const int KS = KT + 4;
+  return ((size_t)4 * KC_C * KS + (32 * KS > KC_C * KC_AS ? 32 * KS : KC_C * KC_AS) + KC_C * KC_AS + KC_C + 4 * KT) * sizeof(float);
 }
-
-static int kda_chunk_effective(int K, int chunk) {
-  // the prepare kernel reuses a [C][K+1] tile for the [C][C+1] inverse, so C <= K; larger
-  // requests run as smaller chunks (same mathematics, different fp32 summation order)
-  int C = chunk < KDA_CMAX ? chunk : KDA_CMAX;
-  if (C > K) C = K;
-  return C < 1 ? 1 : C;
+static size_t kc_scan_smem(int KT) {
+  return ((size_t)3 * KC_C * (KT + 4) + KC_C * KC_AS + KT + 2 * KC_C * KC_VS + KT * KC_VS + 4 * 2 * KC_C * 4 +
+          (256 / KT) * 2 * KT * 4) * sizeof(float) + 3 * sizeof(uint64_t);
+}
+static int kc_padded_k(int K) { return K <= 64 ? 64 : 128; }
+static int64_t kc_workspace_bytes(int B, int T, int HV, int K, int V) {
+  return (int64_t)B * HV * ((T + KC_C - 1) / KC_C) * kc_record_floats(kc_padded_k(K), V) * 4 + 16;   // + alignment of the base
 }
 
 // tensor-core path (kda_mma.cu)
@@ -519,9 +711,8 @@ int kch_kda_chunk_mma(const void* q, const void* k, const void* v, const void* g
 
 extern "C" int64_t kch_kda_chunk_workspace_bytes(int B, int T, int HV, int K, int V, int chunk_size) {
   if (B <= 0 || T <= 0 || HV <= 0 || K <= 0 || V <= 0 || chunk_size < 1) return 0;
-  int C = kda_chunk_effective(K, chunk_size);
-  int NT = (T + C - 1) / C;
-  int64_t need = (int64_t)kda_ws_layout(nullptr, nullptr, B, HV, K, V, C, NT);
+  if (K > 128) return 0;                       // runs as the token recurrence
+  int64_t need = kc_workspace_bytes(B, T, HV, K, V);
   // the dtype is not known here: size for whichever path may run
   if (kch_kda_mma_supported(K, V, chunk_size, 0.f, KCH_BF16)) {
     int64_t m = kch_kda_mma_workspace_bytes(B, T, HV);
@@ -565,30 +756,32 @@ static int kda_chunk_impl(const void* q, const void* k, const void* v, const voi
     }
     return KCH_OK;
   }
-  int C = kda_chunk_effective(K, chunk_size);
-  int NT = (T + C - 1) / C;
-  KdaChunkWs ws;
-  size_t need = kda_ws_layout(&ws, (char*)workspace, B, HV, K, V, C, NT);
-  KCH_REQUIRE(workspace && (size_t)workspace_bytes >= need, "kch_kda_chunk: workspace %lld < %lld bytes",
+  const int NT = (T + KC_C - 1) / KC_C, KT = kc_padded_k(K);
+  const int64_t need = kc_workspace_bytes(B, T, HV, K, V);
+  KCH_REQUIRE(workspace && workspace_bytes >= need, "kch_kda_chunk: workspace %lld < %lld bytes",
               (long long)workspace_bytes, (long long)need);
+  float* ws = (float*)(((uintptr_t)workspace + 15) & ~(uintptr_t)15);
+  unsigned int* status = kch_status_device_ptr();
+  KCH_REQUIRE(status != nullptr, "kch_kda_chunk: cannot resolve the device status word");
   cudaStream_t s = kch_stream(stream);
-  size_t smem1 = ((size_t)3 * C * (K + 1) + (size_t)C * (C + 1) + C) * sizeof(float);
-  int Kp = (K + 3) & ~3;
-  size_t smem2 = ((size_t)3 * KDA_CMAX * Kp + KDA_CMAX * KDA_CMAX + KDA_CMAX * 32 + (size_t)Kp * 32 + Kp) * sizeof(float);
-  dim3 g1(NT, HV, B), g2((V + 31) / 32, HV, B);
-#define GO(T_)                                                                                       \
-  do {                                                                                               \
-    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_prepare_kernel<T_>,                                   \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));      \
-    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_scan_kernel<T_>,                                      \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));      \
-    kda_chunk_prepare_kernel<T_><<<g1, 256, smem1, s>>>((const T_*)q, (const T_*)k, (const T_*)v,    \
-        (const T_*)g, (const T_*)beta, ws, T, H, HV, K, V, C, NT, scale, g_clamp_min, ld_qk, ld_v,    \
-        ld_g, ld_beta);                                                                              \
-    kda_chunk_scan_kernel<T_><<<g2, 256, smem2, s>>>(ws, initial_state, (T_*)o, final_state, T, HV,  \
-        K, V, C, NT);                                                                                \
+  const size_t smem1 = kc_prepare_smem(KT), smem2 = kc_scan_smem(KT);
+  const dim3 g1(NT, HV, B), g2((V + KC_VS - 1) / KC_VS, HV, B);
+#define GO(T_, KT_)                                                                                       \
+  do {                                                                                                    \
+    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_prepare_kernel<T_, KT_>,                                   \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));           \
+    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_scan_kernel<T_, KT_>,                                      \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));           \
+    kda_chunk_prepare_kernel<T_, KT_><<<g1, 4 * KT_, smem1, s>>>((const T_*)q, (const T_*)k,              \
+        (const T_*)v, (const T_*)g, (const T_*)beta, ws, T, H, HV, K, V, NT, scale, g_clamp_min, ld_qk,   \
+        ld_v, ld_g, ld_beta);                                                                             \
+    kda_chunk_scan_kernel<T_, KT_><<<g2, 256, smem2, s>>>(ws, initial_state, (T_*)o, final_state, T, HV,  \
+        K, V, NT, status);                                                                                \
   } while (0)
-  KCH_DISPATCH_FLOAT(dtype, T_, GO(T_));
+  KCH_DISPATCH_FLOAT(dtype, T_, {
+    if (KT == 64) GO(T_, 64);
+    else GO(T_, 128);
+  });
 #undef GO
   kch_note_launch(1);  // two kernels per call
   KCH_LAUNCH_OK();
