@@ -272,6 +272,9 @@ typedef struct kch_attend_args {
                              * e.g. the tail of a cache's ring when a later chunk of a sequence is attended) */
 } kch_attend_args;
 int kch_attend(const kch_attend_args* args, void* stream);
+/* The same for selection lists in which no index occurs twice (what kch_indexer_topk writes): the list may then be
+ * applied as a bit mask over contiguous key tiles instead of being gathered. */
+int kch_attend_distinct(const kch_attend_args* args, void* stream);
 
 /* ---- decode caches ---------------------------------------------------------------------------------- */
 

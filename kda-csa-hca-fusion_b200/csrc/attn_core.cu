@@ -190,11 +190,11 @@ __global__ void __launch_bounds__(256) attn_generic_kernel(AttnArgs a) {
 }
 
 bool kch_attend_mma_supported(const kch_attend_args* p);
-int kch_attend_mma(const kch_attend_args* p, void* stream);
+int kch_attend_mma(const kch_attend_args* p, bool distinct, void* stream);
 bool kch_attend_tc5_enabled();
 int kch_attend_tc5(const kch_attend_args* p, void* stream);
 
-extern "C" int kch_attend(const kch_attend_args* p, void* stream) {
+static int attend_impl(const kch_attend_args* p, bool distinct, void* stream) {
   KCH_REQUIRE(p != nullptr, "kch_attend: null args");
   KCH_REQUIRE(p->nh >= 1, "nh=%d must be >= 1", p->nh);
   KCH_REQUIRE(p->c >= 1 && p->c <= 256, "c=%d must be in [1, 256]", p->c);
@@ -208,7 +208,7 @@ extern "C" int kch_attend(const kch_attend_args* p, void* stream) {
   // tensor-core kernel for the production geometry; KCH_ATTEND=generic forces the fp32 CUDA-core kernel
   static const bool force_generic = [] { const char* e = getenv("KCH_ATTEND"); return e && e[0] == 'g'; }();
   if (!force_generic && kch_attend_mma_supported(p))
-    return kch_attend_tc5_enabled() ? kch_attend_tc5(p, stream) : kch_attend_mma(p, stream);
+    return kch_attend_tc5_enabled() ? kch_attend_tc5(p, stream) : kch_attend_mma(p, distinct, stream);
   AttnArgs a;
   a.q = p->q; a.q_dtype = p->q_dtype; a.q_ld = p->q_ld; a.q_normalize = p->q_normalize;
   a.B = p->B; a.T = p->T; a.nh = p->nh; a.c = p->c;
@@ -247,3 +247,6 @@ extern "C" int kch_attend(const kch_attend_args* p, void* stream) {
   KCH_LAUNCH_OK();
   return KCH_OK;
 }
+
+extern "C" int kch_attend(const kch_attend_args* p, void* stream) { return attend_impl(p, false, stream); }
+extern "C" int kch_attend_distinct(const kch_attend_args* p, void* stream) { return attend_impl(p, true, stream); }

@@ -18,11 +18,13 @@
 #define AM_WARPS 4
 #define AM_TILE 32
 #define AM_C 128
+#define AM_DENSE_GAIN 6                // a gathered entry against a tile entry at 16 heads: 52 ps against 8.1 ps
 #define AM_QLD 136   // padded row of the per-warp query tile (bf16 elements)
 
 struct AttnMmaArgs {
   const bf16* q; int64_t q_ld;
   int B, T, nh;
+  int t_lo;                            // first query of each sequence that the launch covers
   const bf16* comp; int64_t comp_batch_rows; int n_comp;
   const int32_t* sel; int topk;
   int m; int64_t t0; int nvis_fixed;
@@ -64,9 +66,10 @@ template <int AM_STAGES, int MINB>
 __global__ void __launch_bounds__(AM_WARPS * 32, MINB) attn_mma_kernel(AttnMmaArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t bt = (int64_t)blockIdx.x * AM_WARPS + warp;
-  if (bt >= (int64_t)a.B * a.T) return;
-  const int t = (int)(bt % a.T), b = (int)(bt / a.T);
+  const int64_t qn = (int64_t)blockIdx.x * AM_WARPS + warp, per = a.T - a.t_lo;
+  if (qn >= a.B * per) return;
+  const int t = a.t_lo + (int)(qn % per), b = (int)(qn / per);
+  const int64_t bt = (int64_t)b * a.T + t;
   const int g = lane >> 2, j = lane & 3;
   // per-warp shared memory: the key ring; its last stage doubles as the query staging tile until the
   // query fragments are in registers (the prologue only fills stages 0 .. AM_STAGES-2)
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(AD_WARPS * 32, 2) attn_dense_mma_kernel(AttnMm
 int kch_attend_dense_tc5(const bf16* q, int64_t q_ld, int B, int T, int nh, const bf16* comp, int64_t comp_batch_rows,
                          int n_comp, int m, int64_t t0, int nvis_fixed, const bf16* win, int64_t win_ld,
                          int64_t win_batch_rows, int win_size, int win_t0, const void* sink, int sink_dtype, float scale,
-                         bf16* out, cudaStream_t s);
+                         bf16* out, const int32_t* sel, int topk, int q_end, int* q_done, cudaStream_t s);
 
 bool kch_attend_mma_supported(const kch_attend_args* p) {
   if (p->c != AM_C || p->nh > 16 || p->nh < 1) return false;
@@ -414,8 +417,10 @@ bool kch_attend_mma_supported(const kch_attend_args* p) {
   return true;
 }
 
-int kch_attend_mma(const kch_attend_args* p, void* stream) {
+// `distinct`: the caller vouches that no index occurs twice in a selection list, so that the list may become a bit mask
+int kch_attend_mma(const kch_attend_args* p, bool distinct, void* stream) {
   AttnMmaArgs a;
+  a.t_lo = 0;
   a.q = (const bf16*)p->q; a.q_ld = p->q_ld;
   a.B = p->B; a.T = p->T; a.nh = p->nh;
   a.comp = (const bf16*)p->comp; a.comp_batch_rows = p->comp_batch_rows; a.n_comp = p->comp ? p->n_comp : 0;
@@ -433,8 +438,31 @@ int kch_attend_mma(const kch_attend_args* p, void* stream) {
   if (!a.sel && !dense_per_warp && !dense_mma) {
     const int rc = kch_attend_dense_tc5(a.q, a.q_ld, a.B, a.T, a.nh, a.comp, a.comp_batch_rows, a.n_comp, a.m, a.t0, a.nvis_fixed,
                                         a.win, a.win_ld, a.win_batch_rows, a.win_size, a.win_t0, a.sink, a.sink_dtype, a.scale,
-                                        a.out, kch_stream(stream));
+                                        a.out, nullptr, 0, 0, nullptr, kch_stream(stream));
     if (rc != -100) return rc;
+  }
+  // A selection list of distinct indices: contiguous key tiles under the list's bit mask cost per VISIBLE entry, the
+  // gather below per SELECTED one, AM_DENSE_GAIN (twice that for at most 8 heads) times as much each.
+  static const int force_mask = [] { const char* e = getenv("KCH_ATTEND"); return !e ? 0 : e[0] == 'r' ? -1 : e[0] == 'd' ? 1 : 0; }();
+  if (a.sel && distinct && a.topk > 0 && force_mask >= 0) {
+    const int64_t gain = p->nh <= 8 ? 2 * AM_DENSE_GAIN : AM_DENSE_GAIN;
+    const int64_t most = gain * ((int64_t)a.topk + a.win_size) - a.win_size;      // visible blocks up to which tiles win
+    int64_t q_end = a.T;
+    if (!force_mask) {
+      if (a.nvis_fixed >= 0 || a.m <= 0) q_end = (a.nvis_fixed >= 0 && a.nvis_fixed < a.n_comp ? a.nvis_fixed : a.n_comp) <= most ? a.T : 0;
+      else if (a.n_comp > most) q_end = (most + 1) * a.m - 1 - a.t0;              // the first query that sees more
+    }
+    if (q_end > a.T) q_end = a.T;
+    if (q_end > 0) {
+      int done = 0;
+      const int rc = kch_attend_dense_tc5(a.q, a.q_ld, a.B, a.T, a.nh, a.comp, a.comp_batch_rows, a.n_comp, a.m, a.t0, a.nvis_fixed,
+                                          a.win, a.win_ld, a.win_batch_rows, a.win_size, a.win_t0, a.sink, a.sink_dtype, a.scale,
+                                          a.out, a.sel, a.topk, (int)q_end, &done, kch_stream(stream));
+      if (rc != -100) {
+        if (rc != KCH_OK || done >= a.T) return rc;
+        a.t_lo = done;
+      }
+    }
   }
   if (!a.sel && !dense_per_warp) {
     const size_t smem = (size_t)AD_STAGES * AM_TILE * AM_C * 2 + (size_t)AD_WARPS * 16 * AM_QLD * 2;
@@ -444,7 +472,7 @@ int kch_attend_mma(const kch_attend_args* p, void* stream) {
     KCH_LAUNCH_OK();
     return KCH_OK;
   }
-  int64_t nq = (int64_t)p->B * p->T;
+  int64_t nq = (int64_t)p->B * (p->T - a.t_lo);
   unsigned grid = (unsigned)((nq + AM_WARPS - 1) / AM_WARPS);
   // ring depth / resident CTAs per SM: two stages and three CTAs per SM (168 registers) measured fastest on
   // B200 (7.1 ms vs 8.0 ms for three stages / two CTAs at the benchmark size); KCH_ATTN_CFG = 0 | 2 selects

@@ -295,9 +295,10 @@ def mma_attention_eligible(dtype, c, nh, normalize_qk, scale):
 
 def attend(q, comp, *, nh, c, sel=None, m=0, t0=0, n_visible=-1, q_normalize=False, comp_norms=None,
            comp_scales=None, comp_kind=None, win=None, sliding_window=0, win_mode=0, win_len=0, sink=None,
-           scale=1.0, out_dtype=torch.float32, win_t0=0):
+           scale=1.0, out_dtype=torch.float32, win_t0=0, sel_distinct=False):
     """Kernel-level joint-softmax attention.  q ``[B,T,nh*c]`` view (row-strided ok); comp ``[B,n,c]``
-    contiguous or None; win ``[B,Tw,c]`` (row-strided ok) or None."""
+    contiguous or None; win ``[B,Tw,c]`` (row-strided ok) or None.  ``sel_distinct``: no index occurs twice in a
+    list of ``sel`` (true of every list the indexer writes)."""
     lib = _lib.load()
     B, T = q.shape[0], q.shape[1]
     a = _lib.AttendArgs()
@@ -341,7 +342,7 @@ def attend(q, comp, *, nh, c, sel=None, m=0, t0=0, n_visible=-1, q_normalize=Fal
     out = torch.empty(B, T, nh * c, dtype=out_dtype, device=q.device)
     a.out, a.out_dtype = out.data_ptr(), _lib.dtype_tag(out_dtype)
     with torch.cuda.device(q.device):
-        _lib.check(lib.kch_attend(a, _lib.stream()))
+        _lib.check((lib.kch_attend_distinct if sel_distinct else lib.kch_attend)(a, _lib.stream()))
     return out
 
 
@@ -442,7 +443,7 @@ def naive_csa(H, W_aKV, W_bKV, W_aZ, W_bZ, Ba, Bb, W_DQ, W_UQ, W_IUQ, W_w, W_KV_
         local = rownorm(Ca, normalize_qk, kdt) if normalize_qk else Ca
     out = attend(q, C_comp_n if topk > 0 else None, nh=nh, c=c, sel=indices, m=m, t0=q_lo, q_normalize=normalize_qk,
                  win=local, sliding_window=sliding_window, sink=sink_logits, scale=scale, out_dtype=H.dtype,
-                 win_t0=q_lo)
+                 win_t0=q_lo, sel_distinct=True)
     out_final = out[:, :original_T - q_lo]
     res = [out_final]
     if return_projections:

@@ -643,7 +643,7 @@ class HybridDecoding(nn.Module):
                 P = prev.shape[1]
                 local = torch.cat([prev.to(kdt), local], dim=1)
         return attend(q, comp_n, nh=nh, c=c, sel=indices, m=m, t0=t0, q_normalize=True, win=local, sliding_window=win,
-                      sink=layer.sink, scale=1.0, out_dtype=h.dtype, win_t0=P)
+                      sink=layer.sink, scale=1.0, out_dtype=h.dtype, win_t0=P, sel_distinct=True)
 
     def _hca_chunk(self, layer, cache, h):
         cfg = self.cfg

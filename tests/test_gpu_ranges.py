@@ -36,3 +36,65 @@ def test_kda_chunk_fp32_edges(kch, B, T, H, HV, K, V, chunk, gate):
     o, s = kch.naive_chunk_kda(*(x.to(DEV) for x in (q, k, v, g, beta)), initial_state=S0.to(DEV), output_final_state=True,
                                chunk_size=chunk)
     assert md(o, o_ref) <= 2e-5 and md(s, s_ref) <= 2e-5, (md(o, o_ref), md(s, s_ref))
+
+
+def _attend_ref(q, comp, sel, win, m, t0, nvis, window, sink, scale, win_t0):
+    """One softmax over the selected (or all visible) rows, the window and the sink, in 64 bits on the GPU."""
+    B, T, nh, c = q.shape
+    n = comp.shape[1]
+    q, comp, win, out = q.double(), comp.double(), win.double(), torch.zeros(B, T, nh, c, dtype=torch.float64, device=DEV)
+    q = q / q.norm(dim=-1, keepdim=True).clamp_min(1e-12)
+    for t in range(T):
+        v = min(n, nvis if nvis >= 0 else (t0 + t + 1) // m)
+        lo = max(0, t + win_t0 - window + 1)
+        for b in range(B):
+            ids = torch.arange(v, device=DEV) if sel is None else sel[b, t][(sel[b, t] >= 0) & (sel[b, t] < v)].long()
+            keys = torch.cat([comp[b, ids], win[b, lo:t + win_t0 + 1] if window else comp[b, :0]])
+            s = torch.cat([q[b, t] @ keys.T * scale, sink.double()[:, None]], 1)
+            out[b, t] = torch.softmax(s, -1)[:, :-1] @ keys if len(keys) else 0
+    return out.reshape(B, T, nh * c)
+
+
+@pytest.mark.parametrize("B,T,nh,n,topk,m,t0,nvis,window,scale,odd", [
+    (1, 70, 16, 300, 40, 1, 200, -1, 128, 1.0, None), (2, 33, 8, 130, 130, 4, 400, -1, 16, 1.0, None),
+    (1, 17, 5, 64, 7, 4, 0, -1, 8, 4.0, None), (1, 9, 12, 65, 65, 1, 0, 65, 0, 1.0, None),
+    (2, 40, 16, 2500, 30, 1, 900, -1, 20, 1.0, None), (1, 24, 16, 96, 20, 2, 100, -1, 32, 1.0, "nan"),
+    (1, 24, 8, 96, 20, 2, 100, -1, 32, 1.0, "inf")])
+def test_selection_as_mask_matches_gather(kch, B, T, nh, n, topk, m, t0, nvis, window, scale, odd):
+    """A selection list applied as a bit mask over key tiles (few visible rows per selected one), gathered, or split between
+    the two (the case of 2500 rows): operator outputs within 2e-3 of the 64-bit softmax, as everywhere.  Rows that a query
+    does not attend do not reach it even when they are not finite."""
+    from kch_b200.csa import attend
+    g = torch.Generator(device=DEV).manual_seed(T * nh + n)
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s, generator=g, device=DEV), dim=-1).bfloat16()  # noqa: E731
+    win_t0 = 3
+    q, comp, win = torch.randn(B, T, nh, 128, generator=g, device=DEV).bfloat16(), unit(B, n, 128), unit(B, T + win_t0, 128)
+    sink = torch.randn(nh, generator=g, device=DEV)
+    sel = torch.full((B, T, topk), -1, dtype=torch.int32, device=DEV)
+    for t in range(T):
+        v = min(n, nvis if nvis >= 0 else (t0 + t + 1) // m)
+        for b in range(B):
+            ids = torch.randperm(v, generator=g, device=DEV)[:topk]
+            sel[b, t, :len(ids)] = ids.int()
+    bad = None
+    if odd:                                   # a row that half of the queries select, and a token's window row
+        bad = (sel == 5).any(-1)[0]
+        comp[0, 5] = float(odd)
+        win[0, 20] = float(odd)
+        bad |= (torch.arange(T, device=DEV) + win_t0 >= 20) & (torch.arange(T, device=DEV) + win_t0 < 20 + window)
+    kw = dict(nh=nh, c=128, sel=sel, m=m, t0=t0, n_visible=nvis, q_normalize=True, win=win, sliding_window=window, sink=sink,
+              scale=scale, out_dtype=torch.bfloat16, win_t0=win_t0)
+    a = attend(q.reshape(B, T, nh * 128), comp, sel_distinct=True, **kw)
+    b = attend(q.reshape(B, T, nh * 128), comp, **kw)
+    ref = _attend_ref(q, comp, sel, win, m, t0, nvis, window, sink, scale, win_t0)
+    if odd:
+        assert 0 < int(bad.sum()) < T
+        assert not torch.isfinite(a[:, bad].float()).all(-1).any() and torch.isfinite(a[:, ~bad].float()).all()
+        a, b, ref = a[:, ~bad], b[:, ~bad], ref[:, ~bad]
+    assert md(a, ref) <= 2e-3 and md(b, ref) <= 2e-3, (md(a, ref), md(b, ref))
+    dense = attend(q.reshape(B, T, nh * 128), comp, **dict(kw, sel=None))
+    dref = _attend_ref(q, comp, None, win, m, t0, nvis, window, sink, scale, win_t0)
+    if odd:
+        keep = ~bad & (torch.arange(T, device=DEV) < 0)      # every query sees row 5: nothing finite is expected
+        dense, dref = dense[:, keep], dref[:, keep]
+    assert md(dense, dref) <= 2e-3, md(dense, dref)
