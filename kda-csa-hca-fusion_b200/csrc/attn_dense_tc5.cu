@@ -159,7 +159,7 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   extern __shared__ uint8_t dt_raw[];
   DtSmem& sm = *reinterpret_cast<DtSmem*>(((uintptr_t)dt_raw + 1023) & ~(uintptr_t)1023);
   uint32_t* smask = reinterpret_cast<uint32_t*>(&sm + 1);          // [NQ][mask_words]
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform to the compiler)
+  const int tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   auto nvis_of = [&](int tt) -> int {
     int64_t nv64 = a.nvis_fixed >= 0 ? a.nvis_fixed : (a.m > 0 ? (a.t0 + tt + 1) / a.m : a.n_comp);
     return (int)(nv64 < a.n_comp ? nv64 : a.n_comp);
@@ -205,7 +205,7 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 
   if (warp == 8) {
     // ------------------------------ producer: the query tile, then the key tiles -----------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       bool ok = true;
       int g = 0, c = 0;
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++c) {
@@ -234,10 +234,8 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ----------------------------------------------------------------------
-    // The whole warp walks the loop, so that descriptors and addresses are warp-uniform values, and one elected thread
-    // issues: from a branch on the lane number every MMA cost about a hundred cycles (operands moved to uniform registers
-    // one by one), which alone was 1400 cycles a tile.
-    {
+    // (issued from a branch on the lane number, the MMAs took 1400 cycles a tile)
+    if (t5_elect()) {
       const uint32_t id_s = t5_idesc(DT_KT), id_o = t5_idesc(128) | (1u << 16);
       const uint64_t dq = t5_desc(smem_addr_u32(sm.q[0])), dk = t5_desc(smem_addr_u32(sm.k[0][0]));
       const uint64_t dv = t5_desc_mn(smem_addr_u32(sm.k[0][0]), 8192u);
@@ -247,14 +245,11 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         t5_fence_after();
         const uint32_t pa = tS + 64u * (gi & 1);
         const uint64_t vd = dv + (uint64_t)((gi % DT_KSTAGES) * (2 * DT_KT * 64 * 2 >> 4));
-        if (t5_elect()) {
 #pragma unroll
-          for (int ks = 0; ks < DT_KT / 16; ++ks)
-            dt_mma_ts(tO, pa + 32u * (ks >> 1) + 8u * (ks & 1), vd + ks * (2048 >> 4), id_o, first && ks == 0 ? 0u : 1u);
-          t5_commit(&sm.pv_done);
-          t5_commit(&sm.k_empty[gi % DT_KSTAGES]);
-        }
-        __syncwarp();
+        for (int ks = 0; ks < DT_KT / 16; ++ks)
+          dt_mma_ts(tO, pa + 32u * (ks >> 1) + 8u * (ks & 1), vd + ks * (2048 >> 4), id_o, first && ks == 0 ? 0u : 1u);
+        t5_commit(&sm.pv_done);
+        t5_commit(&sm.k_empty[gi % DT_KSTAGES]);
       };
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++c) {
         const Item x = item_of(it);
@@ -268,17 +263,14 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             if (!ok) break;
             t5_fence_after();
             const uint64_t kd = dk + (uint64_t)((g % DT_KSTAGES) * (2 * DT_KT * 64 * 2 >> 4));
-            if (t5_elect()) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k)              // (a panel of 64 channels, four steps of 16)
-                t5_mma(tS + 64u * (g & 1), dq + (k >> 2) * (128 * 64 * 2 >> 4) + 2 * (k & 3), kd + (k >> 2) * (DT_KT * 64 * 2 >> 4) + 2 * (k & 3),
-                       id_s, k ? 1u : 0u);
-              t5_commit(&sm.s_full[g & 1]);
-            }
-            __syncwarp();
+            for (int k = 0; k < 8; ++k)                // (a panel of 64 channels, four steps of 16)
+              t5_mma(tS + 64u * (g & 1), dq + (k >> 2) * (128 * 64 * 2 >> 4) + 2 * (k & 3), kd + (k >> 2) * (DT_KT * 64 * 2 >> 4) + 2 * (k & 3),
+                     id_s, k ? 1u : 0u);
+            t5_commit(&sm.s_full[g & 1]);
             ++g;
           }
-          if ((i == x.ntiles - 1 || x.ntiles == 0) && t5_elect()) t5_commit(&sm.q_empty);      // the query tile has been read
+          if (i == x.ntiles - 1 || x.ntiles == 0) t5_commit(&sm.q_empty);      // the query tile has been read
           if (i == (x.ntiles ? 1 : 0) && c) ok = wait(&sm.o_empty, c - 1);     // the last item's O has been read
           if (i >= 1 && ok) {
             const int gp = i < x.ntiles ? g - 2 : g - 1;                       // tile i - 1 of this item
@@ -286,7 +278,7 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             if (ok) issue_pv(gp, i == 1);
           }
         }
-        if (ok && t5_elect()) t5_commit(&sm.o_full);
+        if (ok) t5_commit(&sm.o_full);
       }
     }
   } else {

@@ -93,7 +93,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t red0 = Cfg::PUSH ? sbase + Cfg::RING : sbase;
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + Cfg::BAR_OFF);      // [0,1] group landed, [2,3] group drained, [4] accumulator complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   const bool split = ksplit > 1;
   const int ks = split ? (int)gd_cluster_rank() : 0;
   const int nb = (int)(blockIdx.x / ksplit);                               // one tile per cluster
@@ -121,7 +121,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     gd_tma_load_3d(a0 + gi * gr * GD_A_BYTES, &map_a, 0, 0, kb_first + r * gr, &bars[gi]);
     gd_tma_load_3d(w0 + gi * gr * Cfg::W_BYTES, &map_w, 0, nb * BN, kb_first + r * gr, &bars[gi]);
   };
-  if (tid == 0) {                                    // the operand copies, first thing
+  if (warp == 0 && t5_elect()) {                     // the operand copies, first thing
     for (int r = 0; r < min(ng, nrounds); ++r) issue_round(r);
   }
 
@@ -141,7 +141,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   // ---- one thread: every MMA of this CTA's share, once the operands have landed ------------------------------------
   bool ok = true;
-  if (tid == 0) {
+  if (warp == 0 && t5_elect()) {
     const uint32_t idesc = t5_idesc(BN);
     for (int r = 0; r < nrounds && ok; ++r) {
       const int gi = r % ng, par = (r / ng) & 1;

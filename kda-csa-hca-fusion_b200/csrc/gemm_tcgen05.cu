@@ -29,6 +29,7 @@
 #include <unordered_map>
 
 #include "kch_common.cuh"
+#include "tc5_utils.cuh"
 
 #define TG_BM 128
 #define TG_BK 64
@@ -206,7 +207,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   constexpr int TG_STAGES = TgSmem<BN, TWO, SK>::STAGES;
   constexpr int A_ROWS = TgSmem<BN, TWO, SK>::A_ROWS;
   constexpr int BM_T = TWO ? 2 * TG_BM : TG_BM;       // rows of a tile: a CTA pair takes 256, each CTA its 128
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = t5_warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = TWO ? cluster_ctarank() : 0u;
   const bool split = SK && ksplit > 1;
   const uint32_t ks = split ? cluster_ctarank() : 0u;
@@ -245,7 +246,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       uint32_t it = 0;
       bool ok = true;
       for (int64_t tile = unit; tile < total_tiles && ok; tile += nunits) {
@@ -275,7 +276,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && t5_elect()) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM_T >> 4) << 24);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
@@ -841,7 +842,7 @@ indexer_logits_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
                               float* __restrict__ logits, int T, int n, int HI, int64_t n_ld, int strips_per_batch) {
   extern __shared__ uint8_t smem_raw[];
   IxSmem& sm = *reinterpret_cast<IxSmem*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = t5_warp_index(), lane = threadIdx.x & 31;
   constexpr uint32_t TMEM_COLS = 2 * IX_BN;
   if (threadIdx.x == 0) {
     for (int s = 0; s < IX_ASTAGES; ++s) { mbar_init(&sm.a_full[s], 1); mbar_init(&sm.a_empty[s], 1); }
@@ -868,7 +869,7 @@ indexer_logits_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       uint32_t ait = 0, bit = 0;
       int strip = 0, cur = -1;
       bool ok = true;
@@ -896,7 +897,7 @@ indexer_logits_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(IX_BN >> 3) << 17) | ((uint32_t)(IX_BM >> 4) << 24);
       uint32_t ait = 0, bit = 0, hcount = 0;
       int strip = 0, cur = -1;

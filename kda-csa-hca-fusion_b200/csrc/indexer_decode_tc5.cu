@@ -43,7 +43,7 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
                           const int32_t* __restrict__ ctr, unsigned int* status) {
   extern __shared__ uint8_t ixd_raw[];
   IxdSmem& sm = *reinterpret_cast<IxdSmem*>(((uintptr_t)ixd_raw + 1023) & ~(uintptr_t)1023);
-  const int b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.y, tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   const int nvis = min(ctr[KCH_CTR_TOKENS] / m, ctr[KCH_CTR_N_BLOCKS]);
   const int r0 = blockIdx.x * IXD_ROWS;
   if (r0 >= nvis) return;                                      // the whole CTA, before any barrier or allocation
@@ -100,7 +100,7 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
 
   if (warp == 4) {
     // ------------------------------ producer: key tiles ------------------------------------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       for (int t = IXD_STAGES; t < ntiles; ++t) {              // the first round was issued at the top
         const int s = t % IXD_STAGES;
         if (!mbarrier_wait_bounded(&sm.empty[s], ((t / IXD_STAGES) & 1) ^ 1, KCH_STATUS_INDEXER_DECODE, IXD_SPIN, status)) break;
@@ -110,7 +110,7 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
     }
   } else if (warp == 5) {
     // ------------------------------ MMA issuer -----------------------------------------------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       const uint32_t idesc = t5_idesc(32);
       const uint64_t bdesc = t5_desc(smem_addr_u32(sm.qb));
       for (int t = 0; t < ntiles; ++t) {

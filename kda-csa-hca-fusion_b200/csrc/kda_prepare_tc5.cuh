@@ -54,7 +54,7 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   const int n = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
   const int G = a.HV / a.H, h = hv / G;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   const int t0 = n * KM_C;
   const int64_t bh = (int64_t)b * a.HV + hv;
   uint8_t* wsc = a.ws + (bh * a.NT + n) * (int64_t)KM_CHUNK_BYTES;
@@ -176,7 +176,7 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
   const uint32_t ai32 = smem_addr_u32(sm + PT_AIMG);
 
   // ---- [A ; Aqk] raw = [EK; QG] Y^T ---------------------------------------------------------------------------------
-  if (tid == 0) {
+  if (warp == 0 && t5_elect()) {
     const uint32_t yb = smem_addr_u32(sm + PT_Y), id64 = t5_idesc(64);
 #pragma unroll
     for (int term = 0; term < 3; ++term) {
@@ -373,7 +373,7 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
 
   // ---- w^T = EK^T Tb^T, u^T = V^T Tb^T (EK and V read as MN-major A operands: rows = tokens, 64-wide panels) -----------
   const uint32_t tW = tmem + 64, tU = tmem + 128;
-  if (ok && tid == 0) {
+  if (ok && warp == 0 && t5_elect()) {
     if (mbarrier_wait_bounded(&bars[1], 0, 62, PT_SPIN, status)) {
       t5_fence_after();
       const uint32_t idm = t5_idesc(64) | (1u << 15);

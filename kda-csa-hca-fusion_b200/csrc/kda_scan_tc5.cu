@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
            *va_ready1 = bars + 10;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   const int hv = blockIdx.x, b = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = t5_warp_index(), lane = threadIdx.x & 31;
   const int64_t bh = (int64_t)b * a.HV + hv;
   const uint8_t* wsb = a.ws + bh * a.NT * (int64_t)T5_CHUNK_BYTES;
   constexpr uint32_t TMEM_COLS = 512;          // S^T 128 | [D1w 64 | D1q 64] of even chunks | the same of odd chunks
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       for (int n = 0; n < a.NT; ++n) {
         const uint8_t* src = wsb + (int64_t)n * T5_CHUNK_BYTES;
         const uint32_t ph = (uint32_t)n & 1;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (t5_elect()) {
       const uint32_t id64 = t5_idesc(64), id128 = t5_idesc(128), id128mn = t5_idesc(128) | (1u << 16);
       const uint32_t sa = smem_addr_u32(sm + T5_SA), va = smem_addr_u32(sm + T5_VA), tw = smem_addr_u32(sm + T5_TW),
                      tk = smem_addr_u32(sm + T5_TK), ta = smem_addr_u32(sm + T5_TA);

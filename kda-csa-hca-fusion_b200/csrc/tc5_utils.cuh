@@ -6,12 +6,16 @@
 __device__ __forceinline__ void t5_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void t5_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void t5_fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// true in one thread of a fully active warp; the compiler keeps warp-uniform operands uniform inside the branch
+// True in one thread of a fully active warp.  The roles that one thread plays (MMA issue, copies) are entered through it
+// and not through `lane == 0`: descriptors, coordinates and addresses then stay in uniform registers, where a branch on
+// the lane number made every tcgen05.mma cost about a hundred issue cycles (the operands moved over one by one) against
+// the 64 it executes in.
 __device__ __forceinline__ bool t5_elect() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
+__device__ __forceinline__ int t5_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }   // uniform to the compiler
 __device__ __forceinline__ void t5_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr_u32(bar)) : "memory");
 }
