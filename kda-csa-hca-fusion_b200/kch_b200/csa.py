@@ -7,6 +7,8 @@ training and is not part of this path; asking for it with gradients enabled rais
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib
@@ -19,12 +21,40 @@ def _as_rows(t):
     if T == 0 or B == 0:
         t = t.contiguous()
         return t, c, T
+    if t.is_contiguous():
+        return t, c, T
     ok = (t.stride(-1) == 1 or c == 1)
     ld = t.stride(1) if T > 1 else max(c, t.stride(1))
     if ok and ld >= c and (B == 1 or (t.stride(0) % ld == 0 and t.stride(0) >= T * ld)):
         return t, ld, (t.stride(0) // ld if B > 1 else T)
     t = t.contiguous()
     return t, c, T
+
+
+def _rows_2d(x, width):
+    """``(tensor, rows, elements between rows)`` of ``x [..., width]`` seen as ``[rows, width]`` with a dense last
+    dimension; copies only when no such view exists."""
+    if x.is_contiguous():
+        return x, x.numel() // width if width else 0, width
+    if x.dim() == 3 and x.stride(2) == 1 and (x.shape[0] == 1 or x.stride(0) == x.shape[1] * x.stride(1)):
+        rows = x.shape[0] * x.shape[1]
+        return x, rows, x.stride(1) if rows > 1 and x.shape[1] > 1 else (x.stride(0) if rows > 1 else width)
+    x = x.reshape(-1, width)
+    if x.stride(-1) != 1 and width > 1:
+        x = x.contiguous()
+    return x, x.shape[0], x.stride(0) if x.shape[0] > 1 else width
+
+
+@functools.lru_cache(maxsize=64)
+def _epilogue(segments, group):
+    """The C form of a list of column segments (read by the call only, so equal lists share one)."""
+    ep = _lib.Epilogue()
+    ep.n_segments, ep.group = len(segments), int(group)
+    end = 0
+    for i, (width, act, param) in enumerate(segments):
+        end += int(width)
+        ep.seg_end[i], ep.seg_act[i], ep.seg_param[i] = end, int(act), float(param)
+    return ep, end
 
 
 def linear(x, W, residual=None, epilogue=None, group=1):
@@ -39,35 +69,27 @@ def linear(x, W, residual=None, epilogue=None, group=1):
         raise ValueError(f"linear: weight shape {tuple(W.shape)} does not match input features {K}")
     if W.dtype != x.dtype:
         raise ValueError(f"linear: weight dtype {W.dtype} does not match input dtype {x.dtype}")
-    lead = x.shape[:-1]
-    x2 = x.reshape(-1, K)
-    if x2.stride(-1) != 1 and K > 1:
-        x2 = x2.contiguous()
-    M = x2.shape[0]
-    lda = x2.stride(0) if M > 1 else K
+    x2, M, lda = _rows_2d(x, K)
     if W.stride(-1) != 1:
         W = W.contiguous()
-    out = torch.empty(M, N, dtype=x.dtype, device=x.device)
+    out = torch.empty((*x.shape[:-1], N), dtype=x.dtype, device=x.device)
     r2, ldr = None, 0
     if residual is not None:
-        r2 = residual.reshape(-1, N)
-        if r2.stride(-1) != 1:
-            r2 = r2.contiguous()
-        ldr = r2.stride(0) if M > 1 else N
+        r2, rows, ldr = _rows_2d(residual, residual.shape[-1])
+        if rows != M or residual.shape[-1] != N:
+            r2 = residual.reshape(-1, N)
+            if r2.stride(-1) != 1:
+                r2 = r2.contiguous()
+            ldr = r2.stride(0) if M > 1 else N
     ep = None
     if epilogue:
-        ep = _lib.Epilogue()
-        ep.n_segments, ep.group = len(epilogue), int(group)
-        end = 0
-        for i, (width, act, param) in enumerate(epilogue):
-            end += int(width)
-            ep.seg_end[i], ep.seg_act[i], ep.seg_param[i] = end, int(act), float(param)
+        ep, end = _epilogue(tuple(map(tuple, epilogue)), group)
         if end != N:
             raise ValueError(f"linear: epilogue segments cover {end} columns, the weight has {N} rows")
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_linear_ex(_lib.ptr(x2), _lib.ptr(W), _lib.ptr(out), _lib.ptr(r2), M, N, K, lda,
                                      W.stride(0), N, ldr, _lib.dtype_tag(x.dtype), ep, _lib.stream()))
-    return out.reshape(*lead, N)
+    return out
 
 
 def linear_kslabs(a_slabs, W, residual=None):
@@ -92,7 +114,7 @@ def linear_kslabs(a_slabs, W, residual=None):
         if r2.stride(-1) != 1:
             r2 = r2.contiguous()
         ldr = r2.stride(0) if M > 1 else N
-    with torch.cuda.device(a_slabs.device):
+    with _lib.device(a_slabs.device):
         _lib.check(lib.kch_linear_kslabs(_lib.ptr(a_slabs), _lib.ptr(W), _lib.ptr(out), _lib.ptr(r2), M, N, K, n_slabs,
                                          W.stride(0), N, ldr, _lib.KCH_BF16, _lib.stream()))
     return out
@@ -115,20 +137,18 @@ def rownorm(x, normalize=True, out_dtype=torch.float32):
         return x.to(out_dtype)
     lib = _lib.load()
     c = x.shape[-1]
-    lead = x.shape[:-1]
     if x.is_contiguous() or x.dim() != 3:
-        x3 = x.contiguous().reshape(1, -1, c)
+        x3, ld = x.contiguous(), c
     else:
-        x3 = x
-    x3, ld, bsr = _as_rows(x3)
-    if bsr != x3.shape[1]:
-        x3, ld = x3.contiguous(), c
-    rows = x3.shape[0] * x3.shape[1]
-    y = torch.empty(rows, c, dtype=out_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+        x3, ld, bsr = _as_rows(x)
+        if bsr != x3.shape[1]:
+            x3, ld = x3.contiguous(), c
+    rows = x3.numel() // c if c else 0
+    y = torch.empty(x.shape, dtype=out_dtype, device=x.device)
+    with _lib.device(x.device):
         _lib.check(lib.kch_rownorm(_lib.ptr(x3), ld, _lib.ptr(y), None, rows, c, _lib.dtype_tag(x.dtype),
                                    _lib.dtype_tag(out_dtype), _lib.stream()))
-    return y.reshape(*lead, c)
+    return y
 
 
 def csa_compress_kv(C, Z, B_pos, m: int):
@@ -148,7 +168,7 @@ def csa_compress_kv(C, Z, B_pos, m: int):
     Bp = B_pos.contiguous()
     n = T // m
     out = torch.empty(B, n, c, dtype=torch.float32, device=C.device)
-    with torch.cuda.device(C.device):
+    with _lib.device(C.device):
         _lib.check(lib.kch_compress_kv(_lib.ptr(C2), _lib.ptr(Z2), _lib.ptr(Bp), _lib.ptr(out), B, T, c, m, ld, bsr,
                                        n * c, _lib.dtype_tag(C.dtype), _lib.dtype_tag(Bp.dtype), _lib.stream()))
     return out
@@ -178,7 +198,7 @@ def csa_compress_kv_overlapped(Ca, Cb, Za, Zb, Ba, Bb, m: int, *, prev_Cb=None, 
         pc, pz = prev_Cb.to(Ca.dtype).contiguous(), prev_Zb.to(Ca.dtype).contiguous()
     n = T // m
     out = torch.empty(B, n, c, dtype=torch.float32, device=Ca.device)
-    with torch.cuda.device(Ca.device):
+    with _lib.device(Ca.device):
         _lib.check(lib.kch_compress_kv_overlapped(
             _lib.ptr(views[0][0]), _lib.ptr(views[1][0]), _lib.ptr(views[2][0]), _lib.ptr(views[3][0]),
             _lib.ptr(Ba_), _lib.ptr(Bb_), _lib.ptr(pc), _lib.ptr(pz), c, _lib.ptr(out), B, T, c, m, ld, bsr, n * c,
@@ -209,7 +229,7 @@ def indexer_topk(q_idx, k_idx, w_idx, topk, *, m=0, t0=0, n_visible=-1, normaliz
         wf = None if w_idx is None else w_idx.float().contiguous()
         nbytes = int(lib.kch_indexer_workspace_bytes_ex(B, T, n, _lib.KCH_BF16))
         ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device(dev):
             _lib.check(lib.kch_indexer_topk_ex(_lib.ptr(q_idx), _lib.KCH_BF16, q_idx.stride(1), 1, _lib.ptr(kn),
                                                _lib.ptr(wf), _lib.ptr(idx), B, T, n, HI, DI, int(topk), float(scale),
                                                int(m), int(t0), int(n_visible), 1 if sorted_output else 0,
@@ -225,7 +245,7 @@ def indexer_topk(q_idx, k_idx, w_idx, topk, *, m=0, t0=0, n_visible=-1, normaliz
     wf = None if w_idx is None else w_idx.float().contiguous()
     nbytes = int(lib.kch_indexer_workspace_bytes(B, T, n, HI, DI))
     ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device(dev):
         _lib.check(lib.kch_indexer_topk(_lib.ptr(qn), _lib.ptr(kn), _lib.ptr(wf), _lib.ptr(idx), B, T, n, HI, DI,
                                         int(topk), float(scale), int(m), int(t0), int(n_visible),
                                         1 if sorted_output else 0, int(k_batch_stride), _lib.ptr(ws), nbytes,
@@ -302,7 +322,7 @@ def attend(q, comp, *, nh, c, sel=None, m=0, t0=0, n_visible=-1, q_normalize=Fal
     lib = _lib.load()
     B, T = q.shape[0], q.shape[1]
     a = _lib.AttendArgs()
-    q3, qld, qbsr = _as_rows(q.reshape(B, T, nh * c))
+    q3, qld, qbsr = _as_rows(q if q.dim() == 3 else q.reshape(B, T, nh * c))
     if qbsr != T:
         q3 = q3.contiguous()
         qld = nh * c
@@ -341,7 +361,7 @@ def attend(q, comp, *, nh, c, sel=None, m=0, t0=0, n_visible=-1, q_normalize=Fal
     a.scale = float(scale)
     out = torch.empty(B, T, nh * c, dtype=out_dtype, device=q.device)
     a.out, a.out_dtype = out.data_ptr(), _lib.dtype_tag(out_dtype)
-    with torch.cuda.device(q.device):
+    with _lib.device(q.device):
         _lib.check((lib.kch_attend_distinct if sel_distinct else lib.kch_attend)(a, _lib.stream()))
     return out
 

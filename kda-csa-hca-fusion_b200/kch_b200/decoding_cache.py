@@ -73,7 +73,7 @@ def _row_norms(x):
     B, n, c = x.shape
     x = x.contiguous()
     out = torch.empty(B, n, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_rownorm(_lib.ptr(x), c, None, _lib.ptr(out), B * n, c, _lib.dtype_tag(x.dtype), _lib.KCH_F32,
                                    _lib.stream()))
     return out
@@ -199,7 +199,7 @@ class _CacheBase:
         a.out, a.out_dtype = out.data_ptr(), _lib.dtype_tag(out_dtype)
         a.counters = self._ctr.data_ptr()
         a.workspace, a.workspace_bytes = self._ws_attn.data_ptr(), self._ws_attn.numel()
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             _lib.check(lib.kch_attend_decode(a, _lib.stream()))
         return out
 
@@ -242,7 +242,7 @@ class _CacheBase:
         B, nb, c = rows_f32.shape
         r = rows_f32.to(self.dtype)
         tmp_norm = torch.empty(B, nb, dtype=torch.float32, device=self.device)
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             if self._kind is None:
                 self._comp[:, start:start + nb] = r
                 _lib.check(lib.kch_rownorm(_lib.ptr(r), c, None, _lib.ptr(tmp_norm), B * nb, c,
@@ -419,7 +419,7 @@ class CSADecodingCache(_CacheBase):
             a.ring, a.ring_pos = self._sw._buf.data_ptr(), self._sw._n % self.win
         a.normalize = int(self._normalize_qk)
         a.counters = self._ctr.data_ptr()
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             _lib.check(lib.kch_cache_append_token_advance(a, _lib.stream()))   # the last CTA advances the device counters
         self._advance(m)
 
@@ -520,7 +520,7 @@ class CSADecodingCache(_CacheBase):
         wf, w_ld = (None, 0) if w_idx is None else rows(w_idx, HI)
         idx = torch.empty(B, 1, topk, dtype=torch.int32, device=self.device)
         scale = 1.0 if normalize_qk else DI ** -0.5
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             _lib.check(lib.kch_decode_indexer_topk(
                 _lib.ptr(qf), _lib.dtype_tag(qf.dtype), q_ld, _lib.ptr(self._kcomp), _lib.dtype_tag(self.dtype),
                 _lib.ptr(self._kcomp_norms), _lib.ptr(wf), 0 if wf is None else _lib.dtype_tag(wf.dtype), w_ld,
@@ -646,7 +646,7 @@ class HCADecodingCache(_CacheBase):
             a.ring, a.ring_pos = self._sw._buf.data_ptr(), self._sw._n % self.win
         a.normalize = int(self._normalize_qk)
         a.counters = self._ctr.data_ptr()
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             _lib.check(lib.kch_cache_append_token_advance(a, _lib.stream()))   # the last CTA advances the device counters
         self._advance(m)
 

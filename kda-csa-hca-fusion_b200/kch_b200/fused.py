@@ -99,7 +99,7 @@ def layernorm(x, weight, bias, eps=1e-5):
     x = x.contiguous()
     d = x.shape[-1]
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_layernorm(_lib.ptr(x), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), x.numel() // d, d,
                                      float(eps), _lib.dtype_tag(x.dtype), _lib.dtype_tag(weight.dtype),
                                      _lib.stream()))
@@ -115,7 +115,7 @@ def short_conv(x, weight, bias, lookback=None):
     b = bias.to(x.dtype).contiguous()
     lb = None if lookback is None else lookback.to(x.dtype).contiguous()
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_short_conv(_lib.ptr(x), _lib.ptr(lb), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), B, T, d,
                                       _lib.dtype_tag(x.dtype), _lib.stream()))
     return y
@@ -138,7 +138,7 @@ def layernorm_short_conv(x, ln_weight, ln_bias, eps, weight, bias, lookback=None
     lw, lbias = ln_weight.contiguous(), ln_bias.contiguous()
     y = torch.empty_like(x)
     new_lb = torch.empty(B, 2, d, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_layernorm_short_conv(_lib.ptr(x), _lib.ptr(lw), _lib.ptr(lbias), float(eps), _lib.ptr(lb),
                                                 _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.ptr(new_lb), B, T, d,
                                                 _lib.dtype_tag(x.dtype), _lib.dtype_tag(lw.dtype), _lib.stream()))
@@ -155,7 +155,7 @@ def short_conv_step(x, weight, bias, lookback):
     w = weight.reshape(d, 3).to(x.dtype).contiguous()
     b = bias.to(x.dtype).contiguous()
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_short_conv_step(_lib.ptr(x), _lib.ptr(lookback), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), B, d,
                                            _lib.dtype_tag(x.dtype), _lib.stream()))
     return y
@@ -177,7 +177,7 @@ def layernorm_short_conv_step(x, ln_weight, ln_bias, eps, weight, bias, lookback
     b = bias.to(x.dtype).contiguous()
     lw, lbias = ln_weight.contiguous(), ln_bias.contiguous()
     y = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_layernorm_short_conv_step(_lib.ptr(x), _lib.ptr(lw), _lib.ptr(lbias), float(eps),
                                                      _lib.ptr(lookback), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), B, d,
                                                      _lib.dtype_tag(x.dtype), _lib.dtype_tag(lw.dtype), _lib.stream()))
@@ -202,7 +202,7 @@ def activation(x, act, *, param=0.0, group=1):
             x2 = x2.contiguous().reshape(-1, cols)
         rows, ldx = x2.shape[0], (x2.stride(0) if x2.shape[0] > 1 else cols)
     y = torch.empty(rows, cols, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.device(x.device):
         _lib.check(lib.kch_activation(_lib.ptr(x2), _lib.ptr(y), rows, cols, act, float(param), int(group),
                                       _lib.dtype_tag(x.dtype), ldx, cols, _lib.stream()))
     return y.reshape(*lead, cols)
@@ -551,7 +551,7 @@ class HybridDecoding(nn.Module):
         model = self.model
         dev = next(model.parameters()).device
         if dev.type == "cuda":
-            with torch.cuda.device(dev):
+            with _lib.device(dev):
                 _lib.raise_on_device_status("HybridDecoding.export_state")      # never checkpoint a broken session
         return {
             "layout": list(model.layout),

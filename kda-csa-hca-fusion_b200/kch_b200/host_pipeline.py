@@ -103,5 +103,5 @@ class HostPipeline:
         without writing their outputs.  Read it where the host waits anyway (the downloads have to complete
         before the caller may use `outputs`), and turn it into an exception instead of silent garbage."""
         from . import _lib
-        with torch.cuda.device(self.device):
+        with _lib.device(self.device):
             _lib.raise_on_device_status("HostPipeline.run")

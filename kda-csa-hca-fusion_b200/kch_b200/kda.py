@@ -18,7 +18,12 @@ _VALID_BACKENDS = {"b200"}
 
 
 def _validate_inputs(q, k, v, g, beta, fn_name):
-    # shape / device / dtype contract of ops_kda.py:28-83
+    # shape / device / dtype contract of ops_kda.py:28-83; the checks one by one only to name the first that fails
+    if (q.dim() == k.dim() == v.dim() == g.dim() == 4 and beta.dim() == 3
+            and q.shape[:2] == k.shape[:2] == v.shape[:2] == g.shape[:2] == beta.shape[:2]
+            and q.device == k.device == v.device == g.device == beta.device
+            and q.dtype == k.dtype == v.dtype == g.dtype == beta.dtype):
+        return
     for name, t, rank in (("q", q, 4), ("k", k, 4), ("v", v, 4), ("g", g, 4), ("beta", beta, 3)):
         if t.dim() != rank:
             expect = ("[B, T, H, K]" if name in ("q", "k") else "[B, T, HV, V]" if name == "v"
@@ -69,6 +74,8 @@ def _validate_shapes(q, k, v, g, beta, fn_name, chunk_size=None):
 def _token_stride(x):
     """``(tensor, elements between consecutive tokens)`` for a ``[B,T,H,K]`` / ``[B,T,HV]`` operand whose heads are
     dense within a token (e.g. a column slice of a fused projection); anything else is made contiguous."""
+    if x.is_contiguous():
+        return x, x.shape[2] * (x.shape[3] if x.dim() == 4 else 1)
     inner = 1
     ok = True
     for d in range(x.dim() - 1, 1, -1):
@@ -101,7 +108,11 @@ def _run(fn_name, q, k, v, g, beta, scale, initial_state, output_final_state, g_
     B, T, H, K = q.shape
     HV, V = v.shape[2], v.shape[-1]
     tag = _lib.dtype_tag(v.dtype)
-    (q, ld_q), (k, ld_k), (v, ld_v), (g, ld_g), (beta, ld_b) = (_token_stride(x) for x in (q, k, v, g, beta))
+    q, ld_q = _token_stride(q)
+    k, ld_k = _token_stride(k)
+    v, ld_v = _token_stride(v)
+    g, ld_g = _token_stride(g)
+    beta, ld_b = _token_stride(beta)
     if ld_q != ld_k:
         q, k = q.contiguous(), k.contiguous()
         ld_q = ld_k = H * K
@@ -125,7 +136,7 @@ def _run(fn_name, q, k, v, g, beta, scale, initial_state, output_final_state, g_
             S = torch.empty(B, HV, K, V, dtype=torch.float32, device=q.device)
     gmin = float(g_clamp_min) if g_clamp_min > -math.inf else -math.inf
     sc = _scale_value(scale, K)
-    with torch.cuda.device(q.device):
+    with _lib.device(q.device):
         if chunk_size is None:
             _lib.check(lib.kch_kda_recurrent(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(g), _lib.ptr(beta),
                                              _lib.ptr(S0), _lib.ptr(o), _lib.ptr(S), B, T, H, HV, K, V, sc, gmin,

@@ -66,7 +66,7 @@ class PeerGather:
         """``flat [rows, width]`` contiguous on this rank -> ``[world, rows, width]`` (rank-major), a view of the buffer."""
         _lib = self._lib
         nbytes = flat.numel() * flat.element_size()
-        with torch.cuda.device(flat.device):
+        with _lib.device(flat.device):
             _lib.check(_lib.load().kch_peer_allgather(_lib.ptr(flat), nbytes, self._bufs, self._flags, self.rank,
                                                       self.world, _lib.stream()))
         out = self.mem[self.flag_bytes:self.flag_bytes + self.world * nbytes].view(flat.dtype)
