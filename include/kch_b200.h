@@ -111,6 +111,13 @@ int kch_linear_ex(const void* A, const void* W, void* C, const void* residual, i
                   int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* epilogue,
                   void* stream);
 
+/* kch_linear_ex for a caller who vouches that the launch just before it on `stream` does not write W (the projections of
+ * a decode step: the launch before is the kernel that produced A).  A decode batch's weights are then under way before
+ * that launch has finished. */
+int kch_linear_settled(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
+                       int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* epilogue,
+                       void* stream);
+
 /* The output projection after an all-gather of per-GPU head slices (no counterpart in the reference, which has no
  * distributed code; mathematically F.linear(concat_heads(A), W), ops_fused.py:609/713/739): A holds the K input
  * columns as `n_slabs` slabs [n_slabs][M][K / n_slabs] one after the other -- the rank-major buffer ncclAllGather

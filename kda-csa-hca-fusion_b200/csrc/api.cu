@@ -29,7 +29,7 @@ int kch_linear_simt(const void* A, const void* W, void* C, const void* residual,
 bool kch_linear_tcgen05_supported(const void* A, const void* W, const void* C, const void* R, int64_t M, int N,
                                   int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype);
 int kch_linear_tcgen05(const void* A, const void* W, void* C, const void* R, int64_t M, int N, int K, int64_t lda,
-                       int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream, int slab_k = 0);
+                       int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream, int slab_k = 0, int w_settled = 0);
 bool kch_linear_tcgen05_epilogue_ok(const kch_epilogue* e, int N);
 
 extern "C" int kch_linear(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
@@ -55,9 +55,9 @@ extern "C" int kch_linear_kslabs(const void* A, const void* W, void* C, const vo
   return kch_linear_tcgen05(A, W, C, residual, M, N, K, slab_k, ldw, ldc, ldr, nullptr, stream, n_slabs > 1 ? slab_k : 0);
 }
 
-extern "C" int kch_linear_ex(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
-                             int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* ep,
-                             void* stream) {
+static int linear_impl(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
+                       int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* ep,
+                       int w_settled, void* stream) {
   KCH_REQUIRE(M >= 0 && N >= 0 && K >= 1, "kch_linear: M=%lld N=%d K=%d", (long long)M, N, K);
   KCH_REQUIRE(lda >= K && ldw >= K && ldc >= N, "kch_linear: leading dimensions lda=%lld ldw=%lld ldc=%lld too small",
               (long long)lda, (long long)ldw, (long long)ldc);
@@ -74,8 +74,8 @@ extern "C" int kch_linear_ex(const void* A, const void* W, void* C, const void* 
   const bool tc = !force_simt && N >= 32 &&
                   kch_linear_tcgen05_supported(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype);
   if (tc && kch_linear_tcgen05_epilogue_ok(ep, N))
-    return kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, ep, stream);
-  int rc = tc ? kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, nullptr, stream)
+    return kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, ep, stream, 0, w_settled);
+  int rc = tc ? kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, nullptr, stream, 0, w_settled)
               : kch_linear_simt(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype, stream);
   if (rc != KCH_OK || !ep || ep->n_segments == 0) return rc;
   // unfused epilogue: the same activations as separate in-place passes over the column segments
@@ -92,4 +92,15 @@ extern "C" int kch_linear_ex(const void* A, const void* W, void* C, const void* 
     start = end;
   }
   return KCH_OK;
+}
+
+extern "C" int kch_linear_ex(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
+                             int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* ep,
+                             void* stream) {
+  return linear_impl(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype, ep, 0, stream);
+}
+extern "C" int kch_linear_settled(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
+                                  int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, const kch_epilogue* ep,
+                                  void* stream) {
+  return linear_impl(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype, ep, 1, stream);
 }

@@ -65,6 +65,8 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_split_kernel(AdArgs a)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ float s_m[4][AD_NH], s_l[4][AD_NH];
   __shared__ float s_acc[4][AD_NH][AD_C];
+  chain_wait();
+  chain_trigger();
   // ---- per-step geometry from the device counters -------------------------------------------------------
   const int nb = a.ctr[KCH_CTR_N_BLOCKS];
   int nvis = a.m > 0 ? a.ctr[KCH_CTR_TOKENS] / a.m : nb;
@@ -207,6 +209,8 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_split_kernel(AdArgs a)
 }
 
 __global__ void __launch_bounds__(AD_THREADS) attn_decode_combine_kernel(AdArgs a, int S) {
+  chain_wait();
+  chain_trigger();
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const float* wsb = a.ws + (int64_t)b * S * a.nh * (AD_C + 2) + h * (AD_C + 2);
   const int64_t stride = (int64_t)a.nh * (AD_C + 2);
@@ -293,6 +297,8 @@ __global__ void __launch_bounds__(ADM_WARPS * 32) attn_decode_mma_kernel(AdArgs 
   uint8_t* wbase = adm_smem + 2 * 16 * ADM_QLD * 2 + (size_t)warp * ((ADM_STAGES + 1) * ADM_STAGE_BYTES);
   const uint32_t ring = smem_addr_u32(wbase);
   const uint32_t work = ring + ADM_STAGES * ADM_STAGE_BYTES;
+  chain_wait();
+  chain_trigger();
   // ---- per-step geometry from the device counters -------------------------------------------------------
   const int nb = a.ctr[KCH_CTR_N_BLOCKS];
   int nvis = a.m > 0 ? a.ctr[KCH_CTR_TOKENS] / a.m : nb;
@@ -658,16 +664,16 @@ extern "C" int kch_attend_decode(const kch_attend_decode_args* p, void* stream) 
     const size_t smem = 2 * 16 * ADM_QLD * 2 + (size_t)ADM_WARPS * ((ADM_STAGES + 1) * ADM_STAGE_BYTES);
     if (p->comp_dtype == KCH_BF16) {
       KCH_CUDA_OK(cudaFuncSetAttribute(attn_decode_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attn_decode_mma_kernel<false><<<dim3(S, p->B), ADM_WARPS * 32, smem, s>>>(a);
+      KCH_CUDA_OK(kch_launch_chained(attn_decode_mma_kernel<false>, dim3(S, p->B), dim3(ADM_WARPS * 32), smem, s, 1, a));
     } else {
       KCH_CUDA_OK(cudaFuncSetAttribute(attn_decode_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attn_decode_mma_kernel<true><<<dim3(S, p->B), ADM_WARPS * 32, smem, s>>>(a);
+      KCH_CUDA_OK(kch_launch_chained(attn_decode_mma_kernel<true>, dim3(S, p->B), dim3(ADM_WARPS * 32), smem, s, 1, a));
     }
   } else {
-    attn_decode_split_kernel<<<dim3(S, p->B), AD_THREADS, 0, s>>>(a);
+    KCH_CUDA_OK(kch_launch_chained(attn_decode_split_kernel, dim3(S, p->B), dim3(AD_THREADS), 0, s, 1, a));
   }
   KCH_LAUNCH_OK();
-  attn_decode_combine_kernel<<<dim3(p->nh, p->B), AD_THREADS, 0, s>>>(a, S);
+  KCH_CUDA_OK(kch_launch_chained(attn_decode_combine_kernel, dim3(p->nh, p->B), dim3(AD_THREADS), 0, s, 1, a, S));
   KCH_LAUNCH_OK();
   return KCH_OK;
 }

@@ -72,6 +72,8 @@ __global__ void __launch_bounds__(128) cache_append_kernel(AppendArgs a) {
   extern __shared__ float srow[];   // [c] compressed row, then [cI]
   __shared__ float red[4];
   const int b = blockIdx.x, tid = threadIdx.x;
+  chain_wait();
+  chain_trigger();
   if (a.counters) {   // the step is replayed from a CUDA graph: the counters live on the device
     a.acc_len = a.counters[KCH_CTR_ACC_LEN];
     a.n_blocks = a.counters[KCH_CTR_N_BLOCKS];
@@ -253,8 +255,8 @@ static int cache_append_launch(const kch_cache_append_args* p, void* stream, int
   a.advance = advance; a.n_ctas = p->B;
   size_t smem = (size_t)(p->c > p->c_I ? p->c : p->c_I) * sizeof(float);
   cudaStream_t s = kch_stream(stream);
-  if (p->dtype == KCH_BF16) cache_append_kernel<bf16><<<p->B, 128, smem, s>>>(a);
-  else cache_append_kernel<float><<<p->B, 128, smem, s>>>(a);
+  if (p->dtype == KCH_BF16) KCH_CUDA_OK(kch_launch_chained(cache_append_kernel<bf16>, dim3(p->B), dim3(128), smem, s, 1, a));
+  else KCH_CUDA_OK(kch_launch_chained(cache_append_kernel<float>, dim3(p->B), dim3(128), smem, s, 1, a));
   KCH_LAUNCH_OK();
   return KCH_OK;
 }

@@ -93,9 +93,10 @@ __device__ __forceinline__ float block_sum_256(float v, float* red) {
 
 template <typename TW>
 __global__ void __launch_bounds__(256)
-layernorm_row_kernel_bf16(const bf16* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b,
-                          bf16* __restrict__ y, int d, float eps) {
+layernorm_row_kernel_bf16(const bf16* x, const TW* w, const TW* b, bf16* y, int d, float eps) {
   __shared__ float red[8];
+  chain_wait();
+  chain_trigger();
   const int c0 = threadIdx.x * 8;
   const bool on = c0 < d;
   const int64_t row = blockIdx.x;
@@ -131,7 +132,7 @@ extern "C" int kch_layernorm(const void* x, const void* weight, const void* bias
   if (dtype == KCH_BF16 && rows <= 512 && (d % 8) == 0 && d <= 2048 &&
       (((uintptr_t)x | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0) {
     cudaStream_t s = kch_stream(stream);
-    KCH_DISPATCH_FLOAT(wdtype, TW, (layernorm_row_kernel_bf16<TW><<<(unsigned)rows, 256, 0, s>>>(
+    KCH_DISPATCH_FLOAT(wdtype, TW, KCH_CUDA_OK(kch_launch_chained(layernorm_row_kernel_bf16<TW>, dim3((unsigned)rows), dim3(256), 0, s, 1,
         (const bf16*)x, (const TW*)weight, (const TW*)bias, (bf16*)y, d, eps)));
     KCH_LAUNCH_OK();
     return KCH_OK;
@@ -432,10 +433,11 @@ extern "C" int kch_short_conv_step(const void* x, void* lookback, const void* we
 // kch_short_conv_step (the normalised row is rounded to bf16 before the taps see it).
 template <typename TW>
 __global__ void __launch_bounds__(256)
-ln_conv_step_kernel_bf16(const bf16* __restrict__ x, const TW* __restrict__ lw, const TW* __restrict__ lb2, float eps,
-                         bf16* lookback, const bf16* __restrict__ cw, const bf16* __restrict__ cb,
-                         bf16* __restrict__ y, int d) {
+ln_conv_step_kernel_bf16(const bf16* x, const TW* lw, const TW* lb2, float eps, bf16* lookback, const bf16* cw, const bf16* cb,
+                         bf16* y, int d) {
   __shared__ float red[8];
+  chain_wait();
+  chain_trigger();
   const int c0 = threadIdx.x * 8;
   const bool on = c0 < d;
   const int64_t row = blockIdx.x;
@@ -495,7 +497,7 @@ extern "C" int kch_layernorm_short_conv_step(const void* x, const void* ln_weigh
   KCH_REQUIRE(((((uintptr_t)ln_weight) | ((uintptr_t)ln_bias)) & 15) == 0,
               "kch_layernorm_short_conv_step: LayerNorm parameters must be 16-byte aligned");
   cudaStream_t s = kch_stream(stream);
-  KCH_DISPATCH_FLOAT(wdtype, TW, (ln_conv_step_kernel_bf16<TW><<<(unsigned)B, 256, 0, s>>>(
+  KCH_DISPATCH_FLOAT(wdtype, TW, KCH_CUDA_OK(kch_launch_chained(ln_conv_step_kernel_bf16<TW>, dim3((unsigned)B), dim3(256), 0, s, 1,
       (const bf16*)x, (const TW*)ln_weight, (const TW*)ln_bias, eps, (bf16*)lookback, (const bf16*)conv_weight,
       (const bf16*)conv_bias, (bf16*)y, d)));
   KCH_LAUNCH_OK();

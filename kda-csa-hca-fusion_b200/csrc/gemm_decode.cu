@@ -77,8 +77,8 @@ __device__ __forceinline__ float gd_silu(float x) { return __fdividef(x, 1.0f + 
 template <int BN>
 __global__ void __launch_bounds__(GD_THREADS)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                   bf16* __restrict__ C, const bf16* __restrict__ R, int M, int N, int kblocks_all, int kper,
-                   int64_t ldc, int64_t ldr, int vec_ok, const GdEpilogue ep, int ksplit, int gr, int ng,
+                   bf16* C, const bf16* R, int M, int N, int kblocks_all, int kper,
+                   int64_t ldc, int64_t ldr, int vec_ok, const GdEpilogue ep, int ksplit, int gr, int ng, int w_settled,
                    unsigned int* status) {
   // `gr` k-blocks per copy (the depth of a tensor-map box), `ng` groups of `gr` stages: ng = 1 when the CTA's whole
   // share fits the ring (one copy per operand), else 2 groups refilled in turn as their MMAs retire
@@ -115,14 +115,29 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const uint32_t tmem = *tmem_slot;
   if (split && Cfg::PUSH) gd_cluster_arrive();       // "my shared memory exists": waited for before the first push
   const int nrounds = (kblocks + gr - 1) / gr;
-  auto issue_round = [&](int r) {                    // k-blocks [r * gr, (r + 1) * gr) of this CTA into group r % ng
+  auto issue_w = [&](int r) {                        // k-blocks [r * gr, (r + 1) * gr) of this CTA into group r % ng
     const int gi = r % ng;
     mbarrier_expect_tx(&bars[gi], (uint32_t)gr * (GD_A_BYTES + Cfg::W_BYTES));       // a box is `gr` k-blocks deep
-    gd_tma_load_3d(a0 + gi * gr * GD_A_BYTES, &map_a, 0, 0, kb_first + r * gr, &bars[gi]);
     gd_tma_load_3d(w0 + gi * gr * Cfg::W_BYTES, &map_w, 0, nb * BN, kb_first + r * gr, &bars[gi]);
   };
-  if (warp == 0 && t5_elect()) {                     // the operand copies, first thing
-    for (int r = 0; r < min(ng, nrounds); ++r) issue_round(r);
+  auto issue_a = [&](int r) {
+    const int gi = r % ng;
+    gd_tma_load_3d(a0 + gi * gr * GD_A_BYTES, &map_a, 0, 0, kb_first + r * gr, &bars[gi]);
+  };
+  // The operand copies, first thing.  Weights that the launch before this one does not write (w_settled) are under way
+  // before that launch has finished: their share of HBM time, and this kernel's set-up, disappear behind it.
+  const int first = min(ng, nrounds);
+  if (w_settled && warp == 0 && t5_elect()) {
+    for (int r = 0; r < first; ++r) issue_w(r);
+  }
+  __syncwarp();
+  chain_wait();
+  chain_trigger();
+  if (warp == 0 && t5_elect()) {
+    for (int r = 0; r < first; ++r) {
+      if (!w_settled) issue_w(r);
+      issue_a(r);
+    }
   }
 
   // ---- the rows this thread finishes, and their residual values (an earlier kernel's output: ready now) ----------
@@ -158,7 +173,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       if (r + ng < nrounds) {                          // refill this group once its MMAs have read it
         t5_commit(&bars[2 + gi]);
         ok = mbarrier_wait_bounded(&bars[2 + gi], par, KCH_STATUS_GEMM_DECODE, GD_SPIN, status);
-        if (ok) issue_round(r + ng);
+        if (ok) { issue_w(r + ng); issue_a(r + ng); }
       }
     }
     if (ok) t5_commit(&bars[4]);
@@ -307,7 +322,7 @@ int kch_make_tensor_map_katoms_bf16(CUtensorMap* map, const void* base, uint64_t
 
 template <int BN>
 static int launch_gd(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int64_t lda, int64_t ldw,
-                     int64_t ldc, int64_t ldr, const GdEpilogue& ep, cudaStream_t s) {
+                     int64_t ldc, int64_t ldr, const GdEpilogue& ep, int w_settled, cudaStream_t s) {
   using Cfg = GdCfg<BN>;
   static int sms = 0;
   if (!sms) {
@@ -337,21 +352,16 @@ static int launch_gd(const void* A, const void* W, void* C, const void* R, int M
   KCH_REQUIRE(status != nullptr, "kch_linear: cannot resolve the device status word");
   const int vec_ok = (ldc % 4 == 0) && (((uintptr_t)C & 7) == 0) && (!R || ((ldr % 4 == 0) && (((uintptr_t)R & 7) == 0)));
   KCH_CUDA_OK(cudaFuncSetAttribute(gemm_decode_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ksplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(tiles * ksplit)); cfg.blockDim = dim3(GD_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM;
-  cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = ksplit > 1 ? 1 : 0;
-  KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_decode_kernel<BN>, ma, mw, (bf16*)C, (const bf16*)R, M, N, kblocks, kper, ldc, ldr,
-                                 vec_ok, ep, ksplit, gr, ng, status));
+  KCH_CUDA_OK(kch_launch_chained(gemm_decode_kernel<BN>, dim3((unsigned)(tiles * ksplit)), dim3(GD_THREADS), Cfg::SMEM, s,
+                                 (unsigned)ksplit, ma, mw, (bf16*)C, (const bf16*)R, M, N, kblocks, kper, ldc, ldr, vec_ok, ep,
+                                 ksplit, gr, ng, w_settled, status));
   kch_note_launch(1);
   return KCH_OK;
 }
 
 // KCH_OK when launched; GD_UNSUPPORTED (-100) when this shape belongs to the general kernel (the caller goes on).
 int kch_linear_decode_tc5(const void* A, const void* W, void* C, const void* R, int64_t M, int N, int K, int64_t lda,
-                          int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream) {
+                          int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, int w_settled, void* stream) {
   static const bool off = [] { const char* v = getenv("KCH_GEMM_DECODE"); return v && v[0] == '0'; }();
   if (off || M < 1 || M > GD_ROWS || N < 8 || K < GD_BK || (K % GD_BK) != 0) return GD_UNSUPPORTED;
   if ((lda % 8) || (ldw % 8) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return GD_UNSUPPORTED;
@@ -366,9 +376,9 @@ int kch_linear_decode_tc5(const void* A, const void* W, void* C, const void* R, 
     }
   }
   cudaStream_t s = kch_stream(stream);
-  if (l2) return launch_gd<128>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, s);
+  if (l2) return launch_gd<128>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, w_settled, s);
   static const int bn = [] { const char* v = getenv("KCH_GD_BN"); return v ? atoi(v) : 32; }();
-  if (bn == 128) return launch_gd<128>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, s);
-  if (bn == 64) return launch_gd<64>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, s);
-  return launch_gd<32>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, s);
+  if (bn == 128) return launch_gd<128>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, w_settled, s);
+  if (bn == 64) return launch_gd<64>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, w_settled, s);
+  return launch_gd<32>(A, W, C, R, (int)M, N, K, lda, ldw, ldc, ldr, ep, w_settled, s);
 }

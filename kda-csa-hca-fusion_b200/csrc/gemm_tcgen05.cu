@@ -748,10 +748,10 @@ bool kch_linear_tcgen05_epilogue_ok(const kch_epilogue* e, int N) {
 }
 
 int kch_linear_decode_tc5(const void* A, const void* W, void* C, const void* R, int64_t M, int N, int K, int64_t lda,
-                          int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream);
+                          int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, int w_settled, void* stream);
 
 int kch_linear_tcgen05(const void* A, const void* W, void* C, const void* R, int64_t M, int N, int K, int64_t lda,
-                       int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream, int slab_k) {
+                       int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream, int slab_k, int w_settled) {
   cudaStream_t s = kch_stream(stream);
   TgEpilogue ep = {};
   if (e && e->n_segments) {
@@ -760,7 +760,7 @@ int kch_linear_tcgen05(const void* A, const void* W, void* C, const void* R, int
   }
   if (M <= 64 && slab_k == 0) {
     // a decode batch: the kernel built for it (one copy per operand, K split over a cluster); -100 = not its shape
-    const int rc = kch_linear_decode_tc5(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, e, stream);
+    const int rc = kch_linear_decode_tc5(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, e, w_settled, stream);
     if (rc != -100) return rc;
   }
   if (M <= TG_BM && N > 128) {

@@ -37,10 +37,11 @@ struct IxdSmem {
 };
 
 __global__ void __launch_bounds__(IXD_THREADS, 3)
-decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* __restrict__ q, int q_dtype, int64_t q_ld,
-                          const float* __restrict__ norms, const void* __restrict__ w, int w_dtype, int64_t w_ld,
-                          float* __restrict__ logits, int64_t cap, int64_t n_ld, int HI, int normalize, float scale, int m,
-                          const int32_t* __restrict__ ctr, unsigned int* status) {
+decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* q, int q_dtype, int64_t q_ld, const float* norms,
+                          const void* w, int w_dtype, int64_t w_ld, float* logits, int64_t cap, int64_t n_ld, int HI,
+                          int normalize, float scale, int m, const int32_t* ctr, unsigned int* status) {
+  chain_wait();
+  chain_trigger();
   extern __shared__ uint8_t ixd_raw[];
   IxdSmem& sm = *reinterpret_cast<IxdSmem*>(((uintptr_t)ixd_raw + 1023) & ~(uintptr_t)1023);
   const int b = blockIdx.y, tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
@@ -188,8 +189,8 @@ int kch_decode_indexer_logits_tc5(const void* q, int q_dtype, int64_t q_ld, cons
   const size_t smem = sizeof(IxdSmem) + 1024;
   KCH_CUDA_OK(cudaFuncSetAttribute(decode_indexer_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)((cap + IXD_ROWS - 1) / IXD_ROWS), (unsigned)B);
-  decode_indexer_tc5_kernel<<<grid, IXD_THREADS, smem, s>>>(kmap, q, q_dtype, q_ld, norms, w, w_dtype, w_ld, logits, cap, n_ld, HI,
-                                                           normalize, scale, m, ctr, status);
+  KCH_CUDA_OK(kch_launch_chained(decode_indexer_tc5_kernel, grid, dim3(IXD_THREADS), smem, s, 1, kmap, q, q_dtype, q_ld, norms, w,
+                                 w_dtype, w_ld, logits, cap, n_ld, HI, normalize, scale, m, ctr, status));
   KCH_LAUNCH_OK();
   return KCH_OK;
 }

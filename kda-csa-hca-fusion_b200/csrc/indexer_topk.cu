@@ -754,8 +754,9 @@ __device__ __forceinline__ int sc_ld_remote(const int* local, uint32_t rank) {
 
 template <int EPT>
 __global__ void __launch_bounds__(256)
-topk_select_cluster_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, int64_t n_ld, int topk,
-                           const int32_t* __restrict__ ctr, int ctr_m) {
+topk_select_cluster_kernel(const float* logits, int32_t* out, int64_t n_ld, int topk, const int32_t* ctr, int ctr_m) {
+  chain_wait();
+  chain_trigger();
   const int n = ctr[KCH_CTR_N_BLOCKS];
   const int nv = min(ctr[KCH_CTR_TOKENS] / ctr_m, n);
   const int b = blockIdx.y, tid = threadIdx.x;
@@ -833,15 +834,10 @@ topk_select_cluster_kernel(const float* __restrict__ logits, int32_t* __restrict
 
 static int launch_topk_select_cluster(const float* logits, int32_t* indices, int B, int64_t n_ld, int topk,
                                       const int32_t* counters, int ctr_m, int ept, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = SC_CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(SC_CTAS, (unsigned)B); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.stream = s;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  if (ept <= 8) KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel<8>, logits, indices, n_ld, topk, counters, ctr_m));
-  else if (ept <= 16) KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel<16>, logits, indices, n_ld, topk, counters, ctr_m));
-  else KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel<32>, logits, indices, n_ld, topk, counters, ctr_m));
+  const dim3 grid(SC_CTAS, (unsigned)B);
+  if (ept <= 8) KCH_CUDA_OK(kch_launch_chained(topk_select_cluster_kernel<8>, grid, dim3(256), 0, s, SC_CTAS, logits, indices, n_ld, topk, counters, ctr_m));
+  else if (ept <= 16) KCH_CUDA_OK(kch_launch_chained(topk_select_cluster_kernel<16>, grid, dim3(256), 0, s, SC_CTAS, logits, indices, n_ld, topk, counters, ctr_m));
+  else KCH_CUDA_OK(kch_launch_chained(topk_select_cluster_kernel<32>, grid, dim3(256), 0, s, SC_CTAS, logits, indices, n_ld, topk, counters, ctr_m));
   kch_note_launch(1);
   return KCH_OK;
 }

@@ -73,6 +73,28 @@ __device__ __forceinline__ float ld_any(const void* p, int64_t i, int dtype) {
   return dtype == KCH_BF16 ? __bfloat162float(((const bf16*)p)[i]) : ((const float*)p)[i];
 }
 
+// ---- chained launches (the kernels of a decode step) ------------------------------------------------------------------
+// A step is ~30 short kernels in a row, each a few microseconds long: launch latency and set-up between two of them cost
+// as much as some of them.  kch_launch_chained lets a kernel start while the one before it drains.  Such a kernel calls
+// chain_wait() in every thread before it touches anything an earlier launch may still write or read: the call returns
+// when all earlier launches have completed and their stores are visible.  chain_trigger() (after the wait, so that a
+// kernel's start implies that everything before its predecessor is complete) lets the next one start.  Both are no-ops in
+// a kernel launched the ordinary way.  Inputs are not `const __restrict__` there: such loads could be moved above the wait.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... K, typename... A>
+static inline cudaError_t kch_launch_chained(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster_x, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster_x; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.attrs = attr; cfg.numAttrs = cluster_x > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 #define KCH_DISPATCH_FLOAT(dtype, T, ...)                       \

@@ -96,9 +96,7 @@ kda_recurrent_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 #define KDS_SMEM (KDS_STATE_BYTES + 128 * 16 + 16)
 template <typename T>
 __global__ void __launch_bounds__(128)
-kda_decode_step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                       const T* __restrict__ g, const T* __restrict__ beta, const float* S0, T* __restrict__ o,
-                       float* S_out, int H, int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v,
+kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int H, int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v,
                        int64_t ld_g, int64_t ld_b, unsigned int* status) {
   constexpr int K = 128, V = 128;
   extern __shared__ __align__(128) uint8_t kds_raw[];
@@ -111,6 +109,10 @@ kda_decode_step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T
   if (tid == 0) {
     mbarrier_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  chain_wait();
+  chain_trigger();
+  if (tid == 0) {
     if (S0) {
       mbarrier_expect_tx(bar, KDS_STATE_BYTES);
       bulk_copy_g2s(st, S0 + sbase, KDS_STATE_BYTES, bar);
@@ -192,9 +194,9 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
     KCH_REQUIRE(status != nullptr, "kch_kda_recurrent: cannot resolve the device status word");
     KCH_DISPATCH_FLOAT(dtype, T_, {
       KCH_CUDA_OK(cudaFuncSetAttribute(kda_decode_step_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, KDS_SMEM));
-      kda_decode_step_kernel<T_><<<dim3(HV, B), 128, KDS_SMEM, s>>>(
+      KCH_CUDA_OK(kch_launch_chained(kda_decode_step_kernel<T_>, dim3(HV, B), dim3(128), KDS_SMEM, s, 1,
         (const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta, initial_state, (T_*)o, final_state, H, HV,
-        scale, g_clamp_min, ld_qk, ld_v, ld_g, ld_beta, status);
+        scale, g_clamp_min, ld_qk, ld_v, ld_g, ld_beta, status));
     });
     KCH_LAUNCH_OK();
     return KCH_OK;

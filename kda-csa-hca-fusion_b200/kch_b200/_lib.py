@@ -75,6 +75,7 @@ PROTOTYPES = {
     "kch_short_conv": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "kch_linear": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i64, _i64, _i, _vp]),
     "kch_linear_ex": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i64, _i64, _i, C.POINTER(Epilogue), _vp]),
+    "kch_linear_settled": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i64, _i64, _i, C.POINTER(Epilogue), _vp]),
     "kch_linear_kslabs": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i64, _i64, _i64, _i, _vp]),
     "kch_peer_gather_flag_words": (_i64, [_i]),
     "kch_peer_allgather": (_i, [_vp, _i64, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), _i, _i, _vp]),

@@ -57,10 +57,11 @@ def _epilogue(segments, group):
     return ep, end
 
 
-def linear(x, W, residual=None, epilogue=None, group=1):
+def linear(x, W, residual=None, epilogue=None, group=1, w_settled=False):
     """``F.linear(x, W)`` (+ residual) through the C ABI.  x ``[..., K]`` (last dim dense), W ``[N, K]``.
     ``epilogue``: list of ``(width, act, param)`` column segments covering all N output columns, applied with
-    the rounding points of the unfused chain (``group`` = head width of the silu+L2-norm activation)."""
+    the rounding points of the unfused chain (``group`` = head width of the silu+L2-norm activation).
+    ``w_settled``: the caller knows that the kernel launched just before does not write ``W``."""
     _lib.require_cuda(x, W, fn="linear")
     lib = _lib.load()
     K = x.shape[-1]
@@ -71,7 +72,7 @@ def linear(x, W, residual=None, epilogue=None, group=1):
         raise ValueError(f"linear: weight dtype {W.dtype} does not match input dtype {x.dtype}")
     x2, M, lda = _rows_2d(x, K)
     if W.stride(-1) != 1:
-        W = W.contiguous()
+        W, w_settled = W.contiguous(), False
     out = torch.empty((*x.shape[:-1], N), dtype=x.dtype, device=x.device)
     r2, ldr = None, 0
     if residual is not None:
@@ -87,8 +88,9 @@ def linear(x, W, residual=None, epilogue=None, group=1):
         if end != N:
             raise ValueError(f"linear: epilogue segments cover {end} columns, the weight has {N} rows")
     with _lib.device(x.device):
-        _lib.check(lib.kch_linear_ex(_lib.ptr(x2), _lib.ptr(W), _lib.ptr(out), _lib.ptr(r2), M, N, K, lda,
-                                     W.stride(0), N, ldr, _lib.dtype_tag(x.dtype), ep, _lib.stream()))
+        _lib.check((lib.kch_linear_settled if w_settled else lib.kch_linear_ex)(
+            _lib.ptr(x2), _lib.ptr(W), _lib.ptr(out), _lib.ptr(r2), M, N, K, lda, W.stride(0), N, ldr,
+            _lib.dtype_tag(x.dtype), ep, _lib.stream()))
     return out
 
 

@@ -214,10 +214,12 @@ class _FusedWeights:
     def __init__(self):
         self._key = None
         self._w = None
+        self.settled = False            # the last `get` launched nothing: the copy was there already
 
     def get(self, *weights):
         key = tuple((w.data_ptr(), w.dtype, w.device, w._version) for w in weights)
-        if key != self._key:
+        self.settled = key == self._key
+        if not self.settled:
             self._w = fuse_rows(*weights)
             self._key = key
         return self._w
@@ -302,12 +304,14 @@ class KDAHybridLayer(nn.Module):
         n_used = 2 * H * K + HV * V + K + HV
         segs = [(H * K, _lib.ACT_SILU_L2NORM, 0.0), (H * K, _lib.ACT_SILU_L2NORM, 0.0), (HV * V, _lib.ACT_SILU, 0.0),
                 (K, 0, 0.0), (HV + (W.shape[0] - n_used), _lib.ACT_SIGMOID, 0.0)]
-        proj = linear(xc, W, epilogue=segs, group=K)
+        # in a one-token step the kernel before each projection is one of ours, which produced its input
+        proj = linear(xc, W, epilogue=segs, group=K, w_settled=fused_step and self._fused.settled)
         q, k, v, gd, beta = proj[..., :n_used].split([H * K, H * K, HV * V, K, HV], dim=-1)
         if raw_gate:     # the chunk kernel applies -softplus(.) * decay_scale when it loads the gate
             g = linear(gd, self.g_up.weight)
         else:
-            g = linear(gd, self.g_up.weight, epilogue=[(HV * K, _lib.ACT_NEG_SOFTPLUS, cfg.kda_decay_scale)])
+            g = linear(gd, self.g_up.weight, epilogue=[(HV * K, _lib.ACT_NEG_SOFTPLUS, cfg.kda_decay_scale)],
+                       w_settled=fused_step)
         return (q.unflatten(-1, (H, K)), k.unflatten(-1, (H, K)), v.unflatten(-1, (HV, V)),
                 g.view(B, T, HV, K), beta, new_lb)
 
@@ -324,7 +328,8 @@ class KDAHybridLayer(nn.Module):
                                    output_final_state=True, chunk_size=cfg.kda_chunk_size, use_chunk=use_chunk,
                                    backend=cfg.kda_backend, state_out=None if use_chunk else state_out,
                                    gate_scale=cfg.kda_decay_scale if raw_gate else None)
-        out = out_projection(o.reshape(B, T, HV * V), self.tp, self.o_proj.weight, residual=residual)
+        out = out_projection(o.reshape(B, T, HV * V), self.tp, self.o_proj.weight, residual=residual,
+                             w_settled=T == 1 and lookback_in_place)
         return out, new_state, new_lb
 
 
@@ -681,7 +686,7 @@ class HybridDecoding(nn.Module):
     def _project_out(self, layer, o_core, residual, B, T):
         if _rows_mode(layer.tp):
             return out_projection_rows(o_core, layer.tp, layer.o_proj.weight, residual, lead=(B, T))
-        return out_projection(o_core, layer.tp, layer.o_proj.weight, residual=residual)
+        return out_projection(o_core, layer.tp, layer.o_proj.weight, residual=residual, w_settled=T == 1)
 
     def _csa(self, i, layer, h, residual):
         cfg = self.cfg
@@ -696,10 +701,12 @@ class HybridDecoding(nn.Module):
             cache.append_step(*proj, layer.Ba, layer.Bb, layer.B_idx)
         else:
             c, cI, dc, nIh, nh = cfg.csa_c, cfg.csa_cI, cfg.csa_dc, cfg.csa_nIh, cfg.csa_nh
-            proj = linear(h, layer.fused_weight())
+            W = layer.fused_weight()
+            proj = linear(h, W, w_settled=layer._fused.settled)
             Ca, Cb, Za, Zb, K_idx, Z_idx, cQ, w_idx = proj[..., :4 * c + 2 * cI + dc + nIh].split(
                 [c, c, c, c, cI, cI, dc, nIh], dim=-1)
-            qq = linear(cQ, layer.q_weight())
+            W = layer.q_weight()
+            qq = linear(cQ, W, w_settled=layer._fused_q.settled)
             q, q_idx = qq[..., :nh * c + nIh * cI].split([nh * c, nIh * cI], dim=-1)
             cache.append_step(Ca, Cb, Za, Zb, K_idx, Z_idx, layer.Ba, layer.Bb, layer.B_idx)
             if cache._decode_attend_ok(nh):
@@ -730,9 +737,10 @@ class HybridDecoding(nn.Module):
             cache.append_step(C, Z, layer.B_pos)
         else:
             c, dc, nh = cfg.hca_c, cfg.hca_dc, cfg.hca_nh
-            proj = linear(h, layer.fused_weight())
+            W = layer.fused_weight()
+            proj = linear(h, W, w_settled=layer._fused.settled)
             C, Z, cQ = proj[..., :2 * c + dc].split([c, c, dc], dim=-1)
-            q = linear(cQ, layer.W_UQ.weight)
+            q = linear(cQ, layer.W_UQ.weight, w_settled=True)
             cache.append_step(C, Z, layer.B_pos)
             if cache._decode_attend_ok(nh):
                 o = cache.forward_step(q.view(B, 1, nh, c), nh=nh, scale=1.0, sink_logits=layer.sink, _q_normalize=True,

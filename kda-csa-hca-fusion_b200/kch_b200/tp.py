@@ -172,14 +172,14 @@ def out_projection_rows(o_rows, ctx: TPContext, W, residual=None, lead=None):
     return out
 
 
-def out_projection(o_local, ctx: TPContext, W, residual=None):
+def out_projection(o_local, ctx: TPContext, W, residual=None, w_settled=False):
     """``o_proj`` of a layer whose heads are sharded: all-gather of the per-rank head outputs ``[..., h_local*c]``,
     then ``F.linear(cat over ranks, W)`` (+ residual) on every rank.  The gather lands rank-major
     (``[world, rows, h_local*c]``); the GEMM walks those slabs along its K loop (``kch_linear_kslabs``), so the
     gathered tensor is never permuted into ``[rows, h*c]``."""
     from .csa import linear, linear_kslabs
     if ctx is None or ctx.world == 1:
-        return linear(o_local, W, residual=residual)
+        return linear(o_local, W, residual=residual, w_settled=w_settled)
     lead = o_local.shape[:-1]
     kl = o_local.shape[-1]
     slab_ok = (o_local.dtype == torch.bfloat16 and W.dtype == torch.bfloat16 and kl % 64 == 0 and W.shape[0] >= 32
