@@ -3,20 +3,23 @@
 //   vt^T = u^T - S^T w^T ;  o^T = S^T qg^T + vt^T Aqk^T ;  S^T <- S^T diag(dl) + vt^T kg
 // with every product as hi*hi + lo*hi + hi*lo of two-term bf16 splits and fp32 accumulation.
 //
-// One CTA per (batch, value head); S^T [128 v x 128 k] fp32 is the accumulator of the update product
-// and never leaves tensor memory between chunks.  Per chunk (the dependent chain is S -> D1w -> vt -> S):
-//   vector warps : read S^T (tcgen05.ld, one row v per thread), write its bf16 hi / lo images into shared
-//                  memory in the MMA operand layout, one 64-channel panel at a time, and write
-//                  S^T diag(dl) back (tcgen05.st)
-//   MMA thread   : [D1w | D1q] = S^T [w; qg]^T   (M = 128 v, N = 64 + 64 tokens, K = 128 channels), starting on a
-//                  panel as soon as the vector warps have finished it
-//   vector warps : vt^T = u^T - D1w -> bf16 hi / lo operand tiles, 16 tokens at a time
+// One CTA per (batch, value head); S^T [128 v x 128 k] fp32 is the accumulator of the update product and never leaves
+// tensor memory between chunks; the bf16 hi / lo images of S^T and of vt^T are A operands there as well (an A operand in
+// tensor memory needs no proxy fence, which cost 300 cycles at each of a chunk's four conversions, and frees the shared
+// memory that lets the operands of a whole chunk be fetched ahead).  Per chunk (the dependent chain is S -> D1w -> vt -> S):
+//   vector warps : read S^T (tcgen05.ld, one row v per thread), write its hi / lo images, one 64-channel panel at a time,
+//                  and S^T diag(dl) back
+//   MMA thread   : [D1w | D1q] = S^T [w; qg]^T (N = 64 + 64 tokens, K = 128 channels), starting on a panel as soon as it
+//                  is there (D1q apart, behind D1w, slowed the vector warps' own tensor-memory accesses by as much)
+//   vector warps : vt^T = u^T - D1w -> hi / lo images, 16 tokens at a time
 //   MMA thread   : S^T += vt^T kg (N = 128, kg read as an MN-major operand, i.e. in its natural [token][channel]
 //                  layout), then D1q += vt^T Aqk^T (N = 64); K = 64 tokens
-//   vector warps : o^T = D1q -> bf16 -> global one chunk later, while the next [D1w | D1q] is being computed
-//                  (the [D1w | D1q] block is double-buffered in tensor memory)
-// A producer warp streams the chunk's operand tiles (written by the prepare kernel in this layout) with 1-D
-// bulk copies.  Every wait is a bounded mbarrier wait that records a status code and leaves the loops.
+//   vector warps : o^T = D1q of the chunk before -> bf16 -> global, while the products of this one run (the [D1w | D1q]
+//                  block is double-buffered)
+// A producer warp streams the chunk's operand tiles (written by the prepare kernel in this layout) with 1-D bulk copies,
+// a whole chunk ahead.  Every wait is a bounded mbarrier wait that records a status code and leaves the loops.
+// Bound: the dependent chain, 4200 cycles a chunk: 1540 of D1 and ~900 of the update on the tensor pipe, the rest the two
+// conversions and four hand-overs of ~250 cycles.  It was 5300 with the images in shared memory and o stored two bytes at a time ahead of vt (1 x 8192 tokens, 16 heads, both stages: 526 -> 433 us).
 //
 // Workspace record of a chunk in this layout (written by kda_prepare_mma_kernel when PrepArgs::umma is set):
 //   0      [w; qg] hi: two 64-channel panels of [128 rows][64] bf16 (rows 0..63 w, 64..127 qg), 128-byte swizzle
@@ -52,34 +55,59 @@ struct T5Args {
   unsigned int* status;
   int T, HV, NT;                     // T: tokens from the first chunk of this launch to the end of the sequence
   int Tb;                            // tokens between consecutive batch entries (the whole sequence length)
+  int o_vec;                         // o is 8-byte aligned
 };
 
 // shared-memory map (bytes, 1024-aligned operand tiles)
-#define T5_SA 0                      // S^T hi: 2 panels [128][64] bf16 (32768), then lo (32768)
-#define T5_VA (T5_SA + 65536)        // vt^T hi [128][64] bf16 (16384), lo (16384)
-#define T5_TW (T5_VA + 32768)        // w hi, w lo, q hi, q lo: 4 x 16384
-#define T5_TK (T5_TW + 65536)        // kg^T hi [128][64] (16384), lo (16384)
+#define T5_TW 0                      // two stages of [w; qg] hi panels, lo panels: 4 x 16384 each
+#define T5_TK 131072                 // kg hi [64][128] (16384), lo (16384)
 #define T5_TA (T5_TK + 32768)        // Aqk hi [64][64] (8192), lo (8192)
-#define T5_DL (T5_TA + 16384)        // dl [128] fp32
-#define T5_BARS (T5_DL + 512)
+#define T5_TU (T5_TA + 16384)        // u^T and dl as in the record (straight from global memory they came 500 cycles too late)
+#define T5_BARS (T5_TU + 32768 + 512)
 #define T5_TOTAL (T5_BARS + 128)
+// tensor-memory columns
+#define T5_CS 0                      // S^T fp32
+#define T5_CSA 128                   // S^T images: hi 64 columns (two channels each), lo 64
+#define T5_CD 256                    // [D1w | D1q] of even chunks, of odd chunks; once a vector warp has read its 32 columns
+                                     // of D1w, the images of the same tokens of vt^T lie there: hi 16, lo 16 columns
+static_assert(T5_TOTAL + 1024 <= 232448, "shared memory of the KDA scan");
+
+__device__ __forceinline__ void t5_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void t5_stn(uint32_t taddr, const uint32_t* r) {
+  if constexpr (N == 16)
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 
 __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   extern __shared__ uint8_t t5_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>(((uintptr_t)t5_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + T5_BARS);
-  uint64_t *w_full = bars + 0, *w_empty = bars + 1, *k_full = bars + 2, *k_empty = bars + 3, *sa_ready0 = bars + 4,
-           *d1_full = bars + 5, *va_ready0 = bars + 6, *s_full = bars + 7, *o_full = bars + 8, *sa_ready1 = bars + 9,
-           *va_ready1 = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t *sa_ready0 = bars + 0, *sa_ready1 = bars + 1, *va_ready0 = bars + 2, *va_ready1 = bars + 3, *d1_full = bars + 4,
+           *s_full = bars + 5, *o_full = bars + 6;
+  uint64_t *w_full = bars + 7, *w_empty = bars + 9, *k_full = bars + 11, *k_empty = bars + 12, *u_full = bars + 13, *u_empty = bars + 14;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   const int hv = blockIdx.x, b = blockIdx.y;
   const int warp = t5_warp_index(), lane = threadIdx.x & 31;
   const int64_t bh = (int64_t)b * a.HV + hv;
   const uint8_t* wsb = a.ws + bh * a.NT * (int64_t)T5_CHUNK_BYTES;
-  constexpr uint32_t TMEM_COLS = 512;          // S^T 128 | [D1w 64 | D1q 64] of even chunks | the same of odd chunks
+  constexpr uint32_t TMEM_COLS = 512;
 
   if (threadIdx.x == 0) {
-    mbarrier_init(w_full, 1); mbarrier_init(w_empty, 1); mbarrier_init(k_full, 1); mbarrier_init(k_empty, 1);
+    for (int i = 0; i < 2; ++i) { mbarrier_init(w_full + i, 1); mbarrier_init(w_empty + i, 1); }
+    mbarrier_init(k_full, 1); mbarrier_init(k_empty, 1); mbarrier_init(u_full, 1); mbarrier_init(u_empty, 8);
     mbarrier_init(sa_ready0, 8); mbarrier_init(sa_ready1, 8); mbarrier_init(d1_full, 1); mbarrier_init(va_ready0, 8); mbarrier_init(va_ready1, 8); mbarrier_init(s_full, 1); mbarrier_init(o_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -91,52 +119,55 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   __syncthreads();
   t5_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tD0 = tmem + 128;
+  const uint32_t tS = tmem + T5_CS, tSA = tmem + T5_CSA, tDD = tmem + T5_CD;
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     if (t5_elect()) {
       for (int n = 0; n < a.NT; ++n) {
         const uint8_t* src = wsb + (int64_t)n * T5_CHUNK_BYTES;
+        const int st = n & 1;
         const uint32_t ph = (uint32_t)n & 1;
-        if (!mbarrier_wait_bounded(w_empty, ph ^ 1, 41, T5_SPIN, a.status)) break;
-        mbarrier_expect_tx(w_full, 4 * 16384 + 512);
-        bulk_copy_g2s(sm + T5_TW, src + T5_OFF_WHI, 4 * 16384, w_full);            // [w; qg] hi panels, then lo panels
-        bulk_copy_g2s(sm + T5_DL, src + T5_OFF_U + 32768, 512, w_full);            // dl sits behind u^T
+        if (!mbarrier_wait_bounded(w_empty + st, ((uint32_t)(n >> 1) & 1) ^ 1, 41, T5_SPIN, a.status)) break;
+        mbarrier_expect_tx(w_full + st, 4 * 16384);
+        bulk_copy_g2s(sm + T5_TW + st * 65536, src + T5_OFF_WHI, 4 * 16384, w_full + st);     // [w; qg] hi panels, then lo panels
+        if (!mbarrier_wait_bounded(u_empty, ph ^ 1, 54, T5_SPIN, a.status)) break;
+        mbarrier_expect_tx(u_full, 32768 + 512);
+        bulk_copy_g2s(sm + T5_TU, src + T5_OFF_U, 32768 + 512, u_full);                       // u^T, dl
         if (!mbarrier_wait_bounded(k_empty, ph ^ 1, 42, T5_SPIN, a.status)) break;
         mbarrier_expect_tx(k_full, 2 * 16384 + 16384);
-        bulk_copy_g2s(sm + T5_TK, src + T5_OFF_KHI, 2 * 16384, k_full);            // kg hi, lo
-        bulk_copy_g2s(sm + T5_TA, src + T5_OFF_AQK, 16384, k_full);                // Aqk hi, lo
+        bulk_copy_g2s(sm + T5_TK, src + T5_OFF_KHI, 2 * 16384, k_full);                       // kg hi, lo
+        bulk_copy_g2s(sm + T5_TA, src + T5_OFF_AQK, 16384, k_full);                           // Aqk hi, lo
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     if (t5_elect()) {
       const uint32_t id64 = t5_idesc(64), id128 = t5_idesc(128), id128mn = t5_idesc(128) | (1u << 16);
-      const uint32_t sa = smem_addr_u32(sm + T5_SA), va = smem_addr_u32(sm + T5_VA), tw = smem_addr_u32(sm + T5_TW),
-                     tk = smem_addr_u32(sm + T5_TK), ta = smem_addr_u32(sm + T5_TA);
+      const uint64_t dw0 = t5_desc(smem_addr_u32(sm + T5_TW)), da0 = t5_desc(smem_addr_u32(sm + T5_TA));
+      const uint64_t dk0 = t5_desc_mn(smem_addr_u32(sm + T5_TK));
       for (int n = 0; n < a.NT; ++n) {
-        const uint32_t ph = (uint32_t)n & 1;
-        const uint32_t tD = tD0 + 128u * ph;                 // [D1w | D1q] of this chunk
-        if (!mbarrier_wait_bounded(w_full, ph, 44, T5_SPIN, a.status)) break;
-        // [D1w | D1q] = S^T [w; qg]^T: terms (S hi, x hi), (S lo, x hi), (S hi, x lo); one 64-channel panel of
-        // S^T at a time, as the vector warps finish it
+        const uint32_t ph = (uint32_t)n & 1, sph = (uint32_t)(n >> 1) & 1;
+        const int st = n & 1;
+        const uint64_t dw = dw0 + (uint64_t)(st * 65536 >> 4);
+        const uint32_t tD = tDD + 128u * ph;                 // [D1w | D1q] of this chunk; vt^T images over D1w
+        if (!mbarrier_wait_bounded(w_full + st, sph, 44, T5_SPIN, a.status)) break;
+        // [D1w | D1q] = S^T [w; qg]^T, a 64-channel panel at a time: terms (S hi, x hi), (S lo, x hi), (S hi, x lo)
         bool ok = true;
 #pragma unroll
         for (int pan = 0; pan < 2; ++pan) {
           if (!mbarrier_wait_bounded(pan ? sa_ready1 : sa_ready0, ph, 43, T5_SPIN, a.status)) { ok = false; break; }
           t5_fence_after();
 #pragma unroll
-          for (int term = 0; term < 3; ++term) {
-            const uint32_t abase = sa + (term == 1 ? 32768u : 0u) + (uint32_t)pan * 16384u;
-            const uint32_t bbase = tw + (term == 2 ? 32768u : 0u) + (uint32_t)pan * 16384u;
+          for (int term = 0; term < 3; ++term)
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) t5_mma(tD, t5_desc(abase) + 2 * ks, t5_desc(bbase) + 2 * ks, id128, (pan | term | ks) ? 1u : 0u);
-          }
+            for (int ks = 0; ks < 4; ++ks)
+              t5_mma_ts(tD, tSA + (term == 1 ? 64u : 0u) + 32u * pan + 8u * ks, dw + ((term == 2 ? 32768u : 0u) + pan * 16384u >> 4) + 2 * ks,
+                        id128, (pan | term | ks) ? 1u : 0u);
         }
         if (!ok) break;
         t5_commit(d1_full);
-        t5_commit(w_empty);
+        t5_commit(w_empty + st);
         if (!mbarrier_wait_bounded(k_full, ph, 46, T5_SPIN, a.status)) break;
         // S^T += vt^T kg   (N = 128 channels, kg read in place as an MN-major operand; K = 64 tokens, the 16-token
         // steps {0, 2} first, {1, 3} second, as the vector warps finish them)
@@ -145,26 +176,21 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
           if (!mbarrier_wait_bounded(part ? va_ready1 : va_ready0, ph, 45, T5_SPIN, a.status)) { ok = false; break; }
           t5_fence_after();
 #pragma unroll
-          for (int term = 0; term < 3; ++term) {
-            const uint32_t abase = va + (term == 1 ? 16384u : 0u);
-            const uint32_t bbase = tk + (term == 2 ? 16384u : 0u);
+          for (int term = 0; term < 3; ++term)
 #pragma unroll
             for (int k2 = 0; k2 < 2; ++k2) {
               const int ks = 2 * k2 + part;
-              t5_mma(tS, t5_desc(abase) + 2 * ks, t5_desc_mn(bbase + (uint32_t)ks * 2048u), id128mn, 1u);
+              t5_mma_ts(tS, tD + (term == 1 ? 16u : 0u) + 32u * (ks >> 1) + 8u * (ks & 1), dk0 + ((term == 2 ? 16384u : 0u) + ks * 2048u >> 4), id128mn, 1u);
             }
-          }
         }
         if (!ok) break;
         t5_commit(s_full);
         // D1q += vt^T Aqk^T
 #pragma unroll
-        for (int term = 0; term < 3; ++term) {
-          const uint32_t abase = va + (term == 1 ? 16384u : 0u);
-          const uint32_t bbase = ta + (term == 2 ? 8192u : 0u);
+        for (int term = 0; term < 3; ++term)
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) t5_mma(tD + 64, t5_desc(abase) + 2 * ks, t5_desc(bbase) + 2 * ks, id64, 1u);
-        }
+          for (int ks = 0; ks < 4; ++ks)
+            t5_mma_ts(tD + 64, tD + (term == 1 ? 16u : 0u) + 32u * (ks >> 1) + 8u * (ks & 1), da0 + ((term == 2 ? 8192u : 0u) >> 4) + 2 * ks, id64, 1u);
         t5_commit(o_full);
         t5_commit(k_empty);
       }
@@ -186,38 +212,59 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       t5_st32(tS + lane_base + 64 * pan + 32 * sub, r);
     }
     t5_wait_st();
+    // o^T rows (this thread: value column v, 32 tokens in `ro`) -> o[token][v].  A 4 x 4 transpose inside each group of four
+    // lanes turns 32 stores of 2 bytes per thread into 8 of 8 bytes (64 contiguous bytes per warp and token either way):
+    // with the former the phase took 1860 cycles of a chunk's 5250.
+    auto store_o = [&](int tok0) {
+      uint32_t p[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t own = pack2_bf16(__uint_as_float(ro[2 * i]), __uint_as_float(ro[2 * i + 1]));     // tokens 2i, 2i + 1
+        const uint32_t oth = __shfl_xor_sync(0xffffffffu, own, 1);
+        p[i] = (lane & 1) ? __byte_perm(oth, own, 0x7632) : __byte_perm(own, oth, 0x5410);               // columns v & ~1, + 1 of token 2i + (lane & 1)
+      }
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, (lane & 2) ? p[2 * m] : p[2 * m + 1], 2);
+        const uint2 o4 = (lane & 2) ? make_uint2(got, p[2 * m + 1]) : make_uint2(p[2 * m], got);
+        const int t = tok0 + 32 * sub + 4 * m + (lane & 3);
+        bf16* dst = a.o + (((int64_t)b * a.Tb + t) * a.HV + hv) * 128 + (v & ~3);
+        if (t < a.T && a.o_vec) *reinterpret_cast<uint2*>(dst) = o4;
+        else if (t < a.T) {
+          const uint32_t w2[2] = {o4.x, o4.y};
+          for (int c = 0; c < 4; ++c) reinterpret_cast<uint16_t*>(dst)[c] = (uint16_t)(w2[c >> 1] >> (16 * (c & 1)));
+        }
+      }
+    };
     bool ok = true;
-    const float* dl = reinterpret_cast<const float*>(sm + T5_DL);
+    const float* dl = reinterpret_cast<const float*>(sm + T5_TU + 32768);
+    const float4* up = reinterpret_cast<const float4*>(sm + T5_TU) + sub * 8 * 128 + v;       // [sub][j][v] float4
     for (int n = 0; n < a.NT && ok; ++n) {
       const uint32_t ph = (uint32_t)n & 1;
-      const uint8_t* src = wsb + (int64_t)n * T5_CHUNK_BYTES;
       if (n > 0 && !mbarrier_wait_bounded(s_full, ph ^ 1, 47, T5_SPIN, a.status)) { ok = false; break; }
-      if (!mbarrier_wait_bounded(w_full, ph, 48, T5_SPIN, a.status)) { ok = false; break; }      // dl has landed
       t5_fence_after();
-      // ---- S^T -> bf16 hi / lo operand images, panel 0 then panel 1; S^T diag(dl) back to tensor memory -----------
+      // ---- S^T -> bf16 hi / lo images, panel 0 then panel 1; then S^T diag(dl) back to tensor memory -------------------
       t5_ld32(tS + lane_base + 32 * sub, r);
       t5_ld32(tS + lane_base + 64 + 32 * sub, r2);
       t5_wait_ld();
 #pragma unroll
       for (int pan = 0; pan < 2; ++pan) {
         uint32_t (&rr)[32] = pan ? r2 : r;
-        const int kc0 = 64 * pan + 32 * sub;                   // first channel of these 32 columns
-        uint8_t* pan_hi = sm + T5_SA + (size_t)pan * 16384;
-        uint8_t* pan_lo = pan_hi + 32768;
+        uint32_t h[16], l[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {                          // four 16-byte chunks of 8 channels
-          uint32_t h[4], l[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            split2_bf16(__uint_as_float(rr[8 * q + 2 * e]), __uint_as_float(rr[8 * q + 2 * e + 1]), h[e], l[e]);
-          const uint32_t off = swz<128>(v, 4 * sub + q);
-          *reinterpret_cast<uint4*>(pan_hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<uint4*>(pan_lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
-        }
-        t5_fence_async_smem();
+        for (int e = 0; e < 16; ++e) split2_bf16(__uint_as_float(rr[2 * e]), __uint_as_float(rr[2 * e + 1]), h[e], l[e]);
+        t5_stn<16>(tSA + lane_base + 32 * pan + 16 * sub, h);
+        t5_stn<16>(tSA + lane_base + 64 + 32 * pan + 16 * sub, l);
+        t5_wait_st();
         t5_fence_before();
         __syncwarp();
         if (lane == 0) mbarrier_arrive(pan ? sa_ready1 : sa_ready0);
+      }
+      if (!mbarrier_wait_bounded(u_full, ph, 48, T5_SPIN, a.status)) { ok = false; break; }      // u^T and dl have landed
+#pragma unroll
+      for (int pan = 0; pan < 2; ++pan) {
+        uint32_t (&rr)[32] = pan ? r2 : r;
+        const int kc0 = 64 * pan + 32 * sub;                   // first channel of these 32 columns
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           const float4 d4 = *reinterpret_cast<const float4*>(dl + kc0 + j);
@@ -228,47 +275,37 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
         }
         t5_st32(tS + lane_base + kc0, rr);
       }
-      // u^T row v, tokens 32*sub .. +31 (fp32, straight from the workspace)
-      float u[32];
-      {
-        const float4* up = reinterpret_cast<const float4*>(src + T5_OFF_U) + sub * 8 * 128 + v;   // [sub][j][v] float4: coalesced
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { const float4 x = up[j * 128]; u[4 * j] = x.x; u[4 * j + 1] = x.y; u[4 * j + 2] = x.z; u[4 * j + 3] = x.w; }
-      }
-      // ---- o^T of the previous chunk -> global: token t, value column v (64 contiguous bytes per warp and token) ----
-      if (n > 0) {
-        if (!mbarrier_wait_bounded(o_full, ph ^ 1, 52, T5_SPIN, a.status)) { ok = false; break; }
-        t5_fence_after();
-        t5_ld32(tD0 + 128u * (ph ^ 1) + 64 + lane_base + 32 * sub, ro);
-        t5_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int t = (n - 1) * 64 + 32 * sub + j;
-          a.o[(((int64_t)b * a.Tb + t) * a.HV + hv) * 128 + v] = __float2bfloat16_rn(__uint_as_float(ro[j]));
-        }
-      }
-      // ---- vt^T = u^T - D1w -> operand images, 16 tokens at a time ---------------------------------------------
+      // ---- vt^T = u^T - D1w -> images, 16 tokens at a time -------------------------------------------------------
       t5_wait_st();                                             // the decayed S^T is in place before the update may start
       if (!mbarrier_wait_bounded(d1_full, ph, 49, T5_SPIN, a.status)) { ok = false; break; }
       t5_fence_after();
-      t5_ld32(tD0 + 128u * ph + lane_base + 32 * sub, r);
+      t5_ld32(tDD + 128u * ph + lane_base + 32 * sub, r);
+      float u[32];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { const float4 x = up[j * 128]; u[4 * j] = x.x; u[4 * j + 1] = x.y; u[4 * j + 2] = x.z; u[4 * j + 3] = x.w; }
       t5_wait_ld();
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t h[4], l[4];
+      for (int q = 0; q < 2; ++q) {                             // 16 tokens: 8 columns of each image
+        uint32_t h[8], l[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          split2_bf16(u[8 * q + 2 * e] - __uint_as_float(r[8 * q + 2 * e]), u[8 * q + 2 * e + 1] - __uint_as_float(r[8 * q + 2 * e + 1]),
+        for (int e = 0; e < 8; ++e)
+          split2_bf16(u[16 * q + 2 * e] - __uint_as_float(r[16 * q + 2 * e]), u[16 * q + 2 * e + 1] - __uint_as_float(r[16 * q + 2 * e + 1]),
                       h[e], l[e]);
-        const uint32_t off = swz<128>(v, 4 * sub + q);
-        *reinterpret_cast<uint4*>(sm + T5_VA + off) = make_uint4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<uint4*>(sm + T5_VA + 16384 + off) = make_uint4(l[0], l[1], l[2], l[3]);
-        if (q & 1) {
-          t5_fence_async_smem();
-          t5_fence_before();
-          __syncwarp();
-          if (lane == 0) mbarrier_arrive(q == 1 ? va_ready0 : va_ready1);
-        }
+        t5_stn<8>(tDD + 128u * ph + lane_base + 32 * sub + 8 * q, h);
+        t5_stn<8>(tDD + 128u * ph + lane_base + 32 * sub + 16 + 8 * q, l);
+        t5_wait_st();
+        t5_fence_before();
+        __syncwarp();
+        if (lane == 0) mbarrier_arrive(q ? va_ready1 : va_ready0);
+      }
+      if (lane == 0) mbarrier_arrive(u_empty);
+      // ---- o^T of the previous chunk -> global, while the products of this one run (its D1q is the other buffer) --------
+      if (n > 0) {
+        if (!mbarrier_wait_bounded(o_full, ph ^ 1, 52, T5_SPIN, a.status)) { ok = false; break; }
+        t5_fence_after();
+        t5_ld32(tDD + 128u * (ph ^ 1) + 64 + lane_base + 32 * sub, ro);
+        t5_wait_ld();
+        store_o((n - 1) * 64);
       }
     }
     // the last products must have finished before o^T and the state are read and tensor memory is released
@@ -276,13 +313,9 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
     if (ok && a.NT > 0 && !mbarrier_wait_bounded(o_full, (uint32_t)(a.NT - 1) & 1, 53, T5_SPIN, a.status)) ok = false;
     if (ok && a.NT > 0) {
       t5_fence_after();
-      t5_ld32(tD0 + 128u * ((uint32_t)(a.NT - 1) & 1) + 64 + lane_base + 32 * sub, ro);
+      t5_ld32(tDD + 128u * ((uint32_t)(a.NT - 1) & 1) + 64 + lane_base + 32 * sub, ro);
       t5_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int t = (a.NT - 1) * 64 + 32 * sub + j;
-        if (t < a.T) a.o[(((int64_t)b * a.Tb + t) * a.HV + hv) * 128 + v] = __float2bfloat16_rn(__uint_as_float(ro[j]));
-      }
+      store_o((a.NT - 1) * 64);
       if (a.S_out) {
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
@@ -315,6 +348,7 @@ int kch_kda_scan_tc5(const void* workspace, const float* initial_state, void* o,
   T5Args a;
   a.ws = (const uint8_t*)workspace; a.S0 = initial_state; a.o = (bf16*)o; a.S_out = final_state; a.status = status;
   a.T = T; a.Tb = Tb; a.HV = HV; a.NT = NT;
+  a.o_vec = ((uintptr_t)o & 7) == 0;
   const int smem = T5_TOTAL + 1024;
   KCH_CUDA_OK(cudaFuncSetAttribute(kda_scan_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   kda_scan_tc5_kernel<<<dim3(HV, B), T5_THREADS, smem, s>>>(a);
