@@ -285,7 +285,20 @@ __device__ __forceinline__ void adm_split(float x0, float x1, uint32_t& hi, uint
   lo = adm_pack(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xFFFF0000u));
 }
 
-template <bool Q8>
+// CL: the CTAs of a sequence are one cluster and finish the softmax themselves -- partial sums cross distributed shared
+// memory (added in rank order, as the combine kernel adds them) instead of a workspace and a second launch, which cost
+// 7 to 9 us of a step.
+__device__ __forceinline__ float ad_ld_remote(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ad_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <bool Q8, bool CL>
 __global__ void __launch_bounds__(ADM_WARPS * 32) attn_decode_mma_kernel(AdArgs a) {
   extern __shared__ __align__(128) uint8_t adm_smem[];
   const int sp = blockIdx.x, S = gridDim.x, b = blockIdx.y;
@@ -586,6 +599,52 @@ __global__ void __launch_bounds__(ADM_WARPS * 32) attn_decode_mma_kernel(AdArgs 
   bool any = false;
 #pragma unroll
   for (int w = 0; w < ADM_WARPS; ++w) any = any || s_any[w] != 0;
+  if constexpr (CL) {
+    float* s_sum = reinterpret_cast<float*>(adm_smem + ADM_WARPS * 16 * 4 + 64);      // [16] row sums of this CTA, then its flag
+    for (int idx = tid; idx < a.nh * AD_C; idx += ADM_WARPS * 32) {                   // this CTA's sums over the first warp's tile
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < ADM_WARPS; ++w) v += s_o[(size_t)w * 16 * AD_C + idx];
+      s_o[idx] = v;
+    }
+    if (tid < a.nh) {
+      float l = 0.f;
+#pragma unroll
+      for (int w = 0; w < ADM_WARPS; ++w) l += s_l[w * 16 + tid];
+      s_sum[tid] = l;
+    }
+    if (tid == 0) s_sum[16] = any ? 1.f : 0.f;
+    ad_cluster_sync();
+    const uint32_t o_addr = smem_addr_u32(s_o), l_addr = smem_addr_u32(s_sum);
+    float anyf = 0.f;
+    for (int r = 0; r < S; ++r) anyf += ad_ld_remote(l_addr + 16 * 4, r);
+    for (int idx = sp * (ADM_WARPS * 32) + tid; idx < a.nh * AD_C; idx += S * (ADM_WARPS * 32)) {
+      const int h = idx >> 7;
+      float o = 0.f, den = 0.f;
+      float ov[8], lv[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        ov[r] = r < S ? ad_ld_remote(o_addr + idx * 4, r) : 0.f;
+        lv[r] = r < S ? ad_ld_remote(l_addr + h * 4, r) : 0.f;
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) { o += ov[r]; den += lv[r]; }
+      if (anyf > 0.f) {
+        if (a.sink) {
+          const float sk = ld_any(a.sink, h, a.sink_dtype);
+          den += expf(sk - fmaxf(ascale, sk));
+        }
+        o /= den;
+      } else {
+        o = 0.f;
+      }
+      const int64_t off = (int64_t)b * a.nh * AD_C + idx;
+      if (a.out_dtype == KCH_BF16) ((bf16*)a.out)[off] = __float2bfloat16_rn(o);
+      else ((float*)a.out)[off] = o;
+    }
+    ad_cluster_sync();                                    // nobody leaves while a neighbour may still read its sums
+    return;
+  }
   float* wsb = a.ws + ((int64_t)b * S + sp) * a.nh * (AD_C + 2);
   for (int idx = tid; idx < a.nh * AD_C; idx += ADM_WARPS * 32) {
     const int h = idx >> 7, d = idx & 127;
@@ -662,12 +721,23 @@ extern "C" int kch_attend_decode(const kch_attend_decode_args* p, void* stream) 
   static const bool force_simt = [] { const char* e = getenv("KCH_ATTEND_DECODE"); return e && e[0] == 's'; }();
   if (!force_simt && attend_decode_mma_ok(p)) {
     const size_t smem = 2 * 16 * ADM_QLD * 2 + (size_t)ADM_WARPS * ((ADM_STAGES + 1) * ADM_STAGE_BYTES);
-    if (p->comp_dtype == KCH_BF16) {
-      KCH_CUDA_OK(cudaFuncSetAttribute(attn_decode_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      KCH_CUDA_OK(kch_launch_chained(attn_decode_mma_kernel<false>, dim3(S, p->B), dim3(ADM_WARPS * 32), smem, s, 1, a));
-    } else {
-      KCH_CUDA_OK(cudaFuncSetAttribute(attn_decode_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      KCH_CUDA_OK(kch_launch_chained(attn_decode_mma_kernel<true>, dim3(S, p->B), dim3(ADM_WARPS * 32), smem, s, 1, a));
+    // One cluster per sequence (at most 8 CTAs, two warps with a ring of three tiles each) while its entries are a few
+    // rounds of those rings, or while 8 CTAs per sequence fill the chip anyway; else more CTAs and a second launch.
+    const int CS = S < 8 ? S : 8;
+    const int64_t entries = (a.sel ? (int64_t)a.topk : a.comp ? a.cap : 0) + (a.win ? a.W : 0);
+    const bool cl = CS > 1 && (entries <= (int64_t)CS * ADM_WARPS * ADM_TILE * ADM_STAGES * 2 || S <= 8);
+#define ADM_GO(Q8_, CL_)                                                                                                         \
+  do {                                                                                                                           \
+    KCH_CUDA_OK(cudaFuncSetAttribute(attn_decode_mma_kernel<Q8_, CL_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    KCH_CUDA_OK(kch_launch_chained(attn_decode_mma_kernel<Q8_, CL_>, dim3(CL_ ? CS : S, p->B), dim3(ADM_WARPS * 32), smem, s,    \
+                                   CL_ ? (unsigned)CS : 1u, a));                                                                 \
+  } while (0)
+    if (p->comp_dtype == KCH_BF16) { if (cl) ADM_GO(false, true); else ADM_GO(false, false); }
+    else { if (cl) ADM_GO(true, true); else ADM_GO(true, false); }
+#undef ADM_GO
+    if (cl) {
+      KCH_LAUNCH_OK();
+      return KCH_OK;
     }
   } else {
     KCH_CUDA_OK(kch_launch_chained(attn_decode_split_kernel, dim3(S, p->B), dim3(AD_THREADS), 0, s, 1, a));

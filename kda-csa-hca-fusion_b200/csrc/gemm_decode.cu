@@ -141,7 +141,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
 
   // ---- the rows this thread finishes, and their residual values (an earlier kernel's output: ready now) ----------
-  const int rows_per = 64 / ksplit;
+  const int rows_per = Cfg::PUSH ? 64 / ksplit : (M + ksplit - 1) / ksplit;     // (a pulled tile is dealt out by its real rows)
   const int items = rows_per * QPR;
   uint2 rpre[4];
 #pragma unroll
@@ -215,11 +215,11 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (split) { gd_cluster_arrive(); gd_cluster_wait(); } else { __syncthreads(); }
 
   // ---- finish this CTA's rows: sum the partials in rank order, activation, residual, store ----------------------------
-  auto finish = [&](const int it, const uint2 rpre_v, const bool have_pre) {
+  auto finish = [&](const int it, const uint2 rpre_v, const bool have_pre, const float (&sum)[4]) {
     const bool live = it < items;                       // uniform over a warp (items is a multiple of 32 where it matters)
     const int rl = live ? it / QPR : 0, q = live ? it % QPR : 0;
     const int row = ks * rows_per + rl;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    float v[4] = {sum[0], sum[1], sum[2], sum[3]};
     if (Cfg::PUSH) {
 #pragma unroll 1
       for (int p = 0; p < ksplit; ++p) {
@@ -228,20 +228,6 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                      : "r"(red0 + (uint32_t)((p * rows_per + rl) * RED_LD + q * 4) * 4u) : "memory");
         v[0] += x0; v[1] += x1; v[2] += x2; v[3] += x3;
       }
-    } else {
-      float x[8][4];
-      const uint32_t off = red0 + (uint32_t)(row * RED_LD + q * 4) * 4u;
-#pragma unroll
-      for (int p = 0; p < 8; ++p) {
-        x[p][0] = x[p][1] = x[p][2] = x[p][3] = 0.f;
-        if (p < ksplit) {
-          const uint32_t src = split ? gd_mapa(off, (uint32_t)p) : off;
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[p][0]), "=f"(x[p][1]), "=f"(x[p][2]), "=f"(x[p][3])
-                       : "r"(src) : "memory");
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < 8; ++p) { v[0] += x[p][0]; v[1] += x[p][1]; v[2] += x[p][2]; v[3] += x[p][3]; }
     }
     const int col = nb * BN + q * 4;
     int act = 0;
@@ -303,11 +289,46 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
   };
+  const float zero4[4] = {0.f, 0.f, 0.f, 0.f};
+  if constexpr (Cfg::PUSH) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (i * GD_THREADS < items) finish(tid + i * GD_THREADS, rpre[i], true);
+    for (int i = 0; i < 4; ++i)
+      if (i * GD_THREADS < items) finish(tid + i * GD_THREADS, rpre[i], true, zero4);
 #pragma unroll 1
-  for (int i = 4; i * GD_THREADS < items; ++i) finish(tid + i * GD_THREADS, make_uint2(0u, 0u), false);
+    for (int i = 4; i * GD_THREADS < items; ++i) finish(tid + i * GD_THREADS, make_uint2(0u, 0u), false, zero4);
+  } else {
+    // Pulled partials: the loads of two items, from every rank, are under way before the first sum (one round trip
+    // through the cluster per pair of items; a load-add-activate sequence per item took 4 us of a 14 us launch)
+#pragma unroll 1
+    for (int i0 = 0; i0 * GD_THREADS < items; i0 += 2) {
+      float x[2][8][4], sum[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int it = tid + (i0 + u) * GD_THREADS, row = ks * rows_per + it / QPR;
+        const uint32_t off = red0 + (uint32_t)(row * RED_LD + (it % QPR) * 4) * 4u;
+        const bool on = it < items && row < M;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+          x[u][p][0] = x[u][p][1] = x[u][p][2] = x[u][p][3] = 0.f;
+          if (on && p < ksplit) {
+            const uint32_t src = split ? gd_mapa(off, (uint32_t)p) : off;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(x[u][p][0]), "=f"(x[u][p][1]), "=f"(x[u][p][2]), "=f"(x[u][p][3]) : "r"(src) : "memory");
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sum[u][e] = 0.f;
+#pragma unroll
+          for (int p = 0; p < 8; ++p) sum[u][e] += x[u][p][e];
+        }
+        if ((i0 + u) * GD_THREADS < items) finish(tid + (i0 + u) * GD_THREADS, i0 == 0 ? rpre[u] : i0 == 2 ? rpre[2 + u] : make_uint2(0u, 0u), i0 <= 2, sum[u]);
+      }
+    }
+  }
   if (split && !Cfg::PUSH) { gd_cluster_arrive(); gd_cluster_wait(); }     // nobody leaves while a peer may still read its partials
   __syncthreads();
   if (warp == 1) {

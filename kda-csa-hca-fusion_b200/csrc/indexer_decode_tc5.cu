@@ -18,7 +18,7 @@
 #include "kch_common.cuh"
 #include "tc5_utils.cuh"
 
-#define IXD_ROWS 1024
+#define IXD_ROWS 1024                 // key rows of a CTA at most
 #define IXD_TILE 128
 #define IXD_STAGES 4
 #define IXD_THREADS 192
@@ -39,16 +39,16 @@ struct IxdSmem {
 __global__ void __launch_bounds__(IXD_THREADS, 3)
 decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* q, int q_dtype, int64_t q_ld, const float* norms,
                           const void* w, int w_dtype, int64_t w_ld, float* logits, int64_t cap, int64_t n_ld, int HI,
-                          int normalize, float scale, int m, const int32_t* ctr, unsigned int* status) {
+                          int normalize, float scale, int m, const int32_t* ctr, int cta_rows, unsigned int* status) {
   chain_wait();
   chain_trigger();
   extern __shared__ uint8_t ixd_raw[];
   IxdSmem& sm = *reinterpret_cast<IxdSmem*>(((uintptr_t)ixd_raw + 1023) & ~(uintptr_t)1023);
   const int b = blockIdx.y, tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   const int nvis = min(ctr[KCH_CTR_TOKENS] / m, ctr[KCH_CTR_N_BLOCKS]);
-  const int r0 = blockIdx.x * IXD_ROWS;
+  const int r0 = blockIdx.x * cta_rows;
   if (r0 >= nvis) return;                                      // the whole CTA, before any barrier or allocation
-  const int ntiles = min(IXD_ROWS / IXD_TILE, (nvis - r0 + IXD_TILE - 1) / IXD_TILE);
+  const int ntiles = min(cta_rows / IXD_TILE, (nvis - r0 + IXD_TILE - 1) / IXD_TILE);
 
   if (tid == 0) {
     for (int s = 0; s < IXD_STAGES; ++s) { mbarrier_init(&sm.full[s], 1); mbarrier_init(&sm.empty[s], 1); }
@@ -138,7 +138,7 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
 #pragma unroll
     for (int t = 0; t < IXD_ROWS / IXD_TILE; ++t) {
       const int row = r0 + t * IXD_TILE + warp * 32 + lane;
-      nv[t] = (normalize && row < nvis) ? nb[row] : 1.f;
+      nv[t] = (normalize && t < ntiles && row < nvis) ? nb[row] : 1.f;
     }
     bool ok = true;
 #pragma unroll
@@ -188,9 +188,13 @@ int kch_decode_indexer_logits_tc5(const void* q, int q_dtype, int64_t q_ld, cons
   KCH_REQUIRE(status != nullptr, "kch_decode_indexer_topk: cannot resolve the device status word");
   const size_t smem = sizeof(IxdSmem) + 1024;
   KCH_CUDA_OK(cudaFuncSetAttribute(decode_indexer_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((cap + IXD_ROWS - 1) / IXD_ROWS), (unsigned)B);
+  // A CTA's set-up (query terms, tensor memory) is worth eight tiles of keys when there are enough of them to fill the chip
+  // (two CTAs per SM); a small batch is spread thinner instead: 8 sequences of 4000 blocks took 11.3 us in 32 CTAs.
+  int rows = IXD_ROWS;
+  while (rows > IXD_TILE && (int64_t)B * ((cap + rows - 1) / rows) < 2 * 148) rows >>= 1;
+  dim3 grid((unsigned)((cap + rows - 1) / rows), (unsigned)B);
   KCH_CUDA_OK(kch_launch_chained(decode_indexer_tc5_kernel, grid, dim3(IXD_THREADS), smem, s, 1, kmap, q, q_dtype, q_ld, norms, w,
-                                 w_dtype, w_ld, logits, cap, n_ld, HI, normalize, scale, m, ctr, status));
+                                 w_dtype, w_ld, logits, cap, n_ld, HI, normalize, scale, m, ctr, rows, status));
   KCH_LAUNCH_OK();
   return KCH_OK;
 }

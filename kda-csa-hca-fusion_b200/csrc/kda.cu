@@ -87,22 +87,27 @@ kda_recurrent_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 
 // One-token step (T = 1, K = V = 128), the form a decode step takes.  The 64 KB state of one (batch, value head) is
 // contiguous: one bulk copy brings it into shared memory (no registers, no per-thread loads: three CTAs per SM keep
-// 192 KB of requests in flight), one thread per value column walks its 128 K rows there -- the two contractions over
-// K (k^T S and q^T S) are private sums, no exchange between warps -- and one bulk copy writes the state back.  Decay,
-// key and scaled query of a K row travel as one float4 broadcast.  The sums are taken in the same order as
-// kda_recurrent_kernel (four runs of 32 rows, added left to right), so both kernels return the same bits.
+// 192 KB of requests in flight) and one bulk copy writes it back.  A thread takes RPT of a
+// value column's four runs of 32 K rows; decay, key and scaled query of a K row travel as one float4 broadcast.  Both contractions over K (k^T S and
+// q^T S) are four private runs added left to right, the order of kda_recurrent_kernel, so both return the same bits.
+// Bound: HBM (128 KB per head) at large batches, where one thread per column (RPT = 4, three CTAs per SM) is enough and
+// more threads only cost residency (25 us against 28 for 1024 heads); with at most two CTAs per SM in all, the chain
+// copy -> two passes over the rows -> copy, whose middle four threads per column (RPT = 1) take from 2.2 to 0.7 us:
+// 128 heads, within a step: 9.7 -> 9.1 us.
 // The wait for the copy is bounded (status word, see kch_device_status).
 #define KDS_STATE_BYTES (128 * 128 * 4)
-#define KDS_SMEM (KDS_STATE_BYTES + 128 * 16 + 16)
-template <typename T>
-__global__ void __launch_bounds__(128)
-kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int H, int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v,
-                       int64_t ld_g, int64_t ld_b, unsigned int* status) {
+#define KDS_SMEM (KDS_STATE_BYTES + 128 * 16 + 2 * 4 * 128 * 4 + 16)
+template <typename T, int RPT>
+__global__ void __launch_bounds__(512 / RPT, RPT == 4 ? 3 : 2)
+kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int H,
+                       int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b,
+                       unsigned int* status) {
   constexpr int K = 128, V = 128;
   extern __shared__ __align__(128) uint8_t kds_raw[];
   float* st = reinterpret_cast<float*>(kds_raw);                                   // [K][V]
   float4* sgkq = reinterpret_cast<float4*>(kds_raw + KDS_STATE_BYTES);             // {exp(g), k, scale * q, -} of K row i
-  uint64_t* bar = reinterpret_cast<uint64_t*>(kds_raw + KDS_STATE_BYTES + 128 * 16);
+  float* sp = reinterpret_cast<float*>(kds_raw + KDS_STATE_BYTES + 128 * 16);      // [2][4][V] sums of the runs
+  uint64_t* bar = reinterpret_cast<uint64_t*>(kds_raw + KDS_STATE_BYTES + 128 * 16 + 2 * 4 * V * 4);
   const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int h = hv / (HV / H);
   const int64_t sbase = ((int64_t)b * HV + hv) * K * V;
@@ -112,60 +117,61 @@ kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* 
   }
   chain_wait();
   chain_trigger();
-  if (tid == 0) {
-    if (S0) {
-      mbarrier_expect_tx(bar, KDS_STATE_BYTES);
-      bulk_copy_g2s(st, S0 + sbase, KDS_STATE_BYTES, bar);
-    }
+  if (tid == 0 && S0) {
+    mbarrier_expect_tx(bar, KDS_STATE_BYTES);
+    bulk_copy_g2s(st, S0 + sbase, KDS_STATE_BYTES, bar);
   }
-  {
+  const int c = tid & 127, run0 = (tid >> 7) * RPT;    // value column, first of this thread's runs of 32 K rows
+  const float bt = ldf(beta + (int64_t)b * ld_b + hv);
+  const float vv = ldf(v + (int64_t)b * ld_v + (int64_t)hv * V + c);
+  if (tid < K) {
     const int64_t qoff = (int64_t)b * ld_qk + (int64_t)h * K, goff = (int64_t)b * ld_g + (int64_t)hv * K;
     sgkq[tid] = make_float4(expf(fmaxf(ldf(g + goff + tid), g_min)), ldf(k + qoff + tid), ldf(q + qoff + tid) * scale, 0.f);
   }
-  const float bt = ldf(beta + (int64_t)b * ld_b + hv);
-  const float vv = ldf(v + (int64_t)b * ld_v + (int64_t)hv * V + tid);
   if (!S0) {
-    for (int i = 0; i < K; ++i) st[i * V + tid] = 0.f;
+    for (int i = 32 * run0; i < 32 * (run0 + RPT); ++i) st[i * V + c] = 0.f;
   }
   __syncthreads();
   bool ok = true;
   if (S0) ok = mbarrier_wait_bounded(bar, 0, KCH_STATUS_KDA_STEP, 1u << 24, status);
-  float* col = st + tid;
-  float p[4], r[4];
 #pragma unroll
-  for (int run = 0; run < 4; ++run) {
+  for (int r = run0; r < run0 + RPT; ++r) {
+    const float* col = st + 32 * r * V + c;
+    const float4* row = sgkq + 32 * r;
     float acc = 0.f;
 #pragma unroll 8
-    for (int i = 32 * run; i < 32 * run + 32; ++i) {
-      const float4 c = sgkq[i];
-      acc = fmaf(c.y, col[i * V] * c.x, acc);
+    for (int i = 0; i < 32; ++i) {
+      const float4 x = row[i];
+      acc = fmaf(x.y, col[i * V] * x.x, acc);
     }
-    p[run] = acc;
+    sp[r * V + c] = acc;
   }
-  const float delta = bt * (vv - (p[0] + p[1] + p[2] + p[3]));
+  __syncthreads();
+  const float delta = bt * (vv - (sp[c] + sp[V + c] + sp[2 * V + c] + sp[3 * V + c]));
 #pragma unroll
-  for (int run = 0; run < 4; ++run) {
+  for (int r = run0; r < run0 + RPT; ++r) {
+    float* col = st + 32 * r * V + c;
+    const float4* row = sgkq + 32 * r;
     float acc = 0.f;
 #pragma unroll 8
-    for (int i = 32 * run; i < 32 * run + 32; ++i) {
-      const float4 c = sgkq[i];
-      const float sv = fmaf(c.y, delta, col[i * V] * c.x);
+    for (int i = 0; i < 32; ++i) {
+      const float4 x = row[i];
+      const float sv = fmaf(x.y, delta, col[i * V] * x.x);
       col[i * V] = sv;
-      acc = fmaf(c.z, sv, acc);
+      acc = fmaf(x.z, sv, acc);
     }
-    r[run] = acc;
+    sp[(4 + r) * V + c] = acc;
   }
-  if (ok) stf(o + ((int64_t)b * HV + hv) * V + tid, r[0] + r[1] + r[2] + r[3]);
-  if (S_out) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the bulk store reads what the threads wrote
-    __syncthreads();
-    if (tid == 0 && ok) {
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                   ::"l"(S_out + sbase), "r"(smem_addr_u32(st)), "r"((uint32_t)KDS_STATE_BYTES) : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory must outlive the copy
-    }
+  if (S_out) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // the bulk store reads what the threads wrote
+  __syncthreads();
+  if (S_out && tid == 0 && ok) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                 ::"l"(S_out + sbase), "r"(smem_addr_u32(st)), "r"((uint32_t)KDS_STATE_BYTES) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
+  if (run0 == 0 && ok)
+    stf(o + ((int64_t)b * HV + hv) * V + c, sp[4 * V + c] + sp[5 * V + c] + sp[6 * V + c] + sp[7 * V + c]);
+  if (S_out && tid == 0 && ok) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory must outlive the copy
 }
 
 extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, const void* g,
@@ -192,12 +198,16 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
   if (T == 1 && K == 128 && V == 128 && !old_step && (((uintptr_t)initial_state | (uintptr_t)final_state) & 15) == 0) {
     unsigned int* status = kch_status_device_ptr();
     KCH_REQUIRE(status != nullptr, "kch_kda_recurrent: cannot resolve the device status word");
-    KCH_DISPATCH_FLOAT(dtype, T_, {
-      KCH_CUDA_OK(cudaFuncSetAttribute(kda_decode_step_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, KDS_SMEM));
-      KCH_CUDA_OK(kch_launch_chained(kda_decode_step_kernel<T_>, dim3(HV, B), dim3(128), KDS_SMEM, s, 1,
-        (const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta, initial_state, (T_*)o, final_state, H, HV,
-        scale, g_clamp_min, ld_qk, ld_v, ld_g, ld_beta, status));
-    });
+#define KDS_GO(T_, RPT_)                                                                                                         \
+  do {                                                                                                                           \
+    KCH_CUDA_OK(cudaFuncSetAttribute(kda_decode_step_kernel<T_, RPT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, KDS_SMEM));  \
+    KCH_CUDA_OK(kch_launch_chained(kda_decode_step_kernel<T_, RPT_>, dim3(HV, B), dim3(512 / RPT_), KDS_SMEM, s, 1,              \
+        (const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta, initial_state, (T_*)o, final_state, H, HV,      \
+        scale, g_clamp_min, ld_qk, ld_v, ld_g, ld_beta, status));                                                                \
+  } while (0)
+    const bool few = (int64_t)HV * B <= 2 * 148;
+    KCH_DISPATCH_FLOAT(dtype, T_, { if (few) KDS_GO(T_, 1); else KDS_GO(T_, 4); });
+#undef KDS_GO
     KCH_LAUNCH_OK();
     return KCH_OK;
   }

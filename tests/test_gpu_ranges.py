@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 from kch_b200 import synthetic as syn  # noqa: E402
 from oracle import kch_oracle as orc  # noqa: E402
 
-DEV = "cuda"
+DEV = "cuda:0"
 
 
 @pytest.fixture(scope="module")
@@ -98,3 +98,47 @@ def test_selection_as_mask_matches_gather(kch, B, T, nh, n, topk, m, t0, nvis, w
         keep = ~bad & (torch.arange(T, device=DEV) < 0)      # every query sees row 5: nothing finite is expected
         dense, dref = dense[:, keep], dref[:, keep]
     assert md(dense, dref) <= 2e-3, md(dense, dref)
+
+
+@pytest.mark.parametrize("M,N", [(1, 256), (7, 400), (33, 6288), (64, 256)])
+def test_decode_gemm_l2norm_rows(kch, M, N):
+    """The 128-wide decode tiles deal their rows out over the CTAs of a cluster by the real row count."""
+    from kch_b200 import _lib
+    from kch_b200.csa import linear
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, W = torch.randn(M, 1, 2048, generator=g, device=DEV).bfloat16(), (torch.randn(N, 2048, generator=g, device=DEV) * 0.02).bfloat16()
+    tail = N % 128
+    segs = [(N - tail, _lib.ACT_SILU_L2NORM, 0.0)] + ([(tail, _lib.ACT_SIGMOID, 0.0)] if tail else [])
+    y = linear(x, W, epilogue=segs, group=128)
+    p = (x.double() @ W.double().T).bfloat16().double()
+    ref = torch.nn.functional.silu(p[..., :N - tail]).bfloat16().double().unflatten(-1, (-1, 128))
+    ref = (ref / ref.norm(dim=-1, keepdim=True).bfloat16().double()).flatten(-2)
+    ref = torch.cat([ref, torch.sigmoid(p[..., N - tail:])], -1)
+    # products within one bf16 rounding, then the rounding of the activation: 2^-7 of the value in all
+    assert bool(((y.double() - ref).abs() <= 2 ** -7 * ref.abs() + 2e-3).all()), md(y, ref)
+
+
+@pytest.mark.parametrize("B,nb,topk,quant", [(1, 40, 16, None), (3, 700, 300, "fp8"), (8, 1500, 1024, None), (70, 64, 64, "int8"),
+                                             (2, 5000, 4500, None)])
+def test_decode_attention_split_or_cluster(kch, B, nb, topk, quant):
+    """Few entries per sequence are merged inside a cluster, many by a second launch; the indexer deals its key rows out by
+    the batch.  Against the oracle of the cache: 2e-4 with bf16 rows, 2e-3 with 8-bit rows, as for the golden streams."""
+    c, cI, m, win, nh, nI = 128, 64, 4, 32, 16, 4
+    g = torch.Generator().manual_seed(nb)
+    T = nb * m + 1
+    w = [(torch.randn(B, T, x, generator=g)).bfloat16() for x in (c, c, c, c, cI, cI)]
+    Ba, Bb, Bi = ((torch.randn(m, x, generator=g) * 0.02).bfloat16() for x in (c, c, cI))
+    cache = kch.CSADecodingCache(B, c, cI, m, win, DEV, torch.bfloat16, kv_quant=quant)
+    ref = orc.CSACacheOracle(B, c, cI, m, win, torch.bfloat16, quant)
+    dw, db = [x.to(DEV) for x in w], [x.to(DEV) for x in (Ba, Bb, Bi)]
+    cache.append_step(*(x[:, :-1] for x in dw), *db)
+    cache.append_step(*(x[:, -1:] for x in dw), *db)
+    ref.append(*(x[:, :-1] for x in w), Ba, Bb, Bi)
+    ref.append(*(x[:, -1:] for x in w), Ba, Bb, Bi)
+    q = torch.nn.functional.normalize(torch.randn(B, 1, nh, c, generator=g), dim=-1)
+    qi, wi, sink = torch.randn(B, 1, nI, cI, generator=g), torch.randn(B, 1, nI, generator=g), torch.randn(nh, generator=g)
+    out, sel = cache.forward_step(q.to(DEV), qi.to(DEV), wi.to(DEV), topk=topk, nh=nh, nIh=nI, scale=1.0, sink_logits=sink.to(DEV),
+                                  use_ste=False, _return_indices=True)
+    want = ref.step(q, qi, wi, topk=topk, sink_logits=sink, scale=1.0)
+    assert (sel.sort(-1).values[:, 0, 1:] > sel.sort(-1).values[:, 0, :-1]).all()
+    assert md(out, want) <= (2e-3 if quant else 2e-4), md(out, want)
