@@ -180,18 +180,111 @@ struct TgSmem {
   static constexpr int EPI_WARPS = BN == 256 ? 8 : 4;   // narrower tiles are stored by warps 2..5 alone
   alignas(1024) bf16 a[STAGES][A_ROWS * TG_BK];
   alignas(1024) bf16 b[STAGES][B_ROWS * TG_BK];
-  alignas(16) uint8_t epi[EPI_WARPS][32 * TG_EPI_LD];   // per epilogue warp: a 32 x 32 bf16 chunk, rows padded to 80 bytes
+  // per epilogue warp: a 32 x 32 bf16 chunk, rows padded to 80 bytes; on CTA pairs also a 32 x 64 one for a bulk-tensor store
+  static constexpr int EPI_BYTES = TWO ? 4096 : 32 * TG_EPI_LD;
+  alignas(TWO ? 1024 : 16) uint8_t epi[EPI_WARPS][EPI_BYTES];
   alignas(8) uint64_t full[STAGES];
   uint64_t empty[STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t res_full[8];                // per epilogue warp: a residual tile has landed (CTA pairs)
   uint32_t tmem_base;
 };
+
+// ---- epilogue of a CTA pair's plain, silu and silu + L2-norm columns -------------------------------------------------------
+// A warp's 32 rows x 128 columns leave as two 32 x 64 tiles through swizzled shared memory and bulk-tensor stores: whole
+// 128-byte lines, no store instructions, and the copy engine clips what lies beyond M and N.  The 128 columns are held as
+// packed bf16, so that the accumulator is released before anything is stored and an L2 norm needs silu once.  A residual
+// tile arrives the same way in the staging tile and is added in place.
+// The K = 128 projections are all epilogue: with 64-byte row segments stored by the warps and the accumulator held
+// meanwhile a 256 x 256 tile took 7100 cycles, now 3400 (131072 x 2048: 253 -> 100 us); products with K = 2048, where it is
+// hidden behind the main loop, still gained (131072 x 2048: 773 -> 689 us, 1.42 -> 1.6 PFLOP/s).
+template <typename SM>
+__device__ __forceinline__ void bulk_residual(SM& sm, int warp, const CUtensorMap& map_r, int col, int row, int64_t M, int N) {
+  if (col >= N || row >= M) return;
+  mbar_expect_tx(&sm.res_full[warp - 2], 32 * 64 * 2);
+  tma_load_2d(sm.epi[warp - 2], &map_r, col, row, &sm.res_full[warp - 2]);
+}
+template <int ACT, typename SM, typename F>
+__device__ __forceinline__ void bulk_tile(SM& sm, int warp, int lane, uint32_t taddr, const CUtensorMap& map_c, const CUtensorMap& map_r,
+                                          bool residual, int col0, int64_t row0, int64_t M, int N, float, uint32_t& rphase, F release) {
+  uint8_t* stg = sm.epi[warp - 2];
+  uint32_t pk[64];
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < 4; c += 2) {
+    uint32_t r[2][32];
+    tc_ld32(taddr + 32 * c, r[0]);
+    tc_ld32(taddr + 32 * c + 32, r[1]);
+    tc_wait_ld();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float x = __uint_as_float(r[h][2 * j]), y = __uint_as_float(r[h][2 * j + 1]);
+        if (ACT != 0) { x = ep_silu(bf16r(x)); y = ep_silu(bf16r(y)); }
+        const uint32_t w = pack2_bf16(x, y);
+        if (ACT == KCH_ACT_SILU_L2NORM) {
+          const float xr = __uint_as_float(w << 16), yr = __uint_as_float(w & 0xFFFF0000u);
+          ss = fmaf(xr, xr, ss);
+          ss = fmaf(yr, yr, ss);
+        }
+        pk[16 * (c + h) + j] = w;
+      }
+  }
+  release();
+  if (ACT == KCH_ACT_SILU_L2NORM) {
+    const float nrm = __fdividef(1.0f, fmaxf(bf16r(sqrtf(ss)), 1e-12f));
+#pragma unroll
+    for (int j = 0; j < 64; ++j) pk[j] = pack2_bf16(__uint_as_float(pk[j] << 16) * nrm, __uint_as_float(pk[j] & 0xFFFF0000u) * nrm);
+  }
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const int col = col0 + 64 * g;
+    const bool any = col < N && row0 < M;
+    if (ACT == 0 && residual) {
+      if (g == 1 && lane == 0) {
+        t5_bulk_wait_read();
+        bulk_residual(sm, warp, map_r, col, (int)row0, M, N);
+      }
+      if (any) {
+        mbar_wait(&sm.res_full[warp - 2], rphase & 1, 5);
+        ++rphase;
+      }
+    } else {
+      if (lane == 0) t5_bulk_wait_read();                // the store before has read the tile
+      __syncwarp();
+    }
+    if (any) {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        uint4* dst = reinterpret_cast<uint4*>(stg + lane * 128 + ((v ^ (lane & 7)) << 4));
+        uint32_t w[4] = {pk[32 * g + 4 * v], pk[32 * g + 4 * v + 1], pk[32 * g + 4 * v + 2], pk[32 * g + 4 * v + 3]};
+        if (ACT == 0 && residual) {
+          const uint4 rv = *dst;
+          const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            w[e] = pack2_bf16(__uint_as_float(w[e] << 16) + __uint_as_float(rw[e] << 16),
+                              __uint_as_float(w[e] & 0xFFFF0000u) + __uint_as_float(rw[e] & 0xFFFF0000u));
+        }
+        *dst = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      t5_fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+                     ::"l"(&map_c), "r"(col), "r"((int)row0), "r"(smem_u32(stg)) : "memory");
+        t5_bulk_commit();
+      }
+    }
+  }
+}
 
 template <int BN, bool TWO, bool SK = false>
 __global__ void __launch_bounds__(TG_THREADS, SK ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                    bf16* __restrict__ C, const bf16* __restrict__ R, int64_t M, int N, int K,
+                    const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_r, int c_bulk, bf16* __restrict__ C, const bf16* __restrict__ R, int64_t M, int N, int K,
                     int64_t ldc, int64_t ldr, int vec_ok, const TgEpilogue ep, int slab_k, int64_t slab_rows,
                     int ksplit) {
   // ksplit > 1 (SK only; launched as clusters of `ksplit` CTAs, one tile per cluster): CTA r of the cluster runs
@@ -227,6 +320,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // pair: the even CTA's `full` counts the bytes of both producers, its `acc_empty` the epilogue warps of both CTAs
     for (int s = 0; s < TG_STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sm.acc_full[i], 1); mbar_init(&sm.acc_empty[i], TWO ? 16 : 8); }
+    if (TWO) for (int i = 0; i < 8; ++i) mbar_init(&sm.res_full[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -324,7 +418,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int half = (warp - 2) >> 2;
     const int c_begin = (BN == 256) ? half * 128 : 0;
     const int c_end = (BN == 256) ? c_begin + 128 : (half == 0 ? BN : 0);
-    uint32_t tcount = 0;
+    uint32_t tcount = 0, rphase = 0;
     bool ok = true;
     if (split) {
       // this CTA's partial sums of rows 0..63, as fp32, to shared memory (the ring is drained: every MMA has retired)
@@ -348,10 +442,47 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int64_t mb = tile / n_tiles;
       const int nb = (int)(tile % n_tiles);
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
+      // the activation of this warp's 128 columns when they have one: 0, silu or silu + L2 norm, which bulk_tile knows; -1 otherwise
+      int act_bulk = -1;
+      if constexpr (TWO) {
+        if (c_bulk) {
+          act_bulk = 0;
+          if (ep.nseg) {
+            const int col = nb * BN + c_begin;
+            int sidx = 0;
+            while (sidx < ep.nseg - 1 && col >= ep.seg_end[sidx]) ++sidx;
+            act_bulk = col + 128 <= ep.seg_end[sidx] || col >= N ? ep.seg_act[sidx] : -1;
+            if (act_bulk != 0 && act_bulk != KCH_ACT_SILU && act_bulk != KCH_ACT_SILU_L2NORM) act_bulk = -1;
+          }
+          if (R && lane == 0) {                          // the first half's residual rows are under way before the product is complete
+            t5_bulk_wait_read();
+            bulk_residual(sm, warp, map_r, nb * BN + c_begin, (int)(mb * BM_T + rank * TG_BM + quarter * 32), M, N);
+          }
+        }
+      }
       if (!mbar_wait(&sm.acc_full[acc], aph, 4)) { ok = false; break; }
       tc_fence_after();
       const int64_t row = mb * BM_T + rank * TG_BM + quarter * 32 + lane;
       const uint32_t tbase = tmem_base + acc * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
+      if constexpr (TWO) {
+        if (act_bulk >= 0) {
+          const int col0 = nb * BN + c_begin;
+          const int64_t row0 = mb * BM_T + rank * TG_BM + quarter * 32;
+          auto release = [&] {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&sm.acc_empty[acc]), 0));
+          };
+          if (act_bulk == 0) bulk_tile<0>(sm, warp, lane, tbase + c_begin, map_c, map_r, R != nullptr, col0, row0, M, N, 0.f, rphase, release);
+          else if (act_bulk == KCH_ACT_SILU) bulk_tile<KCH_ACT_SILU>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, 0.f, rphase, release);
+          else bulk_tile<KCH_ACT_SILU_L2NORM>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, 0.f, rphase, release);
+          continue;
+        }
+        if (c_bulk) {                                    // the staging tile is about to be written by hand
+          if (lane == 0) t5_bulk_wait_read();
+          __syncwarp();
+        }
+      }
       float nrm = 1.f;
       // the accumulator chunk after the current one is already on its way from tensor memory
       uint32_t rn[32];
@@ -461,6 +592,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         else mbar_arrive(&sm.acc_empty[acc]);
       }
     }
+    if (TWO && c_bulk && lane == 0) t5_bulk_wait_read();       // shared memory must outlive the copies
   }
   tc_fence_before();
   __syncthreads();
@@ -675,12 +807,12 @@ static int launch_tg(const void* A, const void* W, void* C, const void* R, int64
         attr[0].val.clusterDim.x = (unsigned)ksplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3((unsigned)(tiles * ksplit)); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem;
         cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 1;
-        KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, false, true>, ma, mw, (bf16*)C, (const bf16*)R, M, N, K,
+        KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, false, true>, ma, mw, ma, ma, 0, (bf16*)C, (const bf16*)R, M, N, K,
                                        ldc, ldr, vec_ok, ep, slab_k, M, ksplit));
         kch_note_launch(1);
         return KCH_OK;
       }
-      gemm_tcgen05_kernel<BN, false, true><<<grid, TG_THREADS, smem, s>>>(ma, mw, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
+      gemm_tcgen05_kernel<BN, false, true><<<grid, TG_THREADS, smem, s>>>(ma, mw, ma, ma, 0, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
                                                                          vec_ok, ep, slab_k, M, 1);
       KCH_LAUNCH_OK();
       return KCH_OK;
@@ -688,7 +820,7 @@ static int launch_tg(const void* A, const void* W, void* C, const void* R, int64
   }
   size_t smem = sizeof(TgSmem<BN>) + 1024;
   KCH_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gemm_tcgen05_kernel<BN, false><<<grid, TG_THREADS, smem, s>>>(ma, mw, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr, vec_ok, ep,
+  gemm_tcgen05_kernel<BN, false><<<grid, TG_THREADS, smem, s>>>(ma, mw, ma, ma, 0, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr, vec_ok, ep,
                                                                slab_k, M, 1);
   KCH_LAUNCH_OK();
   return KCH_OK;
@@ -724,7 +856,13 @@ static int launch_tg_pair(const void* A, const void* W, void* C, const void* R, 
   int pairs = (int)(tiles < max_pairs ? tiles : max_pairs);
   cfg.gridDim = dim3(2 * pairs);
   int vec_ok = (ldc % 8 == 0) && (((uintptr_t)C & 15) == 0) && (!R || ((ldr % 8 == 0) && (((uintptr_t)R & 15) == 0)));
-  KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, true>, ma, mw, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
+  // bulk-tensor stores (and loads of a residual) want 16-byte-aligned rows with a pitch of whole 16 bytes
+  int c_bulk = vec_ok && M <= 0x7FFFFFFFLL - 512;
+  CUtensorMap mc = ma, mr = ma;
+  if (c_bulk && (make_map_2d(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64) ||
+                 (R && make_map_2d(&mr, R, (uint64_t)M, (uint64_t)N, (uint64_t)ldr, 32, 64))))
+    c_bulk = 0;
+  KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, true>, ma, mw, mc, mr, c_bulk, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
                                  vec_ok, ep, slab_k, M, 1));
   kch_note_launch(1);
   return KCH_OK;

@@ -142,3 +142,46 @@ def test_decode_attention_split_or_cluster(kch, B, nb, topk, quant):
     want = ref.step(q, qi, wi, topk=topk, sink_logits=sink, scale=1.0)
     assert (sel.sort(-1).values[:, 0, 1:] > sel.sort(-1).values[:, 0, :-1]).all()
     assert md(out, want) <= (2e-3 if quant else 2e-4), md(out, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(512, 136, 64), (513, 264, 128), (700, 776, 2048), (1153, 2304, 128), (640, 1016, 192)])
+def test_large_gemm_bulk_store_edges(kch, M, N, K):
+    """The bulk-tensor store clips rows beyond M and columns beyond N of a 256 x 256 tile; nothing around C is touched.  Products
+    within one bf16 rounding of the 64-bit value."""
+    from kch_b200 import _lib
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x, W = torch.randn(M, K, generator=g, device=DEV).bfloat16(), (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    ref = x.double() @ W.double().T
+    for ldc in (N, N + 24):
+        C = torch.full((M + 2, ldc), 7.0, device=DEV, dtype=torch.bfloat16)
+        lib = _lib.load()
+        _lib.check(lib.kch_linear(_lib.ptr(x), _lib.ptr(W), C.data_ptr() + 2 * ldc, None, M, N, K, K, K, ldc, 0, _lib.KCH_BF16,
+                                  _lib.stream()))
+        got = C[1:-1, :N].double()
+        assert bool(((got - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()), md(got, ref)
+        assert bool((C[0] == 7).all() and (C[-1] == 7).all() and (C[1:-1, N:] == 7).all())
+
+
+@pytest.mark.parametrize("M,N", [(520, 520), (1100, 400)])
+def test_large_gemm_residual_and_activation_edges(kch, M, N):
+    """Residual tiles arrive and leave by the copy engine; 128-column groups of one activation take its epilogue, mixed ones the
+    general loop.  Product, activation and sum each round once to bf16."""
+    from kch_b200 import _lib
+    from kch_b200.csa import linear
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, W = torch.randn(M, 256, generator=g, device=DEV).bfloat16(), (torch.randn(N, 256, generator=g, device=DEV) / 16).bfloat16()
+    R = torch.randn(M, N + 8, generator=g, device=DEV).bfloat16()[:, :N]
+    p = (x.double() @ W.double().T).bfloat16().double()
+    y = linear(x, W, residual=R)
+    assert bool(((y.double() - (p + R.double())).abs() <= 2 ** -7 * (p.abs() + R.double().abs()) + 1e-5).all())
+    segs = [(128, _lib.ACT_SILU_L2NORM, 0.0), (160, _lib.ACT_SILU, 0.0), (N - 288 - 16, 0, 0.0), (16, _lib.ACT_SIGMOID, 0.0)]
+    if (N - 16) % 32:
+        segs = [(128, _lib.ACT_SILU_L2NORM, 0.0), (160, _lib.ACT_SILU, 0.0), (N - 288, _lib.ACT_SIGMOID, 0.0)]
+    y = linear(x, W, epilogue=segs, group=128)
+    h = torch.nn.functional.silu(p[:, :128]).bfloat16().double()
+    want = [h / h.norm(dim=-1, keepdim=True).bfloat16().double(), torch.nn.functional.silu(p[:, 128:288])]
+    rest = p[:, 288:]
+    want.append(torch.cat([rest[:, :-16], torch.sigmoid(rest[:, -16:])], 1) if len(segs) == 4 else torch.sigmoid(rest))
+    want = torch.cat(want, 1)
+    # the fp32 product may round to the neighbouring bf16 value (2^-7 of it), then silu, norm and result round (2^-9 to 2^-8 each)
+    assert bool(((y.double() - want).abs() <= 2 ** -6 * want.abs() + 2e-3).all()), md(y, want)
