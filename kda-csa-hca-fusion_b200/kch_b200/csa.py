@@ -431,18 +431,20 @@ def naive_csa(H, W_aKV, W_bKV, W_aZ, W_bZ, Ba, Bb, W_DQ, W_UQ, W_IUQ, W_w, W_KV_
             raise ValueError("naive_csa: _q_rows and return_projections cannot be combined")
         H, T = H[:, :q_hi], q_hi
     original_T = T
-    pad = (-T) % m
+    # An incomplete last block is visible to no query, so only whole blocks are compressed and nothing is padded; a sequence
+    # shorter than one block (and a caller who wants the padded stages) is.
+    pad = (-T) % m if (T < m or _aux is not None) else 0
     if pad:
         H = torch.nn.functional.pad(H, (0, 0, 0, pad))
         T += pad
-    n_blocks = T // m
+    Tc = T // m * m
     if _fused_weight is None:
         _fused_weight = fuse_rows(W_aKV, W_bKV, W_aZ, W_bZ, W_KV_idx, W_Z_idx, W_DQ, W_w)
     proj = linear(H, _fused_weight)                                     # [B,T,4c+2cI+dc+nIh (+pad)]
     Ca, Cb, Za, Zb, K_idx_raw, Z_idx, cQ, w_idx = proj[..., :4 * c + 2 * c_I + dc + nIh].split(
         [c, c, c, c, c_I, c_I, dc, nIh], dim=-1)
-    C_comp = csa_compress_kv_overlapped(Ca, Cb, Za, Zb, Ba, Bb, m)      # [B,n,c] fp32
-    K_IComp = csa_compress_kv(K_idx_raw, Z_idx, B_idx, m)               # [B,n,cI] fp32
+    C_comp = csa_compress_kv_overlapped(Ca[:, :Tc], Cb[:, :Tc], Za[:, :Tc], Zb[:, :Tc], Ba, Bb, m)      # [B,n,c] fp32
+    K_IComp = csa_compress_kv(K_idx_raw[:, :Tc], Z_idx[:, :Tc], B_idx, m)                               # [B,n,cI] fp32
     W_q = _fused_q_weight if _fused_q_weight is not None else torch.cat([W_UQ, W_IUQ], dim=0)
     if q_lo:                                                            # the query side for this rank's rows only
         cQ, w_idx = cQ[:, q_lo:], w_idx[:, q_lo:]

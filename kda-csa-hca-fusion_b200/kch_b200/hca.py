@@ -63,7 +63,8 @@ def naive_hca(H, W_KV, W_Z, B_pos, W_DQ, W_UQ, *, m2: int, nh: int, c: int, dc: 
             raise ValueError("naive_hca: _q_rows and return_projections cannot be combined")
         H, T = H[:, :q_hi], q_hi
     original_T = T
-    pad = (-T) % m2
+    # an incomplete last block is visible to no query: only whole blocks are compressed (a sequence shorter than one is padded)
+    pad = (-T) % m2 if T < m2 else 0
     if pad:
         H = torch.nn.functional.pad(H, (0, 0, 0, pad))
         T += pad
@@ -76,7 +77,8 @@ def naive_hca(H, W_KV, W_Z, B_pos, W_DQ, W_UQ, *, m2: int, nh: int, c: int, dc: 
     else:
         C, Z, cQ = proj[..., :2 * c + dc].split([c, c, dc], dim=-1)
         C_loc = C
-    C_comp = csa_compress_kv(C, Z, B_pos, m2)
+    Tc = T // m2 * m2
+    C_comp = csa_compress_kv(C[:, :Tc], Z[:, :Tc], B_pos, m2)
     kdt = torch.bfloat16 if mma_attention_eligible(H.dtype, c, nh, True, scale) else torch.float32
     C_comp_n = rownorm(C_comp, True, kdt)
     q = linear(cQ[:, q_lo:] if q_lo else cQ, W_UQ)

@@ -185,3 +185,25 @@ def test_large_gemm_residual_and_activation_edges(kch, M, N):
     want = torch.cat(want, 1)
     # the fp32 product may round to the neighbouring bf16 value (2^-7 of it), then silu, norm and result round (2^-9 to 2^-8 each)
     assert bool(((y.double() - want).abs() <= 2 ** -6 * want.abs() + 2e-3).all()), md(y, want)
+
+
+@pytest.mark.parametrize("B,T,dtype", [(2, 131, "bf16"), (1, 517, "bf16"), (3, 130, "fp32"), (1, 9, "bf16"), (2, 3, "fp32")])
+def test_ragged_lengths_without_padding(kch, B, T, dtype):
+    """Lengths that are no multiple of a block (4 and 64 tokens) or of the indexer's query tile: same as the oracle, which pads.
+    Operator outputs within 2e-3 (bf16) / 2e-5 (fp32); CSA on the kernel's own selection."""
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    kw = dict(nh=8, c=128, dc=64, nIh=4, c_I=64, m=4)
+    w, sink, H = syn.csa_inputs(T, B, T, 256, **kw, dtype=dt, random_sink=True)
+    args = dict(kw, topk=24, sliding_window=16, normalize_qk=True)
+    dw = {k: v.to(DEV) for k, v in w.items()}
+    out, idx = kch.naive_csa(H.to(DEV), *dw.values(), **args, sink_logits=sink.to(DEV), use_ste=False, _return_indices=True)
+    ref = orc.csa_forward(H, *w.values(), **args, sink_logits=sink,
+                          indices_override=torch.cat([idx.long().cpu(), idx.new_full((B, -T % 4, 24), -1).long().cpu()], 1))
+    assert out.shape == ref.shape and md(out, ref) <= (4e-3 if dtype == "bf16" else 2e-5), md(out, ref)
+    vis = (torch.arange(T) + 1) // 4
+    assert bool(((idx.cpu() >= 0).sum(-1) == vis.clamp(max=24)).all()) and bool((idx.cpu() < vis[None, :, None].clamp(min=1)).all())
+    w, sink, H = syn.hca_inputs(T + 1, B, T, 256, nh=8, c=128, dc=64, m2=64, dtype=dt, random_sink=True)
+    kw = dict(m2=64, nh=8, c=128, dc=64, sliding_window=16)
+    out = kch.naive_hca(H.to(DEV), *(v.to(DEV) for v in w.values()), **kw, sink_logits=sink.to(DEV))
+    ref = orc.hca_forward(H, *w.values(), **kw, sink_logits=sink)
+    assert out.shape == ref.shape and md(out, ref) <= (4e-3 if dtype == "bf16" else 2e-5), md(out, ref)
