@@ -382,6 +382,16 @@ int kch_attend_decode_splits(int B);
 int64_t kch_attend_decode_workspace_bytes(int B, int nh, int c);
 int kch_attend_decode(const kch_attend_decode_args* args, void* stream);
 
+/* A run of `T` tokens at once (ops_decoding_cache.py:700-830): open accumulators, overlap partner, window ring and device
+ * counters, for the streams named in `args` (token t of sequence b at element b*bs_c + t*ld_c, K_idx / Z_idx at
+ * b*bs_i + t*ld_i; args->acc_len, n_blocks and has_prev as they were before).  The rows of the whole blocks are the
+ * caller's: kch_compress_kv(_overlapped) before this call, then kch_cache_store_rows (fp32 rows [B, n, c] into storage
+ * [B, capacity, c] from block `start` on, rounded to `dtype`, with their norms) or kch_quantize_rows. */
+int kch_cache_append_rows(const kch_cache_append_args* args, int64_t T, int64_t bs_c, int64_t bs_i, int64_t ring_n,
+                          int64_t tokens_seen, void* stream);
+int kch_cache_store_rows(const float* rows, int64_t n, int c, int B, void* dst, float* norms, int64_t capacity,
+                         int64_t start, int dtype, void* stream);
+
 /* Block-scaled 8-bit encoding of rows (no counterpart in the reference; it stores the cache dtype only):
  * payload [rows,c], scales [rows,c/64], norms [rows] = max(||dequantised row||, 1e-12). */
 int kch_quantize_rows(const void* x, int64_t ld, void* payload, float* scales, float* norms, int64_t rows,

@@ -329,3 +329,132 @@ extern "C" int kch_quantize_rows(const void* x, int64_t ld, void* payload, float
   KCH_LAUNCH_OK();
   return KCH_OK;
 }
+
+// =====================================================================================================================
+// A run of tokens appended at once (the prompt, or a chunk of it): everything beside the compression of the whole blocks.
+// One launch instead of two dozen copies, concatenations and index writes per cache, and the counters travel as kernel
+// arguments -- an upload of them from pageable memory made the host wait for the device twice per layer and chunk.
+//   part 0 .. 3 (5)  a projection stream (Ca, Cb, Za, Zb, K_idx, Z_idx): the last whole block of the b-branch becomes the
+//                    overlap partner of the next one, then the tokens behind the last whole block open the next
+//                    accumulator; a thread owns a channel, so it reads an old accumulator row before it writes it
+//   last part        the window ring: the last min(win, T) rows, normalised in fp32 (a warp per row)
+// Prompt of 3001 tokens in two chunks: host 3.36 -> 2.69 ms.
+// =====================================================================================================================
+struct BulkArgs {
+  const void* src[6];
+  void* acc[6];
+  void* prev[2];                       // b-branch rows of the last whole block (Cb, Zb)
+  int64_t ld[6], bs[6];                // elements between tokens / sequences
+  int width[6];
+  int parts, m, acc_len, normalize, win, c;
+  int64_t T, nb;                       // new tokens; whole blocks that they (with the open ones) complete
+  void* ring; int64_t ring_n;          // tokens the ring has seen
+  int32_t* ctr; int32_t ctr_new[KCH_CTR_WORDS];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256) cache_append_rows_kernel(BulkArgs a) {
+  const int b = blockIdx.x, part = blockIdx.y, tid = threadIdx.x;
+  if (part < a.parts) {
+    const T* src = (const T*)a.src[part] + (int64_t)b * a.bs[part];
+    const int w = a.width[part];
+    T* acc = (T*)a.acc[part] + (int64_t)b * a.m * w;
+    T* prev = (part == 1 || part == 3) && a.prev[part >> 1] ? (T*)a.prev[part >> 1] + (int64_t)b * a.m * w : nullptr;
+    for (int d = tid; d < w; d += 256) {
+      if (a.nb > 0) {
+        if (prev)
+          for (int j = 0; j < a.m; ++j) {
+            const int64_t t = (a.nb - 1) * a.m + j - a.acc_len;
+            prev[(int64_t)j * w + d] = t < 0 ? acc[(int64_t)(t + a.acc_len) * w + d] : src[t * a.ld[part] + d];
+          }
+        const int64_t t0 = a.nb * a.m - a.acc_len;
+        for (int64_t t = t0; t < a.T; ++t) acc[(t - t0) * w + d] = src[t * a.ld[part] + d];
+      } else {
+        for (int64_t t = 0; t < a.T; ++t) acc[(a.acc_len + t) * w + d] = src[t * a.ld[part] + d];
+      }
+    }
+  } else if (a.ring) {
+    const int warp = tid >> 5, lane = tid & 31;
+    const int64_t k = a.T < a.win ? a.T : a.win;
+    for (int64_t i = warp; i < k; i += 8) {
+      const int64_t t = a.T - k + i;
+      const T* row = (const T*)a.src[0] + (int64_t)b * a.bs[0] + t * a.ld[0];
+      T* dst = (T*)a.ring + ((int64_t)b * a.win + (a.ring_n + t) % a.win) * a.c;
+      float nrm = 1.f;
+      if (a.normalize) {
+        float ss = 0.f;
+        for (int d = lane; d < a.c; d += 32) { const float x = ldf(row + d); ss += x * x; }
+        nrm = fmaxf(sqrtf(warp_sum(ss)), 1e-12f);
+      }
+      for (int d = lane; d < a.c; d += 32) stf(dst + d, ldf(row + d) / nrm);
+    }
+  }
+  if (b == 0 && part == 0 && tid < KCH_CTR_WORDS) a.ctr[tid] = a.ctr_new[tid];
+}
+
+extern "C" int kch_cache_append_rows(const kch_cache_append_args* p, int64_t T, int64_t bs_c, int64_t bs_i, int64_t ring_n,
+                                     int64_t tokens_seen, void* stream) {
+  KCH_REQUIRE(p != nullptr && p->counters != nullptr, "kch_cache_append_rows: needs the cache's device counters");
+  KCH_REQUIRE(p->B >= 1 && p->c >= 1 && p->m >= 1 && T >= 1, "kch_cache_append_rows: B=%d c=%d m=%d T=%lld", p->B, p->c, p->m, (long long)T);
+  KCH_REQUIRE(p->acc_len >= 0 && p->acc_len < p->m, "acc_len=%d out of range for m=%d", p->acc_len, p->m);
+  KCH_REQUIRE(p->Ca && p->Za && p->acc_Ca && p->acc_Za, "kch_cache_append_rows: null projection or accumulator");
+  const bool overlap = p->Cb != nullptr;
+  BulkArgs a = {};
+  auto stream_of = [&](const void* src, void* acc, int64_t ld, int64_t bs, int width) {
+    a.src[a.parts] = src; a.acc[a.parts] = acc; a.ld[a.parts] = ld; a.bs[a.parts] = bs; a.width[a.parts] = width;
+    ++a.parts;
+  };
+  stream_of(p->Ca, p->acc_Ca, p->ld_c, bs_c, p->c);
+  if (overlap) stream_of(p->Cb, p->acc_Cb, p->ld_c, bs_c, p->c);
+  stream_of(p->Za, p->acc_Za, p->ld_c, bs_c, p->c);
+  if (overlap) stream_of(p->Zb, p->acc_Zb, p->ld_c, bs_c, p->c);
+  if (p->K_idx) {
+    stream_of(p->K_idx, p->acc_K_idx, p->ld_i, bs_i, p->c_I);
+    stream_of(p->Z_idx, p->acc_Z_idx, p->ld_i, bs_i, p->c_I);
+  }
+  a.m = p->m; a.acc_len = p->acc_len; a.normalize = p->normalize; a.win = p->win; a.c = p->c;
+  a.T = T; a.nb = (p->acc_len + T) / p->m;
+  if (overlap) { a.prev[0] = p->prev_Cb; a.prev[1] = p->prev_Zb; }
+  a.ring = p->win > 0 ? p->ring : nullptr; a.ring_n = ring_n;
+  a.ctr = const_cast<int32_t*>(p->counters);
+  a.ctr_new[KCH_CTR_ACC_LEN] = (int32_t)(p->acc_len + T - a.nb * p->m);
+  a.ctr_new[KCH_CTR_N_BLOCKS] = (int32_t)(p->n_blocks + a.nb);
+  a.ctr_new[KCH_CTR_RING_N] = p->win > 0 ? (int32_t)(ring_n + T) : 0;
+  a.ctr_new[KCH_CTR_HAS_PREV] = overlap && (p->has_prev || a.nb > 0);
+  a.ctr_new[KCH_CTR_TOKENS] = (int32_t)(tokens_seen + T);
+  const dim3 grid(p->B, a.parts + 1);
+  KCH_DISPATCH_FLOAT(p->dtype, T_, (cache_append_rows_kernel<T_><<<grid, 256, 0, kch_stream(stream)>>>(a)));
+  KCH_LAUNCH_OK();
+  return KCH_OK;
+}
+
+// Rows of fresh blocks (fp32) into a cache's storage at block `start`: rounded to the cache dtype, with the fp32 norm of the
+// rounded row; a warp per row.
+template <typename T>
+__global__ void __launch_bounds__(256) cache_store_rows_kernel(const float* __restrict__ rows, int64_t n, int c, int64_t total, T* dst,
+                                                               float* norms, int64_t cap, int64_t start) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= total) return;
+  const int64_t o = (r / n) * cap + start + r % n;
+  float ss = 0.f;
+  for (int d = lane; d < c; d += 32) {
+    const float x = round_to<T>(rows[r * c + d]);
+    stf(dst + o * c + d, x);
+    ss += x * x;
+  }
+  ss = warp_sum(ss);
+  if (lane == 0) norms[o] = fmaxf(sqrtf(ss), 1e-12f);
+}
+
+extern "C" int kch_cache_store_rows(const float* rows, int64_t n, int c, int B, void* dst, float* norms, int64_t capacity,
+                                    int64_t start, int dtype, void* stream) {
+  KCH_REQUIRE(rows && dst && norms && c >= 1 && B >= 1 && n >= 0 && start >= 0 && start + n <= capacity,
+              "kch_cache_store_rows: %lld rows at block %lld of %lld", (long long)n, (long long)start, (long long)capacity);
+  if (n == 0) return KCH_OK;
+  const int64_t total = (int64_t)B * n;
+  KCH_DISPATCH_FLOAT(dtype, T, (cache_store_rows_kernel<T><<<(unsigned)ceil_div64(total, 8), 256, 0, kch_stream(stream)>>>(
+      rows, n, c, total, (T*)dst, norms, capacity, start)));
+  KCH_LAUNCH_OK();
+  return KCH_OK;
+}

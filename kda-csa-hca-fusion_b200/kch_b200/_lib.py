@@ -99,6 +99,8 @@ PROTOTYPES = {
     "kch_attend_distinct": (_i, [C.POINTER(AttendArgs), _vp]),
     "kch_cache_append_token": (_i, [C.POINTER(CacheAppendArgs), _vp]),
     "kch_cache_append_token_advance": (_i, [C.POINTER(CacheAppendArgs), _vp]),
+    "kch_cache_append_rows": (_i, [C.POINTER(CacheAppendArgs), _i64, _i64, _i64, _i64, _i64, _vp]),
+    "kch_cache_store_rows": (_i, [_vp, _i64, _i, _i, _vp, _vp, _i64, _i64, _i, _vp]),
     "kch_quantize_rows": (_i, [_vp, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _vp]),
     "kch_cache_advance": (_i, [_vp, _i, _vp]),
     "kch_decode_indexer_workspace_bytes": (_i64, [_i, _i64]),

@@ -67,18 +67,6 @@ class _SlidingWindowRingBuffer:
         self._n += Tn
 
 
-def _row_norms(x):
-    """fp32 ``max(||row||, 1e-12)`` of ``x [B,n,c]`` (the divisor the kernels use for a stored row)."""
-    lib = _lib.load()
-    B, n, c = x.shape
-    x = x.contiguous()
-    out = torch.empty(B, n, dtype=torch.float32, device=x.device)
-    with _lib.device(x.device):
-        _lib.check(lib.kch_rownorm(_lib.ptr(x), c, None, _lib.ptr(out), B * n, c, _lib.dtype_tag(x.dtype), _lib.KCH_F32,
-                                   _lib.stream()))
-    return out
-
-
 class _CacheBase:
     # The counters live twice: Python ints (the reference's interface) and an int32 vector on the device that
     # the one-token kernels read, so that a decode step has no host argument that changes between tokens.
@@ -240,21 +228,75 @@ class _CacheBase:
         """rows ``[B,nb,c]`` fp32 -> storage at block offset ``start`` (+ norms of the stored rows)."""
         lib = _lib.load()
         B, nb, c = rows_f32.shape
+        if self._kind is None:
+            self._store_plain(rows_f32, start, self._comp, self._norms)
+            return
         r = rows_f32.to(self.dtype)
         tmp_norm = torch.empty(B, nb, dtype=torch.float32, device=self.device)
+        payload = torch.empty(B, nb, c, dtype=torch.uint8, device=self.device)
+        sc = torch.empty(B, nb, c // 64, dtype=torch.float32, device=self.device)
         with _lib.device(self.device):
-            if self._kind is None:
-                self._comp[:, start:start + nb] = r
-                _lib.check(lib.kch_rownorm(_lib.ptr(r), c, None, _lib.ptr(tmp_norm), B * nb, c,
-                                           _lib.dtype_tag(self.dtype), _lib.KCH_F32, _lib.stream()))
-            else:
-                payload = torch.empty(B, nb, c, dtype=torch.uint8, device=self.device)
-                sc = torch.empty(B, nb, c // 64, dtype=torch.float32, device=self.device)
-                _lib.check(lib.kch_quantize_rows(_lib.ptr(r), c, _lib.ptr(payload), _lib.ptr(sc), _lib.ptr(tmp_norm),
-                                                 B * nb, c, self._kind, _lib.dtype_tag(self.dtype), _lib.stream()))
-                self._comp[:, start:start + nb] = payload
-                self._scales[:, start:start + nb] = sc
+            _lib.check(lib.kch_quantize_rows(_lib.ptr(r), c, _lib.ptr(payload), _lib.ptr(sc), _lib.ptr(tmp_norm),
+                                             B * nb, c, self._kind, _lib.dtype_tag(self.dtype), _lib.stream()))
+        self._comp[:, start:start + nb] = payload
+        self._scales[:, start:start + nb] = sc
         self._norms[:, start:start + nb] = tmp_norm
+
+    def _store_plain(self, rows_f32, start, dst, norms):
+        rows_f32 = rows_f32.float().contiguous()
+        B, nb, c = rows_f32.shape
+        with _lib.device(self.device):
+            _lib.check(_lib.load().kch_cache_store_rows(_lib.ptr(rows_f32), nb, c, B, _lib.ptr(dst), _lib.ptr(norms), dst.shape[1],
+                                                        start, _lib.dtype_tag(self.dtype), _lib.stream()))
+
+    def _blocks_of(self, new, nb, m):
+        """The tokens of the ``nb`` blocks that ``new`` completes, per stream ``[B, nb*m, width]``: views of ``new`` unless
+        a block is open."""
+        if self._acc_len == 0:
+            return [x[:, :nb * m] for x in new]
+        return [torch.cat([a[:, :self._acc_len], x[:, :nb * m - self._acc_len]], dim=1) for a, x in zip(self._acc, new)]
+
+    def _append_rows(self, new, m, c_I):
+        """Open accumulators, overlap partner, window ring and counters after a run of tokens (one launch); the rows of its
+        whole blocks are stored already."""
+        T = new[0].shape[1]
+
+        def strides(group):          # one (token, sequence) stride pair per group of streams
+            pairs = {(x.stride(1) if T > 1 else x.shape[2], x.stride(0) if self.B > 1 else 0) for x in group}
+            if len(pairs) != 1 or any(x.stride(2) != 1 for x in group):
+                group = [x.contiguous() for x in group]
+                pairs = {(group[0].shape[2], T * group[0].shape[2])}
+            return group, *pairs.pop()
+
+        n_c = len(new) - (2 if c_I else 0)
+        rows_c, ld_c, bs_c = strides(new[:n_c])
+        rows_i, ld_i, bs_i = strides(new[n_c:]) if c_I else ([], 0, 0)
+        a = _lib.CacheAppendArgs()
+        a.B, a.c, a.c_I, a.m, a.win, a.dtype = self.B, self.c, c_I, m, self.win, _lib.dtype_tag(self.dtype)
+        a.ld_c, a.ld_i, a.acc_len, a.n_blocks = ld_c, ld_i, self._acc_len, self._n_blocks
+        p = [x.data_ptr() for x in rows_c + rows_i]
+        acc = [x.data_ptr() for x in self._acc]
+        if c_I:
+            a.Ca, a.Cb, a.Za, a.Zb, a.K_idx, a.Z_idx = p
+            a.acc_Ca, a.acc_Cb, a.acc_Za, a.acc_Zb, a.acc_K_idx, a.acc_Z_idx = acc
+            a.prev_Cb, a.prev_Zb, a.has_prev = self._prev[0].data_ptr(), self._prev[1].data_ptr(), int(self._has_prev)
+        else:
+            (a.Ca, a.Za), (a.acc_Ca, a.acc_Za) = p, acc
+        if self._sw is not None:
+            a.ring = self._sw._buf.data_ptr()
+        a.normalize = int(self._normalize_qk)
+        a.counters = self._ctr.data_ptr()
+        ring_n = 0 if self._sw is None else self._sw._n
+        with _lib.device(self.device):
+            _lib.check(_lib.load().kch_cache_append_rows(a, T, bs_c, bs_i, ring_n, self._n_tokens_seen, _lib.stream()))
+        total = self._acc_len + T
+        if self._sw is not None:
+            self._sw._n += T
+        self._n_blocks += total // m
+        self._acc_len = total % m
+        self._n_tokens_seen += T
+        if c_I and total // m:
+            self._has_prev = True
 
     def _dequant(self, nb):
         if self._comp is None:
@@ -424,36 +466,17 @@ class CSADecodingCache(_CacheBase):
         self._advance(m)
 
     def _append_many(self, new, biases):
-        m, T_new = self.m, new[0].shape[1]
-        if self._sw is not None:
-            tail = new[0][:, -self.win:]
-            keys = rownorm(tail, True).to(self.dtype) if self._normalize_qk else tail
-            self._sw._n += T_new - tail.shape[1]
-            self._sw.append(keys)
-        staged = [torch.cat([a[:, :self._acc_len], x], dim=1) for a, x in zip(self._acc, new)]
-        total = staged[0].shape[1]
-        nb = total // m
+        m = self.m
+        nb = (self._acc_len + new[0].shape[1]) // m
         if nb:
             self._grow(self._n_blocks + nb)
-            full = [s[:, :nb * m].contiguous() for s in staged]
+            full = self._blocks_of(new, nb, m)
             rows = csa_compress_kv_overlapped(full[0], full[1], full[2], full[3], biases[0], biases[1], m,
                                               prev_Cb=self._prev[0] if self._has_prev else None,
                                               prev_Zb=self._prev[1] if self._has_prev else None)
             self._store_rows(rows, self._n_blocks)
-            krows = csa_compress_kv(full[4], full[5], biases[2], m).to(self.dtype)
-            self._kcomp[:, self._n_blocks:self._n_blocks + nb] = krows
-            self._kcomp_norms[:, self._n_blocks:self._n_blocks + nb] = _row_norms(krows)
-            self._prev[0].copy_(full[1][:, -m:])
-            self._prev[1].copy_(full[3][:, -m:])
-            self._has_prev = True
-            self._n_blocks += nb
-        rest = total - nb * m
-        for a, s in zip(self._acc, staged):
-            if rest:
-                a[:, :rest] = s[:, nb * m:]
-        self._acc_len = rest
-        self._n_tokens_seen += T_new
-        self._sync_counters()
+            self._store_plain(csa_compress_kv(full[4], full[5], biases[2], m), self._n_blocks, self._kcomp, self._kcomp_norms)
+        self._append_rows(new, m, self.c_I)
 
     # ---- attend -----------------------------------------------------------------------------------------
     def forward_step(self, q, q_idx, w_idx, *, topk, nh, nIh, scale=None, sink_logits=None, use_ste=True,
@@ -651,27 +674,13 @@ class HCADecodingCache(_CacheBase):
         self._advance(m)
 
     def _append_many(self, new, bias):
-        m, T_new = self.m2, new[0].shape[1]
-        if self._sw is not None:
-            tail = new[0][:, -self.win:]
-            keys = rownorm(tail, True).to(self.dtype) if self._normalize_qk else tail
-            self._sw._n += T_new - tail.shape[1]
-            self._sw.append(keys)
-        staged = [torch.cat([a[:, :self._acc_len], x], dim=1) for a, x in zip(self._acc, new)]
-        total = staged[0].shape[1]
-        nb = total // m
+        m = self.m2
+        nb = (self._acc_len + new[0].shape[1]) // m
         if nb:
             self._grow(self._n_blocks + nb)
-            full = [s[:, :nb * m].contiguous() for s in staged]
+            full = self._blocks_of(new, nb, m)
             self._store_rows(csa_compress_kv(full[0], full[1], bias, m), self._n_blocks)
-            self._n_blocks += nb
-        rest = total - nb * m
-        for a, s in zip(self._acc, staged):
-            if rest:
-                a[:, :rest] = s[:, nb * m:]
-        self._acc_len = rest
-        self._n_tokens_seen += T_new
-        self._sync_counters()
+        self._append_rows(new, m, 0)
 
     def forward_step(self, q, *, nh, scale=None, sink_logits=None, normalize_qk=True, _q_normalize=False,
                      _out_dtype=None):

@@ -207,3 +207,46 @@ def test_ragged_lengths_without_padding(kch, B, T, dtype):
     out = kch.naive_hca(H.to(DEV), *(v.to(DEV) for v in w.values()), **kw, sink_logits=sink.to(DEV))
     ref = orc.hca_forward(H, *w.values(), **kw, sink_logits=sink)
     assert out.shape == ref.shape and md(out, ref) <= (4e-3 if dtype == "bf16" else 2e-5), md(out, ref)
+
+
+@pytest.mark.parametrize("B,win,quant,dtype,runs", [(1, 8, None, "bf16", (3, 2, 40, 3, 2)), (3, 5, "int8", "bf16", (1, 7, 3, 6)),
+                                                    (2, 16, None, "fp32", (2, 130, 2, 9)), (2, 0, "fp8", "bf16", (5, 11))])
+def test_bulk_append_leaves_the_cache_of_the_oracle(kch, B, win, quant, dtype, runs):
+    """Runs that close no, one or many blocks, with and without an open one, shorter and longer than the window: what is copied
+    is the same to the bit, rows within one rounding of the storage dtype (fp32: 4 ulp of the softmax sums)."""
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    c, cI, m, m2 = 128, 64, 4, 8
+    rel = 2 ** -7 if dt == torch.bfloat16 else 2e-6          # neighbouring bf16 values are up to 2^-7 of the value apart
+    g = torch.Generator().manual_seed(B)
+    Ba, Bb, Bi, Bh = (torch.randn(r, x, generator=g).mul(0.1).to(dt) for r, x in ((m, c), (m, c), (m, cI), (m2, c)))
+    csa, hca = kch.CSADecodingCache(B, c, cI, m, win, DEV, dt, kv_quant=quant), kch.HCADecodingCache(B, c, m2, win, DEV, dt, kv_quant=quant)
+    rc, rh = orc.CSACacheOracle(B, c, cI, m, win, dt, quant), orc.HCACacheOracle(B, c, m2, win, dt, quant)
+    for i, T in enumerate(runs):
+        wide = torch.randn(B, T, 4 * c + 2 * cI, generator=g).to(dt)         # slices of one projection, as a module passes them
+        if i % 2:
+            wide = wide.transpose(0, 1).contiguous().transpose(0, 1)
+        dev = wide.to(DEV)
+        csa.append_step(*dev.split([c] * 4 + [cI] * 2, -1), *(x.to(DEV) for x in (Ba, Bb, Bi)))
+        rc.append(*wide.split([c] * 4 + [cI] * 2, -1), Ba, Bb, Bi)
+        hca.append_step(dev[..., :c], dev[..., 2 * c:3 * c], Bh.to(DEV))
+        rh.append(wide[..., :c], wide[..., 2 * c:3 * c], Bh)
+        for cache, ref, mm in ((csa, rc, m), (hca, rh, m2)):
+            st, nb, rest = cache.export_state(), ref.tokens // mm, ref.tokens % mm
+            assert (st["n_blocks"], st["acc_len"], st["n_tokens_seen"]) == (nb, rest, ref.tokens)
+            assert cache._ctr.tolist()[:5] == [rest, nb, ref.tokens if win else 0, int(cache is csa and nb > 0), ref.tokens]
+            assert all(torch.equal(a[:, :rest].cpu(), r) for a, r in zip(st["acc"], ref.acc))
+            if win:
+                k = min(win, ref.tokens)
+                slots = torch.arange(ref.tokens - k, ref.tokens) % win
+                got, want = st["ring"].cpu()[:, slots].float(), ref.window.float()
+                assert bool(((got - want).abs() <= rel * want.abs() + 1e-7).all())
+            if nb:
+                if not quant:
+                    got, want = st["comp"].cpu().float(), ref.C_comp.float()
+                    assert bool(((got - want).abs() <= rel * want.abs() + 2e-6).all()), md(got, want)
+                    assert bool(((st["norms"].cpu() - got.norm(dim=-1)).abs() <= 2e-6 * st["norms"].cpu()).all())
+                if cache is csa:
+                    assert torch.equal(st["prev"][0].cpu(), ref.prev_Cb) and torch.equal(st["prev"][1].cpu(), ref.prev_Zb)
+                    got, want = st["kcomp"].cpu().float(), ref.K_IComp.float()
+                    assert bool(((got - want).abs() <= rel * want.abs() + 2e-6).all())
+                    assert bool(((st["kcomp_norms"].cpu() - got.norm(dim=-1)).abs() <= 2e-6 * got.norm(dim=-1)).all())
