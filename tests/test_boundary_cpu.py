@@ -203,3 +203,61 @@ def test_bench_accounting():
     nbytes = bench.decode_state_bytes(bench.C4, 64, 131072, 2)
     assert 0.80e9 < nbytes < 0.90e9          # indexer keys counted at their stored width (bf16 + fp32 norm per row)
     assert bench.decode_state_bytes(bench.C4, 64, 131072, 1.0625) < nbytes
+
+
+def _cpu_cache(cls, **fields):
+    """A cache object without its CUDA requirement: enough for what append_step decides on the host."""
+    cache = object.__new__(cls)
+    cache.__dict__.update(B=2, c=8, win=4, device=torch.device("cpu"), dtype=torch.float32, kv_quant=None, _kind=None,
+                          _normalize_qk=True, **fields)
+    cache.reset()
+    return cache
+
+
+@pytest.mark.parametrize("T", [1, 5])
+@pytest.mark.parametrize("cut", ["narrow", "wide", "batch of one", "larger batch", "flat"])
+def test_append_refuses_a_stream_of_another_shape(T, cut):
+    """The append kernels read every stream with the width and batch of the cache: a stream of another shape is refused before
+    anything is grown or stored, and so is a bias with fewer rows than a block."""
+    import kch_b200
+    x = lambda w: torch.zeros(2, T, w)  # noqa: E731
+
+    def bad(t):
+        return {"narrow": t[..., :-1], "wide": torch.cat([t, t], -1), "batch of one": t[:1], "larger batch": torch.cat([t, t]),
+                "flat": t.flatten(1)[:, None].expand(-1, T, -1)[..., :1]}[cut]
+    csa = _cpu_cache(kch_b200.CSADecodingCache, c_I=4, m=4)
+    biases = [torch.zeros(4, 8), torch.zeros(4, 8), torch.zeros(4, 4)]
+    for i in range(1, 6):
+        streams = [x(8)] * 4 + [x(4)] * 2
+        streams[i] = bad(streams[i])
+        with pytest.raises(ValueError):
+            csa.append_step(*streams, *biases)
+    for i in range(3):
+        with pytest.raises(ValueError, match="must hold"):
+            csa.append_step(*[x(8)] * 4, *[x(4)] * 2, *(b[:-1] if i == j else b for j, b in enumerate(biases)))
+    hca = _cpu_cache(kch_b200.HCADecodingCache, m2=4)
+    with pytest.raises(ValueError):
+        hca.append_step(x(8), bad(x(8)), torch.zeros(4, 8))
+    with pytest.raises(ValueError, match="must hold"):
+        hca.append_step(x(8), x(8), torch.zeros(3, 8))
+    for cache in (csa, hca):
+        assert (cache._n_tokens_seen, cache._n_blocks, cache._acc_len, cache._comp) == (0, 0, 0, None)
+
+
+def test_compression_refuses_streams_of_different_shapes():
+    import kch_b200
+    C, b = torch.zeros(2, 8, 6), torch.zeros(4, 6)
+    for other in (C[:1], C[..., :5], C[:, :4]):
+        with pytest.raises(ValueError, match="shape"):
+            kch_b200.csa_compress_kv(C, other, b, 4)
+        for i in range(3):
+            streams = [C, C, C]
+            streams[i] = other
+            with pytest.raises(ValueError, match="shape"):
+                kch_b200.csa_compress_kv_overlapped(C, *streams, b, b, 4)
+    with pytest.raises(ValueError, match="must hold"):
+        kch_b200.csa_compress_kv(C, C, b[:3], 4)
+    with pytest.raises(ValueError, match="must hold"):
+        kch_b200.csa_compress_kv_overlapped(C, C, C, C, b, b[:3], 4)
+    with pytest.raises(ValueError, match="prev_Cb"):
+        kch_b200.csa_compress_kv_overlapped(C, C, C, C, b, b, 4, prev_Cb=C[:, :3], prev_Zb=C[:, :4])
