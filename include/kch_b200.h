@@ -384,7 +384,8 @@ int kch_attend_decode(const kch_attend_decode_args* args, void* stream);
 
 /* A run of `T` tokens at once (ops_decoding_cache.py:700-830): open accumulators, overlap partner, window ring and device
  * counters, for the streams named in `args` (token t of sequence b at element b*bs_c + t*ld_c, K_idx / Z_idx at
- * b*bs_i + t*ld_i; args->acc_len, n_blocks and has_prev as they were before).  The rows of the whole blocks are the
+ * b*bs_i + t*ld_i; args->acc_len, n_blocks and has_prev as they were before).  Cb comes with Zb, both accumulators and both
+ * prev tensors, K_idx with Z_idx and both accumulators, win > 0 with the ring; anything less is refused.  The rows of the whole blocks are the
  * caller's: kch_compress_kv(_overlapped) before this call, then kch_cache_store_rows (fp32 rows [B, n, c] into storage
  * [B, capacity, c] from block `start` on, rounded to `dtype`, with their norms) or kch_quantize_rows. */
 int kch_cache_append_rows(const kch_cache_append_args* args, int64_t T, int64_t bs_c, int64_t bs_i, int64_t ring_n,

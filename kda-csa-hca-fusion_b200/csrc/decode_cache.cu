@@ -399,6 +399,16 @@ extern "C" int kch_cache_append_rows(const kch_cache_append_args* p, int64_t T, 
   KCH_REQUIRE(p->acc_len >= 0 && p->acc_len < p->m, "acc_len=%d out of range for m=%d", p->acc_len, p->m);
   KCH_REQUIRE(p->Ca && p->Za && p->acc_Ca && p->acc_Za, "kch_cache_append_rows: null projection or accumulator");
   const bool overlap = p->Cb != nullptr;
+  KCH_REQUIRE(overlap ? p->Zb && p->acc_Cb && p->acc_Zb && p->prev_Cb && p->prev_Zb : !p->Zb,
+              "kch_cache_append_rows: Cb goes with Zb, acc_Cb, acc_Zb, prev_Cb and prev_Zb");
+  KCH_REQUIRE(p->K_idx ? p->Z_idx && p->acc_K_idx && p->acc_Z_idx && p->c_I >= 1 : !p->Z_idx,
+              "kch_cache_append_rows: K_idx goes with Z_idx, acc_K_idx, acc_Z_idx and c_I >= 1");
+  KCH_REQUIRE(p->win >= 0 && (p->win == 0 || p->ring), "kch_cache_append_rows: win=%d needs its ring", p->win);
+  KCH_REQUIRE(p->ld_c >= 0 && p->ld_i >= 0 && bs_c >= 0 && bs_i >= 0, "kch_cache_append_rows: negative stride");
+  const int64_t most = 0x7FFFFFFFLL - T;               // the counters are 32-bit words
+  KCH_REQUIRE(T <= 0x7FFFFFFFLL && p->n_blocks >= 0 && ring_n >= 0 && tokens_seen >= 0 && p->n_blocks <= most && ring_n <= most &&
+                  tokens_seen <= most, "kch_cache_append_rows: counters out of range (n_blocks=%d ring_n=%lld tokens_seen=%lld T=%lld)",
+              p->n_blocks, (long long)ring_n, (long long)tokens_seen, (long long)T);
   BulkArgs a = {};
   auto stream_of = [&](const void* src, void* acc, int64_t ld, int64_t bs, int width) {
     a.src[a.parts] = src; a.acc[a.parts] = acc; a.ld[a.parts] = ld; a.bs[a.parts] = bs; a.width[a.parts] = width;

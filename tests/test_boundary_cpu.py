@@ -261,3 +261,36 @@ def test_compression_refuses_streams_of_different_shapes():
         kch_b200.csa_compress_kv_overlapped(C, C, C, C, b, b[:3], 4)
     with pytest.raises(ValueError, match="prev_Cb"):
         kch_b200.csa_compress_kv_overlapped(C, C, C, C, b, b, 4, prev_Cb=C[:, :3], prev_Zb=C[:, :4])
+
+
+def test_bulk_append_refuses_incomplete_arguments():
+    """kch_cache_append_rows: what one stream needs is there, or the call is refused on the host (the pointers below are never
+    followed: every call is wrong in one respect)."""
+    from kch_b200 import _lib
+    lib = _lib.load()
+
+    def call(T=4, ring_n=0, seen=0, bs_c=32, **change):
+        a = _lib.CacheAppendArgs()
+        a.B, a.c, a.c_I, a.m, a.win, a.dtype, a.ld_c, a.ld_i = 1, 8, 4, 4, 4, _lib.KCH_F32, 8, 4
+        for name in ("Ca Cb Za Zb K_idx Z_idx acc_Ca acc_Cb acc_Za acc_Zb acc_K_idx acc_Z_idx prev_Cb prev_Zb ring counters").split():
+            setattr(a, name, 4096)
+        for name, value in change.items():
+            setattr(a, name, value)
+        rc = lib.kch_cache_append_rows(a, T, bs_c, 16, ring_n, seen, None)
+        return rc, lib.kch_last_error().decode()
+    for name in "Zb acc_Cb acc_Zb prev_Cb prev_Zb Cb".split():
+        rc, why = call(**{name: None})
+        assert rc < 0 and "Cb goes with" in why, (name, why)
+    for name in "Z_idx acc_K_idx acc_Z_idx K_idx".split():
+        rc, why = call(**{name: None})
+        assert rc < 0 and "K_idx goes with" in why, (name, why)
+    rc, why = call(c_I=0)
+    assert rc < 0 and "c_I" in why
+    rc, why = call(ring=None)
+    assert rc < 0 and "ring" in why
+    for kw in (dict(ld_c=-8), dict(ld_i=-1), dict(bs_c=-1)):
+        rc, why = call(**kw)
+        assert rc < 0 and "stride" in why, why
+    for kw in (dict(seen=2 ** 31 - 4), dict(ring_n=2 ** 31 - 4), dict(n_blocks=2 ** 31 - 2), dict(T=2 ** 31), dict(seen=-1)):
+        rc, why = call(**kw)
+        assert rc < 0 and "out of range" in why, (kw, why)
