@@ -342,7 +342,7 @@ def attend(q, comp, *, nh, c, sel=None, m=0, t0=0, n_visible=-1, q_normalize=Fal
     lib = _lib.load()
     B, T = q.shape[0], q.shape[1]
     a = _lib.AttendArgs()
-    q3, qld, qbsr = _as_rows(q if q.dim() == 3 else q.reshape(B, T, nh * c))
+    q3, qld, qbsr = _as_rows(q if q.dim() == 3 and q.shape[2] == nh * c else q.reshape(B, T, nh * c))
     if qbsr != T:
         q3 = q3.contiguous()
         qld = nh * c

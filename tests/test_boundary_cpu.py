@@ -294,3 +294,12 @@ def test_bulk_append_refuses_incomplete_arguments():
     for kw in (dict(seen=2 ** 31 - 4), dict(ring_n=2 ** 31 - 4), dict(n_blocks=2 ** 31 - 2), dict(T=2 ** 31), dict(seen=-1)):
         rc, why = call(**kw)
         assert rc < 0 and "out of range" in why, (kw, why)
+
+
+def test_attend_refuses_queries_of_another_width():
+    """The kernels read nh * c query channels per token (naive_hca with a W_UQ of fewer rows arrives here)."""
+    from kch_b200.csa import attend
+    comp = torch.zeros(1, 2, 8)
+    for q in (torch.zeros(1, 3, 24), torch.zeros(1, 3, 40), torch.zeros(1, 3, 3, 8)):
+        with pytest.raises(RuntimeError, match="shape"):
+            attend(q, comp, nh=4, c=8, m=1, q_normalize=True)
