@@ -41,13 +41,12 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
                           const void* w, int w_dtype, int64_t w_ld, float* logits, int64_t cap, int64_t n_ld, int HI,
                           int normalize, float scale, int m, const int32_t* ctr, int cta_rows, unsigned int* status) {
   chain_wait();
-  chain_trigger();
   extern __shared__ uint8_t ixd_raw[];
   IxdSmem& sm = *reinterpret_cast<IxdSmem*>(((uintptr_t)ixd_raw + 1023) & ~(uintptr_t)1023);
   const int b = blockIdx.y, tid = threadIdx.x, warp = t5_warp_index(), lane = tid & 31;
   const int nvis = min(ctr[KCH_CTR_TOKENS] / m, ctr[KCH_CTR_N_BLOCKS]);
   const int r0 = blockIdx.x * cta_rows;
-  if (r0 >= nvis) return;                                      // the whole CTA, before any barrier or allocation
+  if (r0 >= nvis) return;                                      // the whole CTA, before any barrier or allocation (and so triggered)
   const int ntiles = min(cta_rows / IXD_TILE, (nvis - r0 + IXD_TILE - 1) / IXD_TILE);
 
   if (tid == 0) {
@@ -76,6 +75,7 @@ decode_indexer_tc5_kernel(const __grid_constant__ CUtensorMap kmap, const void* 
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   __syncthreads();
+  chain_trigger();                                             // after the allocation (see kch_launch_chained)
   // 32 rows x 8 chunks of 16 bytes: row = term * 8 + head, chunk c holds elements 8c .. 8c+7 of that head's term
   for (int i = tid; i < 32 * 8; i += IXD_THREADS) {
     const int row = i >> 3, ch = i & 7, term = row >> 3, h = row & 7;

@@ -78,7 +78,9 @@ __device__ __forceinline__ float ld_any(const void* p, int64_t i, int dtype) {
 // as much as some of them.  kch_launch_chained lets a kernel start while the one before it drains.  Such a kernel calls
 // chain_wait() in every thread before it touches anything an earlier launch may still write or read: the call returns
 // when all earlier launches have completed and their stores are visible.  chain_trigger() (after the wait, so that a
-// kernel's start implies that everything before its predecessor is complete) lets the next one start.  Both are no-ops in
+// kernel's start implies that everything before its predecessor is complete) lets the next one start.  A kernel that takes
+// tensor memory triggers after it holds it: the next kernel may take its own before its wait, and a CTA still waiting for
+// columns that the next kernel holds, which in turn waits for that CTA, would wait for good.  Both are no-ops in
 // a kernel launched the ordinary way.  Inputs are not `const __restrict__` there: such loads could be moved above the wait.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -303,3 +303,16 @@ def test_attend_refuses_queries_of_another_width():
     for q in (torch.zeros(1, 3, 24), torch.zeros(1, 3, 40), torch.zeros(1, 3, 3, 8)):
         with pytest.raises(RuntimeError, match="shape"):
             attend(q, comp, nh=4, c=8, m=1, q_normalize=True)
+
+
+def test_chained_kernels_take_tensor_memory_before_they_trigger():
+    """A kernel started early may allocate tensor memory before its wait, so the kernel before it has to hold its own by then:
+    in every kernel with both, no trigger stands before the allocation."""
+    csrc = os.path.join(ROOT, "kda-csa-hca-fusion_b200", "csrc")
+    both = []
+    for name in sorted(os.listdir(csrc)):
+        for body in open(os.path.join(csrc, name)).read().split("__global__")[1:]:
+            if "chain_trigger()" in body and "tcgen05.alloc" in body:
+                both.append(name)
+                assert body.index("chain_trigger()") > body.index("tcgen05.alloc"), name
+    assert both == ["gemm_decode.cu", "indexer_decode_tc5.cu"]
