@@ -212,17 +212,26 @@ class _FusedWeights:
     """Row-concatenated copy of several weight matrices, rebuilt when the sources move or change dtype."""
 
     def __init__(self):
-        self._key = None
-        self._w = None
-        self.settled = False            # the last `get` launched nothing: the copy was there already
+        self._fused = (None, None)      # (key, copy), replaced as one: other threads may be reading
 
     def get(self, *weights):
+        return self.get_settled(*weights)[0]
+
+    def get_settled(self, *weights):
+        """``(copy, settled)``; ``settled``: this call launched nothing, the copy was there already."""
         key = tuple((w.data_ptr(), w.dtype, w.device, w._version) for w in weights)
-        self.settled = key == self._key
-        if not self.settled:
-            self._w = fuse_rows(*weights)
-            self._key = key
-        return self._w
+        have, w = self._fused
+        if key == have:
+            return w, True
+        w = fuse_rows(*weights)
+        self._fused = (key, w)
+        return w, False
+
+
+def _at_rest(w):
+    """Is ``w`` a parameter as it lies?  A parametrised weight is computed by the access itself, so the launch just before
+    the product writes it."""
+    return type(w) is nn.Parameter
 
 
 class KDAHybridLayer(nn.Module):
@@ -297,21 +306,21 @@ class KDAHybridLayer(nn.Module):
             else:
                 prev = lb if lb is not None else x.new_zeros(B, 2, d)
                 new_lb = torch.cat([prev.to(x.dtype), x], dim=1)[:, -2:].clone()
-        W = self._fused.get(self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.g_down.weight,
-                            self.beta.weight)
+        W, settled = self._fused.get_settled(self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.g_down.weight,
+                                             self.beta.weight)
         # one GEMM for q|k|v|g_down|beta with the activations of ops_fused.py:571-581 applied in its epilogue
         # (silu + per-head L2 norm, silu, none, sigmoid); q, k, v, beta stay column slices of its output
         n_used = 2 * H * K + HV * V + K + HV
         segs = [(H * K, _lib.ACT_SILU_L2NORM, 0.0), (H * K, _lib.ACT_SILU_L2NORM, 0.0), (HV * V, _lib.ACT_SILU, 0.0),
                 (K, 0, 0.0), (HV + (W.shape[0] - n_used), _lib.ACT_SIGMOID, 0.0)]
         # in a one-token step the kernel before each projection is one of ours, which produced its input
-        proj = linear(xc, W, epilogue=segs, group=K, w_settled=fused_step and self._fused.settled)
+        proj = linear(xc, W, epilogue=segs, group=K, w_settled=fused_step and settled)
         q, k, v, gd, beta = proj[..., :n_used].split([H * K, H * K, HV * V, K, HV], dim=-1)
+        W = self.g_up.weight
         if raw_gate:     # the chunk kernel applies -softplus(.) * decay_scale when it loads the gate
-            g = linear(gd, self.g_up.weight)
+            g = linear(gd, W)
         else:
-            g = linear(gd, self.g_up.weight, epilogue=[(HV * K, _lib.ACT_NEG_SOFTPLUS, cfg.kda_decay_scale)],
-                       w_settled=fused_step)
+            g = linear(gd, W, epilogue=[(HV * K, _lib.ACT_NEG_SOFTPLUS, cfg.kda_decay_scale)], w_settled=fused_step and _at_rest(W))
         return (q.unflatten(-1, (H, K)), k.unflatten(-1, (H, K)), v.unflatten(-1, (HV, V)),
                 g.view(B, T, HV, K), beta, new_lb)
 
@@ -328,8 +337,9 @@ class KDAHybridLayer(nn.Module):
                                    output_final_state=True, chunk_size=cfg.kda_chunk_size, use_chunk=use_chunk,
                                    backend=cfg.kda_backend, state_out=None if use_chunk else state_out,
                                    gate_scale=cfg.kda_decay_scale if raw_gate else None)
-        out = out_projection(o.reshape(B, T, HV * V), self.tp, self.o_proj.weight, residual=residual,
-                             w_settled=T == 1 and lookback_in_place)
+        W = self.o_proj.weight
+        out = out_projection(o.reshape(B, T, HV * V), self.tp, W, residual=residual,
+                             w_settled=T == 1 and lookback_in_place and _at_rest(W))
         return out, new_state, new_lb
 
 
@@ -382,12 +392,18 @@ class CSAHybridLayer(nn.Module):
         self._fused = _FusedWeights()
         self._fused_q = _FusedWeights()
 
+    def q_weight_settled(self):
+        return self._fused_q.get_settled(self.W_UQ.weight, self.W_IUQ.weight)
+
+    def fused_weight_settled(self):
+        return self._fused.get_settled(self.W_aKV.weight, self.W_bKV.weight, self.W_aZ.weight, self.W_bZ.weight,
+                                       self.W_KV_idx.weight, self.W_Z_idx.weight, self.W_DQ.weight, self.W_w.weight)
+
     def q_weight(self):
-        return self._fused_q.get(self.W_UQ.weight, self.W_IUQ.weight)
+        return self.q_weight_settled()[0]
 
     def fused_weight(self):
-        return self._fused.get(self.W_aKV.weight, self.W_bKV.weight, self.W_aZ.weight, self.W_bZ.weight,
-                               self.W_KV_idx.weight, self.W_Z_idx.weight, self.W_DQ.weight, self.W_w.weight)
+        return self.fused_weight_settled()[0]
 
     def core(self, x, *, return_projections=False, q_rows=None):
         cfg = self.cfg
@@ -422,8 +438,11 @@ class HCAHybridLayer(nn.Module):
         self.tp = None
         self._fused = _FusedWeights()
 
+    def fused_weight_settled(self):
+        return self._fused.get_settled(self.W_KV.weight, self.W_Z.weight, self.W_DQ.weight)
+
     def fused_weight(self):
-        return self._fused.get(self.W_KV.weight, self.W_Z.weight, self.W_DQ.weight)
+        return self.fused_weight_settled()[0]
 
     def core(self, x, *, return_projections=False, q_rows=None):
         cfg = self.cfg
@@ -686,7 +705,8 @@ class HybridDecoding(nn.Module):
     def _project_out(self, layer, o_core, residual, B, T):
         if _rows_mode(layer.tp):
             return out_projection_rows(o_core, layer.tp, layer.o_proj.weight, residual, lead=(B, T))
-        return out_projection(o_core, layer.tp, layer.o_proj.weight, residual=residual, w_settled=T == 1)
+        W = layer.o_proj.weight
+        return out_projection(o_core, layer.tp, W, residual=residual, w_settled=T == 1 and _at_rest(W))
 
     def _csa(self, i, layer, h, residual):
         cfg = self.cfg
@@ -701,12 +721,12 @@ class HybridDecoding(nn.Module):
             cache.append_step(*proj, layer.Ba, layer.Bb, layer.B_idx)
         else:
             c, cI, dc, nIh, nh = cfg.csa_c, cfg.csa_cI, cfg.csa_dc, cfg.csa_nIh, cfg.csa_nh
-            W = layer.fused_weight()
-            proj = linear(h, W, w_settled=layer._fused.settled)
+            W, settled = layer.fused_weight_settled()
+            proj = linear(h, W, w_settled=settled)
             Ca, Cb, Za, Zb, K_idx, Z_idx, cQ, w_idx = proj[..., :4 * c + 2 * cI + dc + nIh].split(
                 [c, c, c, c, cI, cI, dc, nIh], dim=-1)
-            W = layer.q_weight()
-            qq = linear(cQ, W, w_settled=layer._fused_q.settled)
+            W, settled = layer.q_weight_settled()
+            qq = linear(cQ, W, w_settled=settled)
             q, q_idx = qq[..., :nh * c + nIh * cI].split([nh * c, nIh * cI], dim=-1)
             cache.append_step(Ca, Cb, Za, Zb, K_idx, Z_idx, layer.Ba, layer.Bb, layer.B_idx)
             if cache._decode_attend_ok(nh):
@@ -737,10 +757,11 @@ class HybridDecoding(nn.Module):
             cache.append_step(C, Z, layer.B_pos)
         else:
             c, dc, nh = cfg.hca_c, cfg.hca_dc, cfg.hca_nh
-            W = layer.fused_weight()
-            proj = linear(h, W, w_settled=layer._fused.settled)
+            W, settled = layer.fused_weight_settled()
+            proj = linear(h, W, w_settled=settled)
             C, Z, cQ = proj[..., :2 * c + dc].split([c, c, dc], dim=-1)
-            q = linear(cQ, layer.W_UQ.weight, w_settled=True)
+            W = layer.W_UQ.weight
+            q = linear(cQ, W, w_settled=_at_rest(W))
             cache.append_step(C, Z, layer.B_pos)
             if cache._decode_attend_ok(nh):
                 o = cache.forward_step(q.view(B, 1, nh, c), nh=nh, scale=1.0, sink_logits=layer.sink, _q_normalize=True,

@@ -316,3 +316,28 @@ def test_chained_kernels_take_tensor_memory_before_they_trigger():
                 both.append(name)
                 assert body.index("chain_trigger()") > body.index("tcgen05.alloc"), name
     assert both == ["gemm_decode.cu", "indexer_decode_tc5.cu"]
+
+
+def test_fused_weights_say_whether_this_call_launched_the_copy():
+    """The early weight fetch of a one-token step rests on it: False on the call that concatenates (first, or after a change in
+    place), True on the next, and the answer is the caller's own, whatever another thread asks in between."""
+    from torch import nn
+    from kch_b200.fused import _at_rest, _FusedWeights
+    a, b = nn.Linear(4, 3, bias=False), nn.Linear(4, 5, bias=False)
+    f = _FusedWeights()
+    W, settled = f.get_settled(a.weight, b.weight)
+    again = f.get_settled(a.weight, b.weight)          # another caller, between the first one's get and its launch
+    assert not settled and again[1] and again[0] is W and f.get(a.weight, b.weight) is W
+    with torch.no_grad():
+        b.weight.mul_(2)
+    W2, settled = f.get_settled(a.weight, b.weight)
+    assert not settled and torch.equal(W2[3:], b.weight.detach()) and f.get_settled(a.weight, b.weight)[1]
+    assert not hasattr(f, "settled")
+    # a parametrised weight is computed when it is read: the launch before the product writes it
+
+    class Twice(nn.Module):
+        def forward(self, w):
+            return w * 2
+    assert _at_rest(a.weight)
+    nn.utils.parametrize.register_parametrization(a, "weight", Twice())
+    assert not _at_rest(a.weight)

@@ -250,3 +250,66 @@ def test_bulk_append_leaves_the_cache_of_the_oracle(kch, B, win, quant, dtype, r
                     got, want = st["kcomp"].cpu().float(), ref.K_IComp.float()
                     assert bool(((got - want).abs() <= rel * want.abs() + 2e-6).all())
                     assert bool(((st["kcomp_norms"].cpu() - got.norm(dim=-1)).abs() <= 2e-6 * got.norm(dim=-1)).all())
+
+
+@pytest.mark.parametrize("M", [1, 7, 64])
+@pytest.mark.parametrize("N,K", [(256, 64), (2304, 128), (2048, 2048)])
+def test_settled_weights_give_the_same_product(kch, M, N, K):
+    """Weights fetched before the launch before has finished, or after it: the same product to the bit."""
+    from kch_b200.csa import linear
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    W, R = (torch.randn(N, K, generator=g, device=DEV) * 0.05).bfloat16(), torch.randn(M, 1, N, generator=g, device=DEV).bfloat16()
+    for _ in range(5):
+        x = torch.randn(M, 1, K, generator=g, device=DEV).bfloat16()
+        assert torch.equal(linear(x, W, residual=R, w_settled=True), linear(x, W, residual=R))
+
+
+_STEP_CFG = dict(d_model=512, n_heads_qk=4, n_heads_v=4, head_dim_k=128, head_dim_v=128, kda_chunk_size=64, csa_m=4, csa_topk=8,
+                 csa_nh=16, csa_c=128, csa_dc=128, csa_nIh=4, csa_cI=64, csa_sliding_window=16, hca_m2=16, hca_nh=16, hca_c=128,
+                 hca_dc=128, hca_sliding_window=16)
+
+
+@pytest.mark.parametrize("names", [("q_proj", "W_aKV", "W_KV"), ("g_up",), ("W_UQ",), ("o_proj",), ("parametrised",)])
+def test_weights_changed_between_one_token_steps(kch, names):
+    """A step right after a change of weights in place (members of a fused projection, or read as they lie), or with weights
+    computed when they are read, is the step of a model built with those weights, to the bit."""
+    from torch.nn.utils import parametrize
+    cfg = kch.HybridConfig(**_STEP_CFG)
+
+    def model_of(params):
+        with torch.device(DEV):
+            m = kch.HybridKCHAttention(cfg, 5)
+        m = m.bfloat16().eval()
+        m.load_state_dict(params, strict=True)
+        return m
+    params = {k: v.to(DEV) for k, v in syn.hybrid_params(7, cfg, 5, dtype=torch.bfloat16).items()}
+    x = syn.hidden_states(8, 3, 48, cfg.d_model, torch.bfloat16).to(DEV)
+
+    class Twice(torch.nn.Module):
+        def forward(self, w):
+            return w * 2
+    with torch.no_grad():
+        model = model_of(params)
+        a = kch.HybridDecoding(model=model)
+        a.reset()
+        a(x[:, :32])
+        a(x[:, 32:33])
+        for t in range(33, 41):
+            st = a.export_state()
+            st = {k: (v.clone() if torch.is_tensor(v) else v) for k, v in st.items()}
+            if names == ("parametrised",):
+                if t == 33:
+                    for layer in model.layers:
+                        for n in ("g_up", "W_UQ", "o_proj"):
+                            if n in dict(layer.named_children()):
+                                parametrize.register_parametrization(getattr(layer, n), "weight", Twice(), unsafe=True)
+                changed = {k: v * 2 if k.split(".")[-2] in ("g_up", "W_UQ", "o_proj") else v for k, v in params.items()}
+            else:
+                changed = {k: v * (-1.5) ** (t - 32) if k.split(".")[-2] in names else v for k, v in params.items()}
+                for k, w in model.named_parameters():
+                    if k.split(".")[-2] in names:
+                        w.copy_(changed[k])
+            got = a(x[:, t:t + 1])
+            b = kch.HybridDecoding(model=model_of(changed))
+            b.import_state(st)
+            assert torch.equal(got, b(x[:, t:t + 1])), t
