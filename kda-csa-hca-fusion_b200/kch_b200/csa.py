@@ -47,13 +47,14 @@ def _rows_2d(x, width):
 
 @functools.lru_cache(maxsize=64)
 def _epilogue(segments, group):
-    """The C form of a list of column segments (read by the call only, so equal lists share one)."""
+    """The C form of a list of column segments (read by the call only, so equal lists share one).  ``segments`` holds plain
+    numbers: a tensor would be compared by identity and may change its value."""
     ep = _lib.Epilogue()
-    ep.n_segments, ep.group = len(segments), int(group)
+    ep.n_segments, ep.group = len(segments), group
     end = 0
     for i, (width, act, param) in enumerate(segments):
-        end += int(width)
-        ep.seg_end[i], ep.seg_act[i], ep.seg_param[i] = end, int(act), float(param)
+        end += width
+        ep.seg_end[i], ep.seg_act[i], ep.seg_param[i] = end, act, param
     return ep, end
 
 
@@ -84,7 +85,7 @@ def linear(x, W, residual=None, epilogue=None, group=1, w_settled=False):
             ldr = r2.stride(0) if M > 1 else N
     ep = None
     if epilogue:
-        ep, end = _epilogue(tuple(map(tuple, epilogue)), group)
+        ep, end = _epilogue(tuple((int(w), int(a), float(p)) for w, a, p in epilogue), int(group))
         if end != N:
             raise ValueError(f"linear: epilogue segments cover {end} columns, the weight has {N} rows")
     with _lib.device(x.device):

@@ -341,3 +341,23 @@ def test_fused_weights_say_whether_this_call_launched_the_copy():
     assert _at_rest(a.weight)
     nn.utils.parametrize.register_parametrization(a, "weight", Twice())
     assert not _at_rest(a.weight)
+
+
+def test_epilogue_segments_are_taken_by_value(monkeypatch):
+    """A parameter given as a tensor and changed in place between two products is read anew."""
+    from kch_b200 import _lib, csa
+    seen = []
+
+    class Lib:
+        def kch_linear_ex(self, *a):
+            seen.append([a[12].seg_param[i] for i in range(a[12].n_segments)])
+            return 0
+    monkeypatch.setattr(_lib, "load", lambda: Lib())
+    monkeypatch.setattr(_lib, "require_cuda", lambda *t, fn="": None)
+    monkeypatch.setattr(_lib, "device", lambda dev: _lib._SAME_DEVICE)
+    monkeypatch.setattr(_lib, "stream", lambda: 0)
+    scale, x, W = torch.tensor(0.5), torch.zeros(2, 8), torch.zeros(4, 8)
+    for value in (0.5, 2.0):
+        scale.fill_(value)
+        csa.linear(x, W, epilogue=[(4, _lib.ACT_NEG_SOFTPLUS, scale)])
+    assert seen == [[0.5], [2.0]]
