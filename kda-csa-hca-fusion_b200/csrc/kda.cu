@@ -233,8 +233,10 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
 
 // =====================================================================================
 // Chunked form in fp32 on CUDA cores, for every geometry the tensor-core kernels do not take (fp32 inputs, K or V other
-// than 128).  Chunks are always 64 tokens (zero rows pad the last one): the mathematics does not depend on the chunk
-// length, and a longer chunk means fewer dependent steps in stage 2.  K is padded to KT = 64 or 128 channels.
+// than 128).  A record holds L tokens: as many whole chunks of C = min(chunk_size, 64, K) as fit into 64 (zero rows pad it
+// to 64 rows), because a longer record means fewer dependent steps in stage 2 and the mathematics does not depend on the
+// length -- but for a gate that grows: the exponent of a pair is clamped at 50 within a chunk of C tokens and exact between
+// chunks, where the state carries it.  K is padded to KT = 64 or 128 channels.
 //
 // Stage 1, one CTA of 4*KT threads per (b, hv, chunk), all chunks in parallel:
 //   gamma = cumsum(g), A (strictly lower), Tm = (I+A)^-1 diag(beta),
@@ -246,7 +248,7 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
 // what underflows is smaller still), halving the blocks from 32 to 4 rows: 8 K exponentials a level and plain products;
 // only the 4 x 4 diagonal blocks take the difference pair by pair.  The inverse is built from 8 x 8 blocks upwards.
 // 1024 tokens, 4 heads, K = V = 128, fp32: 202 -> 42 us.
-// A chunk whose gate is positive or not finite somewhere takes every pair directly (exponent clamped at 50).
+// A record whose gate is positive or not finite somewhere takes every pair directly.
 // =====================================================================================
 #define KC_C 64
 #define KC_AS 68                       // row stride of the 64 x 64 tiles (16-byte rows, 8 rows on 32 banks)
@@ -260,7 +262,7 @@ template <typename T, int KT>
 __global__ void __launch_bounds__(4 * KT)
 kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                          const T* __restrict__ g, const T* __restrict__ beta, float* __restrict__ ws, int T_,
-                         int H, int HV, int K, int V, int NT, float scale, float g_min,
+                         int H, int HV, int K, int V, int NT, int L, int C, float scale, float g_min,
                          int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b) {
   constexpr int NTH = 4 * KT, KS = KT + 4, NW = NTH / 32;
   extern __shared__ __align__(16) float smem[];
@@ -276,7 +278,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   const int n = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
   const int h = hv / (HV / H);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = n * KC_C;
+  const int t0 = n * L, t_end = min(t0 + L, T_);        // this record's tokens; rows behind them are zero
   float* rec = ws + (((int64_t)b * HV + hv) * NT + n) * kc_record_floats(KT, V);
   float* o_w = rec;
   float* o_qg = o_w + KC_C * KS;
@@ -290,7 +292,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   for (int idx = tid; idx < KC_C * KT; idx += NTH) {
     const int i = idx / KT, kk = idx % KT, t = t0 + i;
     float kv = 0.f, qv = 0.f, gv = 0.f;
-    if (t < T_ && kk < K) {
+    if (t < t_end && kk < K) {
       const int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
       kv = ldf(k + qoff);
       qv = ldf(q + qoff) * scale;
@@ -301,7 +303,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     sq[i * KS + kk] = qv;
     sgam[i * KS + kk] = gv;
   }
-  if (tid < KC_C) sbeta[tid] = t0 + tid < T_ ? ldf(beta + ((int64_t)b * T_ + t0 + tid) * ld_b + hv) : 0.f;
+  if (tid < KC_C) sbeta[tid] = t0 + tid < t_end ? ldf(beta + ((int64_t)b * T_ + t0 + tid) * ld_b + hv) : 0.f;
   for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) {
     sA[idx] = 0.f;
     if (idx % KC_AS > idx / KC_AS) o_aqk[idx] = 0.f;
@@ -413,6 +415,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
       if (i * (i + 1) / 2 > p % pairs) --i;
       const int j = blk * side + p % pairs - i * (i + 1) / 2;
       i += blk * side;
+      const bool same_chunk = i / C == j / C;
       float a = 0.f, aq = 0.f;
 #pragma unroll
       for (int c = 0; c < KT / 32; ++c) {
@@ -422,7 +425,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
         if (i != j || direct) {
           float d = sgam[i * KS + kk] - sgam[j * KS + kk];
           for (int s = j >> 4; s < i >> 4; ++s) d += stot[s * KT + kk];
-          e = expf(fminf(d, 50.f)) * kj;
+          e = expf(same_chunk ? fminf(d, 50.f) : d) * kj;
         }
         a = fmaf(sk[i * KS + kk], e, a);
         aq = fmaf(sq[i * KS + kk], e, aq);
@@ -521,7 +524,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 #pragma unroll 4
     for (int idx = tid; idx < KC_C * KT; idx += NTH) {
       const int i = idx / KT, c = idx % KT, t = t0 + i;
-      sx[i * KS + c] = t < T_ && v0 + c < V ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + v0 + c) : 0.f;
+      sx[i * KS + c] = t < t_end && v0 + c < V ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + v0 + c) : 0.f;
     }
     __syncthreads();
     product(acc);
@@ -548,7 +551,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 template <typename T, int KT>
 __global__ void __launch_bounds__(256)
 kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0, T* __restrict__ o,
-                      float* __restrict__ S_out, int T_, int HV, int K, int V, int NT, unsigned int* status) {
+                      float* __restrict__ S_out, int T_, int HV, int K, int V, int NT, int L, unsigned int* status) {
   constexpr int KS = KT + 4, IG = 256 / KT, IR = KC_C / IG;
   extern __shared__ __align__(16) float smem[];
   float* sw = smem;                          // [64][KS], then qg [64][KS]
@@ -671,14 +674,14 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
       reinterpret_cast<float4*>(sS)[2 * kk + c4] = x;
     }
     if (tid < 2 * KC_C) {
-      const int c4 = tid >> 6, t = n * KC_C + r;
+      const int c4 = tid >> 6, t = n * L + r;
       float4 x = red[c4 * KC_C + r];
 #pragma unroll
       for (int p = 1; p < 4; ++p) {
         const float4 y = red[(p * 2 + c4) * KC_C + r];
         x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
       }
-      if (t < T_ && ok) {
+      if (r < L && t < T_ && ok) {
         T* orow = o + (((int64_t)b * T_ + t) * HV + hv) * V + v0 + 4 * c4;
         const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -709,8 +712,18 @@ static size_t kc_scan_smem(int KT) {
           (256 / KT) * 2 * KT * 4) * sizeof(float) + 3 * sizeof(uint64_t);
 }
 static int kc_padded_k(int K) { return K <= 64 ? 64 : 128; }
-static int64_t kc_workspace_bytes(int B, int T, int HV, int K, int V) {
-  return (int64_t)B * HV * ((T + KC_C - 1) / KC_C) * kc_record_floats(kc_padded_k(K), V) * 4 + 16;   // + alignment of the base
+// tokens of a chunk (what the clamp of a growing gate's exponents counts by), and of a record
+static int kc_chunk(int K, int chunk_size) {
+  const int C = chunk_size < KC_C ? chunk_size : KC_C;
+  return C < K ? C : K;
+}
+static int kc_record_tokens(int C) { return KC_C / C * C; }
+static int64_t kc_records(int T, int K, int chunk_size) {
+  const int L = kc_record_tokens(kc_chunk(K, chunk_size));
+  return ((int64_t)T + L - 1) / L;
+}
+static int64_t kc_workspace_bytes(int B, int T, int HV, int K, int V, int chunk_size) {
+  return (int64_t)B * HV * kc_records(T, K, chunk_size) * kc_record_floats(kc_padded_k(K), V) * 4 + 16;   // + alignment of the base
 }
 
 // tensor-core path (kda_mma.cu)
@@ -724,7 +737,7 @@ int kch_kda_chunk_mma(const void* q, const void* k, const void* v, const void* g
 extern "C" int64_t kch_kda_chunk_workspace_bytes(int B, int T, int HV, int K, int V, int chunk_size) {
   if (B <= 0 || T <= 0 || HV <= 0 || K <= 0 || V <= 0 || chunk_size < 1) return 0;
   if (K > 128) return 0;                       // runs as the token recurrence
-  int64_t need = kc_workspace_bytes(B, T, HV, K, V);
+  int64_t need = kc_workspace_bytes(B, T, HV, K, V, chunk_size);
   // the dtype is not known here: size for whichever path may run
   if (kch_kda_mma_supported(K, V, chunk_size, 0.f, KCH_BF16)) {
     int64_t m = kch_kda_mma_workspace_bytes(B, T, HV);
@@ -768,8 +781,8 @@ static int kda_chunk_impl(const void* q, const void* k, const void* v, const voi
     }
     return KCH_OK;
   }
-  const int NT = (T + KC_C - 1) / KC_C, KT = kc_padded_k(K);
-  const int64_t need = kc_workspace_bytes(B, T, HV, K, V);
+  const int C = kc_chunk(K, chunk_size), L = kc_record_tokens(C), NT = (int)kc_records(T, K, chunk_size), KT = kc_padded_k(K);
+  const int64_t need = kc_workspace_bytes(B, T, HV, K, V, chunk_size);
   KCH_REQUIRE(workspace && workspace_bytes >= need, "kch_kda_chunk: workspace %lld < %lld bytes",
               (long long)workspace_bytes, (long long)need);
   float* ws = (float*)(((uintptr_t)workspace + 15) & ~(uintptr_t)15);
@@ -785,10 +798,10 @@ static int kda_chunk_impl(const void* q, const void* k, const void* v, const voi
     KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_scan_kernel<T_, KT_>,                                      \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));           \
     kda_chunk_prepare_kernel<T_, KT_><<<g1, 4 * KT_, smem1, s>>>((const T_*)q, (const T_*)k,              \
-        (const T_*)v, (const T_*)g, (const T_*)beta, ws, T, H, HV, K, V, NT, scale, g_clamp_min, ld_qk,   \
-        ld_v, ld_g, ld_beta);                                                                             \
+        (const T_*)v, (const T_*)g, (const T_*)beta, ws, T, H, HV, K, V, NT, L, C, scale, g_clamp_min,    \
+        ld_qk, ld_v, ld_g, ld_beta);                                                                             \
     kda_chunk_scan_kernel<T_, KT_><<<g2, 256, smem2, s>>>(ws, initial_state, (T_*)o, final_state, T, HV,  \
-        K, V, NT, status);                                                                                \
+        K, V, NT, L, status);                                                                             \
   } while (0)
   KCH_DISPATCH_FLOAT(dtype, T_, {
     if (KT == 64) GO(T_, 64);

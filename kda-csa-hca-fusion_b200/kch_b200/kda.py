@@ -181,7 +181,8 @@ def naive_chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_fin
                     chunk_size: int = 64, *, g_clamp_min: float = -10.0, state_dtype=None, _gate_scale=None):
     """Chunk-parallel KDA; equals :func:`naive_recurrent_kda` up to fp32 round-off.  Chunks larger
     than 64 tokens (or than K) are processed as smaller chunks: the same mathematics in a different
-    summation order.  ``_gate_scale`` (not in the reference): ``g`` is the pre-activation of the layer's gate and
+    summation order.  Where the gate grows, a pair's exponent is clamped at 50 within a chunk, as in the
+    reference (ops_kda.py:414, 516).  ``_gate_scale`` (not in the reference): ``g`` is the pre-activation of the layer's gate and
     the kernel applies ``-softplus(g) * _gate_scale`` itself (see :func:`chunk_gate_supported`)."""
     return _run("naive_chunk_kda", q, k, v, g, beta, scale, initial_state, output_final_state,
                 g_clamp_min, state_dtype, int(chunk_size), gate_scale=_gate_scale)

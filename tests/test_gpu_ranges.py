@@ -38,6 +38,22 @@ def test_kda_chunk_fp32_edges(kch, B, T, H, HV, K, V, chunk, gate):
     assert md(o, o_ref) <= 2e-5 and md(s, s_ref) <= 2e-5, (md(o, o_ref), md(s, s_ref))
 
 
+@pytest.mark.parametrize("T,K,chunk,lo,hi,growth", [
+    (100, 64, 16, 10, 60, 1.0), (130, 64, 64, 0, 64, 1.0), (150, 64, 48, 20, 110, 0.6), (64, 16, 64, 0, 40, 2.0),
+    (100, 64, 32, 10, 60, 1.5), (70, 64, 3, 0, 60, 1.0)])
+def test_kda_chunk_fp32_growing_gate(kch, T, K, chunk, lo, hi, growth):
+    """Where half of the channels grow for a while, exponents are clamped within a chunk of min(chunk_size, 64, K) tokens and
+    exact between chunks, whatever the kernels pack together.  Values reach 1e32; the chunk form in 32 bits on the CPU is up to
+    1.5e-6 (2-norm, relative) from 64 bits here, ten times that is allowed."""
+    q, k, v, g, beta, S0 = syn.kda_inputs(3, 1, T, 1, K, 8, 1, torch.float32, with_state=True)
+    g[:, lo:hi, :, :K // 2] = growth
+    o_ref, s_ref = orc.chunk_kda(*(x.double() for x in (q, k, v, g, beta)), initial_state=S0.double(), chunk_size=min(chunk, 64, K))
+    o, s = kch.naive_chunk_kda(*(x.to(DEV) for x in (q, k, v, g, beta)), initial_state=S0.to(DEV), output_final_state=True,
+                               chunk_size=chunk)
+    for got, want in ((o, o_ref), (s, s_ref)):
+        assert float((got.double().cpu() - want).norm() / want.norm()) <= 1.5e-5
+
+
 def _attend_ref(q, comp, sel, win, m, t0, nvis, window, sink, scale, win_t0):
     """One softmax over the selected (or all visible) rows, the window and the sink, in 64 bits on the GPU."""
     B, T, nh, c = q.shape
