@@ -18,7 +18,7 @@
 #define AM_WARPS 4
 #define AM_TILE 32
 #define AM_C 128
-#define AM_DENSE_GAIN 6                // a gathered entry against a tile entry at 16 heads: 52 ps against 8.1 ps
+#define AM_DENSE_GAIN 6                // a gathered entry against a tile entry at 16 heads, chip full: 52 ps against 8.1 ps
 #define AM_QLD 136   // padded row of the per-warp query tile (bf16 elements)
 
 struct AttnMmaArgs {
@@ -417,6 +417,20 @@ bool kch_attend_mma_supported(const kch_attend_args* p) {
   return true;
 }
 
+// What the two forms of a selection cost, in us, for `queries` (over all sequences) that select `entries` rows each, window
+// included, out of `last` (at most) and `mean` (on average) visible ones.  Few queries wait for one chain: a gathering warp
+// takes 48 ns an entry, a CTA over key tiles 11 ns a visible row and 6.5 ns an index for its mask; many are bound by the
+// chip.  Measured (visible -> mask / gather us): 8 heads, top-k 512, 256 queries: 512 -> 23 / 41, 2000 -> 40 / 43, 6000 ->
+// 84 / 43; 16 heads, top-k 1024, 1024 queries: 2000 -> 42 / 76, 6000 -> 88 / 76.
+static double am_gather_us(double queries, double entries) {
+  const double ns = 52e-3 * queries;
+  return 10. + 1e-3 * entries * (ns > 48. ? ns : 48.);
+}
+static double am_mask_us(double queries, int nh, double topk, double last, double mean) {
+  const double rounds = queries / (nh <= 8 ? 16 : 8) / (2 * 148), chain = 11. * last, chip = (nh <= 8 ? 4.05e-3 : 8.1e-3) * queries * mean;
+  return 10. + 1e-3 * (6.5 * topk * (rounds > 1. ? rounds : 1.) + (chip > chain ? chip : chain));
+}
+
 // `distinct`: the caller vouches that no index occurs twice in a selection list, so that the list may become a bit mask
 int kch_attend_mma(const kch_attend_args* p, bool distinct, void* stream) {
   AttnMmaArgs a;
@@ -442,17 +456,33 @@ int kch_attend_mma(const kch_attend_args* p, bool distinct, void* stream) {
     if (rc != -100) return rc;
   }
   // A selection list of distinct indices: contiguous key tiles under the list's bit mask cost per VISIBLE entry, the
-  // gather below per SELECTED one, AM_DENSE_GAIN (twice that for at most 8 heads) times as much each.
+  // gather below per SELECTED one, AM_DENSE_GAIN (twice that for at most 8 heads) times as much each once the chip is full.
+  // Queries that see few enough rows take the mask and the others are gathered, in two launches; for fewer queries than
+  // fill the chip either launch costs its chain whatever their number, and the cheapest of three ways is taken.
   static const int force_mask = [] { const char* e = getenv("KCH_ATTEND"); return !e ? 0 : e[0] == 'r' ? -1 : e[0] == 'd' ? 1 : 0; }();
   if (a.sel && distinct && a.topk > 0 && force_mask >= 0) {
     const int64_t gain = p->nh <= 8 ? 2 * AM_DENSE_GAIN : AM_DENSE_GAIN;
     const int64_t most = gain * ((int64_t)a.topk + a.win_size) - a.win_size;      // visible blocks up to which tiles win
     int64_t q_end = a.T;
     if (!force_mask) {
-      if (a.nvis_fixed >= 0 || a.m <= 0) q_end = (a.nvis_fixed >= 0 && a.nvis_fixed < a.n_comp ? a.nvis_fixed : a.n_comp) <= most ? a.T : 0;
-      else if (a.n_comp > most) q_end = (most + 1) * a.m - 1 - a.t0;              // the first query that sees more
+      const bool causal = a.nvis_fixed < 0 && a.m > 0;
+      auto sees = [&](int64_t t) -> int64_t {
+        const int64_t v = a.nvis_fixed >= 0 ? a.nvis_fixed : causal ? (a.t0 + t + 1) / a.m : a.n_comp;
+        return v < a.n_comp ? v : a.n_comp;
+      };
+      auto mask_us = [&](int64_t end) {
+        const double w = a.win_size, last = (double)sees(end - 1);
+        return am_mask_us((double)a.B * end, p->nh, a.topk, last + w, 0.5 * ((double)sees(0) + last) + w);
+      };
+      const double entries = (double)a.topk + a.win_size;
+      double best = am_gather_us((double)a.B * a.T, entries);
+      q_end = 0;
+      if (mask_us(a.T) < best) { best = mask_us(a.T); q_end = a.T; }
+      if (causal && a.n_comp > most) {
+        const int64_t split = (most + 1) * a.m - 1 - a.t0;                          // the first query that sees more
+        if (split > 0 && split < a.T && mask_us(split) + am_gather_us((double)a.B * (a.T - split), entries) < best) q_end = split;
+      }
     }
-    if (q_end > a.T) q_end = a.T;
     if (q_end > 0) {
       int done = 0;
       const int rc = kch_attend_dense_tc5(a.q, a.q_ld, a.B, a.T, a.nh, a.comp, a.comp_batch_rows, a.n_comp, a.m, a.t0, a.nvis_fixed,

@@ -116,6 +116,27 @@ def test_selection_as_mask_matches_gather(kch, B, T, nh, n, topk, m, t0, nvis, w
     assert md(dense, dref) <= 2e-3, md(dense, dref)
 
 
+def test_selection_split_between_mask_and_gather(kch):
+    """Enough queries to fill the chip, of which the first see few rows and the others many: the former take the mask, the
+    latter the gather, in two launches.  Each form is within 2e-3 of the 64-bit softmax, so 4e-3 of each other."""
+    from kch_b200.csa import attend
+    B, T, nh, topk = 4, 4096, 16, 256
+    g = torch.Generator(device=DEV).manual_seed(2)
+    q = torch.randn(B, T, nh, 128, generator=g, device=DEV).bfloat16()
+    comp = torch.nn.functional.normalize(torch.randn(B, T, 128, generator=g, device=DEV), dim=-1).bfloat16()
+    sink = torch.randn(nh, generator=g, device=DEV)
+    pos = torch.arange(T, device=DEV)
+    score = torch.rand(B, T, T, generator=g, device=DEV).masked_fill_(pos[None, :] > pos[:, None], -1.0)
+    top = score.topk(topk, -1)
+    sel = torch.where(top.values >= 0, top.indices, -1).int()
+    kw = dict(nh=nh, c=128, m=1, q_normalize=True, sink=sink, scale=1.0, out_dtype=torch.bfloat16)
+    a, b = (attend(q.reshape(B, T, nh * 128), comp, sel=sel, sel_distinct=d, **kw) for d in (True, False))
+    assert md(a, b) <= 4e-3, md(a, b)
+    for t0 in (0, 6 * topk - 8, T - 8):                      # the line between the two lies at six visible rows per selected one
+        ref = _attend_ref(q[:, t0:t0 + 8], comp, sel[:, t0:t0 + 8], comp[:, :0], 1, t0, -1, 0, sink, 1.0, 0)
+        assert md(a[:, t0:t0 + 8], ref) <= 2e-3, md(a[:, t0:t0 + 8], ref)
+
+
 @pytest.mark.parametrize("M,N", [(1, 256), (7, 400), (33, 6288), (64, 256)])
 def test_decode_gemm_l2norm_rows(kch, M, N):
     """The 128-wide decode tiles deal their rows out over the CTAs of a cluster by the real row count."""
