@@ -77,9 +77,9 @@ def _attend_ref(q, comp, sel, win, m, t0, nvis, window, sink, scale, win_t0):
     (2, 40, 16, 2500, 30, 1, 900, -1, 20, 1.0, None), (1, 24, 16, 96, 20, 2, 100, -1, 32, 1.0, "nan"),
     (1, 24, 8, 96, 20, 2, 100, -1, 32, 1.0, "inf")])
 def test_selection_as_mask_matches_gather(kch, B, T, nh, n, topk, m, t0, nvis, window, scale, odd):
-    """A selection list applied as a bit mask over key tiles (few visible rows per selected one), gathered, or split between
-    the two (the case of 2500 rows): operator outputs within 2e-3 of the 64-bit softmax, as everywhere.  Rows that a query
-    does not attend do not reach it even when they are not finite."""
+    """A selection list applied as a bit mask over key tiles (few visible rows per selected one) or gathered (the case of 2500
+    rows): operator outputs within 2e-3 of the 64-bit softmax, as everywhere.  Rows that a query does not attend do not reach
+    it even when they are not finite."""
     from kch_b200.csa import attend
     g = torch.Generator(device=DEV).manual_seed(T * nh + n)
     unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s, generator=g, device=DEV), dim=-1).bfloat16()  # noqa: E731
@@ -108,11 +108,18 @@ def test_selection_as_mask_matches_gather(kch, B, T, nh, n, topk, m, t0, nvis, w
         assert not torch.isfinite(a[:, bad].float()).all(-1).any() and torch.isfinite(a[:, ~bad].float()).all()
         a, b, ref = a[:, ~bad], b[:, ~bad], ref[:, ~bad]
     assert md(a, ref) <= 2e-3 and md(b, ref) <= 2e-3, (md(a, ref), md(b, ref))
+    if odd:                                   # without a list: a row that only the later half of the queries sees
+        late = (t0 + T // 2) // m + 1
+        comp = unit(B, n, 128)
+        comp[0, late] = float(odd)
+        pos = torch.arange(T, device=DEV)
+        bad = ((t0 + pos + 1) // m > late) | ((pos + win_t0 >= 20) & (pos + win_t0 < 20 + window))
     dense = attend(q.reshape(B, T, nh * 128), comp, **dict(kw, sel=None))
     dref = _attend_ref(q, comp, None, win, m, t0, nvis, window, sink, scale, win_t0)
     if odd:
-        keep = ~bad & (torch.arange(T, device=DEV) < 0)      # every query sees row 5: nothing finite is expected
-        dense, dref = dense[:, keep], dref[:, keep]
+        assert 0 < int(bad.sum()) < T
+        assert not torch.isfinite(dense[:, bad].float()).all(-1).any() and torch.isfinite(dense[:, ~bad].float()).all()
+        dense, dref = dense[:, ~bad], dref[:, ~bad]
     assert md(dense, dref) <= 2e-3, md(dense, dref)
 
 
@@ -236,14 +243,14 @@ def test_ragged_lengths_without_padding(kch, B, T, dtype):
     out, idx = kch.naive_csa(H.to(DEV), *dw.values(), **args, sink_logits=sink.to(DEV), use_ste=False, _return_indices=True)
     ref = orc.csa_forward(H, *w.values(), **args, sink_logits=sink,
                           indices_override=torch.cat([idx.long().cpu(), idx.new_full((B, -T % 4, 24), -1).long().cpu()], 1))
-    assert out.shape == ref.shape and md(out, ref) <= (4e-3 if dtype == "bf16" else 2e-5), md(out, ref)
+    assert out.shape == ref.shape and md(out, ref) <= (2e-3 if dtype == "bf16" else 2e-5), md(out, ref)
     vis = (torch.arange(T) + 1) // 4
     assert bool(((idx.cpu() >= 0).sum(-1) == vis.clamp(max=24)).all()) and bool((idx.cpu() < vis[None, :, None].clamp(min=1)).all())
     w, sink, H = syn.hca_inputs(T + 1, B, T, 256, nh=8, c=128, dc=64, m2=64, dtype=dt, random_sink=True)
     kw = dict(m2=64, nh=8, c=128, dc=64, sliding_window=16)
     out = kch.naive_hca(H.to(DEV), *(v.to(DEV) for v in w.values()), **kw, sink_logits=sink.to(DEV))
     ref = orc.hca_forward(H, *w.values(), **kw, sink_logits=sink)
-    assert out.shape == ref.shape and md(out, ref) <= (4e-3 if dtype == "bf16" else 2e-5), md(out, ref)
+    assert out.shape == ref.shape and md(out, ref) <= (2e-3 if dtype == "bf16" else 2e-5), md(out, ref)
 
 
 @pytest.mark.parametrize("B,win,quant,dtype,runs", [(1, 8, None, "bf16", (3, 2, 40, 3, 2)), (3, 5, "int8", "bf16", (1, 7, 3, 6)),
