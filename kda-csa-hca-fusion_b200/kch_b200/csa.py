@@ -154,16 +154,14 @@ def rownorm(x, normalize=True, out_dtype=torch.float32):
     return y
 
 
-def _check_same_shape(fn, shape, **others):
-    for name, t in others.items():
+def _refuse_shapes(fn, shape, streams, m, biases):
+    """Names the first of ``streams`` that is not of ``shape``, or of ``biases`` with fewer values than a block's rows."""
+    for name, t in streams:
         if t.shape != shape:
             raise ValueError(f"{fn}: {name}.shape={tuple(t.shape)} must be {tuple(shape)}")
-
-
-def _check_bias(fn, m, c, **biases):
-    for name, t in biases.items():
-        if t.numel() < m * c:
-            raise ValueError(f"{fn}: {name}.shape={tuple(t.shape)} must hold ({m}, {c}) values")
+    for name, t in biases:
+        if t.numel() < m * shape[-1]:
+            raise ValueError(f"{fn}: {name}.shape={tuple(t.shape)} must hold ({m}, {shape[-1]}) values")
 
 
 def csa_compress_kv(C, Z, B_pos, m: int):
@@ -173,8 +171,8 @@ def csa_compress_kv(C, Z, B_pos, m: int):
         raise ValueError(f"compression factor m={m} must be >= 1")
     if T % m != 0:
         raise ValueError(f"T={T} must be divisible by m={m}")
-    _check_same_shape("csa_compress_kv", C.shape, Z=Z)
-    _check_bias("csa_compress_kv", m, c, B_pos=B_pos)
+    if Z.shape != C.shape or B_pos.numel() < m * c:
+        _refuse_shapes("csa_compress_kv", C.shape, (("Z", Z),), m, (("B_pos", B_pos),))
     _lib.require_cuda(C, Z, B_pos, fn="csa_compress_kv")
     lib = _lib.load()
     C2, ld, bsr = _as_rows(C)
@@ -201,10 +199,10 @@ def csa_compress_kv_overlapped(Ca, Cb, Za, Zb, Ba, Bb, m: int, *, prev_Cb=None, 
         raise ValueError(f"T={T} must be divisible by m={m}")
     if T == 0:
         return Ca.new_zeros(B, 0, c)
-    _check_same_shape("csa_compress_kv_overlapped", Ca.shape, Cb=Cb, Za=Za, Zb=Zb)
-    _check_bias("csa_compress_kv_overlapped", m, c, Ba=Ba, Bb=Bb)
-    if prev_Cb is not None:
-        _check_same_shape("csa_compress_kv_overlapped", (B, m, c), prev_Cb=prev_Cb, prev_Zb=prev_Zb)
+    if not (Ca.shape == Cb.shape == Za.shape == Zb.shape) or Ba.numel() < m * c or Bb.numel() < m * c:
+        _refuse_shapes("csa_compress_kv_overlapped", Ca.shape, (("Cb", Cb), ("Za", Za), ("Zb", Zb)), m, (("Ba", Ba), ("Bb", Bb)))
+    if prev_Cb is not None and not (prev_Cb.shape == prev_Zb.shape == (B, m, c)):
+        _refuse_shapes("csa_compress_kv_overlapped", (B, m, c), (("prev_Cb", prev_Cb), ("prev_Zb", prev_Zb)), m, ())
     _lib.require_cuda(Ca, Cb, Za, Zb, fn="csa_compress_kv_overlapped")
     lib = _lib.load()
     views = [_as_rows(x) for x in (Ca, Cb, Za, Zb)]

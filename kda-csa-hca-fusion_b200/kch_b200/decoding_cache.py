@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .csa import attend, csa_compress_kv, csa_compress_kv_overlapped, indexer_topk, rownorm
+from .csa import _refuse_shapes, attend, csa_compress_kv, csa_compress_kv_overlapped, indexer_topk, rownorm
 
 _QUANT = {None: None, "fp8": _lib.KCH_FP8_E4M3, "int8": _lib.KCH_INT8}
 
@@ -249,17 +249,6 @@ class _CacheBase:
             _lib.check(_lib.load().kch_cache_store_rows(_lib.ptr(rows_f32), nb, c, B, _lib.ptr(dst), _lib.ptr(norms), dst.shape[1],
                                                         start, _lib.dtype_tag(self.dtype), _lib.stream()))
 
-    def _check_streams(self, streams, biases, T_new, m):
-        """Every stream ``[B, T_new, width]`` and every bias of at least ``m`` rows, before anything is stored: the append
-        kernels read all of them with the geometry of the cache.  ``streams``: (name, tensor, width), ``biases`` likewise."""
-        fn = f"{type(self).__name__}.append_step"
-        for name, t, w in streams:
-            if tuple(t.shape) != (self.B, T_new, w):
-                raise ValueError(f"{fn}: {name}.shape={tuple(t.shape)} must be (B, T_new, width)=({self.B}, {T_new}, {w}).")
-        for name, t, w in biases:
-            if t.numel() < m * w:
-                raise ValueError(f"{fn}: {name}.shape={tuple(t.shape)} must hold ({m}, {w}) values.")
-
     def _blocks_of(self, new, nb, m):
         """The tokens of the ``nb`` blocks that ``new`` completes, per stream ``[B, nb*m, width]``: views of ``new`` unless
         a block is open."""
@@ -432,9 +421,12 @@ class CSADecodingCache(_CacheBase):
                                  f"Ca_new.shape[1]={T_new}. All inputs must share the same T_new.")
         if T_new == 0:
             return []
-        self._check_streams((("Cb_new", Cb_new, c), ("Za_new", Za_new, c), ("Zb_new", Zb_new, c), ("K_idx_new", K_idx_new, self.c_I),
-                             ("Z_idx_new", Z_idx_new, self.c_I)),
-                            (("Ba", Ba, c), ("Bb", Bb, c), ("B_idx", B_idx, self.c_I)), T_new, self.m)
+        # the append kernels read every stream and bias with the geometry of the cache: all of them, before anything is stored
+        m, c_I, fn = self.m, self.c_I, "CSADecodingCache.append_step"
+        if not (Ca_new.shape == Cb_new.shape == Za_new.shape == Zb_new.shape) or Ba.numel() < m * c or Bb.numel() < m * c:
+            _refuse_shapes(fn, Ca_new.shape, (("Cb_new", Cb_new), ("Za_new", Za_new), ("Zb_new", Zb_new)), m, (("Ba", Ba), ("Bb", Bb)))
+        if not (K_idx_new.shape == Z_idx_new.shape == (B, T_new, c_I)) or B_idx.numel() < m * c_I:
+            _refuse_shapes(fn, (B, T_new, c_I), (("K_idx_new", K_idx_new), ("Z_idx_new", Z_idx_new)), m, (("B_idx", B_idx),))
         new = [x.to(device=self.device, dtype=self.dtype) for x in (Ca_new, Cb_new, Za_new, Zb_new, K_idx_new, Z_idx_new)]
         biases = [x.to(device=self.device, dtype=self.dtype).contiguous() for x in (Ba, Bb, B_idx)]
         first_new = self._n_blocks
@@ -646,7 +638,8 @@ class HCADecodingCache(_CacheBase):
                              f"C_new.shape[1]={T_new}.")
         if T_new == 0:
             return []
-        self._check_streams((("Z_new", Z_new, c),), (("B_pos", B_pos, c),), T_new, self.m2)
+        if Z_new.shape != C_new.shape or B_pos.numel() < self.m2 * c:
+            _refuse_shapes("HCADecodingCache.append_step", C_new.shape, (("Z_new", Z_new),), self.m2, (("B_pos", B_pos),))
         new = [x.to(device=self.device, dtype=self.dtype) for x in (C_new, Z_new)]
         bias = B_pos.to(device=self.device, dtype=self.dtype).contiguous()
         first_new = self._n_blocks
