@@ -278,7 +278,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   const int n = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
   const int h = hv / (HV / H);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = n * L, t_end = min(t0 + L, T_);        // this record's tokens; rows behind them are zero
+  const int t0 = n * L, t_end = min(t0 + L, T_), rows = t_end - t0;      // this record's tokens; rows behind them are zero
   float* rec = ws + (((int64_t)b * HV + hv) * NT + n) * kc_record_floats(KT, V);
   float* o_w = rec;
   float* o_qg = o_w + KC_C * KS;
@@ -327,6 +327,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   if (!direct) {
 #pragma unroll
     for (int s = 32; s >= 4; s >>= 1) {
+      if (s >= rows) continue;                            // blocks of zero rows only
 #pragma unroll 4
       for (int idx = tid; idx < KC_C * KT; idx += NTH) {
         const int i = idx / KT, kk = idx % KT;
@@ -407,7 +408,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) sT[idx] = 0.f;
   // the 4 x 4 diagonal blocks (every block of the triangle when `direct`): a warp per pair, its lanes over the channels
   {
-    const int side = direct ? KC_C : 4, pairs = side * (side + 1) / 2, blocks = KC_C / side;
+    const int side = direct ? KC_C : 4, pairs = side * (side + 1) / 2, blocks = (rows + side - 1) / side;
     for (int p = warp; p < blocks * pairs; p += NW) {
       const int blk = p / pairs;
       int i = (int)((sqrtf(8.f * (p % pairs) + 1.f) - 1.f) * 0.5f);
@@ -415,7 +416,6 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
       if (i * (i + 1) / 2 > p % pairs) --i;
       const int j = blk * side + p % pairs - i * (i + 1) / 2;
       i += blk * side;
-      const bool same_chunk = i / C == j / C;
       float a = 0.f, aq = 0.f;
 #pragma unroll
       for (int c = 0; c < KT / 32; ++c) {
@@ -425,7 +425,8 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
         if (i != j || direct) {
           float d = sgam[i * KS + kk] - sgam[j * KS + kk];
           for (int s = j >> 4; s < i >> 4; ++s) d += stot[s * KT + kk];
-          e = expf(same_chunk ? fminf(d, 50.f) : d) * kj;
+          if (direct && i / C == j / C) d = fminf(d, 50.f);       // (without `direct` it is at most 0)
+          e = expf(d) * kj;
         }
         a = fmaf(sk[i * KS + kk], e, a);
         aq = fmaf(sq[i * KS + kk], e, aq);
@@ -470,6 +471,7 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   // ... then [[T00, 0], [-T11 A10 T00, T11]] for blocks of 8, 16 and 32
 #pragma unroll
   for (int s = 8; s <= 32; s <<= 1) {
+    if (s >= rows) continue;
     for (int idx = tid; idx < 32 * s; idx += NTH) {
       const int blk = idx / (s * s), i = (idx / s) % s, c = idx % s, r0 = blk * 2 * s;
       float acc = 0.f;
