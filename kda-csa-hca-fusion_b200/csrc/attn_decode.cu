@@ -743,7 +743,13 @@ extern "C" int kch_attend_decode(const kch_attend_decode_args* p, void* stream) 
     KCH_CUDA_OK(kch_launch_chained(attn_decode_split_kernel, dim3(S, p->B), dim3(AD_THREADS), 0, s, 1, a));
   }
   KCH_LAUNCH_OK();
-  KCH_CUDA_OK(kch_launch_chained(attn_decode_combine_kernel, dim3(p->nh, p->B), dim3(AD_THREADS), 0, s, 1, a, S));
+  // The merge is started early only where the CTAs before it leave it room: three of them fill an SM, and a grid that fills
+  // more than nine SMs in ten leaves the early CTAs to crowd on the few others (HCA, 3000 rows a sequence, early / not: 10
+  // sequences x 32 CTAs 18.9 / 20.7 us, 12 x 32 19.5 / 20.7, 32 x 13 26.5 / 22.9, 16 x 27 27.1 / 20.7).
+  if ((int64_t)S * p->B <= 3 * 148 * 9 / 10)
+    KCH_CUDA_OK(kch_launch_chained(attn_decode_combine_kernel, dim3(p->nh, p->B), dim3(AD_THREADS), 0, s, 1, a, S));
+  else
+    attn_decode_combine_kernel<<<dim3(p->nh, p->B), AD_THREADS, 0, s>>>(a, S);
   KCH_LAUNCH_OK();
   return KCH_OK;
 }
