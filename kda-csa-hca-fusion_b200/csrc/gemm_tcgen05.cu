@@ -158,6 +158,8 @@ __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__floa
 // Fast intrinsics (ex2.approx, approximate reciprocal): a few fp32 ulp, far below the bf16 rounding
 // that follows every step, so a fused result differs from the unfused chain by at most one bf16 rounding.
 __device__ __forceinline__ float ep_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+__device__ __forceinline__ float ep_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
+__device__ __forceinline__ float ep_neg_softplus(float x, float prm) { return -bf16r(x > 20.f ? x : __logf(1.0f + __expf(x))) * prm; }
 // Ring depth: as many (A tile + W tile) stages as fit in about 200 KB, so that narrow tiles (small BN) keep
 // the same number of bytes in flight per SM as the 256-wide tile does with 4 stages.
 // row pitch (in floats) of the fp32 partial tile a split-K CTA leaves in shared memory: 16 bytes of padding keep the
@@ -191,7 +193,7 @@ struct TgSmem {
   uint32_t tmem_base;
 };
 
-// ---- epilogue of a CTA pair's plain, silu and silu + L2-norm columns -------------------------------------------------------
+// ---- epilogue of a CTA pair's columns, 128 of one activation at a time ------------------------------------------------------
 // A warp's 32 rows x 128 columns leave as two 32 x 64 tiles through swizzled shared memory and bulk-tensor stores: whole
 // 128-byte lines, no store instructions, and the copy engine clips what lies beyond M and N.  The 128 columns are held as
 // packed bf16, so that the accumulator is released before anything is stored and an L2 norm needs silu once.  A residual
@@ -207,7 +209,7 @@ __device__ __forceinline__ void bulk_residual(SM& sm, int warp, const CUtensorMa
 }
 template <int ACT, typename SM, typename F>
 __device__ __forceinline__ void bulk_tile(SM& sm, int warp, int lane, uint32_t taddr, const CUtensorMap& map_c, const CUtensorMap& map_r,
-                                          bool residual, int col0, int64_t row0, int64_t M, int N, float, uint32_t& rphase, F release) {
+                                          bool residual, int col0, int64_t row0, int64_t M, int N, float prm, uint32_t& rphase, F release) {
   uint8_t* stg = sm.epi[warp - 2];
   uint32_t pk[64];
   float ss = 0.f;
@@ -222,7 +224,9 @@ __device__ __forceinline__ void bulk_tile(SM& sm, int warp, int lane, uint32_t t
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         float x = __uint_as_float(r[h][2 * j]), y = __uint_as_float(r[h][2 * j + 1]);
-        if (ACT != 0) { x = ep_silu(bf16r(x)); y = ep_silu(bf16r(y)); }
+        if (ACT == KCH_ACT_NEG_SOFTPLUS) { x = ep_neg_softplus(bf16r(x), prm); y = ep_neg_softplus(bf16r(y), prm); }
+        else if (ACT == KCH_ACT_SIGMOID) { x = ep_sigmoid(bf16r(x)); y = ep_sigmoid(bf16r(y)); }
+        else if (ACT != 0) { x = ep_silu(bf16r(x)); y = ep_silu(bf16r(y)); }
         const uint32_t w = pack2_bf16(x, y);
         if (ACT == KCH_ACT_SILU_L2NORM) {
           const float xr = __uint_as_float(w << 16), yr = __uint_as_float(w & 0xFFFF0000u);
@@ -281,7 +285,10 @@ __device__ __forceinline__ void bulk_tile(SM& sm, int warp, int lane, uint32_t t
   }
 }
 
-template <int BN, bool TWO, bool SK = false>
+// GATE (CTA pairs): bulk_tile for sigmoid and softplus columns too.  A kernel of its own: their code beside the others cost
+// the plain K = 128 products 3 % (131072 x 2048: 103.3 -> 105.7 us), while without it 128 and more columns of one of them
+// took the general loop (131072 x 2048 x 128: sigmoid 462 us, now 268; softplus 767, now 637).
+template <int BN, bool TWO, bool SK = false, bool GATE = false>
 __global__ void __launch_bounds__(TG_THREADS, SK ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_r, int c_bulk, bf16* __restrict__ C, const bf16* __restrict__ R, int64_t M, int N, int K,
@@ -442,8 +449,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int64_t mb = tile / n_tiles;
       const int nb = (int)(tile % n_tiles);
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
-      // the activation of this warp's 128 columns when they have one: 0, silu or silu + L2 norm, which bulk_tile knows; -1 otherwise
+      // the activation of this warp's 128 columns when they have one that bulk_tile knows; -1 otherwise
       int act_bulk = -1;
+      float prm_bulk = 0.f;
       if constexpr (TWO) {
         if (c_bulk) {
           act_bulk = 0;
@@ -452,7 +460,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int sidx = 0;
             while (sidx < ep.nseg - 1 && col >= ep.seg_end[sidx]) ++sidx;
             act_bulk = col + 128 <= ep.seg_end[sidx] || col >= N ? ep.seg_act[sidx] : -1;
-            if (act_bulk != 0 && act_bulk != KCH_ACT_SILU && act_bulk != KCH_ACT_SILU_L2NORM) act_bulk = -1;
+            if constexpr (GATE) prm_bulk = ep.seg_param[sidx];
+            const bool gate = GATE && (act_bulk == KCH_ACT_SIGMOID || act_bulk == KCH_ACT_NEG_SOFTPLUS);
+            if (act_bulk != 0 && act_bulk != KCH_ACT_SILU && act_bulk != KCH_ACT_SILU_L2NORM && !gate) act_bulk = -1;
           }
           if (R && lane == 0) {                          // the first half's residual rows are under way before the product is complete
             t5_bulk_wait_read();
@@ -473,6 +483,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&sm.acc_empty[acc]), 0));
           };
+          if constexpr (GATE) {
+            if (act_bulk == KCH_ACT_SIGMOID) {
+              bulk_tile<KCH_ACT_SIGMOID>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, 0.f, rphase, release);
+              continue;
+            }
+            if (act_bulk == KCH_ACT_NEG_SOFTPLUS) {
+              bulk_tile<KCH_ACT_NEG_SOFTPLUS>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, prm_bulk, rphase, release);
+              continue;
+            }
+          }
           if (act_bulk == 0) bulk_tile<0>(sm, warp, lane, tbase + c_begin, map_c, map_r, R != nullptr, col0, row0, M, N, 0.f, rphase, release);
           else if (act_bulk == KCH_ACT_SILU) bulk_tile<KCH_ACT_SILU>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, 0.f, rphase, release);
           else bulk_tile<KCH_ACT_SILU_L2NORM>(sm, warp, lane, tbase + c_begin, map_c, map_r, false, col0, row0, M, N, 0.f, rphase, release);
@@ -526,14 +546,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(ep_silu(bf16r(__uint_as_float(r[j]))));
         } else if (act == KCH_ACT_SIGMOID) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            r[j] = __float_as_uint(__fdividef(1.0f, 1.0f + __expf(-bf16r(__uint_as_float(r[j])))));
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(ep_sigmoid(bf16r(__uint_as_float(r[j]))));
         } else if (act == KCH_ACT_NEG_SOFTPLUS) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = bf16r(__uint_as_float(r[j]));
-            r[j] = __float_as_uint(-bf16r(v > 20.f ? v : __logf(1.0f + __expf(v))) * prm);
-          }
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(ep_neg_softplus(bf16r(__uint_as_float(r[j])), prm));
         }
         if (vec_ok && col + 32 <= N) {
           // Transpose the 32 x 32 chunk through shared memory so that a store instruction writes 8 row segments
@@ -838,7 +854,11 @@ static int launch_tg_pair(const void* A, const void* W, void* C, const void* R, 
   rc = make_map_2d(&mw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, BN / 2, TG_BK);
   if (rc) return rc;
   size_t smem = sizeof(TgSmem<BN, true>) + 1024;
-  KCH_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kernel = gemm_tcgen05_kernel<BN, true>;
+  for (int i = 0, start = 0; i < ep.nseg; start = ep.seg_end[i++])        // a whole group of 128 columns under one of these
+    if ((ep.seg_act[i] == KCH_ACT_SIGMOID || ep.seg_act[i] == KCH_ACT_NEG_SOFTPLUS) && (start + 127) / 128 * 128 + 128 <= ep.seg_end[i])
+      kernel = gemm_tcgen05_kernel<BN, true, false, true>;
+  KCH_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -848,7 +868,7 @@ static int launch_tg_pair(const void* A, const void* W, void* C, const void* R, 
   if (!max_pairs) {
     cfg.gridDim = dim3(2);
     int nc = 0;
-    KCH_CUDA_OK(cudaOccupancyMaxActiveClusters(&nc, gemm_tcgen05_kernel<BN, true>, &cfg));
+    KCH_CUDA_OK(cudaOccupancyMaxActiveClusters(&nc, kernel, &cfg));
     KCH_REQUIRE(nc > 0, "kch_linear: no CTA pair of the tcgen05 GEMM fits on this device");
     max_pairs = nc;
   }
@@ -862,7 +882,7 @@ static int launch_tg_pair(const void* A, const void* W, void* C, const void* R, 
   if (c_bulk && (make_map_2d(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64) ||
                  (R && make_map_2d(&mr, R, (uint64_t)M, (uint64_t)N, (uint64_t)ldr, 32, 64))))
     c_bulk = 0;
-  KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, true>, ma, mw, mc, mr, c_bulk, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
+  KCH_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, ma, mw, mc, mr, c_bulk, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
                                  vec_ok, ep, slab_k, M, 1));
   kch_note_launch(1);
   return KCH_OK;

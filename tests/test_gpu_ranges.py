@@ -231,6 +231,24 @@ def test_large_gemm_residual_and_activation_edges(kch, M, N):
     assert bool(((y.double() - want).abs() <= 2 ** -6 * want.abs() + 2e-3).all()), md(y, want)
 
 
+@pytest.mark.parametrize("M,N", [(520, 520), (1100, 384)])
+@pytest.mark.parametrize("act", ["SIGMOID", "NEG_SOFTPLUS"])
+def test_large_gemm_wide_activation(kch, M, N, act):
+    """Column groups of 128 with one elementwise activation leave by the copy engine, the ragged rest of N too.  Product,
+    activation and result round to bf16 (2^-7 of the product, at most as much of the value, then 2^-8 each)."""
+    from kch_b200 import _lib
+    from kch_b200.csa import linear
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, W = torch.randn(M, 128, generator=g, device=DEV).bfloat16(), (torch.randn(N, 128, generator=g, device=DEV) / 6).bfloat16()
+    p = (x.double() @ W.double().T).bfloat16().double()
+    for cut in (N, 256):                     # all columns, or a second group without an activation
+        segs = [(cut, getattr(_lib, "ACT_" + act), 0.5)] + ([(N - cut, 0, 0.0)] if cut < N else [])
+        want = torch.sigmoid(p[:, :cut]) if act == "SIGMOID" else -0.5 * torch.nn.functional.softplus(p[:, :cut])
+        want = torch.cat([want, p[:, cut:]], 1)
+        y = linear(x, W, epilogue=segs)
+        assert bool(((y.double() - want).abs() <= 2 ** -6 * want.abs() + 1e-4).all()), md(y, want)
+
+
 @pytest.mark.parametrize("B,T,dtype", [(2, 131, "bf16"), (1, 517, "bf16"), (3, 130, "fp32"), (1, 9, "bf16"), (2, 3, "fp32")])
 def test_ragged_lengths_without_padding(kch, B, T, dtype):
     """Lengths that are no multiple of a block (4 and 64 tokens) or of the indexer's query tile: same as the oracle, which pads.
