@@ -53,6 +53,7 @@ long long kch_launch_count(int reset);      /* kernels launched by this library 
 #define KCH_STATUS_GEMM_DECODE 0x6D01   /* status word: a wait of the decode-batch GEMM (operands / accumulator) expired */
 #define KCH_STATUS_KDA_STEP 0x6D03       /* status word: the state copy of the one-token KDA step did not arrive */
 #define KCH_STATUS_KDA_CHUNK 0x6D04      /* status word: a chunk record of the fp32 KDA scan did not arrive */
+#define KCH_STATUS_ATTEND_TILES 0x6D05   /* status word: a wait of the attention over key tiles (operands / accumulator) expired */
 #define KCH_STATUS_INDEXER_DECODE 0x6D02 /* status word: a wait of the one-token indexer (key tiles / accumulator) expired */
 int kch_selftest_bounded_wait(unsigned int limit_polls, unsigned int* polls_out, void* stream);
 

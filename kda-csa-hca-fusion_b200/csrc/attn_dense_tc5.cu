@@ -45,7 +45,6 @@
 #define DT_SOFT 256                    // softmax threads
 #define DT_THREADS (DT_SOFT + 64)      // + producer warp, MMA warp
 #define DT_SPIN (1u << 24)
-#define DT_STATUS 0x6D05
 
 struct DtArgs {
   int B, T, nh;
@@ -201,7 +200,7 @@ attn_dense_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   const uint32_t tmem = sm.tmem;
   // S buffers at columns 0 and 64 (P of the same tile over their columns 0..15 and 32..47), O at 128..255
   const uint32_t tS = tmem, tO = tmem + 128;
-  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbarrier_wait_bounded(bar, parity & 1, DT_STATUS, DT_SPIN, a.status); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbarrier_wait_bounded(bar, parity & 1, KCH_STATUS_ATTEND_TILES, DT_SPIN, a.status); };
 
   if (warp == 8) {
     // ------------------------------ producer: the query tile, then the key tiles -----------------------------------
