@@ -61,6 +61,8 @@ def main():
     ap.add_argument("--iters", type=int, default=5)
     ap.add_argument("--warmup", type=int, default=2)
     ap.add_argument("--fp32-queries", action="store_true", help="indexer: fp32 queries (the mma.sync logits kernel)")
+    ap.add_argument("--distinct", action="store_true", help="csa_attend: the lists hold no index twice (as the indexer's do)")
+    ap.add_argument("--fp32", action="store_true", help="kda: fp32 inputs (the CUDA-core chunk kernels)")
     ap.add_argument("--gate-scale", type=float, default=0.1, help="kda: multiplies the synthetic log-decay")
     ap.add_argument("--kv-quant", default=None, choices=[None, "fp8", "int8"])
     ap.add_argument("--graph", action="store_true", help="decode: replay the step from a CUDA graph")
@@ -78,8 +80,9 @@ def main():
         fl = 2.0 * a.M * a.N * a.K
         out.update(M=a.M, N=a.N, K=a.K, ms=ms, tflops=fl / ms / 1e9, algorithmic_bytes=2.0 * (a.M * a.K + a.N * a.K + a.M * a.N))
     elif a.kernel in ("kda_chunk", "kda_recurrent"):
-        q, k, v, gg, beta = (t.to(dev) for t in syn.kda_inputs(0, a.B, a.T, a.H, 128, 128, dtype=torch.bfloat16))
-        gg = (gg.float() * a.gate_scale).bfloat16()     # 0.1: the decay range of the layer's gate (-0.1 softplus)
+        dt = torch.float32 if a.fp32 else torch.bfloat16
+        q, k, v, gg, beta = (t.to(dev) for t in syn.kda_inputs(0, a.B, a.T, a.H, 128, 128, dtype=dt))
+        gg = (gg.float() * a.gate_scale).to(dt)     # 0.1: the decay range of the layer's gate (-0.1 softplus)
         if a.kernel == "kda_chunk":
             fn = lambda: kch_b200.naive_chunk_kda(q, k, v, gg, beta, output_final_state=True)  # noqa: E731
         else:
@@ -101,7 +104,7 @@ def main():
             vis = ((torch.arange(a.T, device=dev) + 1) // m).view(1, -1, 1)
             sel = torch.where(ar < vis, ar, torch.full_like(ar, -1)).to(torch.int32).contiguous()
         fn = lambda: csa.attend(q, comp, nh=nh, c=c, sel=sel, m=m, q_normalize=True, win=win, sliding_window=128,  # noqa: E731
-                                sink=sink, scale=1.0, out_dtype=torch.bfloat16)
+                                sink=sink, scale=1.0, out_dtype=torch.bfloat16, sel_distinct=a.distinct)
         ms = _time(fn, a.iters, a.warmup)
         t = torch.arange(a.T, dtype=torch.float64)
         ent = (torch.minimum((t + 1) // m, torch.tensor(float(a.topk if sel is not None else n))) +
