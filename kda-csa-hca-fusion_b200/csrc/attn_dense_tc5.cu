@@ -20,13 +20,15 @@
 //     MN-major B operand;
 //   * the epilogue divides by the row sum (+ the sink term) and stores 128 contiguous bytes per thread, while the next
 //     item's first scores are computed.
-// A selection list costs nothing but its bit mask: a masked entry is computed and dropped.  That is worth it because a
-// gathered row (attn_mma.cu) is bound by the L2 -> shared-memory path at 256 bytes per (query, entry), while here a
-// key tile is read once for 8 or 16 queries.
-// Bound: the tensor pipe.  A tile takes 780 cycles of an SM, all of it MMA execution: the score product's N = 64 steps run
-// at the rate of N = 128 ones (62 cycles each, the 128 rows of A are read from shared memory either way), the value product
-// at its own (67 cycles, A in tensor memory); ex2 needs 512 and the issue slots of the softmax warps ~600.  It was 2200 with
-// four softmax warps, P in shared memory, one item per CTA and MMAs issued from a branch on the lane number.
+// A selection list costs its bit mask (about 6.5 ns an index of a query tile), and a masked entry is computed and dropped.
+// That is worth it because a gathered row (attn_mma.cu) is bound by the L2 -> shared-memory path at 256 bytes per (query,
+// entry), while here a key tile is read once for 8 or 16 queries; the caller weighs the two (am_mask_us, am_gather_us).
+// Bound: the chain of a tile (score product, hand-over, softmax, hand-over, value product), of which two CTAs keep two under
+// way on an SM: about 1300 cycles a tile and SM, no unit at its limit (CSA, 16384 tokens, top-k 1024: tensor pipe active
+// 43 %, issue slots 49 %).  The score product's N = 64 steps run at the rate of N = 128 ones (62 cycles each, the 128 rows
+// of A are read from shared memory either way), the value product at its own (67 cycles, A in tensor memory), so the
+// pipe's own limit would be 780 cycles a tile; ex2 needs 512 and the issue slots of the softmax warps ~600.  It was 2200
+// with four softmax warps, P in shared memory, one item per CTA and MMAs issued from a branch on the lane number.
 // CSA core, 2 x 10007 tokens, top-k 1024: 1132 us gathered -> 327; 4096 tokens, 8 heads, top-k 512: 164 -> 34; HCA core,
 // 2 x 32768 tokens: 354 -> 288.
 // A masked key multiplies its value row by p = 0, which is no mask for an infinity or a NaN; O shows it (it is not finite

@@ -6,7 +6,7 @@
 // One CTA per (batch, value head); S^T [128 v x 128 k] fp32 is the accumulator of the update product and never leaves
 // tensor memory between chunks; the bf16 hi / lo images of S^T and of vt^T are A operands there as well (an A operand in
 // tensor memory needs no proxy fence, which cost 300 cycles at each of a chunk's four conversions, and frees the shared
-// memory that lets the operands of a whole chunk be fetched ahead).  Per chunk (the dependent chain is S -> D1w -> vt -> S):
+// memory for a second [w; qg] stage).  Per chunk (the dependent chain is S -> D1w -> vt -> S):
 //   vector warps : read S^T (tcgen05.ld, one row v per thread), write its hi / lo images, one 64-channel panel at a time,
 //                  and S^T diag(dl) back
 //   MMA thread   : [D1w | D1q] = S^T [w; qg]^T (N = 64 + 64 tokens, K = 128 channels), starting on a panel as soon as it
@@ -16,10 +16,12 @@
 //                  layout), then D1q += vt^T Aqk^T (N = 64); K = 64 tokens
 //   vector warps : o^T = D1q of the chunk before -> bf16 -> global, while the products of this one run (the [D1w | D1q]
 //                  block is double-buffered)
-// A producer warp streams the chunk's operand tiles (written by the prepare kernel in this layout) with 1-D bulk copies,
-// a whole chunk ahead.  Every wait is a bounded mbarrier wait that records a status code and leaves the loops.
-// Bound: the dependent chain, 4200 cycles a chunk: 1540 of D1 and ~900 of the update on the tensor pipe, the rest the two
-// conversions and four hand-overs of ~250 cycles.  It was 5300 with the images in shared memory and o stored two bytes at a time ahead of vt (1 x 8192 tokens, 16 heads, both stages: 526 -> 433 us).
+// A producer warp streams the chunk's operand tiles (written by the prepare kernel in this layout) with 1-D bulk copies:
+// [w; qg] into two stages, a chunk ahead; u^T with dl, and kg with Aqk, into one stage each, as the chunk before releases it.
+// Every wait is a bounded mbarrier wait that records a status code and leaves the loops.
+// Bound: the dependent chain, 4200 to 4400 cycles a chunk, the tensor pipe active for two thirds of them: 1540 of D1 and ~900
+// of the update, the rest the two conversions and four hand-overs of ~250 cycles.  It was 5300 with the images in shared
+// memory and o stored two bytes at a time ahead of vt (1 x 8192 tokens, 16 heads, both stages: 526 -> 433 us).
 //
 // Workspace record of a chunk in this layout (written by kda_prepare_mma_kernel when PrepArgs::umma is set):
 //   0      [w; qg] hi: two 64-channel panels of [128 rows][64] bf16 (rows 0..63 w, 64..127 qg), 128-byte swizzle
