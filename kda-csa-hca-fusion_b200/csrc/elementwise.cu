@@ -31,45 +31,15 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const TW* __restrict__
     stf(yr + i, (ldf(xr + i) - mean) * rstd * ldf(w + i) + ldf(b + i));
 }
 
-// bf16 fast path for d % 256 == 0 and d <= 4096: 8 values per lane per 256 columns, row kept in registers
-template <typename TW, int NV>
-__global__ void layernorm_kernel_bf16_vec(const bf16* __restrict__ x, const TW* __restrict__ w,
-                                          const TW* __restrict__ b, bf16* __restrict__ y, int64_t rows, int d,
-                                          float eps) {
-  int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const bf16* xr = x + row * d;
-  float v[NV][8];
-  float s = 0.f;
+// 8 bf16 values as they were loaded -> fp32.  The values go through an empty asm statement, so that each use converts again
+// instead of keeping a row's fp32 values (twice the registers) from one pass to the next.
+__device__ __forceinline__ void cvt8(uint4& raw, float (&o)[8]) {
+  asm volatile("" : "+r"(raw.x), "+r"(raw.y), "+r"(raw.z), "+r"(raw.w));
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    uint4 raw = *reinterpret_cast<const uint4*>(xr + i * 256 + lane * 8);
-    const bf16* e = reinterpret_cast<const bf16*>(&raw);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { v[i][k] = __bfloat162float(e[k]); s += v[i][k]; }
-  }
-  const float mean = warp_sum(s) / (float)d;
-  float q = 0.f;
-#pragma unroll
-  for (int i = 0; i < NV; ++i)
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { float t = v[i][k] - mean; q += t * t; }
-  const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)d + eps);
-  bf16* yr = y + row * d;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    uint4 outv;
-    bf16* out = reinterpret_cast<bf16*>(&outv);
-    const int c0 = i * 256 + lane * 8;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = __float2bfloat16_rn((v[i][k] - mean) * rstd * ldf(w + c0 + k) + ldf(b + c0 + k));
-    *reinterpret_cast<uint4*>(yr + c0) = outv;
-  }
+  for (int k = 0; k < 4; ++k) { o[2 * k] = __uint_as_float(w[k] << 16); o[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
 }
-
-// A few rows only (a decode batch): one CTA per row, 8 channels per thread, so every load of the row and of the
-// parameters is issued at once and the launch is one memory round trip plus two block reductions.
+// 8 consecutive parameters; `vec`: they start on a 16-byte boundary (one or two 16-byte loads instead of eight narrow ones)
 template <typename TW>
 __device__ __forceinline__ void ld8p(const TW* p, float (&o)[8]) {
   if constexpr (sizeof(TW) == 2) {
@@ -82,6 +52,64 @@ __device__ __forceinline__ void ld8p(const TW* p, float (&o)[8]) {
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
   }
 }
+template <typename TW>
+__device__ __forceinline__ void ld8p(const TW* p, float (&o)[8], bool vec) {
+  if (vec) { ld8p(p, o); return; }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) o[k] = ldf(p + k);
+}
+
+// bf16 fast path for d % 256 == 0 and d <= 2048: 8 values per lane per 256 columns, the row kept in registers as it lies.
+// Bound: HBM, 131072 x 2048 in 202 us (5.3 TB/s).  It was 355 us with parameters loaded two bytes at a time (more L1
+// instructions than the row itself) and the row held as fp32 values, which left two CTAs an SM.
+template <typename TW, int NV>
+__global__ void __launch_bounds__(256, 3) layernorm_kernel_bf16_vec(const bf16* __restrict__ x, const TW* __restrict__ w,
+                                          const TW* __restrict__ b, bf16* __restrict__ y, int64_t rows, int d,
+                                          float eps, bool pvec) {
+  int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const bf16* xr = x + row * d;
+  uint4 raw[NV];                                             // the row as it lies: half the registers of its fp32 values
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) raw[i] = *reinterpret_cast<const uint4*>(xr + i * 256 + lane * 8);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float v[8];
+    cvt8(raw[i], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += v[k];
+  }
+  const float mean = warp_sum(s) / (float)d;
+  float q = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float v[8];
+    cvt8(raw[i], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { const float t = v[k] - mean; q += t * t; }
+  }
+  const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)d + eps);
+  bf16* yr = y + row * d;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    uint4 outv;
+    bf16* out = reinterpret_cast<bf16*>(&outv);
+    const int c0 = i * 256 + lane * 8;
+    float wv[8], bv[8];
+    ld8p(w + c0, wv, pvec);
+    ld8p(b + c0, bv, pvec);
+    float v[8];
+    cvt8(raw[i], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = __float2bfloat16_rn((v[k] - mean) * rstd * wv[k] + bv[k]);
+    *reinterpret_cast<uint4*>(yr + c0) = outv;
+  }
+}
+
+// A few rows only (a decode batch): one CTA per row, 8 channels per thread, so every load of the row and of the
+// parameters is issued at once and the launch is one memory round trip plus two block reductions.
 // sum over the 256 threads of a CTA; `red` is 8 floats of shared memory (reusable after the call returns)
 __device__ __forceinline__ float block_sum_256(float v, float* red) {
   v = warp_sum(v);
@@ -139,9 +167,10 @@ extern "C" int kch_layernorm(const void* x, const void* weight, const void* bias
   }
   if (dtype == KCH_BF16 && (d % 256) == 0 && d <= 2048 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
     cudaStream_t s = kch_stream(stream);
+    const bool pvec = (((uintptr_t)weight | (uintptr_t)bias) & 15) == 0;
 #define LNV(NV)                                                                                              \
     KCH_DISPATCH_FLOAT(wdtype, TW, (layernorm_kernel_bf16_vec<TW, NV><<<grid, block, 0, s>>>(                 \
-        (const bf16*)x, (const TW*)weight, (const TW*)bias, (bf16*)y, rows, d, eps)))
+        (const bf16*)x, (const TW*)weight, (const TW*)bias, (bf16*)y, rows, d, eps, pvec)))
     switch (d / 256) {
       case 1: LNV(1); break; case 2: LNV(2); break; case 3: LNV(3); break; case 4: LNV(4); break;
       case 5: LNV(5); break; case 6: LNV(6); break; case 7: LNV(7); break; default: LNV(8); break;
@@ -283,15 +312,17 @@ extern "C" int kch_short_conv(const void* x, const void* lookback, const void* w
 // and convolves from there, so the normalised activations never travel to HBM and back.  The two
 // normalised rows that end the sequence are written out as the next call's lookback.
 // HBM traffic per token: d*2 bytes in, d*2 bytes out (+ 2/LC_TT re-read of the halo rows, L2 hits).
+// 131072 x 2048: 319 us (3.4 TB/s), 473 with narrow parameter loads and fp32 rows as above; what is left is the barrier
+// between the two halves of a tile at three CTAs an SM.
 // ---------------------------------------------------------------------------------------
 #define LC_TT 14
 #define LC_ROWS (LC_TT + 2)
 
 template <typename TW, int NV>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 ln_conv_kernel_bf16(const bf16* __restrict__ x, const TW* __restrict__ lw, const TW* __restrict__ lb2, float eps,
                     const bf16* __restrict__ lookback, const bf16* __restrict__ cw, const bf16* __restrict__ cb,
-                    bf16* __restrict__ y, bf16* __restrict__ lb_out, int T_, int d) {
+                    bf16* __restrict__ y, bf16* __restrict__ lb_out, int T_, int d, bool pvec) {
   extern __shared__ __align__(16) uint8_t lc_smem[];
   bf16* sh = reinterpret_cast<bf16*>(lc_smem);               // [LC_ROWS][d] normalised rows t0-2 .. t0+LC_TT-1
   const int b = blockIdx.y, t0 = blockIdx.x * LC_TT;
@@ -310,29 +341,39 @@ ln_conv_kernel_bf16(const bf16* __restrict__ x, const TW* __restrict__ lw, const
       continue;
     }
     const bf16* xr = x + ((int64_t)b * T_ + t) * d;
-    float v[NV][8];
+    uint4 raw[NV];                                             // the row as it lies: half the registers of its fp32 values
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      uint4 raw = *reinterpret_cast<const uint4*>(xr + i * 256 + lane * 8);
-      const bf16* e = reinterpret_cast<const bf16*>(&raw);
+    for (int i = 0; i < NV; ++i) raw[i] = *reinterpret_cast<const uint4*>(xr + i * 256 + lane * 8);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { v[i][k] = __bfloat162float(e[k]); s += v[i][k]; }
+    for (int i = 0; i < NV; ++i) {
+      float v[8];
+      cvt8(raw[i], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s += v[k];
     }
     const float mean = warp_sum(s) / (float)d;
     float q = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
+    for (int i = 0; i < NV; ++i) {
+      float v[8];
+      cvt8(raw[i], v);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { float tt = v[i][k] - mean; q += tt * tt; }
+      for (int k = 0; k < 8; ++k) { const float t = v[k] - mean; q += t * t; }
+    }
     const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)d + eps);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       uint4 outv;
       bf16* out = reinterpret_cast<bf16*>(&outv);
       const int c0 = i * 256 + lane * 8;
+      float wv[8], bv[8];
+      ld8p(lw + c0, wv, pvec);
+      ld8p(lb2 + c0, bv, pvec);
+      float v[8];
+      cvt8(raw[i], v);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) out[k] = __float2bfloat16_rn((v[i][k] - mean) * rstd * ldf(lw + c0 + k) + ldf(lb2 + c0 + k));
+      for (int k = 0; k < 8; ++k) out[k] = __float2bfloat16_rn((v[k] - mean) * rstd * wv[k] + bv[k]);
       *reinterpret_cast<uint4*>(dst + c0) = outv;
       if (lb_out && t >= T_ - 2) *reinterpret_cast<uint4*>(lb_out + ((int64_t)b * 2 + (t - (T_ - 2))) * d + c0) = outv;
     }
@@ -388,6 +429,7 @@ extern "C" int kch_layernorm_short_conv(const void* x, const void* ln_weight, co
   const uintptr_t al = (uintptr_t)x | (uintptr_t)y | (uintptr_t)conv_weight | (uintptr_t)conv_bias | (uintptr_t)lookback |
                        (uintptr_t)lookback_out;
   KCH_REQUIRE((al & 15) == 0, "kch_layernorm_short_conv: operands must be 16-byte aligned");
+  const bool pvec = (((uintptr_t)ln_weight | (uintptr_t)ln_bias) & 15) == 0;
   const size_t smem = (size_t)LC_ROWS * d * 2;
   dim3 grid((unsigned)((T + LC_TT - 1) / LC_TT), B);
   cudaStream_t s = kch_stream(stream);
@@ -395,7 +437,7 @@ extern "C" int kch_layernorm_short_conv(const void* x, const void* ln_weight, co
   KCH_DISPATCH_FLOAT(wdtype, TW, {                                                                                 \
     KCH_CUDA_OK(cudaFuncSetAttribute(ln_conv_kernel_bf16<TW, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     ln_conv_kernel_bf16<TW, NV><<<grid, 256, smem, s>>>((const bf16*)x, (const TW*)ln_weight, (const TW*)ln_bias, eps, \
-        (const bf16*)lookback, (const bf16*)conv_weight, (const bf16*)conv_bias, (bf16*)y, (bf16*)lookback_out, T, d); \
+        (const bf16*)lookback, (const bf16*)conv_weight, (const bf16*)conv_bias, (bf16*)y, (bf16*)lookback_out, T, d, pvec); \
   })
   switch (d / 256) {
     case 1: LCV(1); break; case 2: LCV(2); break; case 3: LCV(3); break; case 4: LCV(4); break;
@@ -513,10 +555,6 @@ extern "C" int kch_layernorm_short_conv_step(const void* x, const void* ln_weigh
 //   KCH_ACT_SILU_L2NORM     y = round(s / max(round(||s||), eps)), s = round(silu(x)), per
 //                           group of `group` consecutive columns         (KDA q,k)
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-
 template <typename T>
 __global__ void act_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int cols, int64_t ldx,
                            int64_t ldy, int act, float param) {

@@ -68,6 +68,11 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// the activations of the projections, in fp32
+__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
+__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
+__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+
 // generic load by runtime dtype tag (slow path helpers)
 __device__ __forceinline__ float ld_any(const void* p, int64_t i, int dtype) {
   return dtype == KCH_BF16 ? __bfloat162float(((const bf16*)p)[i]) : ((const float*)p)[i];
