@@ -26,6 +26,10 @@ extern "C" int kch_abi_version(void) { return 1; }
 
 int kch_linear_simt(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K,
                     int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype, void* stream);
+bool kch_linear_f32_epilogue_ok(const kch_epilogue* e, const void* A, const void* W, int64_t M, int N, int K, int64_t lda,
+                                int64_t ldw, int dtype);
+int kch_linear_f32(const void* A, const void* W, void* C, const void* residual, int64_t M, int N, int K, int64_t lda,
+                   int64_t ldw, int64_t ldc, int64_t ldr, const kch_epilogue* e, void* stream);
 bool kch_linear_tcgen05_supported(const void* A, const void* W, const void* C, const void* R, int64_t M, int N,
                                   int K, int64_t lda, int64_t ldw, int64_t ldc, int64_t ldr, int dtype);
 int kch_linear_tcgen05(const void* A, const void* W, void* C, const void* R, int64_t M, int N, int K, int64_t lda,
@@ -75,6 +79,8 @@ static int linear_impl(const void* A, const void* W, void* C, const void* residu
                   kch_linear_tcgen05_supported(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype);
   if (tc && kch_linear_tcgen05_epilogue_ok(ep, N))
     return kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, ep, stream, 0, w_settled);
+  if (!tc && ep && ep->n_segments && kch_linear_f32_epilogue_ok(ep, A, W, M, N, K, lda, ldw, dtype))
+    return kch_linear_f32(A, W, C, nullptr, M, N, K, lda, ldw, ldc, ldr, ep, stream);
   int rc = tc ? kch_linear_tcgen05(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, nullptr, stream, 0, w_settled)
               : kch_linear_simt(A, W, C, residual, M, N, K, lda, ldw, ldc, ldr, dtype, stream);
   if (rc != KCH_OK || !ep || ep->n_segments == 0) return rc;

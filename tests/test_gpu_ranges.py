@@ -375,3 +375,52 @@ def test_weights_changed_between_one_token_steps(kch, names):
             b = kch.HybridDecoding(model=model_of(changed))
             b.import_state(st)
             assert torch.equal(got, b(x[:, t:t + 1])), t
+
+
+@pytest.mark.parametrize("M,N,K,off", [(1, 1, 4, 0), (31, 63, 28, 4), (32, 64, 32, 0), (33, 65, 36, 0), (662, 840, 256, 0),
+                                       (97, 128, 300, 8), (50, 130, 33, 0), (40, 64, 64, 1)])
+@pytest.mark.parametrize("form", ["plain", "residual", "act", "norm"])
+def test_linear_fp32_edges(kch, M, N, K, off, form):
+    """Tiles of 32 x 64 with steps of 32 in K, operands that 16-byte copies cannot read (odd K, odd offset), and the activation
+    segments in the epilogue.  A chain of K fused multiply-adds is off by at most K 2^-24 sum |a||w|; silu, sigmoid and
+    softplus have slopes below 1.1 and add a few units in the last place of values below max(1, |x|)."""
+    from kch_b200 import _lib
+    from kch_b200.csa import linear
+    gen = torch.Generator(device=DEV).manual_seed(M + N + K)
+    wide = torch.randn(M, K + 2 * off + (-(K + 2 * off)) % (4 if off != 1 else 1), generator=gen, device=DEV)
+    x = wide[:, off:off + K]
+    W = torch.randn(N, K, generator=gen, device=DEV) * K ** -0.5
+    y = x.double() @ W.double().T
+    bound = 1.1 * K * 2.0 ** -24 * (x.double().abs() @ W.double().abs().T) + 2.0 ** -21 * y.abs().clamp_min(1.0)
+    if form == "plain":
+        got, ref = linear(x, W), y
+    elif form == "residual":
+        r = torch.randn(M, N, generator=gen, device=DEV)
+        got, ref = linear(x, W, residual=r), y + r.double()
+        bound = bound + 2.0 ** -23 * r.double().abs()
+    elif form == "act":
+        if N < 4:
+            pytest.skip("four segments")
+        c = [0, N // 4, N // 2, N // 2 + 1, N]
+        acts = [(_lib.ACT_SILU, 0.0), (0, 0.0), (_lib.ACT_SIGMOID, 0.0), (_lib.ACT_NEG_SOFTPLUS, 0.1)]
+        got = linear(x, W, epilogue=[(c[i + 1] - c[i], *acts[i]) for i in range(4)])
+        ref = y.clone()
+        ref[:, :c[1]] = torch.nn.functional.silu(y[:, :c[1]])
+        ref[:, c[2]:c[3]] = torch.sigmoid(y[:, c[2]:c[3]])
+        ref[:, c[3]:] = -0.1 * torch.nn.functional.softplus(y[:, c[3]:])
+    else:
+        if N % 64:
+            pytest.skip("whole groups")
+        for group in (64, 32, 16, 4):
+            got = linear(x, W, epilogue=[(64, _lib.ACT_SILU_L2NORM, 0.0)] + ([(N - 64, _lib.ACT_SILU, 0.0)] if N > 64 else []), group=group)
+            s = torch.nn.functional.silu(y)
+            nrm = s[:, :64].unflatten(-1, (-1, group)).norm(dim=-1, keepdim=True)
+            ref = s.clone()
+            ref[:, :64] = (s[:, :64].unflatten(-1, (-1, group)) / nrm).flatten(1)
+            # a quotient moves by the error of its numerator and of the norm, each relative to the norm
+            e = bound[:, :64].unflatten(-1, (-1, group))
+            b = bound.clone()
+            b[:, :64] = ((e + e.norm(dim=-1, keepdim=True)) / nrm).flatten(1) + group * 2.0 ** -23
+            assert bool(((got.double() - ref).abs() <= b).all()), group
+        return
+    assert bool(((got.double() - ref).abs() <= bound).all()), float(((got.double() - ref).abs() - bound).max())
