@@ -5,6 +5,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "kch_common.cuh"
 #include "mma_utils.cuh"
 
@@ -247,8 +249,11 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
 // factored around a row between the two halves of a block (both factors <= 1 for a decay, so nothing overflows, and
 // what underflows is smaller still), halving the blocks from 32 to 4 rows: 8 K exponentials a level and plain products;
 // only the 4 x 4 diagonal blocks take the difference pair by pair.  The inverse is built from 8 x 8 blocks upwards.
-// 1024 tokens, 4 heads, K = V = 128, fp32: 202 -> 42 us.  What holds zero rows only is skipped (8 tokens: 41 -> 23 us, both
-// stages).
+// Of the 78 K cycles that a chunk then took, 14 K were the diagonal blocks (a warp a pair, two reductions each), 9 K the loads
+// (scalar, a few in flight), 8 K the element-wise outputs, 7 K the loads of v, 10 K the products of the two widest levels (2 x 2
+// tiles: the return path of shared memory): 16-byte loads all under way at once, a warp a diagonal block, 4 x 4 tiles.
+// 1024 tokens, 4 heads, K = V = 128, fp32: 202 -> 42 -> 29 us.  What holds zero rows only is skipped (8 tokens: 41 -> 23 us,
+// both stages).
 // A record whose gate is positive or not finite somewhere takes every pair directly.
 // =====================================================================================
 #define KC_C 64
@@ -259,12 +264,37 @@ __host__ __device__ inline int64_t kc_record_floats(int KT, int V) {
   return 3ll * KC_C * (KT + 4) + KC_C * KC_AS + KT + (int64_t)((V + 7) / 8) * 8 * KC_C;
 }
 
+// four consecutive elements as fp32, from a 16-byte (fp32) or 8-byte (bf16) boundary
+__device__ __forceinline__ float4 kc_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 kc_load4(const bf16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
+}
+// sum of each of N values (a power of two) over groups of G lanes; lane l of a group is left with the N / G sums from l * N / G on
+template <int N, int G>
+__device__ __forceinline__ void kc_reduce(float (&v)[N], int lane) {
+  static_assert(N >= G, "a value per lane at least");
+  int n = N;
+#pragma unroll
+  for (int off = G >> 1; off > 0; off >>= 1) {
+    n >>= 1;
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i < n) {
+        const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+  }
+}
+
 template <typename T, int KT>
 __global__ void __launch_bounds__(4 * KT)
 kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                          const T* __restrict__ g, const T* __restrict__ beta, float* __restrict__ ws, int T_,
                          int H, int HV, int K, int V, int NT, int L, int C, float scale, float g_min,
-                         int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b) {
+                         int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b, int vec) {
   constexpr int NTH = 4 * KT, KS = KT + 4, NW = NTH / 32;
   extern __shared__ __align__(16) float smem[];
   float* sk = smem;                    // [64][KS] k
@@ -289,20 +319,52 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
   float* o_u = o_dl + KT;
 
   bool odd_gate = false;
-#pragma unroll 4
-  for (int idx = tid; idx < KC_C * KT; idx += NTH) {
-    const int i = idx / KT, kk = idx % KT, t = t0 + i;
-    float kv = 0.f, qv = 0.f, gv = 0.f;
-    if (t < t_end && kk < K) {
-      const int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
-      kv = ldf(k + qoff);
-      qv = ldf(q + qoff) * scale;
-      gv = fmaxf(ldf(g + ((int64_t)b * T_ + t) * ld_g + (int64_t)hv * K + kk), g_min);
-      odd_gate |= !(gv <= 0.f && gv > -1e30f);
+  if (vec & 1) {                                         // all twelve loads of a thread are under way before the first is used
+    float4 kv[4], qv[4], gv[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int idx = tid + r * NTH, i = idx / (KT / 4), kk = 4 * (idx % (KT / 4)), t = t0 + i;
+      kv[r] = qv[r] = gv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < t_end && kk < K) {
+        const int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
+        kv[r] = kc_load4(k + qoff);
+        qv[r] = kc_load4(q + qoff);
+        gv[r] = kc_load4(g + ((int64_t)b * T_ + t) * ld_g + (int64_t)hv * K + kk);
+      }
     }
-    sk[i * KS + kk] = kv;
-    sq[i * KS + kk] = qv;
-    sgam[i * KS + kk] = gv;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int idx = tid + r * NTH, i = idx / (KT / 4), kk = 4 * (idx % (KT / 4));
+      if (t0 + i < t_end && kk < K) {
+        float* gp = &gv[r].x;
+        float* qp = &qv[r].x;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          gp[e] = fmaxf(gp[e], g_min);
+          odd_gate |= !(gp[e] <= 0.f && gp[e] > -1e30f);
+          qp[e] *= scale;
+        }
+      }
+      *reinterpret_cast<float4*>(sk + i * KS + kk) = kv[r];
+      *reinterpret_cast<float4*>(sq + i * KS + kk) = qv[r];
+      *reinterpret_cast<float4*>(sgam + i * KS + kk) = gv[r];
+    }
+  } else {
+#pragma unroll 4
+    for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+      const int i = idx / KT, kk = idx % KT, t = t0 + i;
+      float kv = 0.f, qv = 0.f, gv = 0.f;
+      if (t < t_end && kk < K) {
+        const int64_t qoff = ((int64_t)b * T_ + t) * ld_qk + (int64_t)h * K + kk;
+        kv = ldf(k + qoff);
+        qv = ldf(q + qoff) * scale;
+        gv = fmaxf(ldf(g + ((int64_t)b * T_ + t) * ld_g + (int64_t)hv * K + kk), g_min);
+        odd_gate |= !(gv <= 0.f && gv > -1e30f);
+      }
+      sk[i * KS + kk] = kv;
+      sq[i * KS + kk] = qv;
+      sgam[i * KS + kk] = gv;
+    }
   }
   if (tid < KC_C) sbeta[tid] = t0 + tid < t_end ? ldf(beta + ((int64_t)b * T_ + t0 + tid) * ld_b + hv) : 0.f;
   for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) {
@@ -352,7 +414,48 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
         }
       }
       __syncthreads();
-      // 2 x 2 outputs per thread group, the channels of a group dealt out to `split` neighbouring lanes
+      if (s >= 16) {
+        // 4 x 4 outputs of A and of Aqk per thread group, the channels dealt out to SPL neighbouring lanes (a 16-byte read is
+        // four cycles of the return path however many lanes share it: 12 reads feed 128 multiply-adds, 6 fed 32)
+        constexpr int SP32 = NTH / 64;
+        auto tile4 = [&](auto spl_tag) {
+          constexpr int SPL = decltype(spl_tag)::value;
+          const int tile = tid / SPL, ks = tid % SPL, per = (s / 4) * (s / 4), blk = tile / per, tb = tile % per;
+          const int ti = tb / (s / 4), tj = tb % (s / 4);
+          const int i0 = blk * 2 * s + s + 4 * ti, j0 = blk * 2 * s + 4 * tj, y0 = blk * s + 4 * ti;
+          float acc[32] = {};
+          for (int f = ks; f < KT / 4; f += SPL) {
+            float4 xi[4], yi[4], xj[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              xi[e] = *reinterpret_cast<const float4*>(sx + (i0 + e) * KS + 4 * f);
+              yi[e] = *reinterpret_cast<const float4*>(sy + (y0 + e) * KS + 4 * f);
+              xj[e] = *reinterpret_cast<const float4*>(sx + (j0 + e) * KS + 4 * f);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                float& a = acc[4 * e + c];
+                float& aq = acc[16 + 4 * e + c];
+                a = fmaf(xi[e].x, xj[c].x, a); a = fmaf(xi[e].y, xj[c].y, a); a = fmaf(xi[e].z, xj[c].z, a); a = fmaf(xi[e].w, xj[c].w, a);
+                aq = fmaf(yi[e].x, xj[c].x, aq); aq = fmaf(yi[e].y, xj[c].y, aq); aq = fmaf(yi[e].z, xj[c].z, aq); aq = fmaf(yi[e].w, xj[c].w, aq);
+              }
+          }
+          kc_reduce<32, SPL>(acc, lane);
+#pragma unroll
+          for (int u = 0; u < 32 / SPL; ++u) {
+            const int v = ks * (32 / SPL) + u, e = (v & 15) >> 2, c = v & 3;
+            if (v < 16) sA[(i0 + e) * KC_AS + j0 + c] = acc[u] * sbeta[i0 + e];
+            else o_aqk[(i0 + e) * KC_AS + j0 + c] = acc[u];
+          }
+        };
+        if (s == 32) tile4(std::integral_constant<int, SP32>{});
+        else tile4(std::integral_constant<int, 2 * SP32>{});
+        __syncthreads();
+        continue;
+      }
+      // narrower blocks: 2 x 2 outputs per thread group, the channels of a group dealt out to `split` neighbouring lanes
       const int split = NTH / (8 * s);
       const int tile = tid / split, ks = tid % split;
       const int per = (s / 2) * (s / 2);                  // tiles of one block
@@ -407,28 +510,71 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     }
   }
   for (int idx = tid; idx < KC_C * KC_AS; idx += NTH) sT[idx] = 0.f;
-  // the 4 x 4 diagonal blocks (every block of the triangle when `direct`): a warp per pair, its lanes over the channels
-  {
-    const int side = direct ? KC_C : 4, pairs = side * (side + 1) / 2, blocks = (rows + side - 1) / side;
-    for (int p = warp; p < blocks * pairs; p += NW) {
-      const int blk = p / pairs;
-      int i = (int)((sqrtf(8.f * (p % pairs) + 1.f) - 1.f) * 0.5f);
-      if ((i + 1) * (i + 2) / 2 <= p % pairs) ++i;
-      if (i * (i + 1) / 2 > p % pairs) --i;
-      const int j = blk * side + p % pairs - i * (i + 1) / 2;
-      i += blk * side;
+  // V of the first tile of columns: under way while the triangle is finished and inverted
+  float4 vraw[4];
+  if (vec & 2) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int idx = tid + r * NTH, i = idx / (KT / 4), c = 4 * (idx % (KT / 4)), t = t0 + i;
+      vraw[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < t_end && c < V) vraw[r] = kc_load4(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + c);
+    }
+  }
+  if (!direct) {
+    // the 4 x 4 diagonal blocks: a warp per block, its lanes over the channels, the 6 + 10 sums of a block reduced together
+    // (a warp per pair, two reductions each, took a fifth of the stage)
+    for (int blk = warp; blk < (rows + 3) / 4; blk += NW) {
+      const int r0 = 4 * blk;
+      float acc[16] = {};                                 // A (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), then Aqk with the diagonal
+#pragma unroll
+      for (int c = 0; c < KT / 32; ++c) {
+        const int kk = lane + 32 * c;
+        float kr[4], qr[4], gr[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          kr[e] = sk[(r0 + e) * KS + kk];
+          qr[e] = sq[(r0 + e) * KS + kk];
+          gr[e] = sgam[(r0 + e) * KS + kk];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j <= i; ++j) {
+            const float e = i == j ? kr[j] : expf(gr[i] - gr[j]) * kr[j];
+            if (j < i) acc[i * (i - 1) / 2 + j] = fmaf(kr[i], e, acc[i * (i - 1) / 2 + j]);
+            acc[6 + i * (i + 1) / 2 + j] = fmaf(qr[i], e, acc[6 + i * (i + 1) / 2 + j]);
+          }
+      }
+#pragma unroll
+      for (int v = 0; v < 16; ++v) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], 16);
+      kc_reduce<16, 16>(acc, lane);
+      const int v = lane & 15, w = v < 6 ? v : v - 6;
+      if (lane < 16) {
+        if (v < 6) {
+          const int i = 1 + (w >= 1) + (w >= 3), j = w - i * (i - 1) / 2;
+          sA[(r0 + i) * KC_AS + r0 + j] = acc[0] * sbeta[r0 + i];
+        } else {
+          const int i = (w >= 1) + (w >= 3) + (w >= 6), j = w - i * (i + 1) / 2;
+          o_aqk[(r0 + i) * KC_AS + r0 + j] = acc[0];
+        }
+      }
+    }
+  } else {
+    // every pair of the triangle: a warp per pair, its lanes over the channels
+    for (int p = warp; p < KC_C * (KC_C + 1) / 2; p += NW) {
+      int i = (int)((sqrtf(8.f * p + 1.f) - 1.f) * 0.5f);
+      if ((i + 1) * (i + 2) / 2 <= p) ++i;
+      if (i * (i + 1) / 2 > p) --i;
+      const int j = p - i * (i + 1) / 2;
+      if (i >= rows) break;
       float a = 0.f, aq = 0.f;
 #pragma unroll
       for (int c = 0; c < KT / 32; ++c) {
         const int kk = lane + 32 * c;
-        const float kj = sk[j * KS + kk];
-        float e = kj;
-        if (i != j || direct) {
-          float d = sgam[i * KS + kk] - sgam[j * KS + kk];
-          for (int s = j >> 4; s < i >> 4; ++s) d += stot[s * KT + kk];
-          if (direct && i / C == j / C) d = fminf(d, 50.f);       // (without `direct` it is at most 0)
-          e = expf(d) * kj;
-        }
+        float d = sgam[i * KS + kk] - sgam[j * KS + kk];
+        for (int s = j >> 4; s < i >> 4; ++s) d += stot[s * KT + kk];
+        if (i / C == j / C) d = fminf(d, 50.f);
+        const float e = expf(d) * sk[j * KS + kk];
         a = fmaf(sk[i * KS + kk], e, a);
         aq = fmaf(sq[i * KS + kk], e, aq);
       }
@@ -455,18 +601,23 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     }
   }
   // ... meanwhile the element-wise outputs, and exp(gamma) k as the operand of w
+  {
+    const int kk = tid % KT, seg = tid / KT;
+    float before = 0.f, after = stot[seg * KT + kk];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const float x = stot[s * KT + kk];
+      before += s < seg ? x : 0.f;
+      after += s > seg ? x : 0.f;
+    }
 #pragma unroll 4
-  for (int idx = tid; idx < KC_C * KT; idx += NTH) {
-    const int i = idx / KT, kk = idx % KT;
-    const int seg = i >> 4;
-    float gm = sgam[i * KS + kk], rest = stot[seg * KT + kk] - gm;     // gamma, gamma_last - gamma
-    for (int s = 0; s < seg; ++s) gm += stot[s * KT + kk];
-    for (int s = seg + 1; s < 4; ++s) rest += stot[s * KT + kk];
-    const float eg = expf(gm), kv = sk[i * KS + kk];
-    sx[i * KS + kk] = eg * kv;
-    o_qg[i * KS + kk] = sq[i * KS + kk] * eg;
-    o_kg[i * KS + kk] = kv * expf(rest);
-    if (i == KC_C - 1) o_dl[kk] = eg;
+    for (int i = 16 * seg; i < 16 * seg + 16; ++i) {
+      const float gl = sgam[i * KS + kk], kv = sk[i * KS + kk], eg = expf(gl + before);        // gamma; then gamma_last - gamma
+      sx[i * KS + kk] = eg * kv;
+      o_qg[i * KS + kk] = sq[i * KS + kk] * eg;
+      o_kg[i * KS + kk] = kv * expf(after - gl);
+      if (i == KC_C - 1) o_dl[kk] = eg;
+    }
   }
   __syncthreads();
   // ... then [[T00, 0], [-T11 A10 T00, T11]] for blocks of 8, 16 and 32
@@ -524,10 +675,18 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
     *reinterpret_cast<float4*>(o_w + (4 * ti + r) * KS + tc) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
   for (int v0 = 0; v0 < V; v0 += KT) {
     __syncthreads();
+    if (v0 == 0 && (vec & 2)) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int idx = tid + r * NTH;
+        *reinterpret_cast<float4*>(sx + (idx / (KT / 4)) * KS + 4 * (idx % (KT / 4))) = vraw[r];
+      }
+    } else {
 #pragma unroll 4
-    for (int idx = tid; idx < KC_C * KT; idx += NTH) {
-      const int i = idx / KT, c = idx % KT, t = t0 + i;
-      sx[i * KS + c] = t < t_end && v0 + c < V ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + v0 + c) : 0.f;
+      for (int idx = tid; idx < KC_C * KT; idx += NTH) {
+        const int i = idx / KT, c = idx % KT, t = t0 + i;
+        sx[i * KS + c] = t < t_end && v0 + c < V ? ldf(v + ((int64_t)b * T_ + t) * ld_v + (int64_t)hv * V + v0 + c) : 0.f;
+      }
     }
     __syncthreads();
     product(acc);
@@ -541,42 +700,42 @@ kda_chunk_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, const
 }
 
 // =====================================================================================
-// Stage 2 (sequential over chunks): one CTA owns 8 value columns of one (batch, value head) and keeps that slice of
+// Stage 2 (sequential over chunks): one CTA owns VS = 8 or 4 value columns of one (batch, value head) and keeps that slice of
 // the state in shared memory.
 //   vt = u - w S ; o = qg S + Aqk vt ; S <- diag(dl) S + kg^T vt
-// Bound: shared-memory wavefronts (each operand row is read once per 8 columns) and the four barriers of a chunk.
-// 8 columns instead of 32: a chunk's step is shortened, not the chain of chunks, by spreading a head over
-// V / 8 CTAs (a single sequence of a few heads leaves the chip idle otherwise); the next chunk's operands are
+// Bound: shared-memory wavefronts (each operand row is read once per VS columns) and the four barriers of a chunk.
+// Few columns instead of 32: a chunk's step is shortened, not the chain of chunks, by spreading a head over
+// V / VS CTAs (a single sequence of a few heads leaves the chip idle otherwise); the next chunk's operands are
 // bulk-copied into the buffers as each product releases them, so no step waits for memory.
-// 1024 tokens, 4 heads, K = V = 128, fp32: 257 -> 52 us (16 dependent chunks).
+// 1024 tokens, 4 heads, K = V = 128, fp32: 257 -> 52 us with 8 columns -> 37 with 4 (16 dependent chunks); 2 x 2011 tokens, 4
+// heads of 64: 76 -> 48.
 // =====================================================================================
-#define KC_VS 8
-template <typename T, int KT>
+template <typename T, int KT, int VS>
 __global__ void __launch_bounds__(256)
 kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0, T* __restrict__ o,
                       float* __restrict__ S_out, int T_, int HV, int K, int V, int NT, int L, unsigned int* status) {
-  constexpr int KS = KT + 4, IG = 256 / KT, IR = KC_C / IG;
+  constexpr int KS = KT + 4, IG = 256 / KT, IR = KC_C / IG, N4 = VS / 4;
   extern __shared__ __align__(16) float smem[];
   float* sw = smem;                          // [64][KS], then qg [64][KS]
   float* sqg = sw + KC_C * KS;
   float* skg = sqg + KC_C * KS;              // [64][KS]
   float* saqk = skg + KC_C * KS;             // [64][68], dl [KT] behind it as in the record
   float* sdl = saqk + KC_C * KC_AS;
-  float* su = sdl + KT;                      // [64][8]
-  float* sS = su + KC_C * KC_VS;             // [KT][8]
-  float* svt = sS + KT * KC_VS;              // [64][8]
-  float4* red = reinterpret_cast<float4*>(svt + KC_C * KC_VS);      // [4][2][64]: partial sums of w S, then of o
-  float4* red3 = red + 4 * 2 * KC_C;                                // [IG][2][KT]: partial sums of kg^T vt
-  uint64_t* bars = reinterpret_cast<uint64_t*>(red3 + IG * 2 * KT); // w + qg + u | Aqk + dl | kg
+  float* su = sdl + KT;                      // [64][8]: the record keeps u in groups of 8 columns
+  float* sS = su + KC_C * 8;                 // [KT][VS]
+  float* svt = sS + KT * VS;                 // [64][VS]
+  float4* red = reinterpret_cast<float4*>(svt + KC_C * VS);          // [4][N4][64]: partial sums of w S, then of o
+  float4* red3 = red + 4 * N4 * KC_C;                                // [IG][N4][KT]: partial sums of kg^T vt
+  uint64_t* bars = reinterpret_cast<uint64_t*>(red3 + IG * N4 * KT); // w + qg + u | Aqk + dl | kg
   const int vb = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x;
-  const int v0 = vb * KC_VS;
+  const int v0 = vb * VS, u4 = (v0 & 7) / 4;            // first of its columns; its first float4 of a group of 8
   const int64_t bh = (int64_t)b * HV + hv, rf = kc_record_floats(KT, V), sbase = bh * K * V;
   const float* rec = ws + bh * NT * rf;
   auto load_w = [&](int n) {
-    mbarrier_expect_tx(&bars[0], (2 * KC_C * KS + KC_C * KC_VS) * 4);
+    mbarrier_expect_tx(&bars[0], (2 * KC_C * KS + KC_C * 8) * 4);
     bulk_copy_g2s(sw, rec + n * rf, 2 * KC_C * KS * 4, &bars[0]);
-    bulk_copy_g2s(su, rec + n * rf + 3 * KC_C * KS + KC_C * KC_AS + KT + (int64_t)vb * KC_C * KC_VS, KC_C * KC_VS * 4, &bars[0]);
+    bulk_copy_g2s(su, rec + n * rf + 3 * KC_C * KS + KC_C * KC_AS + KT + (int64_t)(v0 / 8) * KC_C * 8, KC_C * 8 * 4, &bars[0]);
   };
   auto load_a = [&](int n) {
     mbarrier_expect_tx(&bars[1], (KC_C * KC_AS + KT) * 4);
@@ -593,8 +752,8 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
     load_a(0);
     load_k(0);
   }
-  for (int idx = tid; idx < KT * KC_VS; idx += 256) {
-    const int kk = idx / KC_VS, c = idx % KC_VS;
+  for (int idx = tid; idx < KT * VS; idx += 256) {
+    const int kk = idx / VS, c = idx % VS;
     sS[idx] = (S0 && kk < K && v0 + c < V) ? S0[sbase + (int64_t)kk * V + v0 + c] : 0.f;
   }
   __syncthreads();
@@ -608,7 +767,7 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
   for (int n = 0; n < NT; ++n) {
     ok = ok && mbarrier_wait_bounded(&bars[0], n & 1, KCH_STATUS_KDA_CHUNK, 1u << 24, status);
     // partial sums of w S and qg S: row r, a quarter of the channels
-    float4 aw[2] = {}, aq[2] = {};
+    float4 aw[N4] = {}, aq[N4] = {};
 #pragma unroll 4
     for (int kk = ks * (KT / 4); kk < (ks + 1) * (KT / 4); kk += 4) {
       const float4 w4 = *reinterpret_cast<const float4*>(sw + r * KS + kk);
@@ -616,23 +775,26 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
       const float wv[4] = {w4.x, w4.y, w4.z, w4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float4 s0 = S4[2 * (kk + e)], s1 = S4[2 * (kk + e) + 1];
-        add4(aw[0], wv[e], s0); add4(aw[1], wv[e], s1);
-        add4(aq[0], qv[e], s0); add4(aq[1], qv[e], s1);
+#pragma unroll
+        for (int c = 0; c < N4; ++c) {
+          const float4 s = S4[N4 * (kk + e) + c];
+          add4(aw[c], wv[e], s);
+          add4(aq[c], qv[e], s);
+        }
       }
     }
-    red[(ks * 2) * KC_C + r] = aw[0];
-    red[(ks * 2 + 1) * KC_C + r] = aw[1];
+#pragma unroll
+    for (int c = 0; c < N4; ++c) red[(ks * N4 + c) * KC_C + r] = aw[c];
     __syncthreads();
-    if (tid < 2 * KC_C) {
+    if (tid < N4 * KC_C) {
       const int c4 = tid >> 6;
-      float4 x = reinterpret_cast<const float4*>(su)[2 * r + c4];
+      float4 x = reinterpret_cast<const float4*>(su)[2 * r + u4 + c4];
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
-        const float4 y = red[(p * 2 + c4) * KC_C + r];
+        const float4 y = red[(p * N4 + c4) * KC_C + r];
         x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
       }
-      reinterpret_cast<float4*>(svt)[2 * r + c4] = x;
+      reinterpret_cast<float4*>(svt)[N4 * r + c4] = x;
     }
     __syncthreads();
     if (tid == 0 && ok && n + 1 < NT) load_w(n + 1);
@@ -643,45 +805,45 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
       const float av[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        add4(aq[0], av[e], vt4[2 * (j + e)]);
-        add4(aq[1], av[e], vt4[2 * (j + e) + 1]);
+#pragma unroll
+        for (int c = 0; c < N4; ++c) add4(aq[c], av[e], vt4[N4 * (j + e) + c]);
       }
     }
-    red[(ks * 2) * KC_C + r] = aq[0];
-    red[(ks * 2 + 1) * KC_C + r] = aq[1];
+#pragma unroll
+    for (int c = 0; c < N4; ++c) red[(ks * N4 + c) * KC_C + r] = aq[c];
     ok = ok && mbarrier_wait_bounded(&bars[2], n & 1, KCH_STATUS_KDA_CHUNK, 1u << 24, status);
     {
       const int kk = tid % KT, ig = tid / KT;
-      float4 as[2] = {};
+      float4 as[N4] = {};
 #pragma unroll 8
       for (int i = ig * IR; i < (ig + 1) * IR; ++i) {
         const float kv = skg[i * KS + kk];
-        add4(as[0], kv, vt4[2 * i]);
-        add4(as[1], kv, vt4[2 * i + 1]);
+#pragma unroll
+        for (int c = 0; c < N4; ++c) add4(as[c], kv, vt4[N4 * i + c]);
       }
-      red3[(ig * 2) * KT + kk] = as[0];
-      red3[(ig * 2 + 1) * KT + kk] = as[1];
+#pragma unroll
+      for (int c = 0; c < N4; ++c) red3[(ig * N4 + c) * KT + kk] = as[c];
     }
     __syncthreads();
     if (tid == 0 && ok && n + 1 < NT) load_k(n + 1);
-    for (int idx = tid; idx < 2 * KT; idx += 256) {
+    for (int idx = tid; idx < N4 * KT; idx += 256) {
       const int kk = idx % KT, c4 = idx / KT;
-      float4 x = reinterpret_cast<float4*>(sS)[2 * kk + c4];
+      float4 x = reinterpret_cast<float4*>(sS)[N4 * kk + c4];
       const float d = sdl[kk];
       x.x *= d; x.y *= d; x.z *= d; x.w *= d;
 #pragma unroll
       for (int p = 0; p < IG; ++p) {
-        const float4 y = red3[(p * 2 + c4) * KT + kk];
+        const float4 y = red3[(p * N4 + c4) * KT + kk];
         x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
       }
-      reinterpret_cast<float4*>(sS)[2 * kk + c4] = x;
+      reinterpret_cast<float4*>(sS)[N4 * kk + c4] = x;
     }
-    if (tid < 2 * KC_C) {
-      const int c4 = tid >> 6, t = n * L + r;
+    if (tid >= 256 - N4 * KC_C) {          // (with four columns: warps that had no share of the state)
+      const int c4 = N4 == 1 ? 0 : (tid - 128) >> 6, t = n * L + r;
       float4 x = red[c4 * KC_C + r];
 #pragma unroll
       for (int p = 1; p < 4; ++p) {
-        const float4 y = red[(p * 2 + c4) * KC_C + r];
+        const float4 y = red[(p * N4 + c4) * KC_C + r];
         x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
       }
       if (r < L && t < T_ && ok) {
@@ -700,8 +862,8 @@ kda_chunk_scan_kernel(const float* __restrict__ ws, const float* __restrict__ S0
     return;
   }
   if (S_out)
-    for (int idx = tid; idx < KT * KC_VS; idx += 256) {
-      const int kk = idx / KC_VS, c = idx % KC_VS;
+    for (int idx = tid; idx < KT * VS; idx += 256) {
+      const int kk = idx / VS, c = idx % VS;
       if (kk < K && v0 + c < V) S_out[sbase + (int64_t)kk * V + v0 + c] = sS[idx];
     }
 }
@@ -710,9 +872,9 @@ static size_t kc_prepare_smem(int KT) {
   const int KS = KT + 4;
   return ((size_t)4 * KC_C * KS + (32 * KS > KC_C * KC_AS ? 32 * KS : KC_C * KC_AS) + KC_C * KC_AS + KC_C + 4 * KT) * sizeof(float);
 }
-static size_t kc_scan_smem(int KT) {
-  return ((size_t)3 * KC_C * (KT + 4) + KC_C * KC_AS + KT + 2 * KC_C * KC_VS + KT * KC_VS + 4 * 2 * KC_C * 4 +
-          (256 / KT) * 2 * KT * 4) * sizeof(float) + 3 * sizeof(uint64_t);
+static size_t kc_scan_smem(int KT, int VS) {
+  return ((size_t)3 * KC_C * (KT + 4) + KC_C * KC_AS + KT + KC_C * 8 + KC_C * VS + KT * VS + 4 * VS * KC_C +
+          (256 / KT) * VS * KT) * sizeof(float) + 3 * sizeof(uint64_t);
 }
 static int kc_padded_k(int K) { return K <= 64 ? 64 : 128; }
 // tokens of a chunk (what the clamp of a growing gate's exponents counts by), and of a record
@@ -792,23 +954,31 @@ static int kda_chunk_impl(const void* q, const void* k, const void* v, const voi
   unsigned int* status = kch_status_device_ptr();
   KCH_REQUIRE(status != nullptr, "kch_kda_chunk: cannot resolve the device status word");
   cudaStream_t s = kch_stream(stream);
-  const size_t smem1 = kc_prepare_smem(KT), smem2 = kc_scan_smem(KT);
-  const dim3 g1(NT, HV, B), g2((V + KC_VS - 1) / KC_VS, HV, B);
-#define GO(T_, KT_)                                                                                       \
+  // value columns of a CTA of the scan: 8, or 4 where twice the CTAs still get an SM each (beyond that two of them would share
+  // one and read every operand row twice as often)
+  const int VS = (int64_t)((V + 3) / 4) * HV * B <= 148 ? 4 : 8;
+  // four elements a load: q, k, g (1), v (2)
+  const int es = dtype == KCH_BF16 ? 2 : 4;
+  const int vec = ((K % 4) == 0 && (ld_qk % 4) == 0 && (ld_g % 4) == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)g) % (4 * es)) == 0 ? 1 : 0) |
+                  ((V % 4) == 0 && (ld_v % 4) == 0 && ((uintptr_t)v % (4 * es)) == 0 ? 2 : 0);
+  const size_t smem1 = kc_prepare_smem(KT), smem2 = kc_scan_smem(KT, VS);
+  const dim3 g1(NT, HV, B), g2((V + VS - 1) / VS, HV, B);
+#define GO(T_, KT_, VS_)                                                                                       \
   do {                                                                                                    \
     KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_prepare_kernel<T_, KT_>,                                   \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));           \
-    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_scan_kernel<T_, KT_>,                                      \
+    KCH_CUDA_OK(cudaFuncSetAttribute(kda_chunk_scan_kernel<T_, KT_, VS_>,                                      \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));           \
     kda_chunk_prepare_kernel<T_, KT_><<<g1, 4 * KT_, smem1, s>>>((const T_*)q, (const T_*)k,              \
         (const T_*)v, (const T_*)g, (const T_*)beta, ws, T, H, HV, K, V, NT, L, C, scale, g_clamp_min,    \
-        ld_qk, ld_v, ld_g, ld_beta);                                                                             \
-    kda_chunk_scan_kernel<T_, KT_><<<g2, 256, smem2, s>>>(ws, initial_state, (T_*)o, final_state, T, HV,  \
+        ld_qk, ld_v, ld_g, ld_beta, vec);                                                                        \
+    kda_chunk_scan_kernel<T_, KT_, VS_><<<g2, 256, smem2, s>>>(ws, initial_state, (T_*)o, final_state, T, HV,  \
         K, V, NT, L, status);                                                                             \
   } while (0)
   KCH_DISPATCH_FLOAT(dtype, T_, {
-    if (KT == 64) GO(T_, 64);
-    else GO(T_, 128);
+    if (KT == 64) { if (VS == 4) GO(T_, 64, 4); else GO(T_, 64, 8); }
+    else if (VS == 4) GO(T_, 128, 4);
+    else GO(T_, 128, 8);
   });
 #undef GO
   kch_note_launch(1);  // two kernels per call

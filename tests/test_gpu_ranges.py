@@ -424,3 +424,21 @@ def test_linear_fp32_edges(kch, M, N, K, off, form):
             assert bool(((got.double() - ref).abs() <= b).all()), group
         return
     assert bool(((got.double() - ref).abs() <= bound).all()), float(((got.double() - ref).abs() - bound).max())
+
+
+@pytest.mark.parametrize("B,T,H,HV,K,V,dtype,off", [
+    (2, 130, 4, 4, 128, 128, torch.float32, 0), (3, 70, 2, 4, 64, 100, torch.float32, 0), (2, 65, 4, 8, 64, 36, torch.bfloat16, 0),
+    (1, 90, 2, 2, 64, 64, torch.bfloat16, 2), (1, 90, 1, 2, 128, 36, torch.float32, 1), (1, 67, 1, 1, 62, 38, torch.float32, 0)])
+def test_kda_chunk_generic_columns(kch, B, T, H, HV, K, V, dtype, off):
+    """Four or eight value columns per CTA of the scan (by the number of CTAs), columns that fill neither, and operands that loads
+    of four elements cannot read (odd widths, an odd offset).  Bounds as in test_kda_chunk_fp32_edges; bf16 adds the rounding
+    of the output."""
+    ins = list(syn.kda_inputs(9 * T + V, B, T, H, K, V, HV, dtype, with_state=True))
+    S0 = ins.pop()
+    o_ref, s_ref = orc.recurrent_kda(*(x.double() for x in ins), initial_state=S0.double())
+    if off:                       # the same values behind an odd offset
+        ins = [torch.cat([x.new_zeros(off), x.flatten()]).to(DEV)[off:].view(x.shape) for x in ins]
+    o, s = kch.naive_chunk_kda(*(x.to(DEV) for x in ins), initial_state=S0.to(DEV), output_final_state=True, chunk_size=64)
+    assert md(s, s_ref) <= 2e-5, md(s, s_ref)
+    d = (o.double().cpu() - o_ref).abs()
+    assert bool((d <= 2e-5 + (o_ref.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0)).all()), float(d.max())
