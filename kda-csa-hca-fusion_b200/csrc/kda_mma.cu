@@ -690,15 +690,46 @@ bool kch_kda_scan_tc5_enabled();      // kda_scan_tc5.cu
 int kch_kda_scan_tc5(const void* workspace, const float* initial_state, void* o, float* final_state, int B, int T,
                      int Tb, int HV, int NT, unsigned int* status, cudaStream_t s);
 
+int kch_kda_scan_segments(int BH, int NT, float* us);
+int64_t kch_kda_scan_split_bytes(int BH, int nseg);
+int kch_kda_scan_tc5_split(const void* workspace, void* split, int nseg, const float* initial_state, void* o, float* final_state,
+                           int B, int T, int HV, int NT, unsigned int* status, cudaStream_t s);
+
 bool kch_kda_mma_supported(int K, int V, int chunk_size, float g_clamp_min, int dtype) {
   static const bool force_generic = [] { const char* e = getenv("KCH_KDA"); return e && e[0] == 'g'; }();
   return !force_generic && dtype == KCH_BF16 && K == KM_K && V == KM_V && chunk_size == KM_C && g_clamp_min >= -10.0f;
 }
 
-// chunk records, then one fp32 state per (batch, head): the carry between the segments of a long sequence
+// Segments scanned side by side (kda_scan_tc5.cu) instead of one chain a head: their number where that is the faster one, else 0.
+// Estimates in us: 0.055 a chunk and head in the prepare stage, 2.25 a chunk in a chain.  The chain overlaps with the prepare
+// stage over three quarters of a sequence of 64 chunks or more, each slowing the other; the segments wait for all of it, and for
+// two passes and the join.
+// Both sides measured, chain / segments (us, both stages, the model's gate), the line between the brackets:
+//   1 head:   12 chunks 69 / 71  [  20: 85 / 79    64: 211 / 114   512: 1263 / 278
+//   16 heads: 12 chunks 71 / 75  [  20: 105 / 101  64: 251 / 183   128: 442 / 306   512: 1440 / 1025
+//   28 heads: 20 chunks 116 / 122 [ 32: 173 / 169  63: 296 / 259  96: 391 / 368  128: 489 / 468  256: 860 / 863
+//   36 heads: 32 chunks 185 / 185 [ 63: 335 / 312 ] 96: 442 / 443  256: 993 / 1086
+// With more heads than a third of the SMs pass 1 no longer fits one wave and the chain stays.
+static int km_split(int B, int T, int HV) {
+  static const int seg_env = [] { const char* e = getenv("KCH_KDA_SPLIT"); return e ? atoi(e) : -1; }();
+  if (seg_env == 0 || !kch_kda_scan_tc5_enabled()) return 0;
+  const int NT = (T + KM_C - 1) / KM_C;
+  if ((int64_t)B * HV > 148) return 0;
+  float scan = 0.f;
+  const int P = kch_kda_scan_segments(B * HV, NT, &scan);
+  if (!P) return 0;
+  const float prep = 0.055f * NT * B * HV, chain = 2.25f * NT;
+  const float plain = NT >= 64 ? prep * 0.25f + fmaxf(prep, chain) * 0.75f + chain * 0.25f + fminf(prep, chain) * 0.35f : prep + chain;
+  const float split = prep + scan + 0.6f * B * HV;
+  return split < plain || seg_env == 1 ? P : 0;
+}
+
+// chunk records, then one fp32 state per (batch, head): the carry between the segments of a long sequence; or what the
+// segments that are scanned side by side need
 int64_t kch_kda_mma_workspace_bytes(int B, int T, int HV) {
   int64_t NT = (T + KM_C - 1) / KM_C;
-  return (int64_t)B * HV * NT * KM_CHUNK_BYTES + (int64_t)B * HV * KM_K * KM_V * 4;
+  const int P = km_split(B, T, HV);
+  return (int64_t)B * HV * NT * KM_CHUNK_BYTES + (P ? kch_kda_scan_split_bytes(B * HV, P) : (int64_t)B * HV * KM_K * KM_V * 4);
 }
 
 // Side stream and events of the segmented driver below (one set per device, created on first use).
@@ -756,6 +787,13 @@ int kch_kda_chunk_mma(const void* q, const void* k, const void* v, const void* g
   int nsegs = seg_env > 0 ? seg_env : (NT >= 64 ? 4 : 1);
   if (nsegs > KM_MAX_SEG) nsegs = KM_MAX_SEG;
   if (nsegs > NT) nsegs = NT > 0 ? NT : 1;
+  const int split = pa.umma && !prep_mma && seg_env == 0 ? km_split(B, T, HV) : 0;
+  if (split) {
+    int rc = launch_kda_prepare_tc5(pa, B, status, s);
+    if (rc != KCH_OK) return rc;
+    return kch_kda_scan_tc5_split(workspace, (uint8_t*)workspace + (int64_t)B * HV * NT * KM_CHUNK_BYTES, split, initial_state, o,
+                                  final_state, B, T, HV, NT, status, s);
+  }
   if (pa.umma && !prep_mma && nsegs > 1) {
     KmSideStream* ss = nullptr;
     int rc = km_side_stream(&ss);

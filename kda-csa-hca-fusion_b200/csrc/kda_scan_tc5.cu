@@ -58,6 +58,11 @@ struct T5Args {
   int T, HV, NT;                     // T: tokens from the first chunk of this launch to the end of the sequence
   int Tb;                            // tokens between consecutive batch entries (the whole sequence length)
   int o_vec;                         // o is 8-byte aligned
+  // A sequence in `nseg` segments of `per` chunks, scanned side by side (0: the whole sequence in one CTA, see the host part)
+  int nseg, per, pass;
+  float* starts;                     // [nseg][B * HV] states at the start of each segment, [k][v]
+  float* trans;                      // [nseg][B * HV] transition of each segment, transposed: [k'][k]
+  const uint32_t* serial;            // [B * HV] != 0: a transition expands, segments 1 .. nseg - 1 are one chain
 };
 
 // shared-memory map (bytes, 1024-aligned operand tiles)
@@ -104,8 +109,35 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   const int hv = blockIdx.x, b = blockIdx.y;
   const int warp = t5_warp_index(), lane = threadIdx.x & 31;
   const int64_t bh = (int64_t)b * a.HV + hv;
-  const uint8_t* wsb = a.ws + bh * a.NT * (int64_t)T5_CHUNK_BYTES;
   constexpr uint32_t TMEM_COLS = 512;
+  // this CTA's run of chunks, what it starts from and what it leaves behind
+  int n0 = 0, NT = a.NT;
+  const float* S0 = a.S0 ? a.S0 + bh * (128 * 128) : nullptr;
+  float* S_out = a.S_out ? a.S_out + bh * (128 * 128) : nullptr;
+  bool with_o = true, with_u = true;                             // with_u false: rows of the identity instead of values
+  if (a.nseg) {
+    const int z = blockIdx.z, seg = a.pass == 1 ? (z + 1) / 2 : z + 1;
+    const int64_t slot = (int64_t)gridDim.x * gridDim.y;
+    n0 = seg * a.per;
+    NT = min(a.per, a.NT - n0);
+    if (a.pass == 1) {
+      S_out = a.starts + ((int64_t)(seg + 1) * slot + bh) * (128 * 128);
+      if (seg > 0) {
+        S0 = nullptr;
+        with_o = false;
+        with_u = z & 1;
+        if (!with_u) S_out = a.trans + ((int64_t)seg * slot + bh) * (128 * 128);
+      }
+    } else {
+      const bool chain = a.serial[bh] != 0u;
+      if (chain && seg > 1) return;
+      S0 = a.starts + ((int64_t)seg * slot + bh) * (128 * 128);
+      if (chain) NT = a.NT - n0;
+      else if (seg + 1 < a.nseg) S_out = nullptr;
+    }
+  }
+  const int T_left = a.T - n0 * 64;                              // tokens from this run's first chunk to the end of the sequence
+  const uint8_t* wsb = a.ws + (bh * a.NT + n0) * (int64_t)T5_CHUNK_BYTES;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbarrier_init(w_full + i, 1); mbarrier_init(w_empty + i, 1); }
@@ -126,20 +158,25 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     if (t5_elect()) {
-      for (int n = 0; n < a.NT; ++n) {
+      for (int n = 0; n < NT; ++n) {
         const uint8_t* src = wsb + (int64_t)n * T5_CHUNK_BYTES;
         const int st = n & 1;
         const uint32_t ph = (uint32_t)n & 1;
         if (!mbarrier_wait_bounded(w_empty + st, ((uint32_t)(n >> 1) & 1) ^ 1, 41, T5_SPIN, a.status)) break;
-        mbarrier_expect_tx(w_full + st, 4 * 16384);
-        bulk_copy_g2s(sm + T5_TW + st * 65536, src + T5_OFF_WHI, 4 * 16384, w_full + st);     // [w; qg] hi panels, then lo panels
+        mbarrier_expect_tx(w_full + st, with_o ? 4 * 16384 : 4 * 8192);
+        if (with_o) {
+          bulk_copy_g2s(sm + T5_TW + st * 65536, src + T5_OFF_WHI, 4 * 16384, w_full + st);   // [w; qg] hi panels, then lo panels
+        } else {                                                                              // w only
+          for (int i = 0; i < 4; ++i) bulk_copy_g2s(sm + T5_TW + st * 65536 + i * 16384, src + T5_OFF_WHI + i * 16384, 8192, w_full + st);
+        }
         if (!mbarrier_wait_bounded(u_empty, ph ^ 1, 54, T5_SPIN, a.status)) break;
-        mbarrier_expect_tx(u_full, 32768 + 512);
-        bulk_copy_g2s(sm + T5_TU, src + T5_OFF_U, 32768 + 512, u_full);                       // u^T, dl
+        mbarrier_expect_tx(u_full, with_u ? 32768 + 512 : 512);                               // u^T, dl
+        if (with_u) bulk_copy_g2s(sm + T5_TU, src + T5_OFF_U, 32768 + 512, u_full);
+        else bulk_copy_g2s(sm + T5_TU + 32768, src + T5_OFF_U + 32768, 512, u_full);
         if (!mbarrier_wait_bounded(k_empty, ph ^ 1, 42, T5_SPIN, a.status)) break;
-        mbarrier_expect_tx(k_full, 2 * 16384 + 16384);
+        mbarrier_expect_tx(k_full, with_o ? 2 * 16384 + 16384 : 2 * 16384);
         bulk_copy_g2s(sm + T5_TK, src + T5_OFF_KHI, 2 * 16384, k_full);                       // kg hi, lo
-        bulk_copy_g2s(sm + T5_TA, src + T5_OFF_AQK, 16384, k_full);                           // Aqk hi, lo
+        if (with_o) bulk_copy_g2s(sm + T5_TA, src + T5_OFF_AQK, 16384, k_full);               // Aqk hi, lo
       }
     }
   } else if (warp == 1) {
@@ -148,13 +185,14 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       const uint32_t id64 = t5_idesc(64), id128 = t5_idesc(128), id128mn = t5_idesc(128) | (1u << 16);
       const uint64_t dw0 = t5_desc(smem_addr_u32(sm + T5_TW)), da0 = t5_desc(smem_addr_u32(sm + T5_TA));
       const uint64_t dk0 = t5_desc_mn(smem_addr_u32(sm + T5_TK));
-      for (int n = 0; n < a.NT; ++n) {
+      for (int n = 0; n < NT; ++n) {
         const uint32_t ph = (uint32_t)n & 1, sph = (uint32_t)(n >> 1) & 1;
         const int st = n & 1;
         const uint64_t dw = dw0 + (uint64_t)(st * 65536 >> 4);
         const uint32_t tD = tDD + 128u * ph;                 // [D1w | D1q] of this chunk; vt^T images over D1w
         if (!mbarrier_wait_bounded(w_full + st, sph, 44, T5_SPIN, a.status)) break;
-        // [D1w | D1q] = S^T [w; qg]^T, a 64-channel panel at a time: terms (S hi, x hi), (S lo, x hi), (S hi, x lo)
+        // [D1w | D1q] = S^T [w; qg]^T (D1w alone without an output), a 64-channel panel at a time: terms (S hi, x hi),
+        // (S lo, x hi), (S hi, x lo)
         bool ok = true;
 #pragma unroll
         for (int pan = 0; pan < 2; ++pan) {
@@ -165,7 +203,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
               t5_mma_ts(tD, tSA + (term == 1 ? 64u : 0u) + 32u * pan + 8u * ks, dw + ((term == 2 ? 32768u : 0u) + pan * 16384u >> 4) + 2 * ks,
-                        id128, (pan | term | ks) ? 1u : 0u);
+                        with_o ? id128 : id64, (pan | term | ks) ? 1u : 0u);
         }
         if (!ok) break;
         t5_commit(d1_full);
@@ -187,13 +225,15 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
         }
         if (!ok) break;
         t5_commit(s_full);
-        // D1q += vt^T Aqk^T
+        if (with_o) {
+          // D1q += vt^T Aqk^T
 #pragma unroll
-        for (int term = 0; term < 3; ++term)
+          for (int term = 0; term < 3; ++term)
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            t5_mma_ts(tD + 64, tD + (term == 1 ? 16u : 0u) + 32u * (ks >> 1) + 8u * (ks & 1), da0 + ((term == 2 ? 8192u : 0u) >> 4) + 2 * ks, id64, 1u);
-        t5_commit(o_full);
+            for (int ks = 0; ks < 4; ++ks)
+              t5_mma_ts(tD + 64, tD + (term == 1 ? 16u : 0u) + 32u * (ks >> 1) + 8u * (ks & 1), da0 + ((term == 2 ? 8192u : 0u) >> 4) + 2 * ks, id64, 1u);
+          t5_commit(o_full);
+        }
         t5_commit(k_empty);
       }
     }
@@ -209,7 +249,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int kc = 64 * pan + 32 * sub + j;
-        r[j] = a.S0 ? __float_as_uint(a.S0[bh * (128 * 128) + (int64_t)kc * 128 + v]) : 0u;
+        r[j] = S0 ? __float_as_uint(S0[(int64_t)kc * 128 + v]) : (!with_u && kc == v ? __float_as_uint(1.f) : 0u);
       }
       t5_st32(tS + lane_base + 64 * pan + 32 * sub, r);
     }
@@ -230,9 +270,9 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
         const uint32_t got = __shfl_xor_sync(0xffffffffu, (lane & 2) ? p[2 * m] : p[2 * m + 1], 2);
         const uint2 o4 = (lane & 2) ? make_uint2(got, p[2 * m + 1]) : make_uint2(p[2 * m], got);
         const int t = tok0 + 32 * sub + 4 * m + (lane & 3);
-        bf16* dst = a.o + (((int64_t)b * a.Tb + t) * a.HV + hv) * 128 + (v & ~3);
-        if (t < a.T && a.o_vec) *reinterpret_cast<uint2*>(dst) = o4;
-        else if (t < a.T) {
+        bf16* dst = a.o + (((int64_t)b * a.Tb + n0 * 64 + t) * a.HV + hv) * 128 + (v & ~3);
+        if (t < T_left && a.o_vec) *reinterpret_cast<uint2*>(dst) = o4;
+        else if (t < T_left) {
           const uint32_t w2[2] = {o4.x, o4.y};
           for (int c = 0; c < 4; ++c) reinterpret_cast<uint16_t*>(dst)[c] = (uint16_t)(w2[c >> 1] >> (16 * (c & 1)));
         }
@@ -241,7 +281,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
     bool ok = true;
     const float* dl = reinterpret_cast<const float*>(sm + T5_TU + 32768);
     const float4* up = reinterpret_cast<const float4*>(sm + T5_TU) + sub * 8 * 128 + v;       // [sub][j][v] float4
-    for (int n = 0; n < a.NT && ok; ++n) {
+    for (int n = 0; n < NT && ok; ++n) {
       const uint32_t ph = (uint32_t)n & 1;
       if (n > 0 && !mbarrier_wait_bounded(s_full, ph ^ 1, 47, T5_SPIN, a.status)) { ok = false; break; }
       t5_fence_after();
@@ -284,7 +324,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       t5_ld32(tDD + 128u * ph + lane_base + 32 * sub, r);
       float u[32];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { const float4 x = up[j * 128]; u[4 * j] = x.x; u[4 * j + 1] = x.y; u[4 * j + 2] = x.z; u[4 * j + 3] = x.w; }
+      for (int j = 0; j < 8; ++j) { const float4 x = with_u ? up[j * 128] : make_float4(0.f, 0.f, 0.f, 0.f); u[4 * j] = x.x; u[4 * j + 1] = x.y; u[4 * j + 2] = x.z; u[4 * j + 3] = x.w; }
       t5_wait_ld();
 #pragma unroll
       for (int q = 0; q < 2; ++q) {                             // 16 tokens: 8 columns of each image
@@ -302,7 +342,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       }
       if (lane == 0) mbarrier_arrive(u_empty);
       // ---- o^T of the previous chunk -> global, while the products of this one run (its D1q is the other buffer) --------
-      if (n > 0) {
+      if (n > 0 && with_o) {
         if (!mbarrier_wait_bounded(o_full, ph ^ 1, 52, T5_SPIN, a.status)) { ok = false; break; }
         t5_fence_after();
         t5_ld32(tDD + 128u * (ph ^ 1) + 64 + lane_base + 32 * sub, ro);
@@ -311,21 +351,28 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       }
     }
     // the last products must have finished before o^T and the state are read and tensor memory is released
-    if (ok && a.NT > 0 && !mbarrier_wait_bounded(s_full, (uint32_t)(a.NT - 1) & 1, 51, T5_SPIN, a.status)) ok = false;
-    if (ok && a.NT > 0 && !mbarrier_wait_bounded(o_full, (uint32_t)(a.NT - 1) & 1, 53, T5_SPIN, a.status)) ok = false;
-    if (ok && a.NT > 0) {
+    if (ok && NT > 0 && !mbarrier_wait_bounded(s_full, (uint32_t)(NT - 1) & 1, 51, T5_SPIN, a.status)) ok = false;
+    if (ok && NT > 0 && with_o && !mbarrier_wait_bounded(o_full, (uint32_t)(NT - 1) & 1, 53, T5_SPIN, a.status)) ok = false;
+    if (ok && NT > 0) {
       t5_fence_after();
-      t5_ld32(tDD + 128u * ((uint32_t)(a.NT - 1) & 1) + 64 + lane_base + 32 * sub, ro);
-      t5_wait_ld();
-      store_o((a.NT - 1) * 64);
-      if (a.S_out) {
+      if (with_o) {
+        t5_ld32(tDD + 128u * ((uint32_t)(NT - 1) & 1) + 64 + lane_base + 32 * sub, ro);
+        t5_wait_ld();
+        store_o((NT - 1) * 64);
+      }
+      if (S_out) {
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
           t5_ld32(tS + lane_base + 64 * sub + c0, r);
           t5_wait_ld();
+          if (with_u) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            a.S_out[bh * (128 * 128) + (int64_t)(64 * sub + c0 + j) * 128 + v] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) S_out[(int64_t)(64 * sub + c0 + j) * 128 + v] = __uint_as_float(r[j]);
+          } else {                                               // a transition, transposed: the rows that the join reads side by side
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<uint4*>(S_out + (int64_t)v * 128 + 64 * sub + c0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+          }
         }
       }
     }
@@ -345,15 +392,123 @@ bool kch_kda_scan_tc5_enabled() {
   return on;
 }
 
+// ---- segments of a sequence side by side -----------------------------------------------------------------------------
+// The update of a chunk is linear in the state, so a segment of chunks maps its start state to S -> M S + b.  Pass 1 finds b
+// (the scan from a zero state) and M (the scan of the identity's rows, without values) of every segment but the first, which
+// is scanned as it is, and the last, whose end nobody needs; the join walks the segments' start states; pass 2 scans all but
+// the first segment from their start states.  Chain: 2 / nseg of the sequence's chunks instead of all of them, on
+// (1 + 2 (nseg - 2)) CTAs a head instead of one.  All of it in the arithmetic of the plain scan, the join in fp32.
+// A transition that expands (an entry beyond 4, or not finite: a gate that grows, keys far from unit length) could lose in M
+// what the plain scan keeps; the segments of such a head run as one chain in pass 2.
+// 1 x 8192 tokens, 16 heads, 5 segments: the scan alone 290 us as one chain; two passes of ~60 us and 19 of the join.
+// km_split (kda_mma.cu) holds the rule.
+// A CTA of the join walks the segments for 16 columns of a head's state; the transitions (64 KB each) are copied two steps ahead.
+#define KJ_COLS 16
+#define KJ_SMEM (2 * 128 * 128 * 4 + 128 * KJ_COLS * 4)
+__global__ void __launch_bounds__(256) kda_join_kernel(float* starts, const float* trans, uint32_t* serial, int nseg) {
+  extern __shared__ __align__(16) float kj_smem[];
+  float4* sS = reinterpret_cast<float4*>(kj_smem + 2 * 128 * 128);      // [128][KJ_COLS / 4]
+  const int64_t slot = (int64_t)gridDim.y * gridDim.z, bh = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
+  const int tid = threadIdx.x, k = tid & 127, half = tid >> 7, c0 = blockIdx.x * KJ_COLS + 8 * half;
+  const uint32_t sm32 = smem_addr_u32(kj_smem);
+  chain_wait();
+  auto fetch = [&](int s) {
+    if (s + 1 < nseg) {
+      const float* src = trans + ((int64_t)s * slot + bh) * (128 * 128);
+      const uint32_t dst = sm32 + (uint32_t)(s & 1) * 65536u;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (tid + 256 * i) * 16u), "l"(src + (tid + 256 * i) * 4) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(1);
+  fetch(2);
+  {
+    const float4* p = reinterpret_cast<const float4*>(starts + (slot + bh) * (128 * 128) + (int64_t)k * 128 + c0);
+    sS[k * (KJ_COLS / 4) + 2 * half] = p[0];
+    sS[k * (KJ_COLS / 4) + 2 * half + 1] = p[1];
+  }
+  bool expands = false;
+  for (int s = 1; s + 1 < nseg; ++s) {
+    float4* out = reinterpret_cast<float4*>(starts + ((int64_t)(s + 1) * slot + bh) * (128 * 128) + (int64_t)k * 128 + c0);
+    const float4 b0 = out[0], b1 = out[1];
+    float acc[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const float* mt = kj_smem + (s & 1) * (128 * 128) + k;
+    float big = 0.f;
+#pragma unroll 16
+    for (int j = 0; j < 128; ++j) {
+      const float m = mt[j * 128];
+      big = fmaxf(big, fabsf(m));
+      expands |= m != m;
+      const float4 x = sS[j * (KJ_COLS / 4) + 2 * half], y = sS[j * (KJ_COLS / 4) + 2 * half + 1];
+      acc[0] = fmaf(m, x.x, acc[0]); acc[1] = fmaf(m, x.y, acc[1]); acc[2] = fmaf(m, x.z, acc[2]); acc[3] = fmaf(m, x.w, acc[3]);
+      acc[4] = fmaf(m, y.x, acc[4]); acc[5] = fmaf(m, y.y, acc[5]); acc[6] = fmaf(m, y.z, acc[6]); acc[7] = fmaf(m, y.w, acc[7]);
+    }
+    expands |= big > 4.f;
+    __syncthreads();
+    fetch(s + 2);
+    const float4 n0 = make_float4(acc[0], acc[1], acc[2], acc[3]), n1 = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    out[0] = sS[k * (KJ_COLS / 4) + 2 * half] = n0;
+    out[1] = sS[k * (KJ_COLS / 4) + 2 * half + 1] = n1;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  expands = __syncthreads_or(expands);             // every CTA of a head has read all of its transitions: they agree
+  if (blockIdx.x == 0 && tid == 0) serial[bh] = expands ? 1u : 0u;
+}
+
+// Segments for the scan of NT chunks of BH heads (0: one CTA a head), and what the scan then takes: both passes (a chunk of
+// pass 1 computes no output) and ~2 us a segment in the join.  Pass 1 stays within one wave of CTAs.
+int kch_kda_scan_segments(int BH, int NT, float* us) {
+  int best = 0;
+  for (int P = 3; BH > 0 && (int64_t)BH * (1 + 2 * (P - 2)) <= 148 && P <= NT; ++P) {
+    const int per = (NT + P - 1) / P;
+    if ((NT + per - 1) / per != P) continue;         // the last segment would be empty
+    const float t = (1.75f + 2.25f) * per + 8.f + 2.f * P;
+    if (!best || t < *us) { best = P; *us = t; }
+  }
+  return best;
+}
+// start states and transitions of the segments, then a flag per head
+int64_t kch_kda_scan_split_bytes(int BH, int nseg) {
+  return nseg ? (int64_t)2 * nseg * BH * 128 * 128 * 4 + (((int64_t)BH * 4 + 15) & ~(int64_t)15) : 0;
+}
+
+static int scan_launch(const T5Args& a, dim3 grid, cudaStream_t s) {
+  const int smem = T5_TOTAL + 1024;
+  KCH_CUDA_OK(cudaFuncSetAttribute(kda_scan_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kda_scan_tc5_kernel<<<grid, T5_THREADS, smem, s>>>(a);
+  KCH_LAUNCH_OK();
+  return KCH_OK;
+}
+
+int kch_kda_scan_tc5_split(const void* workspace, void* split, int nseg, const float* initial_state, void* o, float* final_state,
+                           int B, int T, int HV, int NT, unsigned int* status, cudaStream_t s) {
+  T5Args a = {};
+  a.ws = (const uint8_t*)workspace; a.S0 = initial_state; a.o = (bf16*)o; a.S_out = final_state; a.status = status;
+  a.T = T; a.Tb = T; a.HV = HV; a.NT = NT;
+  a.o_vec = ((uintptr_t)o & 7) == 0;
+  const int64_t states = (int64_t)nseg * B * HV * 128 * 128;
+  a.nseg = nseg; a.per = (NT + nseg - 1) / nseg; a.starts = (float*)split; a.trans = a.starts + states;
+  uint32_t* serial = reinterpret_cast<uint32_t*>(a.trans + states);
+  a.serial = serial;
+  a.pass = 1;
+  int rc = scan_launch(a, dim3(HV, B, 1 + 2 * (nseg - 2)), s);
+  if (rc != KCH_OK) return rc;
+  KCH_CUDA_OK(cudaFuncSetAttribute(kda_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KJ_SMEM));
+  KCH_CUDA_OK(kch_launch_chained(kda_join_kernel, dim3(128 / KJ_COLS, HV, B), dim3(256), KJ_SMEM, s, 1, a.starts, (const float*)a.trans, serial, nseg));
+  KCH_LAUNCH_OK();
+  a.pass = 2;
+  return scan_launch(a, dim3(HV, B, nseg - 1), s);
+}
+
 int kch_kda_scan_tc5(const void* workspace, const float* initial_state, void* o, float* final_state, int B, int T,
                      int Tb, int HV, int NT, unsigned int* status, cudaStream_t s) {
-  T5Args a;
+  T5Args a = {};
   a.ws = (const uint8_t*)workspace; a.S0 = initial_state; a.o = (bf16*)o; a.S_out = final_state; a.status = status;
   a.T = T; a.Tb = Tb; a.HV = HV; a.NT = NT;
   a.o_vec = ((uintptr_t)o & 7) == 0;
-  const int smem = T5_TOTAL + 1024;
-  KCH_CUDA_OK(cudaFuncSetAttribute(kda_scan_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kda_scan_tc5_kernel<<<dim3(HV, B), T5_THREADS, smem, s>>>(a);
-  KCH_LAUNCH_OK();
-  return KCH_OK;
+  return scan_launch(a, dim3(HV, B), s);
 }

@@ -442,3 +442,36 @@ def test_kda_chunk_generic_columns(kch, B, T, H, HV, K, V, dtype, off):
     assert md(s, s_ref) <= 2e-5, md(s, s_ref)
     d = (o.double().cpu() - o_ref).abs()
     assert bool((d <= 2e-5 + (o_ref.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0)).all()), float(d.max())
+
+
+@pytest.mark.parametrize("B,T,H,HV,state,gate", [
+    (1, 2049, 2, 2, True, "model"), (1, 3000, 1, 2, False, "model"), (1, 2500, 2, 2, True, "op"), (2, 1700, 1, 1, True, "mixed"),
+    (1, 2049, 1, 2, True, "clamped"), (1, 2200, 1, 1, True, "grows"), (1, 129, 1, 1, True, "op"), (1, 2048, 1, 1, True, "none")])
+def test_kda_chunk_segments(kch, B, T, H, HV, state, gate):
+    """Few heads and many chunks: the segments of a sequence are scanned side by side.  Gates from the model's (-0.1 softplus)
+    over the operator's own (a chunk decays by 2^-74 on average, past the half-way centre in some channels) to the clamp,
+    none at all, and one that grows for 300 tokens (e^6: its segments run as one chain).  Operands in two bf16 terms: 2^-16
+    relative to the values, which stay around 1 but for the growing gate; the output is rounded to bf16 once."""
+    q, k, v, g, beta, S0 = syn.kda_inputs(T + HV, B, T, H, 128, 128, HV, torch.bfloat16, with_state=True)
+    S0 = S0 if state else None
+    gf = g.float()
+    if gate == "model":
+        gf = gf * 0.1
+    elif gate == "mixed":                      # a run beyond 2^-192 a chunk, which the mma.sync stage prepares
+        gf = gf * 0.3
+        gf[:, 500:900] *= 12.0
+    elif gate == "clamped":
+        gf = gf * 40.0
+    elif gate == "grows":
+        gf = gf * 0.1
+        gf[:, 700:1000] = 0.02
+    elif gate == "none":
+        gf = gf * 0.0
+    g = gf.bfloat16()
+    o_ref, s_ref = orc.recurrent_kda(*(x.double() for x in (q, k, v, g, beta)), initial_state=None if S0 is None else S0.double())
+    o, s = kch.naive_chunk_kda(*(x.to(DEV) for x in (q, k, v, g, beta)), initial_state=None if S0 is None else S0.to(DEV),
+                               output_final_state=True, chunk_size=64)
+    assert kch._lib.device_status() == 0
+    assert float((s.double().cpu() - s_ref).norm() / s_ref.norm()) <= 1e-4
+    d = (o.double().cpu() - o_ref).abs()
+    assert bool((d <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(d.max())
