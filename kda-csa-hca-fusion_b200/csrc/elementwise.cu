@@ -696,11 +696,52 @@ __global__ void rownorm_kernel(const T* __restrict__ x, int64_t ld, TO* __restri
     for (int i = lane; i < c; i += 32) stf(y + row * c + i, ldf(xr + i) / nrm);
 }
 
+// The same for rows of c = 8 * lpr elements on 16-byte boundaries (lpr a power of two): lpr lanes a row, 8 elements a lane, so a
+// warp has 32 / lpr rows in flight.  Bound: HBM; 65536 bf16 rows of 128: 11.3 us (an element a lane and load: 17.2).
+template <typename T, typename TO>
+__global__ void __launch_bounds__(256) rownorm_vec_kernel(const T* __restrict__ x, int64_t ld, TO* __restrict__ y, float* __restrict__ norms,
+                                                         int64_t rows, int lpr) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, row = i / lpr;
+  const int part = (int)(i % lpr);
+  const bool on = row < rows;
+  float v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = 0.f;
+  if (on) ld8p(x + row * ld + 8 * part, v);
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
+  for (int o = lpr >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!on) return;
+  const float nrm = fmaxf(sqrtf(ss), 1e-12f);
+  if (norms && part == 0) norms[row] = nrm;
+  if (!y) return;
+  TO* dst = y + (row * lpr + part) * 8;
+  if constexpr (sizeof(TO) == 2) {
+    uint4 o4;
+    bf16* o = reinterpret_cast<bf16*>(&o4);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = __float2bfloat16_rn(v[k] / nrm);
+    *reinterpret_cast<uint4*>(dst) = o4;
+  } else {
+    reinterpret_cast<float4*>(dst)[0] = make_float4(v[0] / nrm, v[1] / nrm, v[2] / nrm, v[3] / nrm);
+    reinterpret_cast<float4*>(dst)[1] = make_float4(v[4] / nrm, v[5] / nrm, v[6] / nrm, v[7] / nrm);
+  }
+}
+
 extern "C" int kch_rownorm(const void* x, int64_t ld, void* y, float* norms, int64_t rows, int c,
                            int dtype, int out_dtype, void* stream) {
   KCH_REQUIRE(rows >= 0 && c >= 1 && ld >= c, "kch_rownorm: rows=%lld c=%d ld=%lld", (long long)rows, c,
               (long long)ld);
   if (rows == 0) return KCH_OK;
+  const int lpr = c / 8;
+  if (c % 8 == 0 && lpr <= 32 && (lpr & (lpr - 1)) == 0 && ld % 8 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
+    const unsigned g = (unsigned)ceil_div64(rows * lpr, 256);
+    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(out_dtype, TO,
+        (rownorm_vec_kernel<T, TO><<<g, 256, 0, kch_stream(stream)>>>((const T*)x, ld, (TO*)y, norms, rows, lpr))));
+    KCH_LAUNCH_OK();
+    return KCH_OK;
+  }
   dim3 grid((unsigned)ceil_div64(rows, 8)), block(256);
   KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(out_dtype, TO,
       (rownorm_kernel<T, TO><<<grid, block, 0, kch_stream(stream)>>>((const T*)x, ld, (TO*)y, norms, rows, c))));

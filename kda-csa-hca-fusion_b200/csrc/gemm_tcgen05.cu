@@ -975,21 +975,27 @@ struct IxSmem {
   uint32_t tmem_base;
 };
 
-__global__ void indexer_coef_kernel(const bf16* __restrict__ q, int64_t q_ld, const float* __restrict__ w,
-                                    float* __restrict__ coef, int64_t rows, int HI, float scale, int normalize) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  for (int h = 0; h < HI; ++h) {
-    const uint32_t raw = *reinterpret_cast<const uint32_t*>(q + row * q_ld + h * IX_D + 2 * lane);
-    const float x = __uint_as_float(raw << 16), y = __uint_as_float(raw & 0xFFFF0000u);
-    float ss = x * x + y * y;
+// c[t,h]: eight lanes a (query, head), 16 bytes a lane: four of them a warp instead of one after the other (2 x 10007 queries, 4
+// heads: 9.4 -> 5.0 us)
+__global__ void __launch_bounds__(256) indexer_coef_kernel(const bf16* __restrict__ q, int64_t q_ld, const float* __restrict__ w,
+                                                           float* __restrict__ coef, int64_t rows, int HI, float scale, int normalize) {
+  const int64_t i = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);      // query * HI + head
+  const int part = threadIdx.x & 7;
+  const bool on = i < rows * HI;
+  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+  if (on) raw = *reinterpret_cast<const uint4*>(q + (i / HI) * q_ld + (i % HI) * IX_D + 8 * part);
+  const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
+  float ss = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) {
-      const float nrm = normalize ? fmaxf(sqrtf(ss), 1e-12f) : 1.f;
-      coef[row * HI + h] = (w ? w[row * HI + h] : 1.f) * scale / nrm;
-    }
+  for (int e = 0; e < 4; ++e) {
+    const float x = __uint_as_float(r[e] << 16), y = __uint_as_float(r[e] & 0xFFFF0000u);
+    ss += x * x + y * y;
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (on && part == 0) {
+    const float nrm = normalize ? fmaxf(sqrtf(ss), 1e-12f) : 1.f;
+    coef[i] = (w ? w[i] : 1.f) * scale / nrm;
   }
 }
 
@@ -1153,7 +1159,7 @@ int kch_indexer_logits_tcgen05(const void* q, int64_t q_ld, int q_normalize, con
                                const void* kl, const float* w, float* coef, float* logits, int B, int T, int n, int HI,
                                int64_t n_ld, float scale, int m, int64_t t0, int n_visible, cudaStream_t s) {
   const int64_t rows = (int64_t)B * T;
-  indexer_coef_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const bf16*)q, q_ld, w, coef, rows, HI, scale, q_normalize);
+  indexer_coef_kernel<<<(unsigned)((rows * HI + 31) / 32), 256, 0, s>>>((const bf16*)q, q_ld, w, coef, rows, HI, scale, q_normalize);
   KCH_LAUNCH_OK();
   CUtensorMap mq, mkh, mkm, mkl;
   int rc = make_map_2d(&mq, q, (uint64_t)rows, (uint64_t)HI * IX_D, (uint64_t)q_ld, IX_BM, IX_D);

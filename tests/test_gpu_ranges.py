@@ -475,3 +475,23 @@ def test_kda_chunk_segments(kch, B, T, H, HV, state, gate):
     assert float((s.double().cpu() - s_ref).norm() / s_ref.norm()) <= 1e-4
     d = (o.double().cpu() - o_ref).abs()
     assert bool((d <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(d.max())
+
+
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16),
+                                       (torch.float32, torch.float32)])
+@pytest.mark.parametrize("rows,c,ld,off", [(1, 8, 8, 0), (33, 16, 40, 0), (67, 128, 128, 0), (5, 256, 264, 8), (9, 264, 264, 0), (7, 24, 24, 0),
+                                           (31, 128, 130, 0), (31, 128, 136, 1)])
+def test_rownorm_rows(kch, dtype, out, rows, c, ld, off):
+    """Rows of 8 to 256 elements on 16-byte boundaries (several rows a warp) and the others (a warp a row).  fp32 arithmetic: a sum
+    of c squares, a root and a division, 2^-23 * (c / 8 + 8) of the value at most; a bf16 result is rounded once (eight
+    significant bits: half a unit in the last place is up to 2^-8 of the value)."""
+    from kch_b200 import _lib
+    x = torch.randn(rows * ld + off, generator=torch.Generator().manual_seed(c)).to(dtype).to(DEV)[off:].view(rows, ld)
+    x[rows // 2] = 0.0
+    y, norms = torch.empty(rows, c, dtype=out, device=DEV), torch.empty(rows, device=DEV)
+    _lib.check(_lib.load().kch_rownorm(_lib.ptr(x), ld, _lib.ptr(y), _lib.ptr(norms), rows, c, _lib.dtype_tag(dtype), _lib.dtype_tag(out), 0))
+    torch.cuda.synchronize()
+    ref_n = x[:, :c].double().norm(dim=-1).clamp_min(1e-12)
+    ref, eps = x[:, :c].double() / ref_n.unsqueeze(-1), 2.0 ** -23 * (c / 8 + 8)
+    assert bool(((norms.double() - ref_n).abs() <= eps * ref_n).all())
+    assert bool(((y.double() - ref).abs() <= ref.abs() * (eps + (2.0 ** -8 if out == torch.bfloat16 else 0.0))).all())
