@@ -12,9 +12,14 @@
 //                         between the warps of a block of tokens (m = 128 uses all 256 threads of a CTA
 //                         on one block: 16 row subsets x 16 channel chunks).
 //   compress_kernel     : any dtype / width: a thread owns one (batch, block, channel), two passes.
+//   compress_subset_kernel: the same for few or long blocks: a CTA owns 32 channels of a block, a warp every eighth of its rows.
+//                         Bound: the latency of a row's loads, which a thread of the kernel above meets m times in turn
+//                         (10 blocks of 64 fp32 tokens, 128 channels: 25 -> 8 us).
 #include <math.h>
 
 #include "kch_common.cuh"
+
+#define CR_SUBS 8
 
 template <typename T, typename TB, bool OVERLAP>
 __global__ void compress_kernel(const T* __restrict__ Ca, const T* __restrict__ Za,
@@ -62,6 +67,70 @@ __global__ void compress_kernel(const T* __restrict__ Ca, const T* __restrict__ 
       accb = fmaf(e, ldf(pc + off), accb);
     }
   out[(int64_t)b * out_batch_stride + (int64_t)n * c + ch] = acc / den + accb / den;
+}
+
+template <typename T, typename TB, bool OVERLAP>
+__global__ void __launch_bounds__(32 * CR_SUBS)
+compress_subset_kernel(const T* __restrict__ Ca, const T* __restrict__ Za, const T* __restrict__ Cb, const T* __restrict__ Zb,
+                const TB* __restrict__ Ba, const TB* __restrict__ Bb, const T* __restrict__ prevCb, const T* __restrict__ prevZb,
+                float* __restrict__ out, int64_t ld, int64_t batch_stride_rows, int B, int nblk, int c, int m, int64_t out_batch_stride,
+                int64_t prev_ld) {
+  __shared__ float red[3][CR_SUBS][32];
+  const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
+  const int cgroups = (c + 31) / 32;
+  const int64_t unit = blockIdx.x / cgroups;
+  const int ch = (int)(blockIdx.x % cgroups) * 32 + lane;
+  const bool live = ch < c;
+  const int n = (int)(unit % nblk), b = (int)(unit / nblk);
+  const int64_t row0 = (int64_t)b * batch_stride_rows + (int64_t)n * m;
+  const T* pc = nullptr;
+  const T* pz = nullptr;
+  int64_t pld = ld, prow = 0;
+  if (OVERLAP) {
+    if (n > 0) { pc = Cb; pz = Zb; prow = row0 - m; }
+    else if (prevCb) { pc = prevCb; pz = prevZb; pld = prev_ld; prow = (int64_t)b * m; }
+  }
+  // maximum, then sums, exactly as a dense softmax would do it
+  float mx = -INFINITY;
+  if (live) {
+#pragma unroll 4
+    for (int j = sub; j < m; j += CR_SUBS) mx = fmaxf(mx, ldf(Za + (row0 + j) * ld + ch) + ldf(Ba + (int64_t)j * c + ch));
+    if (pc)
+#pragma unroll 4
+      for (int j = sub; j < m; j += CR_SUBS) mx = fmaxf(mx, ldf(pz + (prow + j) * pld + ch) + ldf(Bb + (int64_t)j * c + ch));
+  }
+  red[0][sub][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < CR_SUBS; ++w) mx = fmaxf(mx, red[0][w][lane]);
+  __syncthreads();
+  float den = 0.f, acc = 0.f, accb = 0.f;
+  if (live) {
+#pragma unroll 4
+    for (int j = sub; j < m; j += CR_SUBS) {
+      const int64_t off = (row0 + j) * ld + ch;
+      const float e = expf(ldf(Za + off) + ldf(Ba + (int64_t)j * c + ch) - mx);
+      den += e;
+      acc = fmaf(e, ldf(Ca + off), acc);
+    }
+    if (pc)
+#pragma unroll 4
+      for (int j = sub; j < m; j += CR_SUBS) {
+        const int64_t off = (prow + j) * pld + ch;
+        const float e = expf(ldf(pz + off) + ldf(Bb + (int64_t)j * c + ch) - mx);
+        den += e;
+        accb = fmaf(e, ldf(pc + off), accb);
+      }
+  }
+  red[0][sub][lane] = den;
+  red[1][sub][lane] = acc;
+  red[2][sub][lane] = accb;
+  __syncthreads();
+  if (sub == 0 && live) {
+#pragma unroll
+    for (int w = 1; w < CR_SUBS; ++w) { den += red[0][w][lane]; acc += red[1][w][lane]; accb += red[2][w][lane]; }
+    out[(int64_t)b * out_batch_stride + (int64_t)n * c + ch] = acc / den + accb / den;
+  }
 }
 
 // running softmax-weighted sum over rows, 8 channels per thread
@@ -201,16 +270,23 @@ static int launch_compress(const void* Ca, const void* Za, const void* Cb, const
       return KCH_OK;
     }
   }
-  dim3 grid((unsigned)ceil_div64(total, 128)), block(128);
+  // A CTA a block and 32 channels where a block is long, or where such CTAs are few; fp32 tokens of 128 channels, us, thread a
+  // channel / subsets: m = 64: 45 / 11 at 2048 tokens, 79 / 57 at 131072; m = 16: 16 / 8 and 66 / 104; m = 8: 12 / 8 at 2048, 14 / 25
+  // at 16384; m = 4: 8 / 10 and 61 / 242.
+  const int64_t ctas = (int64_t)B * nblk * ((c + 31) / 32);
+  const bool subsets = m >= 64 ? ctas <= 0x7FFFFFFF : m >= CR_SUBS && ctas <= 8 * 148;
+  dim3 grid((unsigned)(subsets ? ctas : ceil_div64(total, 128))), block(subsets ? 32 * CR_SUBS : 128);
 #define GO(T, TB, OV)                                                                           \
-  compress_kernel<T, TB, OV><<<grid, block, 0, s>>>(                                      \
-      (const T*)Ca, (const T*)Za, (const T*)Cb, (const T*)Zb, (const TB*)Ba, (const TB*)Bb,     \
-      (const T*)prevCb, (const T*)prevZb, out, ld, batch_stride_rows, B, nblk, c, m,            \
-      out_batch_stride, prev_ld)
+  do {                                                                                          \
+    auto kernel = subsets ? compress_subset_kernel<T, TB, OV> : compress_kernel<T, TB, OV>;     \
+    kernel<<<grid, block, 0, s>>>((const T*)Ca, (const T*)Za, (const T*)Cb, (const T*)Zb,       \
+        (const TB*)Ba, (const TB*)Bb, (const T*)prevCb, (const T*)prevZb, out, ld,              \
+        batch_stride_rows, B, nblk, c, m, out_batch_stride, prev_ld);                           \
+  } while (0)
   if (overlap) {
-    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(bdtype, TB, (GO(T, TB, true))));
+    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(bdtype, TB, GO(T, TB, true)));
   } else {
-    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(bdtype, TB, (GO(T, TB, false))));
+    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(bdtype, TB, GO(T, TB, false)));
   }
 #undef GO
   KCH_LAUNCH_OK();

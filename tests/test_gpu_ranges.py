@@ -495,3 +495,17 @@ def test_rownorm_rows(kch, dtype, out, rows, c, ld, off):
     ref, eps = x[:, :c].double() / ref_n.unsqueeze(-1), 2.0 ** -23 * (c / 8 + 8)
     assert bool(((norms.double() - ref_n).abs() <= eps * ref_n).all())
     assert bool(((y.double() - ref).abs() <= ref.abs() * (eps + (2.0 ** -8 if out == torch.bfloat16 else 0.0))).all())
+
+
+@pytest.mark.parametrize("T,c,m", [(64, 33, 8), (7 * 9, 31, 9), (130, 1, 65), (21, 70, 7), (128, 32, 128), (9472, 32, 16), (9600, 5, 8)])
+def test_compress_subsets(kch, T, c, m):
+    """Blocks whose rows eight warps share (m >= 64, or m >= 8 and at most 1184 groups of 32 channels) and, on either side of that
+    line, those that a thread walks; widths that fill no group.  Bound as in test_compress_matches_oracle, by the values: 2e-6."""
+    g = torch.Generator().manual_seed(T + c)
+    t = [torch.randn(2, T, c, generator=g) for _ in range(4)]
+    t[2][0, :m], t[3][0, :m] = -1e30, 40.0
+    Ba, Bb = [torch.randn(m, c, generator=g) * 0.3 for _ in range(2)]
+    a = kch.csa_compress_kv_overlapped(*[x.to(DEV) for x in t], Ba.to(DEV), Bb.to(DEV), m)
+    assert md(a, orc.compress_kv_overlapped(*t, Ba, Bb, m)) <= 2e-6
+    b = kch.csa_compress_kv(t[0].to(DEV), t[2].to(DEV), Ba.to(DEV), m)
+    assert md(b, orc.compress_kv(t[0], t[2], Ba, m)) <= 2e-6
