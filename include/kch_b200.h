@@ -399,6 +399,113 @@ int kch_cache_store_rows(const float* rows, int64_t n, int c, int B, void* dst, 
 int kch_quantize_rows(const void* x, int64_t ld, void* payload, float* scales, float* norms, int64_t rows,
                       int c, int kind, int dtype, void* stream);
 
+/* ---- whole layers ------------------------------------------------------------------------------------------- */
+
+/* The launches of one layer over several tokens from one call; every step is one of the entry points above with the
+ * arguments that the layer gives it, intermediate results in the caller's workspace (256-byte aligned,
+ * kch_*_layer_workspace_bytes of the same arguments).  Common part: x [B*T, d] rows ld_x apart; the pre-norm
+ * (norm_w == NULL: x is normalised already); the output projection [d_out, heads * width] and the residual
+ * (W_o == NULL: `out` receives the heads' outputs; not for kch_kda_layer). */
+typedef struct kch_layer_common {
+  int B, T, d, dtype;
+  const void* x;
+  int64_t ld_x;
+  const void *norm_w, *norm_b;
+  int norm_dtype;
+  float eps;
+  const void* W_o;
+  int64_t ld_wo;
+  int d_out;
+  const void* residual;      /* [B*T, d_out] rows ld_res apart, or NULL */
+  int64_t ld_res;
+  void* out;
+  void* workspace;
+  int64_t workspace_bytes;
+} kch_layer_common;
+
+typedef struct kch_weight_part {     /* `rows` rows of a weight, ld elements apart, 16-byte aligned */
+  const void* w;
+  int64_t ld;
+  int rows;
+} kch_weight_part;
+
+/* naive_csa (ops_csa.py:576-1184) with cosine scoring, or CSAHybridLayer (ops_fused.py:612-713), from T >= m tokens on.
+ * W: the row-fused input projection [n_w, d] (a | b keys, a | b gates, indexer key | gate, query down-projection, indexer
+ * weights, padding) and Wq [n_q, dc] (queries, indexer queries); where they are NULL, parts[0..7] and parts[8..9] are
+ * fused here.  proj [B*T, n_w], comp fp32 [B, T_blocks, c] and kcomp fp32 [B, T_blocks, c_I] receive the projections
+ * and the compressed rows (NULL: kept in the workspace).  T_blocks = T / m. */
+typedef struct kch_csa_layer_args {
+  kch_layer_common l;
+  int c, c_I, dc, nh, nIh, m, topk, sliding_window, T_blocks;
+  float scale;
+  const void* W;
+  int64_t ld_w;
+  int n_w;
+  const void* Wq;
+  int64_t ld_wq;
+  int n_q;
+  kch_weight_part parts[10];
+  const void *Ba, *Bb, *B_idx;
+  int bias_dtype;
+  const void* sink;
+  int sink_dtype;
+  void* proj;
+  float *comp, *kcomp;
+} kch_csa_layer_args;
+int64_t kch_csa_layer_workspace_bytes(const kch_csa_layer_args* args);
+int kch_csa_layer(const kch_csa_layer_args* args, void* stream);
+
+/* naive_hca (ops_hca.py:26-192) or HCAHybridLayer (ops_fused.py:716-739), from T >= m2 tokens on.  W [n_w, d]: keys, gates,
+ * query down-projection (NULL: parts[0..2]); Wq [nh * c, dc]. */
+typedef struct kch_hca_layer_args {
+  kch_layer_common l;
+  int c, dc, nh, m2, sliding_window, T_blocks;
+  float scale;
+  const void* W;
+  int64_t ld_w;
+  int n_w;
+  const void* Wq;
+  int64_t ld_wq;
+  kch_weight_part parts[3];
+  const void* B_pos;
+  int bias_dtype;
+  const void* sink;
+  int sink_dtype;
+  void* proj;
+  float* comp;
+} kch_hca_layer_args;
+int64_t kch_hca_layer_workspace_bytes(const kch_hca_layer_args* args);
+int kch_hca_layer(const kch_hca_layer_args* args, void* stream);
+
+/* KDAHybridLayer (ops_fused.py:316-609) over T >= 2 tokens: W [n_w, d] = q | k | v | gate down | beta | padding, W_gup
+ * [HV * K, K], conv_w [d, 3].  lookback [B, 2, d] (or NULL) and lookback_out hold normalised rows; state / state_out fp32
+ * [B, HV, K, V] (state may be NULL).  T < chunk_size runs the token recurrence. */
+typedef struct kch_kda_layer_args {
+  kch_layer_common l;
+  int H, HV, K, V, chunk_size;
+  float scale, decay_scale, g_clamp_min;
+  const void* lookback;
+  void* lookback_out;
+  const void *conv_w, *conv_b;
+  const void* W;
+  int64_t ld_w;
+  int n_w;
+  const void* W_gup;
+  int64_t ld_wg;
+  const float* state;
+  float* state_out;
+} kch_kda_layer_args;
+int64_t kch_kda_layer_workspace_bytes(const kch_kda_layer_args* args);
+int kch_kda_layer(const kch_kda_layer_args* args, void* stream);
+
+/* A run of T tokens into a cache whose accumulator is empty and which stores its rows in `dtype`: kch_compress_kv(_overlapped)
+ * of the whole blocks (or `rows` fp32 [B, T / m, c] and `key_rows` fp32 [B, T / m, c_I] where the caller has them already,
+ * e.g. from kch_csa_layer), kch_cache_store_rows, kch_cache_append_rows.  Biases in `dtype`. */
+int64_t kch_cache_append_prompt_workspace_bytes(const kch_cache_append_args* args, int64_t T);
+int kch_cache_append_prompt(const kch_cache_append_args* args, int64_t T, int64_t bs_c, int64_t bs_i, int64_t ring_n,
+                            int64_t tokens_seen, const float* rows, const float* key_rows, void* workspace,
+                            int64_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -57,6 +57,39 @@ class AttendDecodeArgs(C.Structure):
                 ("counters", _vp), ("workspace", _vp), ("workspace_bytes", _i64)]
 
 
+class LayerCommon(C.Structure):
+    _fields_ = [("B", _i), ("T", _i), ("d", _i), ("dtype", _i), ("x", _vp), ("ld_x", _i64),
+                ("norm_w", _vp), ("norm_b", _vp), ("norm_dtype", _i), ("eps", _f),
+                ("W_o", _vp), ("ld_wo", _i64), ("d_out", _i), ("residual", _vp), ("ld_res", _i64),
+                ("out", _vp), ("workspace", _vp), ("workspace_bytes", _i64)]
+
+
+class WeightPart(C.Structure):
+    _fields_ = [("w", _vp), ("ld", _i64), ("rows", _i)]
+
+
+class CsaLayerArgs(C.Structure):
+    _fields_ = [("l", LayerCommon),
+                ("c", _i), ("c_I", _i), ("dc", _i), ("nh", _i), ("nIh", _i), ("m", _i), ("topk", _i), ("sliding_window", _i),
+                ("T_blocks", _i), ("scale", _f), ("W", _vp), ("ld_w", _i64), ("n_w", _i), ("Wq", _vp), ("ld_wq", _i64), ("n_q", _i),
+                ("parts", WeightPart * 10), ("Ba", _vp), ("Bb", _vp), ("B_idx", _vp), ("bias_dtype", _i),
+                ("sink", _vp), ("sink_dtype", _i), ("proj", _vp), ("comp", _vp), ("kcomp", _vp)]
+
+
+class HcaLayerArgs(C.Structure):
+    _fields_ = [("l", LayerCommon),
+                ("c", _i), ("dc", _i), ("nh", _i), ("m2", _i), ("sliding_window", _i), ("T_blocks", _i), ("scale", _f),
+                ("W", _vp), ("ld_w", _i64), ("n_w", _i), ("Wq", _vp), ("ld_wq", _i64), ("parts", WeightPart * 3),
+                ("B_pos", _vp), ("bias_dtype", _i), ("sink", _vp), ("sink_dtype", _i), ("proj", _vp), ("comp", _vp)]
+
+
+class KdaLayerArgs(C.Structure):
+    _fields_ = [("l", LayerCommon),
+                ("H", _i), ("HV", _i), ("K", _i), ("V", _i), ("chunk_size", _i), ("scale", _f), ("decay_scale", _f), ("g_clamp_min", _f),
+                ("lookback", _vp), ("lookback_out", _vp), ("conv_w", _vp), ("conv_b", _vp), ("W", _vp), ("ld_w", _i64), ("n_w", _i),
+                ("W_gup", _vp), ("ld_wg", _i64), ("state", _vp), ("state_out", _vp)]
+
+
 # indices into a cache's device counters (include/kch_b200.h KCH_CTR_*)
 CTR_ACC_LEN, CTR_N_BLOCKS, CTR_RING_N, CTR_HAS_PREV, CTR_TOKENS, CTR_ARRIVALS, CTR_WORDS = 0, 1, 2, 3, 4, 5, 8
 STATUS_CACHE_CAPACITY = 64
@@ -112,6 +145,14 @@ PROTOTYPES = {
     "kch_attend_decode_splits": (_i, [_i]),
     "kch_attend_decode_workspace_bytes": (_i64, [_i, _i, _i]),
     "kch_attend_decode": (_i, [C.POINTER(AttendDecodeArgs), _vp]),
+    "kch_cache_append_prompt_workspace_bytes": (_i64, [C.POINTER(CacheAppendArgs), _i64]),
+    "kch_cache_append_prompt": (_i, [C.POINTER(CacheAppendArgs), _i64, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp]),
+    "kch_csa_layer_workspace_bytes": (_i64, [C.POINTER(CsaLayerArgs)]),
+    "kch_csa_layer": (_i, [C.POINTER(CsaLayerArgs), _vp]),
+    "kch_hca_layer_workspace_bytes": (_i64, [C.POINTER(HcaLayerArgs)]),
+    "kch_hca_layer": (_i, [C.POINTER(HcaLayerArgs), _vp]),
+    "kch_kda_layer_workspace_bytes": (_i64, [C.POINTER(KdaLayerArgs)]),
+    "kch_kda_layer": (_i, [C.POINTER(KdaLayerArgs), _vp]),
 }
 
 _lib = None

@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from . import _lib
+from . import _lib, layers
 
 
 def _as_rows(t):
@@ -439,6 +439,16 @@ def naive_csa(H, W_aKV, W_bKV, W_aZ, W_bZ, Ba, Bb, W_DQ, W_UQ, W_IUQ, W_w, W_KV_
         if w.shape[1] != d:
             raise ValueError(f"naive_csa: {name}.shape={tuple(w.shape)} — second dim (in_features) must "
                              f"equal d={d} (H.shape[-1]).")
+    if normalize_qk and _q_rows is None and _aux is None and not _return_indices:
+        # the ordinary call: every launch issued by the library
+        got = layers.csa_layer(H, (W_aKV, W_bKV, W_aZ, W_bZ, W_KV_idx, W_Z_idx, W_DQ, W_w, W_UQ, W_IUQ), Ba, Bb, B_idx, sink_logits,
+                               m=m, topk=topk, nh=nh, nIh=nIh, c=c, c_I=c_I, dc=dc, scale=1.0 if scale is None else float(scale),
+                               sliding_window=sliding_window, W=_fused_weight, Wq=_fused_q_weight, want_proj=return_projections)
+        if got is not None:
+            out, proj, _ = got
+            if not return_projections:
+                return out
+            return out, proj[..., :4 * c + 2 * c_I].split([c, c, c, c, c_I, c_I], dim=-1)
     q_lo = 0
     if _q_rows is not None:
         q_lo, q_hi = int(_q_rows[0]), int(_q_rows[1])

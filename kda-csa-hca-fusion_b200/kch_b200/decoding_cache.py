@@ -12,6 +12,8 @@ kept next to it; the ring holds ``dtype(normalize(fp32(Ca)))`` (725-730) and is 
 """
 from __future__ import annotations
 
+import math
+
 import torch
 
 from . import _lib
@@ -34,12 +36,12 @@ def _validate_cache_dtype(dtype):
 class _SlidingWindowRingBuffer:
     """Last ``win`` keys per sequence, written at slot ``n_written % win``."""
 
-    def __init__(self, B, win, c, device, dtype):
+    def __init__(self, B, win, c, device, dtype, buf=None):
         if win < 1:
             raise ValueError(f"_SlidingWindowRingBuffer: win={win} must be >= 1")
         self.B, self.win, self.c = B, win, c
         self.device, self.dtype = torch.device(device), dtype
-        self._buf = torch.zeros(B, win, c, device=self.device, dtype=dtype)
+        self._buf = torch.zeros(B, win, c, device=self.device, dtype=dtype) if buf is None else buf
         self._n = 0
 
     def reset(self):
@@ -65,6 +67,15 @@ class _SlidingWindowRingBuffer:
         pos = (torch.arange(self._n + Tn - k, self._n + Tn, device=self.device) % self.win)
         self._buf.index_copy_(1, pos, x)
         self._n += Tn
+
+
+def _zeros(device, dtype, *shapes):
+    """Zeroed tensors of these shapes: pieces of one allocation (a launch and an allocation each took longer than the rest of
+    a cache's set-up), each starting on 256 bytes."""
+    step = 256 // torch.empty((), dtype=dtype).element_size()
+    sizes = [-(-math.prod(s) // step) * step for s in shapes]
+    pieces = torch.zeros(sum(sizes), dtype=dtype, device=device).split(sizes)
+    return [p[:math.prod(s)].view(s) for p, s in zip(pieces, shapes)]
 
 
 class _CacheBase:
@@ -256,9 +267,9 @@ class _CacheBase:
             return [x[:, :nb * m] for x in new]
         return [torch.cat([a[:, :self._acc_len], x[:, :nb * m - self._acc_len]], dim=1) for a, x in zip(self._acc, new)]
 
-    def _append_rows(self, new, m, c_I):
-        """Open accumulators, overlap partner, window ring and counters after a run of tokens (one launch); the rows of its
-        whole blocks are stored already."""
+    def _append_rows(self, new, m, c_I, biases=None, rows=None):
+        """A run of tokens: open accumulators, overlap partner, window ring and counters (one launch).  With ``biases`` the rows
+        of its whole blocks come first (``rows``: fp32, where the caller has them), else they are stored already."""
         T = new[0].shape[1]
 
         def strides(group):          # one (token, sequence) stride pair per group of streams
@@ -287,9 +298,26 @@ class _CacheBase:
         a.normalize = int(self._normalize_qk)
         a.counters = self._ctr.data_ptr()
         ring_n = 0 if self._sw is None else self._sw._n
-        with _lib.device(self.device):
-            _lib.check(_lib.load().kch_cache_append_rows(a, T, bs_c, bs_i, ring_n, self._n_tokens_seen, _lib.stream()))
         total = self._acc_len + T
+        lib = _lib.load()
+        with _lib.device(self.device):
+            if biases is not None:
+                if total // m:
+                    self._grow(self._n_blocks + total // m)
+                    a.comp, a.comp_norms, a.capacity = self._comp.data_ptr(), self._norms.data_ptr(), self._comp.shape[1]
+                    if c_I:
+                        a.kcomp, a.kcomp_norms = self._kcomp.data_ptr(), self._kcomp_norms.data_ptr()
+                a.comp_kind = a.dtype
+                a.Ba = biases[0].data_ptr()
+                if c_I:
+                    a.Bb, a.B_idx = biases[1].data_ptr(), biases[2].data_ptr()
+                need = 0 if rows is not None else int(lib.kch_cache_append_prompt_workspace_bytes(a, T))
+                ws = torch.empty(need, dtype=torch.uint8, device=self.device) if need else None
+                r = rows if rows is not None else (None, None)
+                _lib.check(lib.kch_cache_append_prompt(a, T, bs_c, bs_i, ring_n, self._n_tokens_seen, _lib.ptr(r[0]), _lib.ptr(r[1]),
+                                                       _lib.ptr(ws), need, _lib.stream()))
+            else:
+                _lib.check(lib.kch_cache_append_rows(a, T, bs_c, bs_i, ring_n, self._n_tokens_seen, _lib.stream()))
         if self._sw is not None:
             self._sw._n += T
         self._n_blocks += total // m
@@ -297,6 +325,12 @@ class _CacheBase:
         self._n_tokens_seen += T
         if c_I and total // m:
             self._has_prev = True
+
+    def _whole_blocks(self, new):
+        """Can ``kch_cache_append_prompt`` take these streams?  No block is open, rows are stored as they are, and the streams are
+        slices whose sequences lie a whole number of token strides apart."""
+        return (self._acc_len == 0 and self._kind is None
+                and all(x.stride(2) == 1 and x.stride(1) >= x.shape[2] and (self.B == 1 or x.stride(0) % x.stride(1) == 0) for x in new))
 
     def _dequant(self, nb):
         if self._comp is None:
@@ -351,13 +385,13 @@ class CSADecodingCache(_CacheBase):
 
     def reset(self):
         B, m, c, cI, dev, dt = self.B, self.m, self.c, self.c_I, self.device, self.dtype
-        self._acc = [torch.zeros(B, m, w, dtype=dt, device=dev) for w in (c, c, c, c, cI, cI)]
+        *new, ring = _zeros(dev, dt, *((B, m, w) for w in (c, c, c, c, cI, cI, c, c)), (B, self.win, c))
+        self._acc, self._prev = new[:6], new[6:]
         self._acc_len = 0
-        self._prev = [torch.zeros(B, m, c, dtype=dt, device=dev) for _ in range(2)]
         self._has_prev = False
         self._comp = self._scales = self._norms = None
         self._kcomp = self._kcomp_norms = None
-        self._sw = _SlidingWindowRingBuffer(B, self.win, c, dev, dt) if self.win > 0 else None
+        self._sw = _SlidingWindowRingBuffer(B, self.win, c, dev, dt, ring) if self.win > 0 else None
         self._n_tokens_seen = 0
         self._n_blocks = 0
         self._init_counters()
@@ -404,7 +438,9 @@ class CSADecodingCache(_CacheBase):
         return self
 
     # ---- append ---------------------------------------------------------------------------------------
-    def append_step(self, Ca_new, Cb_new, Za_new, Zb_new, K_idx_new, Z_idx_new, Ba, Bb, B_idx):
+    def append_step(self, Ca_new, Cb_new, Za_new, Zb_new, K_idx_new, Z_idx_new, Ba, Bb, B_idx, *, _rows=None):
+        """``_rows``: the compressed rows and indexer keys of the new tokens' blocks in fp32, of a caller who has them (only for an
+        empty accumulator, with biases of the cache's type)."""
         B, T_new, c = Ca_new.shape
         if B != self.B:
             raise ValueError(f"CSADecodingCache.append_step: batch size {B} does not match cache's B={self.B}. "
@@ -433,7 +469,7 @@ class CSADecodingCache(_CacheBase):
         if T_new == 1:
             self._append_one(new, biases)
         else:
-            self._append_many(new, biases)
+            self._append_many(new, biases, _rows)
         return list(range(first_new, self._n_blocks))
 
     def _append_one(self, new, biases):
@@ -471,8 +507,11 @@ class CSADecodingCache(_CacheBase):
             _lib.check(lib.kch_cache_append_token_advance(a, _lib.stream()))   # the last CTA advances the device counters
         self._advance(m)
 
-    def _append_many(self, new, biases):
+    def _append_many(self, new, biases, rows=None):
         m = self.m
+        if self._whole_blocks(new):
+            self._append_rows(new, m, self.c_I, biases, rows)
+            return
         nb = (self._acc_len + new[0].shape[1]) // m
         if nb:
             self._grow(self._n_blocks + nb)
@@ -591,10 +630,10 @@ class HCADecodingCache(_CacheBase):
 
     def reset(self):
         B, m, c, dev, dt = self.B, self.m2, self.c, self.device, self.dtype
-        self._acc = [torch.zeros(B, m, c, dtype=dt, device=dev) for _ in range(2)]
+        *self._acc, ring = _zeros(dev, dt, (B, m, c), (B, m, c), (B, self.win, c))
         self._acc_len = 0
         self._comp = self._scales = self._norms = None
-        self._sw = _SlidingWindowRingBuffer(B, self.win, c, dev, dt) if self.win > 0 else None
+        self._sw = _SlidingWindowRingBuffer(B, self.win, c, dev, dt, ring) if self.win > 0 else None
         self._n_tokens_seen = 0
         self._n_blocks = 0
         self._init_counters()
@@ -626,7 +665,8 @@ class HCADecodingCache(_CacheBase):
             raise NotImplementedError("HCADecodingCache(b200).to(device=...): caches are bound to their GPU")
         return self
 
-    def append_step(self, C_new, Z_new, B_pos):
+    def append_step(self, C_new, Z_new, B_pos, *, _rows=None):
+        """``_rows``: as in ``CSADecodingCache.append_step``."""
         B, T_new, c = C_new.shape
         if B != self.B:
             raise ValueError(f"HCADecodingCache.append_step: batch size {B} does not match cache's B={self.B}. "
@@ -646,7 +686,7 @@ class HCADecodingCache(_CacheBase):
         if T_new == 1:
             self._append_one(new, bias)
         else:
-            self._append_many(new, bias)
+            self._append_many(new, bias, _rows)
         return list(range(first_new, self._n_blocks))
 
     def _append_one(self, new, bias):
@@ -681,8 +721,11 @@ class HCADecodingCache(_CacheBase):
             _lib.check(lib.kch_cache_append_token_advance(a, _lib.stream()))   # the last CTA advances the device counters
         self._advance(m)
 
-    def _append_many(self, new, bias):
+    def _append_many(self, new, bias, rows=None):
         m = self.m2
+        if self._whole_blocks(new):
+            self._append_rows(new, m, 0, [bias], rows)
+            return
         nb = (self._acc_len + new[0].shape[1]) // m
         if nb:
             self._grow(self._n_blocks + nb)

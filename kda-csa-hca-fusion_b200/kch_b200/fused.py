@@ -17,7 +17,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, layers
 from .csa import attend, fuse_rows, indexer_topk, linear, mma_attention_eligible, naive_csa, rownorm
 from .decoding_cache import CSADecodingCache, HCADecodingCache
 from .hca import naive_hca
@@ -228,6 +228,15 @@ class _FusedWeights:
         return w, False
 
 
+def _plain_norm(norm):
+    """A LayerNorm of the stack that nobody watches or replaces: its arithmetic may move into the layer's call."""
+    return type(norm) is _Fp32LayerNorm and not (norm._forward_hooks or norm._forward_pre_hooks)
+
+
+def _unwatched(layer):
+    return type(layer) in (CSAHybridLayer, HCAHybridLayer) and not (layer._forward_hooks or layer._forward_pre_hooks)
+
+
 def _at_rest(w):
     """Is ``w`` a parameter as it lies?  A parametrised weight is computed by the access itself, so the launch just before
     the product writes it."""
@@ -266,9 +275,9 @@ class KDAHybridLayer(nn.Module):
     def reset_conv_state(self):
         self._conv_lookback = None
 
-    def forward(self, x, state=None, residual=None, state_out=None, lookback_in_place=False, norm=None):
-        o, new_state, lb = self.forward_functional(x, state, self._conv_lookback, residual=residual,
-                                                   state_out=state_out, lookback_in_place=lookback_in_place, norm=norm)
+    def forward(self, x, state=None, residual=None, state_out=None, lookback_in_place=False, norm=None, _final_state=None):
+        o, new_state, lb = self.forward_functional(x, state, self._conv_lookback, residual=residual, state_out=state_out,
+                                                   lookback_in_place=lookback_in_place, norm=norm, _final_state=_final_state)
         self._conv_lookback = lb
         return o, new_state
 
@@ -325,10 +334,20 @@ class KDAHybridLayer(nn.Module):
                 g.view(B, T, HV, K), beta, new_lb)
 
     def forward_functional(self, x, state, conv_lookback, *, detach_lookback=True, residual=None, state_out=None,
-                           lookback_in_place=False, norm=None):
+                           lookback_in_place=False, norm=None, _final_state=None):
+        """``_final_state``: where the caller would like the final state of a call over several tokens; the state that is
+        returned tells whether it went there."""
         cfg = self.cfg
         B, T, _ = x.shape
         HV, V = cfg.n_heads_v, cfg.head_dim_v
+        if T >= 2 and _single(self.tp) and not lookback_in_place and (norm is None or _plain_norm(norm)):
+            lb = conv_lookback if conv_lookback is None or conv_lookback.shape[0] == B else None
+            got = layers.kda_layer(x, cfg, self._fused.get(self.q_proj.weight, self.k_proj.weight, self.v_proj.weight,
+                                                           self.g_down.weight, self.beta.weight),
+                                   self.g_up.weight, self.o_proj.weight, self.short_conv.weight, self.short_conv.bias, state, lb,
+                                   scale=self._scale_value(), norm=norm, residual=residual, state_out=_final_state)
+            if got is not None:
+                return got
         use_chunk = cfg.kda_chunk_size >= 1 and T >= cfg.kda_chunk_size
         raw_gate = use_chunk and cfg.kda_decay_scale > 0 and chunk_gate_supported(
             cfg.head_dim_k, cfg.head_dim_v, cfg.kda_chunk_size, -10.0, x.dtype)
@@ -341,6 +360,10 @@ class KDAHybridLayer(nn.Module):
         out = out_projection(o.reshape(B, T, HV * V), self.tp, W, residual=residual,
                              w_settled=T == 1 and lookback_in_place and _at_rest(W))
         return out, new_state, new_lb
+
+
+def _single(tp):
+    return tp is None or tp.world == 1
 
 
 def _rows_mode(tp):
@@ -415,9 +438,21 @@ class CSAHybridLayer(nn.Module):
                          normalize_qk=True, return_projections=return_projections,
                          _fused_weight=self.fused_weight(), _fused_q_weight=self.q_weight(), _q_rows=q_rows)
 
-    def forward(self, x, state=None, residual=None):
+    def forward(self, x, state=None, residual=None, norm=None):
+        """``norm``: the pre-norm, where ``x`` is the un-normalised residual stream."""
+        if norm is not None and not (_plain_norm(norm) and _single(self.tp)):
+            x, norm = norm(x), None
         if _rows_mode(self.tp):
             return _forward_by_rows(self, x, residual), None
+        if _single(self.tp) and "core" not in self.__dict__ and type(self).core is CSAHybridLayer.core:
+            cfg = self.cfg
+            got = layers.csa_layer(x, None, self.Ba, self.Bb, self.B_idx, self.sink, m=cfg.csa_m, topk=cfg.csa_topk, nh=cfg.csa_nh,
+                                   nIh=cfg.csa_nIh, c=cfg.csa_c, c_I=cfg.csa_cI, dc=cfg.csa_dc, scale=1.0,
+                                   sliding_window=cfg.csa_sliding_window, W=self.fused_weight(), Wq=self.q_weight(), norm=norm,
+                                   W_o=self.o_proj.weight, residual=residual)
+            if got is not None:
+                return got[0], None
+        x = x if norm is None else norm(x)
         return out_projection(self.core(x), self.tp, self.o_proj.weight, residual=residual), None
 
 
@@ -451,9 +486,20 @@ class HCAHybridLayer(nn.Module):
                          sliding_window=cfg.hca_sliding_window, sink_logits=self.sink,
                          return_projections=return_projections, _fused_weight=self.fused_weight(), _q_rows=q_rows)
 
-    def forward(self, x, state=None, residual=None):
+    def forward(self, x, state=None, residual=None, norm=None):
+        """``norm``: the pre-norm, where ``x`` is the un-normalised residual stream."""
+        if norm is not None and not (_plain_norm(norm) and _single(self.tp)):
+            x, norm = norm(x), None
         if _rows_mode(self.tp):
             return _forward_by_rows(self, x, residual), None
+        if _single(self.tp) and "core" not in self.__dict__ and type(self).core is HCAHybridLayer.core:
+            cfg = self.cfg
+            got = layers.hca_layer(x, None, self.B_pos, self.sink, m2=cfg.hca_m2, nh=cfg.hca_nh, c=cfg.hca_c, dc=cfg.hca_dc,
+                                   scale=1.0, sliding_window=cfg.hca_sliding_window, W=self.fused_weight(), Wq=self.W_UQ.weight,
+                                   norm=norm, W_o=self.o_proj.weight, residual=residual)
+            if got is not None:
+                return got[0], None
+        x = x if norm is None else norm(x)
         return out_projection(self.core(x), self.tp, self.o_proj.weight, residual=residual), None
 
 
@@ -525,17 +571,34 @@ class HybridKCHAttention(nn.Module):
                              f"but the model has {self.n_kda_layers} KDA layers.")
         ki = 0
         new_lbs = []
+        final = self._final_states(x)
         for layer, norm, kind in zip(self.layers, self.norms, self.layout):
             if kind == "kda":
                 # the pre-norm goes into the layer: LayerNorm + short conv are one kernel there
-                x, st, lb = layer.forward_functional(x, states[ki], lookbacks[ki], residual=x, norm=norm)
+                x, st, lb = layer.forward_functional(x, states[ki], lookbacks[ki], residual=x, norm=norm,
+                                                     _final_state=None if final is None else final[ki])
                 states[ki] = st
                 new_lbs.append(lb)
                 ki += 1
             else:
-                x, _ = layer(norm(x), None, residual=x)
-        new_state = torch.stack(states, dim=0) if self.n_kda_layers > 0 else None
-        return x, new_state, new_lbs
+                # a layer that is watched by hooks sees what it always saw
+                x, _ = layer(x, None, residual=x, norm=norm) if _unwatched(layer) else layer(norm(x), None, residual=x)
+        return x, self._stacked(states, final), new_lbs
+
+    def _final_states(self, x):
+        """One buffer for the final states of all KDA layers of a call over several tokens."""
+        if self.n_kda_layers == 0 or x.shape[1] < 2 or not x.is_cuda:
+            return None
+        cfg = self.cfg
+        return torch.empty(self.n_kda_layers, x.shape[0], cfg.n_heads_v, cfg.head_dim_k, cfg.head_dim_v, dtype=torch.float32,
+                           device=x.device)
+
+    def _stacked(self, states, final):
+        if self.n_kda_layers == 0:
+            return None
+        if final is not None and all(s.data_ptr() == f.data_ptr() and s.shape == f.shape for s, f in zip(states, final)):
+            return final
+        return torch.stack(states, dim=0)
 
 
 class HybridDecoding(nn.Module):
@@ -708,6 +771,38 @@ class HybridDecoding(nn.Module):
         W = layer.o_proj.weight
         return out_projection(o_core, layer.tp, W, residual=residual, w_settled=T == 1 and _at_rest(W))
 
+    def _prompt(self, i, layer, norm, x):
+        """The first tokens of a session through a CSA / HCA layer: pre-norm, operator, output projection and residual in one
+        call, whose projections and compressed rows fill the cache.  None where that call does not apply."""
+        if (not _single(layer.tp) or not _plain_norm(norm) or type(layer) not in (CSAHybridLayer, HCAHybridLayer)
+                or "core" in layer.__dict__):
+            return None
+        cache = self._cache(i, layer, x)
+        if cache.n_tokens_seen > 0:
+            return None
+        cfg = self.cfg
+        if type(layer) is CSAHybridLayer:
+            c, cI = cfg.csa_c, cfg.csa_cI
+            got = layers.csa_layer(x, None, layer.Ba, layer.Bb, layer.B_idx, layer.sink, m=cfg.csa_m, topk=cfg.csa_topk, nh=cfg.csa_nh,
+                                   nIh=cfg.csa_nIh, c=c, c_I=cI, dc=cfg.csa_dc, scale=1.0, sliding_window=cfg.csa_sliding_window,
+                                   W=layer.fused_weight(), Wq=layer.q_weight(), norm=norm, W_o=layer.o_proj.weight, residual=x,
+                                   want_proj=True, want_rows=True)
+            if got is None:
+                return None
+            out, proj, rows = got
+            cache.append_step(*proj[..., :4 * c + 2 * cI].split([c, c, c, c, cI, cI], dim=-1), layer.Ba, layer.Bb, layer.B_idx,
+                              _rows=rows if layer.Ba.dtype == cache.dtype else None)
+            return out
+        c = cfg.hca_c
+        got = layers.hca_layer(x, None, layer.B_pos, layer.sink, m2=cfg.hca_m2, nh=cfg.hca_nh, c=c, dc=cfg.hca_dc, scale=1.0,
+                               sliding_window=cfg.hca_sliding_window, W=layer.fused_weight(), Wq=layer.W_UQ.weight, norm=norm,
+                               W_o=layer.o_proj.weight, residual=x, want_proj=True, want_rows=True)
+        if got is None:
+            return None
+        out, proj, rows = got
+        cache.append_step(proj[..., :c], proj[..., c:2 * c], layer.B_pos, _rows=rows if layer.B_pos.dtype == cache.dtype else None)
+        return out
+
     def _csa(self, i, layer, h, residual):
         cfg = self.cfg
         B_all = h.shape[0]
@@ -859,19 +954,21 @@ class HybridDecoding(nn.Module):
         in_place = (T == 1 and stacked is not None and stacked.dtype == torch.float32 and stacked.is_contiguous()
                     and stacked.device == x.device and model.cfg.kda_chunk_size != 1)
         ki = 0
+        final = model._final_states(x)
         for i, (layer, norm, kind) in enumerate(zip(model.layers, model.norms, model.layout)):
             if T == 0:
                 continue
             if kind == "kda":
                 # in place: the state and the conv lookback keep their addresses from token to token
                 x, st = layer(x, states[ki], residual=x, state_out=states[ki] if in_place else None,
-                              lookback_in_place=in_place, norm=norm)
+                              lookback_in_place=in_place, norm=norm, _final_state=None if final is None else final[ki])
                 states[ki] = st
                 ki += 1
-            elif kind == "csa":
-                x = self._csa(i, layer, norm(x), x)
             else:
-                x = self._hca(i, layer, norm(x), x)
+                y = self._prompt(i, layer, norm, x) if T > 1 else None
+                if y is None:
+                    y = (self._csa if kind == "csa" else self._hca)(i, layer, norm(x), x)
+                x = y
         if T > 0 and not in_place:
-            model._kda_state = torch.stack(states, dim=0) if model.n_kda_layers > 0 else None
+            model._kda_state = model._stacked(states, final)
         return x

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _lib, layers
 from .csa import attend, csa_compress_kv, fuse_rows, linear, mma_attention_eligible, rownorm
 
 
@@ -54,6 +54,12 @@ def naive_hca(H, W_KV, W_Z, B_pos, W_DQ, W_UQ, *, m2: int, nh: int, c: int, dc: 
             return out_empty, (torch.zeros(B_, 0, c, dtype=H.dtype, device=device),
                                torch.zeros(B_, 0, c, dtype=H.dtype, device=device))
         return out_empty
+    if W_KV_local is None and _q_rows is None:
+        got = layers.hca_layer(H, (W_KV, W_Z, W_DQ), B_pos, sink_logits, m2=m2, nh=nh, c=c, dc=dc, scale=float(scale),
+                               sliding_window=sliding_window, W=_fused_weight, Wq=W_UQ, want_proj=return_projections)
+        if got is not None:
+            out, proj, _ = got
+            return (out, (proj[..., :c], proj[..., c:2 * c])) if return_projections else out
     q_lo = 0
     if _q_rows is not None:
         q_lo, q_hi = int(_q_rows[0]), int(_q_rows[1])

@@ -361,3 +361,61 @@ def test_epilogue_segments_are_taken_by_value(monkeypatch):
         scale.fill_(value)
         csa.linear(x, W, epilogue=[(4, _lib.ACT_NEG_SOFTPLUS, scale)])
     assert seen == [[0.5], [2.0]]
+
+
+def test_layer_calls_refuse_on_the_host():
+    """The structures of the one-call layers reach the library field by field (sizes and messages depend on the last ones), and
+    calls that are wrong in one respect are refused before anything is launched (the pointers are never followed)."""
+    from kch_b200 import _lib
+    lib = _lib.load()
+
+    def csa(**kw):
+        a = _lib.CsaLayerArgs()
+        a.l.B, a.l.T, a.l.d, a.l.dtype, a.l.x, a.l.ld_x, a.l.out = 2, 100, 64, _lib.KCH_BF16, 4096, 64, 4096
+        a.c, a.c_I, a.dc, a.nh, a.nIh, a.m, a.topk, a.sliding_window, a.T_blocks, a.scale = 32, 16, 24, 4, 2, 16, 3, 5, 6, 1.0
+        a.W = a.Wq = a.Ba = a.Bb = a.B_idx = 4096
+        a.n_w, a.n_q, a.ld_w, a.ld_wq = 192, 160, 64, 24
+        for k, v in kw.items():
+            setattr(a.l if k in ("B", "norm_w", "W_o", "out") else a, k, v)
+        return a
+    full = lib.kch_csa_layer_workspace_bytes(csa())
+    assert full - lib.kch_csa_layer_workspace_bytes(csa(proj=4096)) == 2 * 100 * 192 * 2
+    assert full - lib.kch_csa_layer_workspace_bytes(csa(comp=4096)) == 2 * 6 * 32 * 4
+    assert full - lib.kch_csa_layer_workspace_bytes(csa(kcomp=4096)) == 2 * 6 * 16 * 4
+    assert lib.kch_csa_layer_workspace_bytes(csa(W=None)) - full == 192 * 64 * 2
+    for kw, why in ((dict(), "workspace"), (dict(B=0), "B=0"), (dict(T_blocks=5), "T_blocks=5"), (dict(n_w=180), "fused widths"),
+                    (dict(norm_w=4096), "come together"), (dict(m=0), "m=0"), (dict(B_idx=None), "biases"), (dict(W_o=4096, out=None), "`out`")):
+        assert lib.kch_csa_layer(csa(**kw), None) < 0 and why in lib.kch_last_error().decode(), (kw, lib.kch_last_error())
+
+    def hca(**kw):
+        a = _lib.HcaLayerArgs()
+        a.l.B, a.l.T, a.l.d, a.l.dtype, a.l.x, a.l.ld_x, a.l.out = 1, 70, 64, _lib.KCH_F32, 4096, 64, 4096
+        a.c, a.dc, a.nh, a.m2, a.sliding_window, a.T_blocks, a.scale, a.n_w, a.W, a.Wq, a.B_pos = 32, 16, 2, 32, 0, 2, 1.0, 80, 4096, 4096, 4096
+        for k, v in kw.items():
+            setattr(a, k, v)
+        return a
+    full = lib.kch_hca_layer_workspace_bytes(hca())
+    assert full - lib.kch_hca_layer_workspace_bytes(hca(comp=4096)) == 256 and full - lib.kch_hca_layer_workspace_bytes(hca(proj=4096)) == 22528
+    for kw, why in ((dict(), "workspace"), (dict(T_blocks=1), "T_blocks=1"), (dict(n_w=79), "fused width"), (dict(B_pos=None), "fused width")):
+        assert lib.kch_hca_layer(hca(**kw), None) < 0 and why in lib.kch_last_error().decode(), (kw, lib.kch_last_error())
+
+    def kda(**kw):
+        a = _lib.KdaLayerArgs()
+        a.l.B, a.l.T, a.l.d, a.l.dtype, a.l.x, a.l.ld_x, a.l.out, a.l.W_o = 1, 40, 64, _lib.KCH_F32, 4096, 64, 4096, 4096
+        a.H, a.HV, a.K, a.V, a.chunk_size, a.n_w, a.scale, a.decay_scale, a.g_clamp_min = 2, 2, 16, 16, 64, 120, 0.25, 0.1, -10.0
+        a.W = a.W_gup = a.conv_w = a.conv_b = a.lookback_out = 4096
+        for k, v in kw.items():
+            setattr(a.l if k in ("T",) else a, k, v)
+        return a
+    assert lib.kch_kda_layer_workspace_bytes(kda()) == 4 * 40 * (64 + 120 + 32 + 32)       # every piece a multiple of 256 here
+    for kw, why in ((dict(), "workspace"), (dict(T=1), "T=1"), (dict(HV=3), "HV=3"), (dict(n_w=113), "fused width"), (dict(lookback_out=None), "fused width")):
+        assert lib.kch_kda_layer(kda(**kw), None) < 0 and why in lib.kch_last_error().decode(), (kw, lib.kch_last_error())
+    a = _lib.CacheAppendArgs()
+    a.B, a.c, a.c_I, a.m, a.dtype, a.comp_kind, a.acc_len = 1, 8, 4, 4, _lib.KCH_F32, _lib.KCH_F32, 1
+    assert lib.kch_cache_append_prompt(a, 8, 64, 32, 0, 0, None, None, None, 0, None) < 0 and b"open block" in lib.kch_last_error()
+    a.acc_len = 0
+    a.comp_kind = _lib.KCH_FP8_E4M3
+    assert lib.kch_cache_append_prompt(a, 8, 64, 32, 0, 0, None, None, None, 0, None) < 0 and b"8-bit" in lib.kch_last_error()
+    a.comp_kind = _lib.KCH_F32
+    assert lib.kch_cache_append_prompt(a, 8, 64, 32, 0, 0, None, None, None, 0, None) < 0 and b"no room" in lib.kch_last_error()
+    assert lib.kch_cache_append_prompt_workspace_bytes(a, 8) == 512

@@ -509,3 +509,70 @@ def test_compress_subsets(kch, T, c, m):
     assert md(a, orc.compress_kv_overlapped(*t, Ba, Bb, m)) <= 2e-6
     b = kch.csa_compress_kv(t[0].to(DEV), t[2].to(DEV), Ba.to(DEV), m)
     assert md(b, orc.compress_kv(t[0], t[2], Ba, m)) <= 2e-6
+
+
+
+@pytest.mark.parametrize("geometry,dtype,B,T", [
+    ("small", torch.float32, 2, 97), ("small", torch.bfloat16, 1, 130), ("small", torch.float32, 1, 64), ("small", torch.bfloat16, 2, 20),
+    ("wide", torch.bfloat16, 2, 203), ("wide", torch.bfloat16, 1, 129), ("wide", torch.float32, 1, 70), ("narrow", torch.float32, 1, 150)])
+@pytest.mark.parametrize("path", ["stack", "prompt", "op"])
+def test_layer_calls_match_the_steps(kch, monkeypatch, geometry, dtype, B, T, path):
+    """The one-call form of the layers against the same launches issued one by one: the same kernels with the same arguments, so
+    the same bits.  Lengths below and above the blocks and chunks, ragged ones, and a geometry whose widths are not multiples
+    of 8 (which the calls leave to the steps)."""
+    from kch_b200 import layers
+    geo = {"small": dict(d_model=64, n_heads_qk=2, n_heads_v=4, head_dim_k=32, head_dim_v=16, csa_nh=4, csa_c=32, csa_dc=24, csa_nIh=2,
+                         csa_cI=16, csa_m=16, csa_topk=3, csa_sliding_window=5, hca_m2=32, hca_nh=2, hca_c=32, hca_dc=16,
+                         hca_sliding_window=0),
+           "wide": dict(d_model=256, n_heads_qk=2, n_heads_v=2, head_dim_k=128, head_dim_v=128, csa_nh=4, csa_c=128, csa_dc=64, csa_nIh=2,
+                        csa_cI=64, csa_m=4, csa_topk=16, csa_sliding_window=16, hca_m2=16, hca_nh=4, hca_c=128, hca_dc=64,
+                        hca_sliding_window=16),
+           "narrow": dict(d_model=36, n_heads_qk=1, n_heads_v=1, head_dim_k=12, head_dim_v=20, csa_nh=1, csa_c=12, csa_dc=10, csa_nIh=1,
+                          csa_cI=6, csa_m=8, csa_topk=4, csa_sliding_window=3, hca_m2=16, hca_nh=1, hca_c=12, hca_dc=10,
+                          hca_sliding_window=3)}[geometry]
+    cfg = kch.HybridConfig(**geo)
+    params = syn.hybrid_params(3, cfg, 5, dtype=dtype, random_sink=True)
+    x = syn.hidden_states(4, B, T, cfg.d_model, dtype).to(DEV)
+    model = kch.HybridKCHAttention(cfg, 5)
+    model.load_state_dict(params, strict=True)
+    model = model.to(dtype).to(DEV).eval()
+
+    def run():
+        if path == "stack":
+            y, S, lbs = model.forward_functional(x, None, [None] * 3)
+            return [y, S, *lbs, *model.forward_functional(x[:, : T // 2 + 2].contiguous(), S, lbs)[:2]]
+        if path == "op":
+            csa, hca = model.layers[3], model.layers[4]
+            w = {k: getattr(csa, k).weight for k in ("W_aKV", "W_bKV", "W_aZ", "W_bZ")}
+            got = kch.naive_csa(x, *w.values(), csa.Ba, csa.Bb, csa.W_DQ.weight, csa.W_UQ.weight, csa.W_IUQ.weight, csa.W_w.weight,
+                                csa.W_KV_idx.weight, csa.W_Z_idx.weight, csa.B_idx, m=cfg.csa_m, topk=cfg.csa_topk, nh=cfg.csa_nh,
+                                nIh=cfg.csa_nIh, c=cfg.csa_c, c_I=cfg.csa_cI, dc=cfg.csa_dc, sliding_window=cfg.csa_sliding_window,
+                                sink_logits=csa.sink, use_ste=False, normalize_qk=True, return_projections=True)
+            got2 = kch.naive_hca(x, hca.W_KV.weight, hca.W_Z.weight, hca.B_pos, hca.W_DQ.weight, hca.W_UQ.weight, m2=cfg.hca_m2,
+                                 nh=cfg.hca_nh, c=cfg.hca_c, dc=cfg.hca_dc, sliding_window=cfg.hca_sliding_window, sink_logits=hca.sink,
+                                 return_projections=True)
+            return [got[0], *got[1], got2[0], *got2[1], csa(x)[0], hca(x, residual=x)[0]]
+        dec = kch.HybridDecoding(model=model)
+        dec.reset()
+        out = [dec(x[:, : T - 7]), dec(x[:, T - 7: T - 1]), dec(x[:, T - 1:]), model._kda_state]
+        for c in dec._caches.values():
+            st = c.export_state()
+            out += [t for t in (*st["acc"], st["comp"], st["norms"], st["ring"], *st.get("prev", []), st.get("kcomp"), c._ctr) if t is not None]
+        return out
+    with torch.no_grad():
+        calls = {}
+        for name in ("csa_layer", "hca_layer", "kda_layer"):
+            def spy(*a, _f=getattr(layers, name), _n=name, **kw):
+                got = _f(*a, **kw)
+                calls[_n] = calls.get(_n, 0) + (got is not None)
+                return got
+            monkeypatch.setattr(layers, name, spy)
+        one = run()
+        if geometry != "narrow" and T >= 64:
+            assert all(calls.get(n, 0) > 0 for n in (("csa_layer", "hca_layer") if path == "op" else ("csa_layer", "hca_layer", "kda_layer"))), calls
+        for name in ("csa_layer", "hca_layer", "kda_layer"):
+            monkeypatch.setattr(layers, name, lambda *a, **kw: None)
+        steps = run()
+    assert len(one) == len(steps)
+    for a, b in zip(one, steps):
+        assert a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b), (a.shape, float((a.double() - b.double()).abs().max()))
