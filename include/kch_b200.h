@@ -167,6 +167,16 @@ int kch_kda_recurrent(const void* q, const void* k, const void* v, const void* g
                       int HV, int K, int V, float scale, float g_clamp_min, int dtype, int64_t ld_qk,
                       int64_t ld_v, int64_t ld_g, int64_t ld_beta, void* stream);
 
+/* One token (T = 1) of the same recurrence for bf16, K = V = 128, with the gate's up-projection and activation folded in: gate_x
+ * [B, K] is the output of g_down (rows ld_gate apart), W_gup [HV * K, K], and g = round(-round(softplus(round(W_gup gate_x))) *
+ * gate_scale) (KDAHybridLayer, ops_fused.py:575-578).  `w_settled`: as kch_linear_settled.  16-byte aligned gate operands and
+ * states; B * HV up to 296 (kch_kda_step_gate_supported). */
+int kch_kda_step_gate_supported(int B, int HV, int K, int V, int dtype);
+int kch_kda_step_gate(const void* q, const void* k, const void* v, const void* gate_x, const void* W_gup, const void* beta,
+                      const float* initial_state, void* o, float* final_state, int B, int H, int HV, int K, int V, float scale,
+                      float g_clamp_min, float gate_scale, int dtype, int64_t ld_qk, int64_t ld_v, int64_t ld_gate, int64_t ld_wg,
+                      int64_t ld_beta, int w_settled, void* stream);
+
 /* naive_chunk_kda, ops_kda.py:340-536 (prepare 375-424, chain 509-535, finalize 440-461).  Same
  * tensors as above.  Needs a workspace of kch_kda_chunk_workspace_bytes(...) bytes. */
 int64_t kch_kda_chunk_workspace_bytes(int B, int T, int HV, int K, int V, int chunk_size);

@@ -99,11 +99,17 @@ kda_recurrent_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 // The wait for the copy is bounded (status word, see kch_device_status).
 #define KDS_STATE_BYTES (128 * 128 * 4)
 #define KDS_SMEM (KDS_STATE_BYTES + 128 * 16 + 2 * 4 * 128 * 4 + 16)
-template <typename T, int RPT>
+struct KdsGate {                         // the gate's up-projection and activation, for a step that brings their input
+  const bf16 *x, *W;                     // [B, 128] rows ld_x apart; [HV * 128, 128] rows ld_w apart
+  int64_t ld_x, ld_w;
+  float scale;                           // g = round(-round(softplus(round(W x))) * scale), the rounding points of the layer
+  int settled;                           // the launch before does not write W
+};
+template <typename T, int RPT, bool GATE>
 __global__ void __launch_bounds__(512 / RPT, RPT == 4 ? 3 : 2)
 kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int H,
                        int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b,
-                       unsigned int* status) {
+                       const KdsGate gate, unsigned int* status) {
   constexpr int K = 128, V = 128;
   extern __shared__ __align__(128) uint8_t kds_raw[];
   float* st = reinterpret_cast<float*>(kds_raw);                                   // [K][V]
@@ -117,16 +123,55 @@ kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* 
     mbarrier_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // the head's 128 x 128 gate weights: four threads a row, 64 bytes each
+  static_assert(!GATE || RPT == 1, "one row of the gate's weights per four threads");
+  uint4 wraw[4];
+  auto load_gate_weights = [&]() {
+    const uint4* p = reinterpret_cast<const uint4*>(gate.W + ((int64_t)hv * K + (tid >> 2)) * gate.ld_w + 32 * (tid & 3));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wraw[i] = p[i];
+  };
+  if (GATE && gate.settled) load_gate_weights();
   chain_wait();
   chain_trigger();
   if (tid == 0 && S0) {
     mbarrier_expect_tx(bar, KDS_STATE_BYTES);
     bulk_copy_g2s(st, S0 + sbase, KDS_STATE_BYTES, bar);
   }
+  if (GATE && !gate.settled) load_gate_weights();
   const int c = tid & 127, run0 = (tid >> 7) * RPT;    // value column, first of this thread's runs of 32 K rows
   const float bt = ldf(beta + (int64_t)b * ld_b + hv);
   const float vv = ldf(v + (int64_t)b * ld_v + (int64_t)hv * V + c);
-  if (tid < K) {
+  if constexpr (GATE) {
+    uint4 xraw[4];
+    const uint4* xp = reinterpret_cast<const uint4*>(gate.x + (int64_t)b * gate.ld_x + 32 * (tid & 3));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xraw[i] = xp[i];
+    if (tid < K) {
+      const int64_t qoff = (int64_t)b * ld_qk + (int64_t)h * K;
+      reinterpret_cast<float*>(sgkq + tid)[1] = ldf(k + qoff + tid);
+      reinterpret_cast<float*>(sgkq + tid)[2] = ldf(q + qoff + tid) * scale;
+    }
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t w4[4] = {wraw[i].x, wraw[i].y, wraw[i].z, wraw[i].w};
+      const uint32_t x4[4] = {xraw[i].x, xraw[i].y, xraw[i].z, xraw[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        dot = fmaf(__uint_as_float(w4[e] << 16), __uint_as_float(x4[e] << 16), dot);
+        dot = fmaf(__uint_as_float(w4[e] & 0xFFFF0000u), __uint_as_float(x4[e] & 0xFFFF0000u), dot);
+      }
+    }
+    dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+    dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+    if ((tid & 3) == 0) {
+      // the activation as the projection's epilogue applies it (gemm_decode.cu)
+      const float t = round_to<bf16>(dot);
+      const float gv = round_to<bf16>(-round_to<bf16>(t > 20.f ? t : __logf(1.0f + __expf(t))) * gate.scale);
+      reinterpret_cast<float*>(sgkq + (tid >> 2))[0] = expf(fmaxf(gv, g_min));
+    }
+  } else if (tid < K) {
     const int64_t qoff = (int64_t)b * ld_qk + (int64_t)h * K, goff = (int64_t)b * ld_g + (int64_t)hv * K;
     sgkq[tid] = make_float4(expf(fmaxf(ldf(g + goff + tid), g_min)), ldf(k + qoff + tid), ldf(q + qoff + tid) * scale, 0.f);
   }
@@ -176,6 +221,56 @@ kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* 
   if (S_out && tid == 0 && ok) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory must outlive the copy
 }
 
+// Steps of up to two heads an SM: one row a thread, and the form that projects the gate itself.  Beyond that the 32 KB of weights
+// that every CTA reads cost as much as the launch that they save (64 sequences, 16 heads, whole step: 356 us with the launch, 360
+// without; 8 sequences: 199 and 185).
+static bool kds_few(int B, int HV) { return (int64_t)HV * B <= 2 * 148; }
+
+template <typename T, bool GATE>
+static int launch_kda_step(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int B, int H,
+                           int HV, float scale, float g_min, int64_t ld_qk, int64_t ld_v, int64_t ld_g, int64_t ld_b, const KdsGate& gate,
+                           cudaStream_t s) {
+  unsigned int* status = kch_status_device_ptr();
+  KCH_REQUIRE(status != nullptr, "kch_kda_recurrent: cannot resolve the device status word");
+#define KDS_GO(RPT_)                                                                                                               \
+  do {                                                                                                                             \
+    KCH_CUDA_OK(cudaFuncSetAttribute(kda_decode_step_kernel<T, RPT_, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, KDS_SMEM)); \
+    KCH_CUDA_OK(kch_launch_chained(kda_decode_step_kernel<T, RPT_, GATE>, dim3(HV, B), dim3(512 / RPT_), KDS_SMEM, s, 1, q, k, v, g,  \
+                                   beta, S0, o, S_out, H, HV, scale, g_min, ld_qk, ld_v, ld_g, ld_b, gate, status));               \
+  } while (0)
+  if constexpr (GATE) {
+    KDS_GO(1);
+  } else {
+    if (kds_few(B, HV)) KDS_GO(1);
+    else KDS_GO(4);
+  }
+#undef KDS_GO
+  KCH_LAUNCH_OK();
+  return KCH_OK;
+}
+
+extern "C" int kch_kda_step_gate_supported(int B, int HV, int K, int V, int dtype) {
+  return dtype == KCH_BF16 && K == 128 && V == 128 && B >= 1 && HV >= 1 && kds_few(B, HV);
+}
+
+// The one-token step of a layer whose gate has not been projected up yet (see KdsGate).  As a launch of its own the up-projection
+// (0.5 MB of weights) took 4.5 us of a step between the two it depends on; here its weights are under way before the launch
+// before has finished, and its 16 K products a head hide behind the copy of the state.
+extern "C" int kch_kda_step_gate(const void* q, const void* k, const void* v, const void* gate_x, const void* W_gup, const void* beta,
+                                 const float* initial_state, void* o, float* final_state, int B, int H, int HV, int K, int V, float scale,
+                                 float g_clamp_min, float gate_scale, int dtype, int64_t ld_qk, int64_t ld_v, int64_t ld_gate, int64_t ld_wg,
+                                 int64_t ld_beta, int w_settled, void* stream) {
+  KCH_REQUIRE(kch_kda_step_gate_supported(B, HV, K, V, dtype),
+              "kch_kda_step_gate: bf16 with K = V = 128 and B * HV from 1 to 296 only (dtype tag %d, K=%d, V=%d, B=%d, HV=%d)", dtype, K, V, B, HV);
+  KCH_REQUIRE(H >= 1 && HV % H == 0, "kch_kda_step_gate: H=%d HV=%d", H, HV);
+  KCH_REQUIRE(q && k && v && gate_x && W_gup && beta && o, "kch_kda_step_gate: an operand is missing");
+  KCH_REQUIRE(((((uintptr_t)gate_x | (uintptr_t)W_gup | (uintptr_t)initial_state | (uintptr_t)final_state) & 15) == 0) && (ld_gate % 8) == 0 && (ld_wg % 8) == 0,
+              "kch_kda_step_gate: gate input, weights and states must be 16-byte aligned with strides that are multiples of 8 elements");
+  const KdsGate gate = {(const bf16*)gate_x, (const bf16*)W_gup, ld_gate, ld_wg, gate_scale, w_settled};
+  return launch_kda_step<bf16, true>((const bf16*)q, (const bf16*)k, (const bf16*)v, nullptr, (const bf16*)beta, initial_state, (bf16*)o,
+                                     final_state, B, H, HV, scale, g_clamp_min, ld_qk, ld_v, 0, ld_beta, gate, kch_stream(stream));
+}
+
 extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, const void* g,
                                  const void* beta, const float* initial_state, void* o,
                                  float* final_state, int B, int T, int H, int HV, int K, int V,
@@ -198,20 +293,10 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
   // (KCH_KDA_DECODE=o keeps the general kernel for the one-token step, for comparison)
   static const bool old_step = [] { const char* e = getenv("KCH_KDA_DECODE"); return e && e[0] == 'o'; }();
   if (T == 1 && K == 128 && V == 128 && !old_step && (((uintptr_t)initial_state | (uintptr_t)final_state) & 15) == 0) {
-    unsigned int* status = kch_status_device_ptr();
-    KCH_REQUIRE(status != nullptr, "kch_kda_recurrent: cannot resolve the device status word");
-#define KDS_GO(T_, RPT_)                                                                                                         \
-  do {                                                                                                                           \
-    KCH_CUDA_OK(cudaFuncSetAttribute(kda_decode_step_kernel<T_, RPT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, KDS_SMEM));  \
-    KCH_CUDA_OK(kch_launch_chained(kda_decode_step_kernel<T_, RPT_>, dim3(HV, B), dim3(512 / RPT_), KDS_SMEM, s, 1,              \
-        (const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta, initial_state, (T_*)o, final_state, H, HV,      \
-        scale, g_clamp_min, ld_qk, ld_v, ld_g, ld_beta, status));                                                                \
-  } while (0)
-    const bool few = (int64_t)HV * B <= 2 * 148;
-    KCH_DISPATCH_FLOAT(dtype, T_, { if (few) KDS_GO(T_, 1); else KDS_GO(T_, 4); });
-#undef KDS_GO
-    KCH_LAUNCH_OK();
-    return KCH_OK;
+    const KdsGate none = {};
+    KCH_DISPATCH_FLOAT(dtype, T_, return (launch_kda_step<T_, false>((const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta,
+                                                                     initial_state, (T_*)o, final_state, B, H, HV, scale, g_clamp_min, ld_qk,
+                                                                     ld_v, ld_g, ld_beta, none, s)));
   }
   int kpt = (K + 3) / 4;
 #define GO(T_, KPT)                                                                              \

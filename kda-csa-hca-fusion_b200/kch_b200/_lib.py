@@ -115,6 +115,8 @@ PROTOTYPES = {
     "kch_activation": (_i, [_vp, _vp, _i64, _i, _i, _f, _i, _i, _i64, _i64, _vp]),
     "kch_rownorm": (_i, [_vp, _i64, _vp, _vp, _i64, _i, _i, _i, _vp]),
     "kch_kda_recurrent": (_i, [_vp] * 8 + [_i] * 6 + [_f, _f, _i, _i64, _i64, _i64, _i64, _vp]),
+    "kch_kda_step_gate_supported": (_i, [_i] * 5),
+    "kch_kda_step_gate": (_i, [_vp] * 9 + [_i] * 5 + [_f, _f, _f, _i, _i64, _i64, _i64, _i64, _i64, _i, _vp]),
     "kch_kda_chunk_workspace_bytes": (_i64, [_i] * 6),
     "kch_kda_chunk": (_i, [_vp] * 8 + [_i] * 7 + [_f, _f, _i, _i64, _i64, _i64, _i64, _vp, _i64, _vp]),
     "kch_kda_chunk_gate_supported": (_i, [_i, _i, _i, _f, _i]),

@@ -21,7 +21,7 @@ from . import _lib, layers
 from .csa import attend, fuse_rows, indexer_topk, linear, mma_attention_eligible, naive_csa, rownorm
 from .decoding_cache import CSADecodingCache, HCADecodingCache
 from .hca import naive_hca
-from .kda import chunk_gate_supported, kda_forward, validate_kda_backend
+from .kda import chunk_gate_supported, kda_forward, step_gate, step_gate_supported, validate_kda_backend
 from .tp import gather_heads, out_projection, out_projection_rows, row_span  # noqa: F401
 
 
@@ -281,9 +281,11 @@ class KDAHybridLayer(nn.Module):
         self._conv_lookback = lb
         return o, new_state
 
-    def project(self, x, conv_lookback, lookback_in_place=False, norm=None, raw_gate=False):
+    def project(self, x, conv_lookback, lookback_in_place=False, norm=None, raw_gate=False, gate_later=False):
         """conv + fused projection + activations -> (q, k, v, g, beta, new_lookback).  With
         ``lookback_in_place`` a one-token call slides ``conv_lookback`` where it lies and returns it.
+        ``gate_later``: the gate's low-rank input comes back in the place of ``g``, and behind the rest whether the conv step ran
+        as one kernel.
         ``norm``: the sub-layer's pre-norm when ``x`` is the un-normalised residual stream; LayerNorm and the
         convolution then run as one kernel where the shape allows."""
         cfg = self.cfg
@@ -325,6 +327,8 @@ class KDAHybridLayer(nn.Module):
         # in a one-token step the kernel before each projection is one of ours, which produced its input
         proj = linear(xc, W, epilogue=segs, group=K, w_settled=fused_step and settled)
         q, k, v, gd, beta = proj[..., :n_used].split([H * K, H * K, HV * V, K, HV], dim=-1)
+        if gate_later:
+            return (q.unflatten(-1, (H, K)), k.unflatten(-1, (H, K)), v.unflatten(-1, (HV, V)), gd, beta, new_lb, fused_step)
         W = self.g_up.weight
         if raw_gate:     # the chunk kernel applies -softplus(.) * decay_scale when it loads the gate
             g = linear(gd, W)
@@ -351,8 +355,21 @@ class KDAHybridLayer(nn.Module):
         use_chunk = cfg.kda_chunk_size >= 1 and T >= cfg.kda_chunk_size
         raw_gate = use_chunk and cfg.kda_decay_scale > 0 and chunk_gate_supported(
             cfg.head_dim_k, cfg.head_dim_v, cfg.kda_chunk_size, -10.0, x.dtype)
-        q, k, v, g, beta, new_lb = self.project(x, conv_lookback, lookback_in_place, norm, raw_gate)
-        o, new_state = kda_forward(q, k, v, g, beta, scale=self._scale_value(), initial_state=state,
+        W = self.g_up.weight
+        if T == 1 and not use_chunk and x.is_cuda and W.dtype == x.dtype and step_gate_supported(B, HV, cfg.head_dim_k, V, x.dtype):
+            validate_kda_backend(cfg.kda_backend)
+            q, k, v, gd, beta, new_lb, fused_step = self.project(x, conv_lookback, lookback_in_place, norm, gate_later=True)
+            # (the kernel before is the fused projection, which does not write the gate's weights)
+            got = step_gate(q, k, v, gd, W, beta, scale=self._scale_value(), initial_state=state, state_out=state_out,
+                            gate_scale=cfg.kda_decay_scale, w_settled=fused_step and _at_rest(W))
+            if got is None:
+                g = linear(gd, W, epilogue=[(HV * cfg.head_dim_k, _lib.ACT_NEG_SOFTPLUS, cfg.kda_decay_scale)])
+                got = kda_forward(q, k, v, g.view(B, T, HV, cfg.head_dim_k), beta, scale=self._scale_value(), initial_state=state,
+                                  output_final_state=True, backend=cfg.kda_backend, state_out=state_out)
+        else:
+            got = None
+            q, k, v, g, beta, new_lb = self.project(x, conv_lookback, lookback_in_place, norm, raw_gate)
+        o, new_state = got if got is not None else kda_forward(q, k, v, g, beta, scale=self._scale_value(), initial_state=state,
                                    output_final_state=True, chunk_size=cfg.kda_chunk_size, use_chunk=use_chunk,
                                    backend=cfg.kda_backend, state_out=None if use_chunk else state_out,
                                    gate_scale=cfg.kda_decay_scale if raw_gate else None)

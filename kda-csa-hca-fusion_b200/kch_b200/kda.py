@@ -169,6 +169,47 @@ def naive_recurrent_kda(q, k, v, g, beta, scale=None, initial_state=None, output
                 g_clamp_min, state_dtype, None, state_out)
 
 
+def step_gate_supported(B, HV, K, V, dtype):
+    """Can ``step_gate`` take this geometry?"""
+    return dtype == torch.bfloat16 and bool(_lib.load().kch_kda_step_gate_supported(int(B), int(HV), int(K), int(V), _lib.KCH_BF16))
+
+
+def step_gate(q, k, v, gate_x, W_gup, beta, *, scale, initial_state, state_out, gate_scale, w_settled=False):
+    """One token of ``naive_recurrent_kda`` whose gate is ``-softplus(W_gup gate_x) * gate_scale``, projected in the same launch
+    (bf16, heads of 128).  ``(o, state)``, or None for a call that is not of this form."""
+    B, T, H, K = q.shape
+    HV, V = v.shape[2], v.shape[3]
+    if T != 1 or HV % H or q.dtype != torch.bfloat16 or not q.is_cuda or not step_gate_supported(B, HV, K, V, q.dtype):
+        return None
+    if not (k.shape == q.shape and v.shape[:2] == (B, 1) and beta.shape == (B, 1, HV) and gate_x.shape == (B, 1, K)
+            and W_gup.shape == (HV * K, K) and q.dtype == k.dtype == v.dtype == beta.dtype == gate_x.dtype == W_gup.dtype
+            and q.device == k.device == v.device == beta.device == gate_x.device == W_gup.device):
+        return None
+    S0, S = initial_state, state_out
+    for t in (S0, S):
+        if t is not None and not (t.dtype == torch.float32 and t.shape == (B, HV, K, V) and t.is_contiguous() and t.device == q.device
+                                  and t.data_ptr() % 16 == 0):
+            return None
+    if gate_x.stride(2) != 1 or W_gup.stride(1) != 1 or W_gup.stride(0) % 8 or gate_x.data_ptr() % 16 or W_gup.data_ptr() % 16:
+        return None
+    ld_x = gate_x.stride(0) if B > 1 else K
+    q, ld_q = _token_stride(q)
+    k, ld_k = _token_stride(k)
+    v, ld_v = _token_stride(v)
+    beta, ld_b = _token_stride(beta)
+    if ld_q != ld_k or ld_x % 8 or ld_x < K:
+        return None
+    o = torch.empty(B, 1, HV, V, dtype=v.dtype, device=q.device)
+    if S is None:
+        S = torch.empty(B, HV, K, V, dtype=torch.float32, device=q.device)
+    with _lib.device(q.device):
+        _lib.check(_lib.load().kch_kda_step_gate(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(gate_x), _lib.ptr(W_gup), _lib.ptr(beta),
+                                                 _lib.ptr(S0), _lib.ptr(o), _lib.ptr(S), B, H, HV, K, V, float(scale), -10.0,
+                                                 float(gate_scale), _lib.KCH_BF16, ld_q, ld_v, ld_x, W_gup.stride(0), ld_b,
+                                                 int(w_settled), _lib.stream()))
+    return o, S
+
+
 def chunk_gate_supported(K, V, chunk_size, g_clamp_min, dtype):
     """Can ``naive_chunk_kda`` take the gate's pre-activation (``_gate_scale``) for this geometry?"""
     if dtype != torch.bfloat16:

@@ -576,3 +576,33 @@ def test_layer_calls_match_the_steps(kch, monkeypatch, geometry, dtype, B, T, pa
     assert len(one) == len(steps)
     for a, b in zip(one, steps):
         assert a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b), (a.shape, float((a.double() - b.double()).abs().max()))
+
+
+@pytest.mark.parametrize("B,H,HV,state,stride,settled", [(1, 1, 1, False, 0, True), (2, 4, 8, True, 8, False), (37, 8, 8, True, 0, True),
+                                                         (37, 2, 4, True, 136, True), (18, 16, 16, False, 24, False)])
+def test_kda_step_gate(kch, B, H, HV, state, stride, settled):
+    """One token whose gate is projected in the same launch: from one head to the 296 that take that form, grouped heads, gate
+    inputs that lie inside a wider row.  The pre-activation (|t| <= 5 here), its softplus and their product
+    with the scale are rounded to bf16 each: the gate is within 7 * 2^-8 of itself, exp(gate) within 0.37 of that; the
+    intrinsic exponential and logarithm stay far below a rounding."""
+    from kch_b200.kda import step_gate, step_gate_supported
+    assert step_gate_supported(B, HV, 128, 128, torch.bfloat16) and not step_gate_supported(297, 1, 128, 128, torch.bfloat16)
+    q, k, v, _, beta, S0 = (x.to(DEV) for x in syn.kda_inputs(B + HV, B, 1, H, 128, 128, HV, torch.bfloat16, with_state=True))
+    gen = torch.Generator().manual_seed(B)
+    x = torch.randn(B, 1, 128 + stride, generator=gen).bfloat16().to(DEV)[..., stride // 16 * 8:][..., :128]
+    W = (torch.randn(HV * 128, 128, generator=gen) * 0.08).bfloat16().to(DEV)
+    S0 = S0 if state else None
+    o, S = step_gate(q, k, v, x, W, beta, scale=128 ** -0.5, initial_state=S0, state_out=None, gate_scale=0.3, w_settled=settled)
+    t = x.double() @ W.double().T
+    assert float(t.abs().max()) <= 5.0
+    decay = torch.exp((-0.3 * torch.nn.functional.softplus(t)).clamp(min=-10.0)).view(B, HV, 128, 1)
+    qd, kd = (y.double()[:, 0].repeat_interleave(HV // H, 1) for y in (q, k))
+    vd, bd = v.double()[:, 0], beta.double()[:, 0].unsqueeze(-1)
+    prev = (torch.zeros(B, HV, 128, 128, device=DEV, dtype=torch.float64) if S0 is None else S0.double()) * decay
+    S_ref = prev + kd.unsqueeze(-1) * (bd * (vd - torch.einsum("bhk,bhkv->bhv", kd, prev))).unsqueeze(-2)
+    off = 0.37 * 7 * 2.0 ** -8 * (torch.zeros_like(prev) if S0 is None else S0.double().abs())
+    off = off + kd.abs().unsqueeze(-1) * (bd * torch.einsum("bhk,bhkv->bhv", kd.abs(), off)).unsqueeze(-2)
+    assert bool(((S.double() - S_ref).abs() <= off + 1e-5).all()), float(((S.double() - S_ref).abs() - off).max())
+    o_ref = torch.einsum("bhk,bhkv->bhv", qd, S_ref) * 128 ** -0.5
+    off = torch.einsum("bhk,bhkv->bhv", qd.abs(), off) * 128 ** -0.5 + o_ref.abs() * 2.0 ** -8
+    assert bool(((o[:, 0].double() - o_ref).abs() <= off + 1e-5).all())
