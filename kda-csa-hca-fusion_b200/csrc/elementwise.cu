@@ -675,20 +675,24 @@ extern "C" int kch_activation(const void* x, void* y, int64_t rows, int cols, in
 
 // ---------------------------------------------------------------------------------------
 // L2 row normalisation into fp32:  y = fp32(x) / max(||fp32(x)||, 1e-12)   (F.normalize).
-// Input rows may be strided (ld elements between rows); one warp per row.
+// Input rows may be strided: `groups` rows of c elements one after the other, the next `groups` of them ld elements on.
 // `norms` (optional) receives max(||x||,eps) per row; `y` may be null when only norms are wanted.
+// A row's squares are summed in one order in every form: element i is added to the sum of its i mod 32 (i ascending), and
+// those 32 sums are added by halves.  What a row's norm is does not depend on where the row lies, and a selection between
+// blocks that score alike does not depend on the path.
 // ---------------------------------------------------------------------------------------
+// one warp per row
 template <typename T, typename TO>
-__global__ void rownorm_kernel(const T* __restrict__ x, int64_t ld, TO* __restrict__ y,
+__global__ void rownorm_kernel(const T* __restrict__ x, int64_t ld, int groups, TO* __restrict__ y,
                                float* __restrict__ norms, int64_t rows, int c) {
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
   if (row >= rows) return;
-  const T* xr = x + row * ld;
+  const T* xr = x + (row / groups) * ld + (row % groups) * c;
   float ss = 0.f;
   for (int i = lane; i < c; i += 32) {
     float v = ldf(xr + i);
-    ss += v * v;
+    ss = fmaf(v, v, ss);
   }
   float nrm = fmaxf(sqrtf(warp_sum(ss)), 1e-12f);
   if (norms && lane == 0) norms[row] = nrm;
@@ -696,27 +700,63 @@ __global__ void rownorm_kernel(const T* __restrict__ x, int64_t ld, TO* __restri
     for (int i = lane; i < c; i += 32) stf(y + row * c + i, ldf(xr + i) / nrm);
 }
 
-// The same for rows of c = 8 * lpr elements on 16-byte boundaries (lpr a power of two): lpr lanes a row, 8 elements a lane, so a
-// warp has 32 / lpr rows in flight.  Bound: HBM; 65536 bf16 rows of 128: 11.3 us (an element a lane and load: 17.2).
-template <typename T, typename TO>
-__global__ void __launch_bounds__(256) rownorm_vec_kernel(const T* __restrict__ x, int64_t ld, TO* __restrict__ y, float* __restrict__ norms,
-                                                         int64_t rows, int lpr) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, row = i / lpr;
-  const int part = (int)(i % lpr);
+// Sum of the squares of a row of 8 * LPR elements, eight consecutive ones in each of LPR neighbouring lanes, in the order above.
+// Lanes 4 apart hold the elements that go into the same sums: they are dealt out among those LPR / 4 lanes first (a transpose,
+// 8 shuffles for 128 elements), then the 32 sums are halved across lanes and registers.
+template <int LPR>
+__device__ __forceinline__ float row_square_sum(float (&v)[8], int part) {
+  constexpr int KR = LPR >= 4 ? LPR / 4 : 1, OWN = 8 / KR;      // elements of a sum; sums of a lane
+#pragma unroll
+  for (int kb = KR / 2; kb >= 1; kb >>= 1) {
+    const bool up = (part >> 2) & kb;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int eb = kb * OWN;
+      if (j & eb) continue;
+      const float got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + eb], 4 * kb);
+      if (up) v[j] = got;
+      else v[j + eb] = got;
+    }
+  }
+  float s[OWN];
+#pragma unroll
+  for (int j = 0; j < OWN; ++j) {
+    s[j] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KR; ++k) s[j] = fmaf(v[k * OWN + j], v[k * OWN + j], s[j]);
+    if (LPR > 2) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 2);
+    if (LPR > 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 1);
+  }
+#pragma unroll
+  for (int eb = 4; eb >= 1; eb >>= 1) {
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+      if (eb >= OWN) s[j] += __shfl_xor_sync(0xffffffffu, s[j], 4 * (eb / OWN));
+      else if (!(j & eb)) s[j] += s[j + eb];
+    }
+  }
+  return s[0];
+}
+
+// The same for rows of c = 8 * LPR elements on 16-byte boundaries: LPR lanes a row, 8 elements a lane, so a warp has 32 / LPR
+// rows in flight.  Bound: HBM; 262144 bf16 rows of 128: 37 us (an element a lane and load: 60).
+template <typename T, typename TO, int LPR>
+__global__ void __launch_bounds__(256) rownorm_vec_kernel(const T* __restrict__ x, int64_t ld, int groups, TO* __restrict__ y,
+                                                         float* __restrict__ norms, int64_t rows) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, row = i / LPR;
+  const int part = (int)(i % LPR);
   const bool on = row < rows;
-  float v[8];
+  float v[8], w[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = 0.f;
-  if (on) ld8p(x + row * ld + 8 * part, v);
-  float ss = 0.f;
+  if (on) ld8p(x + (groups == 1 ? row * ld : (row / groups) * ld + (row % groups) * (8 * LPR)) + 8 * part, v);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
-  for (int o = lpr >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  for (int k = 0; k < 8; ++k) w[k] = v[k];
+  const float nrm = fmaxf(sqrtf(row_square_sum<LPR>(w, part)), 1e-12f);
   if (!on) return;
-  const float nrm = fmaxf(sqrtf(ss), 1e-12f);
   if (norms && part == 0) norms[row] = nrm;
   if (!y) return;
-  TO* dst = y + (row * lpr + part) * 8;
+  TO* dst = y + (row * LPR + part) * 8;
   if constexpr (sizeof(TO) == 2) {
     uint4 o4;
     bf16* o = reinterpret_cast<bf16*>(&o4);
@@ -729,22 +769,35 @@ __global__ void __launch_bounds__(256) rownorm_vec_kernel(const T* __restrict__ 
   }
 }
 
-extern "C" int kch_rownorm(const void* x, int64_t ld, void* y, float* norms, int64_t rows, int c,
-                           int dtype, int out_dtype, void* stream) {
-  KCH_REQUIRE(rows >= 0 && c >= 1 && ld >= c, "kch_rownorm: rows=%lld c=%d ld=%lld", (long long)rows, c,
-              (long long)ld);
+// `rows` counts the groups' rows
+int kch_rownorm_groups(const void* x, int64_t ld, int groups, void* y, float* norms, int64_t rows, int c, int dtype,
+                       int out_dtype, void* stream) {
   if (rows == 0) return KCH_OK;
+  cudaStream_t s = kch_stream(stream);
   const int lpr = c / 8;
   if (c % 8 == 0 && lpr <= 32 && (lpr & (lpr - 1)) == 0 && ld % 8 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
     const unsigned g = (unsigned)ceil_div64(rows * lpr, 256);
-    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(out_dtype, TO,
-        (rownorm_vec_kernel<T, TO><<<g, 256, 0, kch_stream(stream)>>>((const T*)x, ld, (TO*)y, norms, rows, lpr))));
+#define RNV(LPR)                                                                                                         \
+    KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(out_dtype, TO,                                                       \
+        (rownorm_vec_kernel<T, TO, LPR><<<g, 256, 0, s>>>((const T*)x, ld, groups, (TO*)y, norms, rows))))
+    switch (lpr) {
+      case 1: RNV(1); break; case 2: RNV(2); break; case 4: RNV(4); break;
+      case 8: RNV(8); break; case 16: RNV(16); break; default: RNV(32); break;
+    }
+#undef RNV
     KCH_LAUNCH_OK();
     return KCH_OK;
   }
   dim3 grid((unsigned)ceil_div64(rows, 8)), block(256);
   KCH_DISPATCH_FLOAT(dtype, T, KCH_DISPATCH_FLOAT(out_dtype, TO,
-      (rownorm_kernel<T, TO><<<grid, block, 0, kch_stream(stream)>>>((const T*)x, ld, (TO*)y, norms, rows, c))));
+      (rownorm_kernel<T, TO><<<grid, block, 0, s>>>((const T*)x, ld, groups, (TO*)y, norms, rows, c))));
   KCH_LAUNCH_OK();
   return KCH_OK;
+}
+
+extern "C" int kch_rownorm(const void* x, int64_t ld, void* y, float* norms, int64_t rows, int c,
+                           int dtype, int out_dtype, void* stream) {
+  KCH_REQUIRE(rows >= 0 && c >= 1 && ld >= c, "kch_rownorm: rows=%lld c=%d ld=%lld", (long long)rows, c,
+              (long long)ld);
+  return kch_rownorm_groups(x, ld, 1, y, norms, rows, c, dtype, out_dtype, stream);
 }

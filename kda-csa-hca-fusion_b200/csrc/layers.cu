@@ -7,6 +7,9 @@
 
 #include "kch_common.cuh"
 
+int kch_rownorm_groups(const void* x, int64_t ld, int groups, void* y, float* norms, int64_t rows, int c, int dtype,
+                       int out_dtype, void* stream);      // elementwise.cu
+
 namespace {
 struct Carve {                            // 256-byte aligned pieces of a workspace; with a null base it only counts
   uint8_t* base;
@@ -56,22 +59,6 @@ template <typename T>
 __global__ void widen_rows_kernel(const T* __restrict__ x, int64_t ld, float* __restrict__ y, int64_t rows, int width) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < rows * width) y[i] = ldf(x + (i / width) * ld + i % width);
-}
-
-// F.normalize of the `groups` groups of c elements in each row, as dense fp32 [rows * groups, c]; a warp per group
-template <typename T>
-__global__ void rownorm_groups_kernel(const T* __restrict__ x, int64_t ld, float* __restrict__ y, int64_t rows, int groups, int c) {
-  const int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (g >= rows * groups) return;
-  const T* xr = x + (g / groups) * ld + (g % groups) * c;
-  float ss = 0.f;
-  for (int i = lane; i < c; i += 32) {
-    const float v = ldf(xr + i);
-    ss += v * v;
-  }
-  const float nrm = fmaxf(sqrtf(warp_sum(ss)), 1e-12f);
-  for (int i = lane; i < c; i += 32) y[g * c + i] = ldf(xr + i) / nrm;
 }
 
 static int concat_rows(const kch_weight_part* parts, int count, void* dst, int K, int n, int dtype, cudaStream_t s) {
@@ -204,9 +191,7 @@ extern "C" int kch_csa_layer(const kch_csa_layer_args* a, void* stream) {
       LY_GO(kch_indexer_topk_ex(qi, KCH_BF16, a->n_q, 1, (const float*)w.kn, (const float*)w.wf, (int32_t*)w.idx, B, T, n, a->nIh, cI,
                                 a->topk, 1.f, a->m, 0, -1, 0, 0, w.topk, w.topk_bytes, stream));
     } else {
-      KCH_DISPATCH_FLOAT(dt, T_, (rownorm_groups_kernel<T_><<<(unsigned)ceil_div64(rows * a->nIh, 8), 256, 0, s>>>(
-          (const T_*)qi, a->n_q, (float*)w.qn, rows, a->nIh, cI)));
-      KCH_LAUNCH_OK();
+      LY_GO(kch_rownorm_groups(qi, a->n_q, a->nIh, w.qn, nullptr, rows * a->nIh, cI, dt, KCH_F32, stream));
       LY_GO(kch_indexer_topk((const float*)w.qn, (const float*)w.kn, (const float*)w.wf, (int32_t*)w.idx, B, T, n, a->nIh, cI, a->topk,
                              1.f, a->m, 0, -1, 0, 0, w.topk, w.topk_bytes, stream));
     }
