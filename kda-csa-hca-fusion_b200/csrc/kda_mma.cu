@@ -19,6 +19,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <mutex>
+
 #include "mma_utils.cuh"
 
 #define KM_K 128
@@ -732,28 +734,44 @@ int64_t kch_kda_mma_workspace_bytes(int B, int T, int HV) {
   return (int64_t)B * HV * NT * KM_CHUNK_BYTES + (P ? kch_kda_scan_split_bytes(B * HV, P) : (int64_t)B * HV * KM_K * KM_V * 4);
 }
 
-// Side stream and events of the segmented driver below (one set per device, created on first use).
+// Side stream and events of the segmented driver below, one set per device, created on first use.  A call holds `lock` from
+// its first record to its last wait: a wait takes the event as it was recorded last, so another host thread's call in between
+// would put its own work in the place of this one's.
 #define KM_MAX_SEG 8
 struct KmSideStream {
+  std::mutex lock;
   cudaStream_t hp = nullptr;
   cudaEvent_t prep_done[KM_MAX_SEG] = {};
   cudaEvent_t scan_done = nullptr;
 };
-static int km_side_stream(KmSideStream** out) {
+static int km_side_stream(KmSideStream** out, std::unique_lock<std::mutex>* held) {
   static KmSideStream per_dev[16];
   int dev = 0;
   KCH_CUDA_OK(cudaGetDevice(&dev));
   KCH_REQUIRE(dev >= 0 && dev < 16, "kch_kda_chunk: device ordinal %d", dev);
   KmSideStream& ss = per_dev[dev];
+  *held = std::unique_lock<std::mutex>(ss.lock);
   if (!ss.hp) {
+    for (int i = 0; i < KM_MAX_SEG; ++i)
+      if (!ss.prep_done[i]) KCH_CUDA_OK(cudaEventCreateWithFlags(&ss.prep_done[i], cudaEventDisableTiming));
+    if (!ss.scan_done) KCH_CUDA_OK(cudaEventCreateWithFlags(&ss.scan_done, cudaEventDisableTiming));
     int least = 0, greatest = 0;
     KCH_CUDA_OK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     KCH_CUDA_OK(cudaStreamCreateWithPriority(&ss.hp, cudaStreamNonBlocking, greatest));
-    for (int i = 0; i < KM_MAX_SEG; ++i) KCH_CUDA_OK(cudaEventCreateWithFlags(&ss.prep_done[i], cudaEventDisableTiming));
-    KCH_CUDA_OK(cudaEventCreateWithFlags(&ss.scan_done, cudaEventDisableTiming));
   }
   *out = &ss;
   return KCH_OK;
+}
+// A call under capture leaves the side stream in that capture until it ends; only calls of the same capture may use it then.
+static bool km_side_stream_free(const KmSideStream& ss, cudaStream_t s) {
+  cudaStreamCaptureStatus side = cudaStreamCaptureStatusNone, own = cudaStreamCaptureStatusNone;
+  unsigned long long side_id = 0, own_id = 0;
+  bool ok = cudaStreamGetCaptureInfo(ss.hp, &side, &side_id) == cudaSuccess;
+  if (ok && side == cudaStreamCaptureStatusNone) return true;
+  ok = ok && cudaStreamGetCaptureInfo(s, &own, &own_id) == cudaSuccess && side == cudaStreamCaptureStatusActive &&
+       own == cudaStreamCaptureStatusActive && side_id == own_id;
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 int kch_kda_chunk_mma(const void* q, const void* k, const void* v, const void* g, const void* beta,
@@ -794,10 +812,18 @@ int kch_kda_chunk_mma(const void* q, const void* k, const void* v, const void* g
     return kch_kda_scan_tc5_split(workspace, (uint8_t*)workspace + (int64_t)B * HV * NT * KM_CHUNK_BYTES, split, initial_state, o,
                                   final_state, B, T, HV, NT, status, s);
   }
+  KmSideStream* ss = nullptr;
+  std::unique_lock<std::mutex> held;
   if (pa.umma && !prep_mma && nsegs > 1) {
-    KmSideStream* ss = nullptr;
-    int rc = km_side_stream(&ss);
+    int rc = km_side_stream(&ss, &held);
     if (rc != KCH_OK) return rc;
+    if (!km_side_stream_free(*ss, s)) {                // the two stages one after the other, on the caller's stream
+      ss = nullptr;
+      held.unlock();
+    }
+  }
+  if (ss) {
+    int rc = KCH_OK;
     const int per = (NT + nsegs - 1) / nsegs;
     float* carry = final_state ? final_state
                                : reinterpret_cast<float*>((uint8_t*)workspace + (int64_t)B * HV * NT * KM_CHUNK_BYTES);
