@@ -249,8 +249,14 @@ static int launch_kda_step(const T* q, const T* k, const T* v, const T* g, const
   return KCH_OK;
 }
 
+// KCH_KDA_DECODE=o keeps the general kernel for the one-token step, behind a gate projected by a launch of its own, for comparison
+static bool kds_general() {
+  static const bool on = [] { const char* e = getenv("KCH_KDA_DECODE"); return e && e[0] == 'o'; }();
+  return on;
+}
+
 extern "C" int kch_kda_step_gate_supported(int B, int HV, int K, int V, int dtype) {
-  return dtype == KCH_BF16 && K == 128 && V == 128 && B >= 1 && HV >= 1 && kds_few(B, HV);
+  return dtype == KCH_BF16 && K == 128 && V == 128 && B >= 1 && HV >= 1 && kds_few(B, HV) && !kds_general();
 }
 
 // The one-token step of a layer whose gate has not been projected up yet (see KdsGate).  As a launch of its own the up-projection
@@ -290,9 +296,7 @@ extern "C" int kch_kda_recurrent(const void* q, const void* k, const void* v, co
   if (T == 0 && !final_state) return KCH_OK;
   dim3 grid((V + 31) / 32, HV, B), block(128);
   cudaStream_t s = kch_stream(stream);
-  // (KCH_KDA_DECODE=o keeps the general kernel for the one-token step, for comparison)
-  static const bool old_step = [] { const char* e = getenv("KCH_KDA_DECODE"); return e && e[0] == 'o'; }();
-  if (T == 1 && K == 128 && V == 128 && !old_step && (((uintptr_t)initial_state | (uintptr_t)final_state) & 15) == 0) {
+  if (T == 1 && K == 128 && V == 128 && !kds_general() && (((uintptr_t)initial_state | (uintptr_t)final_state) & 15) == 0) {
     const KdsGate none = {};
     KCH_DISPATCH_FLOAT(dtype, T_, return (launch_kda_step<T_, false>((const T_*)q, (const T_*)k, (const T_*)v, (const T_*)g, (const T_*)beta,
                                                                      initial_state, (T_*)o, final_state, B, H, HV, scale, g_clamp_min, ld_qk,

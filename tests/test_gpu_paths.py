@@ -103,3 +103,36 @@ def test_kda_parts_beside_a_capture(kch):
     torch.cuda.synchronize()
     for r in (first, second):
         assert torch.equal(r[0], want[0][0]) and torch.equal(r[1], want[0][1])
+
+
+@pytest.mark.parametrize("B,H,HV,gate_scale", [(1, 1, 1, 0.1), (3, 2, 4, 0.1), (37, 8, 8, 1.0)])
+def test_kda_step_gate_matches_the_two_launches(kch, B, H, HV, gate_scale):
+    """The step that projects its gate against the recurrence on the gate of the same products, rounded at the layer's three points.
+    The only liberty is the order of the 128 products: a pre-activation within 2^-17 (128 x 2^-24) of the middle between two
+    bf16 values may round to the other one.  Channels whose pre-activation is not that close agree as two fp32 recurrences do:
+    1e-5 of values below 10."""
+    from kch_b200.kda import step_gate
+    q, k, v, _, beta, S0 = (x.to(DEV) for x in syn.kda_inputs(B + HV, B, 1, H, 128, 128, HV, torch.bfloat16, with_state=True))
+    gen = torch.Generator().manual_seed(B)
+    x = torch.randn(B, 1, 128, generator=gen).bfloat16().to(DEV)
+    W = (torch.randn(HV * 128, 128, generator=gen) * 0.08).bfloat16().to(DEV)
+    t = (x.double() @ W.double().T).view(B, 1, HV, 128)
+    tr = t.bfloat16()                                     # one rounding of the exact sum
+    ulp = torch.ldexp(torch.ones_like(t), (torch.frexp(t).exponent - 8).int())
+    away = (t - tr.double()).abs()
+    close = (ulp * 0.5 - away) <= 2.0 ** -17 * (x.double().abs() @ W.double().abs().T).view_as(t)
+    sp = torch.nn.functional.softplus(tr.double())
+    spr = sp.bfloat16()
+    ulp2 = torch.ldexp(torch.ones_like(sp), (torch.frexp(sp).exponent - 8).int())
+    close |= (ulp2 * 0.5 - (sp - spr.double()).abs()) <= 2.0 ** -20 * sp.clamp_min(1.0)      # (the intrinsic logarithm)
+    g = (-spr.float() * gate_scale).bfloat16()
+    g = torch.where(close, torch.zeros_like(g), g)
+    # channels that may go either way leave the comparison: no state, no key, no query there
+    keep = ~close.any(dim=2, keepdim=True)                # [B, 1, 1, 128]
+    q, k = q * keep, k * keep
+    S0 = S0 * keep.view(B, 1, 128, 1)
+    assert float(keep.float().mean()) > 0.5
+    o, S = step_gate(q, k, v, x, W, beta, scale=128 ** -0.5, initial_state=S0, state_out=None, gate_scale=gate_scale)
+    o2, S2 = kch.naive_recurrent_kda(q, k, v, g, beta, scale=128 ** -0.5, initial_state=S0, output_final_state=True)
+    assert float((S - S2).abs().max()) <= 1e-5, float((S - S2).abs().max())
+    assert bool(((o.float() - o2.float()).abs() <= 1e-5 + o2.float().abs() * 2.0 ** -8).all())
