@@ -136,3 +136,54 @@ def test_kda_step_gate_matches_the_two_launches(kch, B, H, HV, gate_scale):
     o2, S2 = kch.naive_recurrent_kda(q, k, v, g, beta, scale=128 ** -0.5, initial_state=S0, output_final_state=True)
     assert float((S - S2).abs().max()) <= 1e-5, float((S - S2).abs().max())
     assert bool(((o.float() - o2.float()).abs() <= 1e-5 + o2.float().abs() * 2.0 ** -8).all())
+
+
+@pytest.mark.parametrize("state", [True, False])
+def test_kda_parts_of_many_heads(kch, state):
+    """64 heads and 65 chunks: too many heads for segments side by side, so the sequence goes in four parts, prepared on the caller's
+    stream and scanned on another, the state carried through memory (the caller's final state, or the workspace where none is
+    wanted).  Bounds as in test_kda_chunk_segments: operands in two bf16 terms."""
+    B, T, H = 4, 4100, 16
+    ins = list(syn.kda_inputs(64, B, T, H, 128, 128, H, torch.bfloat16, with_state=True))
+    S0 = ins.pop() if state else (ins.pop(), None)[1]
+    ins[3] = (ins[3].float() * 0.1).bfloat16()
+    d = [x.to(DEV) for x in ins]
+    S0d = None if S0 is None else S0.to(DEV)
+    o, s = kch.naive_chunk_kda(*d, initial_state=S0d, output_final_state=True, chunk_size=64)
+    o_only, none = kch.naive_chunk_kda(*d, initial_state=S0d, output_final_state=False, chunk_size=64)
+    assert none is None and torch.equal(o, o_only)
+
+    def check(o, s, o_ref, s_ref):
+        assert float((s.double() - s_ref).norm() / s_ref.norm()) <= 1e-4
+        e = (o.double() - o_ref).abs()
+        assert bool((e <= o_ref.abs() * 2.0 ** -7 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(e.max())
+    o2, s2 = kch.naive_recurrent_kda(*d, initial_state=S0d, output_final_state=True)
+    check(o, s, o2.double(), s2.double())
+    for b, h in ((0, 0), (3, 15)):                        # heads do not meet: two of them against the oracle in 64 bits
+        one = [x[b:b + 1, :, h:h + 1].double() for x in ins]
+        o_ref, s_ref = orc.chunk_kda(*one, initial_state=None if S0 is None else S0[b:b + 1, h:h + 1].double(), chunk_size=64)
+        check(o[b:b + 1, :, h:h + 1].cpu(), s[b:b + 1, h:h + 1].cpu(), o_ref, s_ref)
+
+
+def test_kda_chain_and_segments_agree(kch, tmp_path):
+    """512 chunks of two heads as one chain (KCH_KDA_SPLIT=0 in a child process) and in segments: both against the oracle."""
+    import os
+    import subprocess
+    import sys
+    B, T, H = 1, 32768, 2
+    q, k, v, g, beta = syn.kda_inputs(512, B, T, H, 128, 128, H, torch.bfloat16)
+    g = (g.float() * 0.1).bfloat16()
+    ins, outs = tmp_path / "in.pt", tmp_path / "out.pt"
+    torch.save((q, k, v, g, beta), ins)
+    code = ("import sys, torch\nsys.path.insert(0, sys.argv[3])\nimport kch_b200\n"
+            "t = [x.cuda() for x in torch.load(sys.argv[1])]\n"
+            "o, s = kch_b200.naive_chunk_kda(*t, output_final_state=True, chunk_size=64)\n"
+            "assert kch_b200._lib.device_status() == 0\ntorch.save((o.cpu(), s.cpu()), sys.argv[2])\n")
+    pkg = os.path.dirname(os.path.dirname(kch.__file__))
+    subprocess.run([sys.executable, "-c", code, str(ins), str(outs), pkg], check=True, env=dict(os.environ, KCH_KDA_SPLIT="0"), timeout=300)
+    o_ref, s_ref = orc.chunk_kda(*(x.double() for x in (q, k, v, g, beta)), chunk_size=64)
+    seg = kch.naive_chunk_kda(*(x.to(DEV) for x in (q, k, v, g, beta)), output_final_state=True, chunk_size=64)
+    for o, s in (torch.load(outs), [x.cpu() for x in seg]):
+        assert float((s.double() - s_ref).norm() / s_ref.norm()) <= 1e-4
+        e = (o.double() - o_ref).abs()
+        assert bool((e <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(e.max())
