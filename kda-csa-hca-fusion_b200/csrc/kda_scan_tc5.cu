@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
               t5_mma_ts(tD + 64, tD + (term == 1 ? 16u : 0u) + 32u * (ks >> 1) + 8u * (ks & 1), da0 + ((term == 2 ? 8192u : 0u) >> 4) + 2 * ks, id64, 1u);
-          t5_commit(o_full);
+          if (n + 1 == NT) t5_commit(o_full);
         }
         t5_commit(k_empty);
       }
@@ -342,9 +342,10 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       }
       if (lane == 0) mbarrier_arrive(u_empty);
       // ---- o^T of the previous chunk -> global, while the products of this one run (its D1q is the other buffer) --------
+      // Its products lie before D1 of this chunk in the MMA thread's order, so the wait for d1_full above covers them.  A barrier
+      // of their own could not be waited for here: the MMA thread has what it needs for the products of this chunk, and a warp
+      // that it overtook by one phase would wait for a phase that nothing completes.
       if (n > 0 && with_o) {
-        if (!mbarrier_wait_bounded(o_full, ph ^ 1, 52, T5_SPIN, a.status)) { ok = false; break; }
-        t5_fence_after();
         t5_ld32(tDD + 128u * (ph ^ 1) + 64 + lane_base + 32 * sub, ro);
         t5_wait_ld();
         store_o((n - 1) * 64);
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
     }
     // the last products must have finished before o^T and the state are read and tensor memory is released
     if (ok && NT > 0 && !mbarrier_wait_bounded(s_full, (uint32_t)(NT - 1) & 1, 51, T5_SPIN, a.status)) ok = false;
-    if (ok && NT > 0 && with_o && !mbarrier_wait_bounded(o_full, (uint32_t)(NT - 1) & 1, 53, T5_SPIN, a.status)) ok = false;
+    if (ok && NT > 0 && with_o && !mbarrier_wait_bounded(o_full, 0, 53, T5_SPIN, a.status)) ok = false;
     if (ok && NT > 0) {
       t5_fence_after();
       if (with_o) {

@@ -187,3 +187,18 @@ def test_kda_chain_and_segments_agree(kch, tmp_path):
         assert float((s.double() - s_ref).norm() / s_ref.norm()) <= 1e-4
         e = (o.double() - o_ref).abs()
         assert bool((e <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(e.max())
+
+
+@pytest.mark.parametrize("B,T,H", [(4, 4096, 16), (1, 8175, 64), (1, 4033, 50)])
+def test_kda_chunks_over_and_over(kch, B, T, H):
+    """The scan's hand-overs between its warps hold whatever a warp is held up by: many calls back to back, beside the prepare stage of
+    their next part or call, with the same bits from each and no wait that expires."""
+    ins = list(syn.kda_inputs(90 + H, B, T, H, 128, 128, H, torch.bfloat16, with_state=True))
+    ins[3] = (ins[3].float() * 0.1).bfloat16()
+    d = [x.to(DEV) for x in ins]
+    want = _chunk(kch, d)
+    for _ in range(8):
+        got = [_chunk(kch, d) for _ in range(8)]
+        torch.cuda.synchronize()
+        assert kch._lib.device_status() == 0
+        assert all(torch.equal(o, want[0]) and torch.equal(s, want[1]) for o, s in got)
