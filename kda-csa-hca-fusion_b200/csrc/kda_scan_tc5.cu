@@ -98,6 +98,10 @@ __device__ __forceinline__ void t5_stn(uint32_t taddr, const uint32_t* r) {
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
+// SEG: segments of a sequence side by side (see the host part).  A kernel of its own: with the choices of a segment made at run
+// time, the chain of a whole sequence took 1.5 us more before its first chunk and 1 % of both stages (64 heads: 2 chunks 29.8 us, 31.6
+// with them; 128 chunks 842, 850).
+template <bool SEG>
 __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   extern __shared__ uint8_t t5_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>(((uintptr_t)t5_raw + 1023) & ~(uintptr_t)1023);
@@ -114,8 +118,8 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   int n0 = 0, NT = a.NT;
   const float* S0 = a.S0 ? a.S0 + bh * (128 * 128) : nullptr;
   float* S_out = a.S_out ? a.S_out + bh * (128 * 128) : nullptr;
-  bool with_o = true, with_u = true;                             // with_u false: rows of the identity instead of values
-  if (a.nseg) {
+  bool out_wanted = true, values = true;
+  if constexpr (SEG) {
     const int z = blockIdx.z, seg = a.pass == 1 ? (z + 1) / 2 : z + 1;
     const int64_t slot = (int64_t)gridDim.x * gridDim.y;
     n0 = seg * a.per;
@@ -124,9 +128,9 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       S_out = a.starts + ((int64_t)(seg + 1) * slot + bh) * (128 * 128);
       if (seg > 0) {
         S0 = nullptr;
-        with_o = false;
-        with_u = z & 1;
-        if (!with_u) S_out = a.trans + ((int64_t)seg * slot + bh) * (128 * 128);
+        out_wanted = false;
+        values = z & 1;
+        if (!values) S_out = a.trans + ((int64_t)seg * slot + bh) * (128 * 128);
       }
     } else {
       const bool chain = a.serial[bh] != 0u;
@@ -136,6 +140,8 @@ __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
       else if (seg + 1 < a.nseg) S_out = nullptr;
     }
   }
+  // (constants where the sequence is one chain); with_u false: rows of the identity instead of values
+  const bool with_o = !SEG || out_wanted, with_u = !SEG || values;
   const int T_left = a.T - n0 * 64;                              // tokens from this run's first chunk to the end of the sequence
   const uint8_t* wsb = a.ws + (bh * a.NT + n0) * (int64_t)T5_CHUNK_BYTES;
 
@@ -479,8 +485,9 @@ int64_t kch_kda_scan_split_bytes(int BH, int nseg) {
 
 static int scan_launch(const T5Args& a, dim3 grid, cudaStream_t s) {
   const int smem = T5_TOTAL + 1024;
-  KCH_CUDA_OK(cudaFuncSetAttribute(kda_scan_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kda_scan_tc5_kernel<<<grid, T5_THREADS, smem, s>>>(a);
+  auto kernel = a.nseg ? kda_scan_tc5_kernel<true> : kda_scan_tc5_kernel<false>;
+  KCH_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kernel<<<grid, T5_THREADS, smem, s>>>(a);
   KCH_LAUNCH_OK();
   return KCH_OK;
 }
