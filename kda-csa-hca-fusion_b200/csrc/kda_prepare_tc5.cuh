@@ -13,12 +13,14 @@
 // units); entries above the diagonal may overflow but are never read.  Down to -2 PT_GMAX, where the gate never grows, the
 // channels beyond are centred half way (EK and QG times 2^-c, Y times 2^c, w times 2^c again): the operator's own gates,
 // -softplus(N(0, 1)), decay a chunk by 2^-74 on average and past 2^-96 in some channel of one chunk in 40, and one CTA on the
-// other path holds up a whole wave (1 x 8192 tokens, 16 heads: 180 us, 158 now).  Beyond that the CTA runs the mma.sync path,
+// other path holds up a whole wave (64 heads, 32 chunks, both stages: 262 us on that path, 240 now).  The centre is taken out of a channel's
+// prefix and total, outside the loop over elements, and whether the gate grows is asked in such chunks only: a chunk of the
+// model's gate pays for neither (240 us; 246 with both in its loops and an image loop for each).  Beyond that the CTA runs the mma.sync path,
 // which re-centres the exponents per 16 x 16 block.  Each product is hi*hi + lo*hi + hi*lo of two-term bf16 splits
 // with fp32 accumulation in tensor memory, as everywhere in the KDA kernels.
 //
 // Data movement: g, k, q are read once by the threads that turn them into operand images (registers -> swizzled
-// shared-memory tiles, the KG image also straight to the chunk record, the QG image from its tile by bulk copy); V arrives
+// shared-memory tiles, the QG / KG images also straight to the chunk record); V arrives
 // through a tensor map (cp.async.bulk.tensor, 128-byte swizzle) while the triangular solve runs; w leaves through shared memory as bulk
 // copies; u^T and Aqk are written from the tensor-memory epilogues.  EK serves twice: K-major as the row operand of
 // the first product, MN-major (the same bytes) as the A operand of the second.
@@ -85,7 +87,7 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
     }
   }
   // ---- log-decay: activation, clamp, running sum (log2 units) -------------------------------------------------
-  float gam[4][8], gmax = 0.f;                       // gmax: a gate that grows (one that is not a number shows in the sum)
+  float gam[4][8];
   {
     float run[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -100,7 +102,6 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
           const float sp = __bfloat162float(__float2bfloat16_rn(gx > 20.f ? gx : __logf(1.0f + __expf(gx))));
           gx = __bfloat162float(__float2bfloat16_rn(-sp * a.gate_scale));
         }
-        gmax = fmaxf(gmax, ok ? gx : 0.f);
         run[x] += ok ? fmaxf(gx, a.g_min) * KM_LOG2E : 0.f;
         gam[s][x] = run[x];
       }
@@ -131,16 +132,28 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
     const float4 u = l4[0], v = l4[1];
     gl[0] = u.x; gl[1] = u.y; gl[2] = u.z; gl[3] = u.w; gl[4] = v.x; gl[5] = v.y; gl[6] = v.z; gl[7] = v.w;
   }
-  bool far = false, strong = gmax > 0.f;
+  bool far = false;
 #pragma unroll
-  for (int x = 0; x < 8; ++x) {
-    far |= !(gl[x] >= -PT_GMAX);
-    strong |= !(gl[x] >= -2.f * PT_GMAX);
-  }
+  for (int x = 0; x < 8; ++x) far |= !(gl[x] >= -PT_GMAX);
   far = __syncthreads_or(far);                       // uniform: some channel decays beyond PT_GMAX
-  if (far && __syncthreads_or(strong)) {             // ... and the half-way centre is not enough: the re-centring path
-    kda_prepare_chunk_mma(a, pt_raw, n, hv, b);
-    return;
+  if (far) {
+    bool strong = false;                             // the half-way centre is not enough, or the gate grows
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      strong |= !(gl[x] >= -2.f * PT_GMAX) || !(gam[0][x] <= 0.f);
+#pragma unroll
+      for (int s = 1; s < 4; ++s) strong |= !(gam[s][x] <= gam[s - 1][x]);
+    }
+    if (__syncthreads_or(strong)) {                  // the whole chunk takes the re-centring path
+      kda_prepare_chunk_mma(a, pt_raw, n, hv, b);
+      return;
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      const float c = pt_centre(gl[x]);
+      pre[x] -= c;
+      gl[x] -= c;
+    }
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr_u32(tmem_slot)), "r"(256u) : "memory");
@@ -148,51 +161,47 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
   }
 
   // ---- the four operand images of the block ----------------------------------------------------------------------
-  auto images = [&](auto centred) {
-    constexpr bool CEN = decltype(centred)::value;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = 4 * rg + s;
-      const bf16* ke = reinterpret_cast<const bf16*>(&kreg[s]);
-      const bf16* qe = reinterpret_cast<const bf16*>(&qreg[s]);
-      uint32_t ekh[4], ekl[4], qgh[4], qgl[4], yh[4], yl[4], kgh[4], kgl[4];
+  for (int s = 0; s < 4; ++s) {
+    const int i = 4 * rg + s;
+    const bf16* ke = reinterpret_cast<const bf16*>(&kreg[s]);
+    const bf16* qe = reinterpret_cast<const bf16*>(&qreg[s]);
+    uint32_t ekh[4], ekl[4], qgh[4], qgl[4], yh[4], yl[4], kgh[4], kgl[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float ga0 = pre[2 * e] + gam[s][2 * e], ga1 = pre[2 * e + 1] + gam[s][2 * e + 1];
+      const float k0 = __bfloat162float(ke[2 * e]), k1 = __bfloat162float(ke[2 * e + 1]);
+      const float q0 = __bfloat162float(qe[2 * e]) * a.scale, q1 = __bfloat162float(qe[2 * e + 1]) * a.scale;
+      const float d0 = ex2_fast(ga0), d1 = ex2_fast(ga1);
+      split2_bf16(k0 * d0, k1 * d1, ekh[e], ekl[e]);
+      split2_bf16(q0 * d0, q1 * d1, qgh[e], qgl[e]);
+      split2_bf16(k0 * ex2_fast(-ga0), k1 * ex2_fast(-ga1), yh[e], yl[e]);
+      split2_bf16(k0 * ex2_fast(gl[2 * e] - ga0), k1 * ex2_fast(gl[2 * e + 1] - ga1), kgh[e], kgl[e]);
+    }
+    const uint32_t pan = (uint32_t)(c8 >> 3), inner = swz<128>(i, c8 & 7);
+    uint8_t* ai = sm + PT_AIMG + pan * 16384u + inner;
+    *reinterpret_cast<uint4*>(ai) = make_uint4(ekh[0], ekh[1], ekh[2], ekh[3]);
+    *reinterpret_cast<uint4*>(ai + 32768) = make_uint4(ekl[0], ekl[1], ekl[2], ekl[3]);
+    *reinterpret_cast<uint4*>(ai + 8192) = make_uint4(qgh[0], qgh[1], qgh[2], qgh[3]);
+    *reinterpret_cast<uint4*>(ai + 32768 + 8192) = make_uint4(qgl[0], qgl[1], qgl[2], qgl[3]);
+    uint8_t* yi = sm + PT_Y + pan * 8192u + inner;
+    *reinterpret_cast<uint4*>(yi) = make_uint4(yh[0], yh[1], yh[2], yh[3]);
+    *reinterpret_cast<uint4*>(yi + 16384) = make_uint4(yl[0], yl[1], yl[2], yl[3]);
+    // the record of the sequential stage: the qg halves of the [w; qg] panels (without the centre), the kg panels
+    if (far) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float ga0 = pre[2 * e] + gam[s][2 * e], ga1 = pre[2 * e + 1] + gam[s][2 * e + 1];
-        const float k0 = __bfloat162float(ke[2 * e]), k1 = __bfloat162float(ke[2 * e + 1]);
-        const float q0 = __bfloat162float(qe[2 * e]) * a.scale, q1 = __bfloat162float(qe[2 * e + 1]) * a.scale;
-        const float c0 = CEN ? pt_centre(gl[2 * e]) : 0.f, c1 = CEN ? pt_centre(gl[2 * e + 1]) : 0.f;
-        const float d0 = ex2_fast(CEN ? ga0 - c0 : ga0), d1 = ex2_fast(CEN ? ga1 - c1 : ga1);
-        split2_bf16(k0 * d0, k1 * d1, ekh[e], ekl[e]);
-        split2_bf16(q0 * d0, q1 * d1, qgh[e], qgl[e]);
-        split2_bf16(k0 * ex2_fast(CEN ? c0 - ga0 : -ga0), k1 * ex2_fast(CEN ? c1 - ga1 : -ga1), yh[e], yl[e]);
-        split2_bf16(k0 * ex2_fast(gl[2 * e] - ga0), k1 * ex2_fast(gl[2 * e + 1] - ga1), kgh[e], kgl[e]);
+        const float c0 = pt_centre(tot[16 * 128 + 8 * c8 + 2 * e]), c1 = pt_centre(tot[16 * 128 + 8 * c8 + 2 * e + 1]);
+        split2_bf16(__bfloat162float(qe[2 * e]) * a.scale * ex2_fast(pre[2 * e] + gam[s][2 * e] + c0),
+                    __bfloat162float(qe[2 * e + 1]) * a.scale * ex2_fast(pre[2 * e + 1] + gam[s][2 * e + 1] + c1), qgh[e], qgl[e]);
       }
-      const uint32_t pan = (uint32_t)(c8 >> 3), inner = swz<128>(i, c8 & 7);
-      uint8_t* ai = sm + PT_AIMG + pan * 16384u + inner;
-      *reinterpret_cast<uint4*>(ai) = make_uint4(ekh[0], ekh[1], ekh[2], ekh[3]);
-      *reinterpret_cast<uint4*>(ai + 32768) = make_uint4(ekl[0], ekl[1], ekl[2], ekl[3]);
-      *reinterpret_cast<uint4*>(ai + 8192) = make_uint4(qgh[0], qgh[1], qgh[2], qgh[3]);
-      *reinterpret_cast<uint4*>(ai + 32768 + 8192) = make_uint4(qgl[0], qgl[1], qgl[2], qgl[3]);
-      uint8_t* yi = sm + PT_Y + pan * 8192u + inner;
-      *reinterpret_cast<uint4*>(yi) = make_uint4(yh[0], yh[1], yh[2], yh[3]);
-      *reinterpret_cast<uint4*>(yi + 16384) = make_uint4(yl[0], yl[1], yl[2], yl[3]);
-      // the record of the sequential stage: kg panels; the qg halves of the [w; qg] panels leave as bulk copies below, or from here
-      // where the operand is not what the record wants
-      if constexpr (CEN) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          split2_bf16(__bfloat162float(qe[2 * e]) * a.scale * ex2_fast(pre[2 * e] + gam[s][2 * e]),
-                      __bfloat162float(qe[2 * e + 1]) * a.scale * ex2_fast(pre[2 * e + 1] + gam[s][2 * e + 1]), qgh[e], qgl[e]);
-        *reinterpret_cast<uint4*>(wsc + pan * 16384u + 8192u + inner) = make_uint4(qgh[0], qgh[1], qgh[2], qgh[3]);
-        *reinterpret_cast<uint4*>(wsc + 32768u + pan * 16384u + 8192u + inner) = make_uint4(qgl[0], qgl[1], qgl[2], qgl[3]);
-      }
-      *reinterpret_cast<uint4*>(wsc + KM_OFF_KHI + pan * 8192u + inner) = make_uint4(kgh[0], kgh[1], kgh[2], kgh[3]);
-      *reinterpret_cast<uint4*>(wsc + KM_OFF_KLO + pan * 8192u + inner) = make_uint4(kgl[0], kgl[1], kgl[2], kgl[3]);
     }
-  };
-  if (far) images(std::true_type{});
-  else images(std::false_type{});
+      *reinterpret_cast<uint4*>(wsc + pan * 16384u + 8192u + inner) = make_uint4(qgh[0], qgh[1], qgh[2], qgh[3]);
+      *reinterpret_cast<uint4*>(wsc + 32768u + pan * 16384u + 8192u + inner) = make_uint4(qgl[0], qgl[1], qgl[2], qgl[3]);
+
+    *reinterpret_cast<uint4*>(wsc + KM_OFF_KHI + pan * 8192u + inner) = make_uint4(kgh[0], kgh[1], kgh[2], kgh[3]);
+    *reinterpret_cast<uint4*>(wsc + KM_OFF_KLO + pan * 8192u + inner) = make_uint4(kgl[0], kgl[1], kgl[2], kgl[3]);
+  }
   if (tid < KM_K) reinterpret_cast<float*>(wsc + KM_OFF_U + 32768)[tid] = ex2_fast(tot[16 * 128 + tid]);
   t5_fence_async_smem();
   t5_fence_before();
@@ -215,14 +224,6 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
                  (term | pan | ks) ? 1u : 0u);
     }
     t5_commit(&bars[0]);
-    // rows 64..127 of the [w; qg] panels lie in the operand tiles as the record wants them: four bulk copies (stored by the threads,
-    // 16 bytes at a time, they were half of the stage's store instructions)
-    if (!far) {
-#pragma unroll
-      for (int p = 0; p < 4; ++p) t5_bulk_store(wsc + p * 16384 + 8192, sm + PT_AIMG + p * 16384 + 8192, 8192);
-      t5_bulk_commit();
-      t5_bulk_wait_read();                                        // (V and T take their place next)
-    }
   }
   bool ok = true;
   if (tid == 0) ok = mbarrier_wait_bounded(&bars[0], 0, 61, PT_SPIN, status);   // one poller; the others sleep at the barrier
@@ -439,11 +440,15 @@ kda_prepare_tc5_kernel(PrepArgs a, const __grid_constant__ CUtensorMap vmap, uns
       uint8_t* wl = wh + 16384;
       const int cc = c & 63;
       // 2^centre, exactly: takes the centre out of EK again
-      const float un = __uint_as_float((uint32_t)(127 + (int)pt_centre(tot[16 * 128 + c])) << 23);
+      if (far) {
+        const float un = __uint_as_float((uint32_t)(127 + (int)pt_centre(tot[16 * 128 + c])) << 23);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * un);
+      }
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         bf16 hi, lo;
-        split1_bf16(__uint_as_float(r[j]) * un, hi, lo);
+        split1_bf16(__uint_as_float(r[j]), hi, lo);
         const uint32_t off = swz<128>(32 * hh + j, cc >> 3) + 2 * (cc & 7);
         *reinterpret_cast<bf16*>(wh + off) = hi;
         *reinterpret_cast<bf16*>(wl + off) = lo;

@@ -202,3 +202,25 @@ def test_kda_chunks_over_and_over(kch, B, T, H):
         torch.cuda.synchronize()
         assert kch._lib.device_status() == 0
         assert all(torch.equal(o, want[0]) and torch.equal(s, want[1]) for o, s in got)
+
+
+@pytest.mark.parametrize("total", [95.5, 96.5, 150.0, 191.0, 193.0])
+@pytest.mark.parametrize("growth", [0.0, 1e-5, 0.02])
+def test_kda_chunks_at_the_lines_of_the_centre(kch, total, growth):
+    """Chunks whose decay (2^-total in every second channel, a few units in the others) lies on either side of where the exponents are
+    centred half way and of where that is not enough, with a gate that never grows, hardly, or does for 20 tokens.  Two chunks
+    and a tail, 64 heads (one chain).  Bounds as in test_kda_chunk_segments."""
+    B, T, H = 2, 150, 32
+    q, k, v, g, beta, S0 = syn.kda_inputs(int(total), B, T, H, 128, 128, H, torch.bfloat16, with_state=True)
+    gf = g.float() * 0.1
+    gf[..., ::2] = -total * 0.6931471805599453 / 64
+    if growth:
+        gf[:, 70:90, :, 1::4] = growth
+    g = gf.bfloat16()
+    o, s = kch.naive_chunk_kda(*(x.to(DEV) for x in (q, k, v, g, beta)), initial_state=S0.to(DEV), output_final_state=True, chunk_size=64)
+    for b, h in ((0, 0), (1, 31)):
+        one = [x[b:b + 1, :, h:h + 1].double() for x in (q, k, v, g, beta)]
+        o_ref, s_ref = orc.recurrent_kda(*one, initial_state=S0[b:b + 1, h:h + 1].double())
+        assert float((s[b:b + 1, h:h + 1].double().cpu() - s_ref).norm() / s_ref.norm()) <= 1e-4
+        e = (o[b:b + 1, :, h:h + 1].double().cpu() - o_ref).abs()
+        assert bool((e <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(e.max())
