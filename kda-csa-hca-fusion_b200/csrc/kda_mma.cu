@@ -692,7 +692,7 @@ bool kch_kda_scan_tc5_enabled();      // kda_scan_tc5.cu
 int kch_kda_scan_tc5(const void* workspace, const float* initial_state, void* o, float* final_state, int B, int T,
                      int Tb, int HV, int NT, unsigned int* status, cudaStream_t s);
 
-int kch_kda_scan_segments(int BH, int NT, float* us);
+int kch_kda_scan_segments(int BH, int NT);
 int64_t kch_kda_scan_split_bytes(int BH, int nseg);
 int kch_kda_scan_tc5_split(const void* workspace, void* split, int nseg, const float* initial_state, void* o, float* final_state,
                            int B, int T, int HV, int NT, unsigned int* status, cudaStream_t s);
@@ -703,27 +703,26 @@ bool kch_kda_mma_supported(int K, int V, int chunk_size, float g_clamp_min, int 
 }
 
 // Segments scanned side by side (kda_scan_tc5.cu) instead of one chain a head: their number where that is the faster one, else 0.
-// Estimates in us: 0.055 a chunk and head in the prepare stage, 2.25 a chunk in a chain.  The chain overlaps with the prepare
-// stage over three quarters of a sequence of 64 chunks or more, each slowing the other; the segments wait for all of it, and for
-// two passes and the join.
-// Both sides measured, chain / segments (us, both stages, the model's gate), the line between the brackets:
-//   1 head:   12 chunks 69 / 71  [  20: 85 / 79    64: 211 / 114   512: 1263 / 278
-//   16 heads: 12 chunks 71 / 75  [  20: 105 / 101  64: 251 / 183   128: 442 / 306   512: 1440 / 1025
-//   28 heads: 20 chunks 116 / 122 [ 32: 173 / 169  63: 296 / 259  96: 391 / 368  128: 489 / 468  256: 860 / 863
-//   36 heads: 32 chunks 185 / 185 [ 63: 335 / 312 ] 96: 442 / 443  256: 993 / 1086
-// With more heads than a third of the SMs pass 1 no longer fits one wave and the chain stays.
+// The two passes and the join cost ~25 us and the longer the more heads there are, so the sequence has to be long; with more than
+// 24 heads the passes are bound by their records' way from HBM (beyond ~3000 of them L2 no longer holds them between the stages),
+// and from 64 chunks on a chain overlaps with the prepare stage, so there the sequence must not be too long.
+// Both sides measured, chain / segments (us, both stages, the model's gate), the rule's line between the brackets:
+//    1 head:   12 chunks 51 / 57  16: 61 / 62  [  20: 70 / 66    64: 190 / 99    512: 1203 / 273
+//    8 heads:  12 chunks 52 / 58  16: 61 / 62  [  20: 74 / 70    64: 203 / 136   512: 1293 / 591
+//   16 heads:  16 chunks 66 / 67  20: 88 / 92  [  24: 105 / 102  64: 236 / 176   512: 1408 / 1017
+//   24 heads:  24 chunks 119 / 122  28: 138 / 137 [ 40: 182 / 171  64: 259 / 240  512: 1528 / 1493
+//   28 heads:  28 chunks 147 / 148 [ 40: 193 / 183  64: 273 / 262  128: 471 / 458 ] 200: 675 / 674  512: 1590 / 1650
+//   32 heads:  40 chunks 204 / 201 [ 48: 241 / 230  63: 304 / 282 ] 64: 294 / 287  128: 484 / 521  300: 1025 / 1158
+//   40 heads:  48 chunks 262 / 259 [ 56: 309 / 301  63: 343 / 331 ] 64: 339 / 335  128: 577 / 609  300: 1221 / 1353
+//   49 heads:  56 chunks 340 / 338  63: 377 / 369  80: 454 / 457  128: 671 / 699: no segments
 static int km_split(int B, int T, int HV) {
   static const int seg_env = [] { const char* e = getenv("KCH_KDA_SPLIT"); return e ? atoi(e) : -1; }();
   if (seg_env == 0 || !kch_kda_scan_tc5_enabled()) return 0;
   const int NT = (T + KM_C - 1) / KM_C;
-  if ((int64_t)B * HV > 148) return 0;
-  float scan = 0.f;
-  const int P = kch_kda_scan_segments(B * HV, NT, &scan);
-  if (!P) return 0;
-  const float prep = 0.055f * NT * B * HV, chain = 2.25f * NT;
-  const float plain = NT >= 64 ? prep * 0.25f + fmaxf(prep, chain) * 0.75f + chain * 0.25f + fminf(prep, chain) * 0.35f : prep + chain;
-  const float split = prep + scan + 0.6f * B * HV;
-  return split < plain || seg_env == 1 ? P : 0;
+  const int64_t heads = (int64_t)B * HV;
+  if (heads > 148) return 0;
+  const bool pays = NT >= 20 && 5 * (int64_t)NT >= 7 * heads && heads <= 40 && (heads <= 24 || NT <= (heads <= 28 ? 128 : 63));
+  return pays || seg_env == 1 ? kch_kda_scan_segments((int)heads, NT) : 0;
 }
 
 // chunk records, then one fp32 state per (batch, head): the carry between the segments of a long sequence; or what the

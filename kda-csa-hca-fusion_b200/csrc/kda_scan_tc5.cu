@@ -407,7 +407,7 @@ bool kch_kda_scan_tc5_enabled() {
 // (1 + 2 (nseg - 2)) CTAs a head instead of one.  All of it in the arithmetic of the plain scan, the join in fp32.
 // A transition that expands (an entry beyond 4, or not finite: a gate that grows, keys far from unit length) could lose in M
 // what the plain scan keeps; the segments of such a head run as one chain in pass 2.
-// 1 x 8192 tokens, 16 heads, 5 segments: the scan alone 290 us as one chain; two passes of ~60 us and 19 of the join.
+// 1 x 8192 tokens, 16 heads, 6 segments: the scan alone 290 us as one chain; two passes of ~60 us and 19 of the join.
 // km_split (kda_mma.cu) holds the rule.
 // A CTA of the join walks the segments for 16 columns of a head's state; the transitions (64 KB each) are copied two steps ahead.
 #define KJ_COLS 16
@@ -466,15 +466,16 @@ __global__ void __launch_bounds__(256) kda_join_kernel(float* starts, const floa
   if (blockIdx.x == 0 && tid == 0) serial[bh] = expands ? 1u : 0u;
 }
 
-// Segments for the scan of NT chunks of BH heads (0: one CTA a head), and what the scan then takes: both passes (a chunk of
-// pass 1 computes no output) and ~2 us a segment in the join.  Pass 1 stays within one wave of CTAs.
-int kch_kda_scan_segments(int BH, int NT, float* us) {
+// Segments for the scan of NT chunks of BH heads (0: none fit): both passes (1.75 and 2.25 us a chunk; pass 1 computes no output)
+// and ~2 us a segment in the join take the least.  Pass 1 stays within one wave of CTAs.
+int kch_kda_scan_segments(int BH, int NT) {
   int best = 0;
+  float best_us = 0.f;
   for (int P = 3; BH > 0 && (int64_t)BH * (1 + 2 * (P - 2)) <= 148 && P <= NT; ++P) {
     const int per = (NT + P - 1) / P;
     if ((NT + per - 1) / per != P) continue;         // the last segment would be empty
-    const float t = (1.75f + 2.25f) * per + 8.f + 2.f * P;
-    if (!best || t < *us) { best = P; *us = t; }
+    const float us = (1.75f + 2.25f) * per + 2.f * P;
+    if (!best || us < best_us) { best = P; best_us = us; }
   }
   return best;
 }
