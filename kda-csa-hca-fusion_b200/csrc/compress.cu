@@ -270,11 +270,16 @@ static int launch_compress(const void* Ca, const void* Za, const void* Cb, const
       return KCH_OK;
     }
   }
-  // A CTA a block and 32 channels where a block is long, or where such CTAs are few; fp32 tokens of 128 channels, us, thread a
-  // channel / subsets: m = 64: 45 / 11 at 2048 tokens, 79 / 57 at 131072; m = 16: 16 / 8 and 66 / 104; m = 8: 12 / 8 at 2048, 14 / 25
-  // at 16384; m = 4: 8 / 10 and 61 / 242.
-  const int64_t ctas = (int64_t)B * nblk * ((c + 31) / 32);
-  const bool subsets = m >= 64 ? ctas <= 0x7FFFFFFF : m >= CR_SUBS && ctas <= 8 * 148;
+  // A CTA a block and 32 channels where such CTAs are few, or where a block is long; its length counts by the lanes that have a
+  // channel.  fp32 tokens, us with the call, thread a channel / subsets:
+  //   few: m = 64: 19 / 11, with the overlap 17 / 13, at 2048 tokens of 128 channels; m = 48: 15 / 11 and 14 / 13 at 8192
+  //   many, m = 64: 63 / 48 at 131072 tokens of 128 channels, 72 / 85 at 524288 of 33 (half of the lanes idle)
+  //   many, with the overlap (twice the rows a CTA): m = 64: 21 / 25 at 32768 of 128, 97 / 96 at 131072; 103 / 169 at 524288 of 33;
+  //     m = 100: 135 / 98 at 131072 of 128; m = 128: 107 / 92 of 128, 105 / 158 of 33
+  //   many short blocks: m = 16: 66 / 104 at 131072; m = 8: 14 / 25 at 16384; m = 4: 61 / 242.
+  const int cgroups = (c + 31) / 32;
+  const int64_t ctas = (int64_t)B * nblk * cgroups, length = (int64_t)m * c / (32 * cgroups);
+  const bool subsets = ctas <= 0x7FFFFFFF && m >= CR_SUBS && (ctas <= 8 * 148 || (m >= 64 && length >= (overlap ? 100 : 50)));
   dim3 grid((unsigned)(subsets ? ctas : ceil_div64(total, 128))), block(subsets ? 32 * CR_SUBS : 128);
 #define GO(T, TB, OV)                                                                           \
   do {                                                                                          \

@@ -224,3 +224,17 @@ def test_kda_chunks_at_the_lines_of_the_centre(kch, total, growth):
         assert float((s[b:b + 1, h:h + 1].double().cpu() - s_ref).norm() / s_ref.norm()) <= 1e-4
         e = (o[b:b + 1, :, h:h + 1].double().cpu() - o_ref).abs()
         assert bool((e <= o_ref.abs() * 2.0 ** -8 + 5e-4 * o_ref.abs().max().clamp_min(1.0)).all()), float(e.max())
+
+
+@pytest.mark.parametrize("c,m,blocks", [(128, 64, 300), (128, 100, 300), (33, 128, 600), (33, 100, 600), (64, 64, 600), (65, 72, 400)])
+def test_compression_of_many_long_blocks(kch, c, m, blocks):
+    """More than 1184 groups of 32 channels, blocks on either side of the lengths from which their rows are shared between warps, with
+    the overlap and without, and widths that leave lanes idle.  Bound as in test_compress_subsets."""
+    g = torch.Generator().manual_seed(c + m)
+    t = [torch.randn(2, blocks * m, c, generator=g) for _ in range(4)]
+    t[2][1, -m:], t[3][0, m:2 * m] = -1e30, 40.0
+    Ba, Bb = [torch.randn(m, c, generator=g) * 0.3 for _ in range(2)]
+    a = kch.csa_compress_kv_overlapped(*[x.to(DEV) for x in t], Ba.to(DEV), Bb.to(DEV), m)
+    assert float((a.double().cpu() - orc.compress_kv_overlapped(*t, Ba, Bb, m).double()).abs().max()) <= 2e-6
+    b = kch.csa_compress_kv(t[0].to(DEV), t[2].to(DEV), Ba.to(DEV), m)
+    assert float((b.double().cpu() - orc.compress_kv(t[0], t[2], Ba, m).double()).abs().max()) <= 2e-6
