@@ -228,13 +228,26 @@ class _FusedWeights:
         return w, False
 
 
+_every_module = torch.nn.modules.module      # hooks registered for all modules live there
+
+
+def _as_written(module, *methods):
+    """Does calling ``module`` run its class's code and nothing else?  Not where it is watched (by hooks of its own or for all
+    modules) or where its ``forward``, or one of ``methods``, was put on the instance."""
+    return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or _every_module._global_forward_hooks or _every_module._global_forward_pre_hooks
+                or _every_module._global_backward_hooks or _every_module._global_backward_pre_hooks
+                or "forward" in module.__dict__ or any(name in module.__dict__ for name in methods))
+
+
 def _plain_norm(norm):
     """A LayerNorm of the stack that nobody watches or replaces: its arithmetic may move into the layer's call."""
-    return type(norm) is _Fp32LayerNorm and not (norm._forward_hooks or norm._forward_pre_hooks)
+    return type(norm) is _Fp32LayerNorm and _as_written(norm)
 
 
-def _unwatched(layer):
-    return type(layer) in (CSAHybridLayer, HCAHybridLayer) and not (layer._forward_hooks or layer._forward_pre_hooks)
+def _plain_layer(layer):
+    """A layer of the stack that nobody watches or replaces: it may be called with the keywords of its own class."""
+    return type(layer) in (KDAHybridLayer, CSAHybridLayer, HCAHybridLayer) and _as_written(layer, "forward_functional")
 
 
 def _at_rest(w):
@@ -275,9 +288,9 @@ class KDAHybridLayer(nn.Module):
     def reset_conv_state(self):
         self._conv_lookback = None
 
-    def forward(self, x, state=None, residual=None, state_out=None, lookback_in_place=False, norm=None, _final_state=None):
+    def forward(self, x, state=None, residual=None, state_out=None, lookback_in_place=False, norm=None, **final):
         o, new_state, lb = self.forward_functional(x, state, self._conv_lookback, residual=residual, state_out=state_out,
-                                                   lookback_in_place=lookback_in_place, norm=norm, _final_state=_final_state)
+                                                   lookback_in_place=lookback_in_place, norm=norm, **final)
         self._conv_lookback = lb
         return o, new_state
 
@@ -593,13 +606,13 @@ class HybridKCHAttention(nn.Module):
             if kind == "kda":
                 # the pre-norm goes into the layer: LayerNorm + short conv are one kernel there
                 x, st, lb = layer.forward_functional(x, states[ki], lookbacks[ki], residual=x, norm=norm,
-                                                     _final_state=None if final is None else final[ki])
+                                                     **self._final_state(layer, final, ki))
                 states[ki] = st
                 new_lbs.append(lb)
                 ki += 1
             else:
-                # a layer that is watched by hooks sees what it always saw
-                x, _ = layer(x, None, residual=x, norm=norm) if _unwatched(layer) else layer(norm(x), None, residual=x)
+                # a layer that is watched or replaced sees what it always saw
+                x, _ = layer(x, None, residual=x, norm=norm) if _plain_layer(layer) else layer(norm(x), None, residual=x)
         return x, self._stacked(states, final), new_lbs
 
     def _final_states(self, x):
@@ -609,6 +622,11 @@ class HybridKCHAttention(nn.Module):
         cfg = self.cfg
         return torch.empty(self.n_kda_layers, x.shape[0], cfg.n_heads_v, cfg.head_dim_k, cfg.head_dim_v, dtype=torch.float32,
                            device=x.device)
+
+    @staticmethod
+    def _final_state(layer, final, ki):
+        """The keyword that offers a KDA layer its place in that buffer."""
+        return {"_final_state": final[ki]} if final is not None and _plain_layer(layer) else {}
 
     def _stacked(self, states, final):
         if self.n_kda_layers == 0:
@@ -978,7 +996,7 @@ class HybridDecoding(nn.Module):
             if kind == "kda":
                 # in place: the state and the conv lookback keep their addresses from token to token
                 x, st = layer(x, states[ki], residual=x, state_out=states[ki] if in_place else None,
-                              lookback_in_place=in_place, norm=norm, _final_state=None if final is None else final[ki])
+                              lookback_in_place=in_place, norm=norm, **model._final_state(layer, final, ki))
                 states[ki] = st
                 ki += 1
             else:

@@ -238,3 +238,90 @@ def test_compression_of_many_long_blocks(kch, c, m, blocks):
     assert float((a.double().cpu() - orc.compress_kv_overlapped(*t, Ba, Bb, m).double()).abs().max()) <= 2e-6
     b = kch.csa_compress_kv(t[0].to(DEV), t[2].to(DEV), Ba.to(DEV), m)
     assert float((b.double().cpu() - orc.compress_kv(t[0], t[2], Ba, m).double()).abs().max()) <= 2e-6
+
+
+def _small(kch, seed=3, T=70):
+    cfg = kch.HybridConfig(d_model=64, n_heads_qk=2, n_heads_v=2, head_dim_k=32, head_dim_v=32, csa_nh=2, csa_c=32, csa_dc=32, csa_nIh=2,
+                           csa_cI=16, csa_m=4, csa_topk=4, csa_sliding_window=8, hca_m2=16, hca_nh=2, hca_c=32, hca_dc=32,
+                           hca_sliding_window=8)
+    model = kch.HybridKCHAttention(cfg, 5)
+    model.load_state_dict(syn.hybrid_params(seed, cfg, 5, dtype=torch.float32, random_sink=True), strict=True)
+    return model.to(DEV).eval(), syn.hidden_states(seed + 1, 2, T, cfg.d_model, torch.float32).to(DEV)
+
+
+def _served(kch, model, x):
+    dec = kch.HybridDecoding(model=model)
+    dec.reset()
+    return torch.cat([dec(x[:, :60]), dec(x[:, 60:69]), dec(x[:, 69:])], 1)
+
+
+@pytest.mark.parametrize("where", [0, 3, 4])
+def test_a_layer_whose_forward_is_replaced_is_called_as_it_always_was(kch, where):
+    """A ``forward`` put on one layer of the stack: it gets the arguments that it got before the layers' own keywords came, for CSA
+    and HCA the normalised input, and its result is the sub-layer's."""
+    model, x = _small(kch)
+    want = model(x)
+    layer, seen = model.layers[where], []
+    plain = type(layer).forward if where else type(layer).forward_functional
+    if where == 0:          # the stack calls a KDA layer's functional form
+        def functional(x, state, lookback, *, residual=None, norm=None):
+            seen.append(x)
+            return plain(layer, x, state, lookback, residual=residual, norm=norm)
+        layer.forward_functional = functional
+    else:
+        def forward(x, state=None, residual=None):
+            seen.append(x)
+            return plain(layer, x, state, residual)
+        layer.forward = forward
+    model.reset_state()
+    got = model(x)
+    assert len(seen) == 1 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("how", ["instance", "hook", "pre_hook", "every"])
+@pytest.mark.parametrize("path", ["stack", "served"])
+def test_a_watched_or_replaced_norm_runs(kch, how, path):
+    """The pre-norms of the CSA and HCA layers, replaced on the instance, hooked, or hooked for all modules: what the program put there
+    takes part in every pass."""
+    model, x = _small(kch)
+    run = (lambda: model(x)) if path == "stack" else (lambda: _served(kch, model, x))
+    base = run()
+    model.reset_state()
+    calls, handles = [], []
+    for norm in (model.norms[3], model.norms[4]):
+        if how == "instance":
+            def forward(h, _n=norm):
+                calls.append(h.shape[1])
+                return type(_n).forward(_n, h) * 2.0
+            norm.forward = forward
+        elif how == "hook":
+            handles.append(norm.register_forward_hook(lambda mod, a, out: (calls.append(a[0].shape[1]), out * 2.0)[1]))
+        elif how == "pre_hook":
+            handles.append(norm.register_forward_pre_hook(lambda mod, a: (calls.append(a[0].shape[1]), (a[0].flip(-1),))[1]))
+    if how == "every":
+        watched = {id(model.norms[3]), id(model.norms[4])}
+        handles.append(torch.nn.modules.module.register_module_forward_hook(
+            lambda mod, a, out: (calls.append(a[0].shape[1]), out * 2.0)[1] if id(mod) in watched else None))
+    try:
+        got = run()
+    finally:
+        for h in handles:
+            h.remove()
+    assert calls == ([70, 70] if path == "stack" else [60, 60, 9, 9, 1, 1])
+    assert float((got - base).abs().max()) > 1e-3
+
+
+def test_hooks_for_all_modules_see_the_layers(kch):
+    """A hook registered for all modules meets the CSA and HCA layers with the input they always had, the normalised one."""
+    model, x = _small(kch)
+    want, seen = model(x), []
+    model.reset_state()
+    types = (type(model.layers[3]), type(model.layers[4]))
+    h = torch.nn.modules.module.register_module_forward_pre_hook(lambda mod, a: seen.append(a[0]) if isinstance(mod, types) else None)
+    try:
+        got = model(x)
+    finally:
+        h.remove()
+    assert torch.equal(got, want) and len(seen) == 2
+    for s in seen:
+        assert float(s.mean(-1).abs().max()) <= 1e-5 and abs(float(s.var(-1, unbiased=False).mean()) - 1.0) <= 1e-3
