@@ -357,7 +357,9 @@ class KDAHybridLayer(nn.Module):
         cfg = self.cfg
         B, T, _ = x.shape
         HV, V = cfg.n_heads_v, cfg.head_dim_v
-        if T >= 2 and _single(self.tp) and not lookback_in_place and (norm is None or _plain_norm(norm)):
+        # a program's own `project` is what runs, with the arguments that it always had
+        own = "project" not in self.__dict__ and type(self).project is KDAHybridLayer.project
+        if T >= 2 and own and _single(self.tp) and not lookback_in_place and (norm is None or _plain_norm(norm)):
             lb = conv_lookback if conv_lookback is None or conv_lookback.shape[0] == B else None
             got = layers.kda_layer(x, cfg, self._fused.get(self.q_proj.weight, self.k_proj.weight, self.v_proj.weight,
                                                            self.g_down.weight, self.beta.weight),
@@ -369,7 +371,7 @@ class KDAHybridLayer(nn.Module):
         raw_gate = use_chunk and cfg.kda_decay_scale > 0 and chunk_gate_supported(
             cfg.head_dim_k, cfg.head_dim_v, cfg.kda_chunk_size, -10.0, x.dtype)
         W = self.g_up.weight
-        if T == 1 and not use_chunk and x.is_cuda and W.dtype == x.dtype and step_gate_supported(B, HV, cfg.head_dim_k, V, x.dtype):
+        if T == 1 and own and not use_chunk and x.is_cuda and W.dtype == x.dtype and step_gate_supported(B, HV, cfg.head_dim_k, V, x.dtype):
             validate_kda_backend(cfg.kda_backend)
             q, k, v, gd, beta, new_lb, fused_step = self.project(x, conv_lookback, lookback_in_place, norm, gate_later=True)
             # (the kernel before is the fused projection, which does not write the gate's weights)

@@ -278,6 +278,21 @@ def test_a_layer_whose_forward_is_replaced_is_called_as_it_always_was(kch, where
     assert len(seen) == 1 and torch.equal(got, want)
 
 
+def test_a_kda_layer_whose_projection_is_replaced(kch):
+    """``project`` put on a KDA layer is what its passes run, over several tokens and over one."""
+    model, x = _small(kch)
+    layer, calls = model.layers[1], []
+    own = type(layer).project
+    want = _served(kch, model, x)
+
+    def project(x, conv_lookback, lookback_in_place=False, norm=None, raw_gate=False):
+        calls.append(x.shape[1])
+        return own(layer, x, conv_lookback, lookback_in_place, norm, raw_gate)
+    layer.project = project
+    got = _served(kch, model, x)
+    assert calls == [60, 9, 1] and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("how", ["instance", "hook", "pre_hook", "every"])
 @pytest.mark.parametrize("path", ["stack", "served"])
 def test_a_watched_or_replaced_norm_runs(kch, how, path):
