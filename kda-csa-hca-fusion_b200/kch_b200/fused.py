@@ -355,6 +355,7 @@ class KDAHybridLayer(nn.Module):
         """``_final_state``: where the caller would like the final state of a call over several tokens; the state that is
         returned tells whether it went there."""
         cfg = self.cfg
+        validate_kda_backend(cfg.kda_backend)       # for every path below
         B, T, _ = x.shape
         HV, V = cfg.n_heads_v, cfg.head_dim_v
         # a program's own `project` is what runs, with the arguments that it always had
@@ -372,7 +373,6 @@ class KDAHybridLayer(nn.Module):
             cfg.head_dim_k, cfg.head_dim_v, cfg.kda_chunk_size, -10.0, x.dtype)
         W = self.g_up.weight
         if T == 1 and own and not use_chunk and x.is_cuda and W.dtype == x.dtype and step_gate_supported(B, HV, cfg.head_dim_k, V, x.dtype):
-            validate_kda_backend(cfg.kda_backend)
             q, k, v, gd, beta, new_lb, fused_step = self.project(x, conv_lookback, lookback_in_place, norm, gate_later=True)
             # (the kernel before is the fused projection, which does not write the gate's weights)
             got = step_gate(q, k, v, gd, W, beta, scale=self._scale_value(), initial_state=state, state_out=state_out,

@@ -340,3 +340,12 @@ def test_hooks_for_all_modules_see_the_layers(kch):
     assert torch.equal(got, want) and len(seen) == 2
     for s in seen:
         assert float(s.mean(-1).abs().max()) <= 1e-5 and abs(float(s.var(-1, unbiased=False).mean()) - 1.0) <= 1e-3
+
+
+@pytest.mark.parametrize("T", [1, 5, 70])
+def test_an_unknown_kda_backend_is_refused_for_every_length(kch, T):
+    """A backend set after the configuration was made is named by the first pass, over one token, few or many."""
+    model, x = _small(kch)
+    model.cfg.kda_backend = "fla"
+    with pytest.raises(ValueError, match="kda_backend='fla'"):
+        model(x[:, :T])
