@@ -11,15 +11,19 @@ int kch_rownorm_groups(const void* x, int64_t ld, int groups, void* y, float* no
                        int out_dtype, void* stream);      // elementwise.cu
 
 namespace {
-struct Carve {                            // 256-byte aligned pieces of a workspace; with a null base it only counts
+// 256-byte aligned pieces of a workspace; with a null base it only counts.  The pieces behind `again(mark)` lie where those
+// behind `mark` did, which are not read any more when they are written (one stream, launch after launch).
+struct Carve {
   uint8_t* base;
-  int64_t used = 0;
+  int64_t used = 0, most = 0;
   explicit Carve(void* p) : base((uint8_t*)p) {}
   void* take(int64_t bytes) {
     void* p = base ? base + used : nullptr;
     used += (bytes + 255) & ~(int64_t)255;
+    if (used > most) most = used;
     return p;
   }
+  void again(int64_t mark) { used = mark; }
 };
 inline int64_t esize(int dtype) { return dtype == KCH_BF16 ? 2 : 4; }
 inline const void* at(const void* p, int64_t elems, int dtype) { return (const uint8_t*)p + elems * esize(dtype); }
@@ -118,20 +122,20 @@ static int64_t csa_carve(const kch_csa_layer_args* a, void* base, CsaWs* w) {
   const int64_t rows = (int64_t)l->B * l->T, es = esize(l->dtype), nb = (int64_t)l->B * a->T_blocks;
   const int64_t ks = esize(attend_key_dtype(l->dtype, a->c, a->nh, a->scale));
   Carve c(base);
-  w->xn = l->norm_w ? c.take(rows * l->d * es) : nullptr;
   w->w = a->W ? nullptr : c.take((int64_t)a->n_w * l->d * es);
   w->wq = a->Wq ? nullptr : c.take((int64_t)a->n_q * a->dc * es);
   w->proj = a->proj ? a->proj : c.take(rows * a->n_w * es);
   w->qq = c.take(rows * a->n_q * es);
   w->comp = a->comp ? a->comp : (float*)c.take(nb * a->c * 4);
   w->kcomp = a->kcomp ? a->kcomp : (float*)c.take(nb * a->c_I * 4);
-  w->comp_n = c.take(nb * a->c * ks);
-  w->local = a->sliding_window > 0 ? c.take(rows * a->c * ks) : nullptr;
-  w->core = a->l.W_o ? c.take(rows * a->nh * a->c * es) : nullptr;
-  w->idx = w->qn = w->kn = w->wf = w->topk = nullptr;
+  w->idx = a->topk > 0 ? c.take(rows * a->topk * 4) : nullptr;
+  // the input projection's operand, then what the selection needs, then what the attention does
+  const int64_t mark = c.used;
+  w->xn = l->norm_w ? c.take(rows * l->d * es) : nullptr;
+  c.again(mark);
+  w->qn = w->kn = w->wf = w->topk = nullptr;
   w->topk_bytes = 0;
   if (a->topk > 0) {
-    w->idx = c.take(rows * a->topk * 4);
     w->kn = c.take(nb * a->c_I * 4);
     w->wf = c.take(rows * a->nIh * 4);
     if (csa_raw_q(a)) {
@@ -142,7 +146,11 @@ static int64_t csa_carve(const kch_csa_layer_args* a, void* base, CsaWs* w) {
     }
     w->topk = c.take(w->topk_bytes);
   }
-  return c.used;
+  c.again(mark);
+  w->comp_n = c.take(nb * a->c * ks);
+  w->local = a->sliding_window > 0 ? c.take(rows * a->c * ks) : nullptr;
+  w->core = a->l.W_o ? c.take(rows * a->nh * a->c * es) : nullptr;
+  return c.most;
 }
 static int csa_checks(const kch_csa_layer_args* a) {
   LY_GO(layer_checks(&a->l, "kch_csa_layer"));
@@ -223,15 +231,17 @@ static int64_t hca_carve(const kch_hca_layer_args* a, void* base, HcaWs* w) {
   const int64_t rows = (int64_t)l->B * l->T, es = esize(l->dtype), nb = (int64_t)l->B * a->T_blocks;
   const int64_t ks = esize(attend_key_dtype(l->dtype, a->c, a->nh, a->scale));
   Carve c(base);
-  w->xn = l->norm_w ? c.take(rows * l->d * es) : nullptr;
   w->w = a->W ? nullptr : c.take((int64_t)a->n_w * l->d * es);
   w->proj = a->proj ? a->proj : c.take(rows * a->n_w * es);
   w->q = c.take(rows * a->nh * a->c * es);
   w->comp = a->comp ? a->comp : (float*)c.take(nb * a->c * 4);
+  const int64_t mark = c.used;            // the input projection's operand, then what the attention needs
+  w->xn = l->norm_w ? c.take(rows * l->d * es) : nullptr;
+  c.again(mark);
   w->comp_n = c.take(nb * a->c * ks);
   w->local = a->sliding_window > 0 ? c.take(rows * a->c * ks) : nullptr;
   w->core = l->W_o ? c.take(rows * a->nh * a->c * es) : nullptr;
-  return c.used;
+  return c.most;
 }
 extern "C" int64_t kch_hca_layer_workspace_bytes(const kch_hca_layer_args* a) {
   HcaWs w;
@@ -290,14 +300,16 @@ static int64_t kda_carve(const kch_kda_layer_args* a, void* base, KdaWs* w) {
   const kch_layer_common* l = &a->l;
   const int64_t rows = (int64_t)l->B * l->T, es = esize(l->dtype);
   Carve c(base);
-  w->xn = l->norm_w && !kda_fused_norm(a) ? c.take(rows * l->d * es) : nullptr;
-  w->xc = c.take(rows * l->d * es);
   w->proj = c.take(rows * a->n_w * es);
   w->g = c.take(rows * a->HV * a->K * es);
   w->o = c.take(rows * a->HV * a->V * es);
+  const int64_t mark = c.used;            // the input projection's operand, then the chunk records
+  w->xn = l->norm_w && !kda_fused_norm(a) ? c.take(rows * l->d * es) : nullptr;
+  w->xc = c.take(rows * l->d * es);
+  c.again(mark);
   w->chunk_bytes = kda_chunked(a) ? kch_kda_chunk_workspace_bytes(l->B, l->T, a->HV, a->K, a->V, a->chunk_size) : 0;
   w->chunk = c.take(w->chunk_bytes);
-  return c.used;
+  return c.most;
 }
 extern "C" int64_t kch_kda_layer_workspace_bytes(const kch_kda_layer_args* a) {
   KdaWs w;

@@ -618,8 +618,9 @@ class HybridKCHAttention(nn.Module):
         return x, self._stacked(states, final), new_lbs
 
     def _final_states(self, x):
-        """One buffer for the final states of all KDA layers of a call over several tokens."""
-        if self.n_kda_layers == 0 or x.shape[1] < 2 or not x.is_cuda:
+        """One buffer for the final states of all KDA layers of a call over several tokens (a rank of several holds only its heads'
+        states, which the steps give)."""
+        if self.n_kda_layers == 0 or x.shape[1] < 2 or not x.is_cuda or not all(_single(getattr(layer, "tp", None)) for layer in self.layers):
             return None
         cfg = self.cfg
         return torch.empty(self.n_kda_layers, x.shape[0], cfg.n_heads_v, cfg.head_dim_k, cfg.head_dim_v, dtype=torch.float32,

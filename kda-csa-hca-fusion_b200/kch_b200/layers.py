@@ -1,14 +1,21 @@
 """One call per layer: the argument structures of ``kch_csa_layer``, ``kch_hca_layer`` and ``kch_kda_layer``.
 
 Each function takes a call whose shapes are the ordinary ones of its layer and returns ``None`` for any other, which the
-caller then runs step by step (and which names what is wrong with it, where something is).  Same kernels, same order, same
-results either way; here the launches are issued by the library instead of by Python.
+caller then runs step by step (and which names what is wrong with it, where something is).  The same results to the bit either
+way: the operators are the same kernels with the same operands, and what Python leaves to torch between them (weights laid one
+after the other, a slice widened to fp32) is exact.  Here the launches are issued by the library instead of by Python.
 """
 from __future__ import annotations
 
 import torch
 
 from . import _lib
+
+
+# Bytes of intermediate results up to which a call is issued as one.  They come as one block that lives as long as the call; step
+# by step each is freed as soon as it has been read, and the host work that one call saves (0.2 ms a layer) hides behind the
+# kernels long before: writing this much takes longer.
+WORKSPACE_LIMIT = 1 << 30
 
 
 def _tag(dt):
@@ -74,9 +81,12 @@ def _out_ok(W_o, width, residual, x):
 def _run(a, size_fn, call_fn, x):
     with _lib.device(x.device):
         need = size_fn(a)
+        if need > WORKSPACE_LIMIT:
+            return False
         ws = torch.empty(need, dtype=torch.uint8, device=x.device)       # (the caching allocator's blocks start on 512 bytes)
         a.l.workspace, a.l.workspace_bytes = ws.data_ptr(), need
         _lib.check(call_fn(a, _lib.stream()))
+    return True
 
 
 def csa_layer(x, weights, Ba, Bb, B_idx, sink, *, m, topk, nh, nIh, c, c_I, dc, scale, sliding_window, W=None, Wq=None, norm=None,
@@ -128,7 +138,8 @@ def csa_layer(x, weights, Ba, Bb, B_idx, sink, *, m, topk, nh, nIh, c, c_I, dc, 
     if sink is not None:
         a.sink, a.sink_dtype = sink.data_ptr(), _tag(sink.dtype)
     lib = _lib.load()
-    _run(a, lib.kch_csa_layer_workspace_bytes, lib.kch_csa_layer, x)
+    if not _run(a, lib.kch_csa_layer_workspace_bytes, lib.kch_csa_layer, x):
+        return None
     return out, proj, rows
 
 
@@ -170,7 +181,8 @@ def hca_layer(x, weights, B_pos, sink, *, m2, nh, c, dc, scale, sliding_window, 
     if sink is not None:
         a.sink, a.sink_dtype = sink.data_ptr(), _tag(sink.dtype)
     lib = _lib.load()
-    _run(a, lib.kch_hca_layer_workspace_bytes, lib.kch_hca_layer, x)
+    if not _run(a, lib.kch_hca_layer_workspace_bytes, lib.kch_hca_layer, x):
+        return None
     return out, proj, rows
 
 
@@ -207,5 +219,6 @@ def kda_layer(x, cfg, W, W_gup, W_o, conv_w, conv_b, state, lookback, *, scale, 
     a.W, a.ld_w, a.n_w, a.W_gup, a.ld_wg = W.data_ptr(), W.stride(0), W.shape[0], W_gup.data_ptr(), W_gup.stride(0)
     a.state, a.state_out = _lib.ptr(state), new_state.data_ptr()
     lib = _lib.load()
-    _run(a, lib.kch_kda_layer_workspace_bytes, lib.kch_kda_layer, x)
+    if not _run(a, lib.kch_kda_layer_workspace_bytes, lib.kch_kda_layer, x):
+        return None
     return out, new_state, new_lookback

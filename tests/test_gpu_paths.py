@@ -349,3 +349,50 @@ def test_an_unknown_kda_backend_is_refused_for_every_length(kch, T):
     model.cfg.kda_backend = "fla"
     with pytest.raises(ValueError, match="kda_backend='fla'"):
         model(x[:, :T])
+
+
+def _peak(f):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    f()
+    torch.cuda.synchronize()
+    return torch.cuda.max_memory_allocated() - base
+
+
+@pytest.mark.parametrize("kind", ["kda", "csa", "hca"])
+@pytest.mark.parametrize("B,T", [(1, 4096), (2, 16384)])
+def test_layer_calls_hold_no_more_memory_than_the_steps(kch, monkeypatch, kind, B, T):
+    """A layer of width 1024 as one call and step by step.  The one call allocates its output before its intermediate results instead
+    of behind them, and rounds each of those (a dozen) up to 512 bytes: that much more at its peak and no further; calls whose
+    intermediate results pass the limit of the one-call form hold what the steps hold."""
+    from kch_b200 import layers
+    cfg = kch.HybridConfig(d_model=1024, n_heads_qk=8, n_heads_v=8, head_dim_k=128, head_dim_v=128, csa_nh=8, csa_c=128, csa_dc=128,
+                           csa_nIh=4, csa_cI=64, csa_m=4, csa_topk=512, csa_sliding_window=128, hca_m2=128, hca_nh=8, hca_c=128,
+                           hca_dc=128, hca_sliding_window=128)
+    model = kch.HybridKCHAttention(cfg, 5).bfloat16().to(DEV).eval()
+    i = {"kda": 0, "csa": 3, "hca": 4}[kind]
+    layer, norm = model.layers[i], model.norms[i]
+    x = syn.hidden_states(5, B, T, cfg.d_model, torch.bfloat16).to(DEV)
+
+    def run():
+        with torch.no_grad():
+            if kind == "kda":
+                return layer.forward_functional(x, None, None, residual=x, norm=norm)
+            return layer(x, None, residual=x, norm=norm)
+    run()
+    names = ("csa_layer", "hca_layer", "kda_layer")
+    own, taken = {n: getattr(layers, n) for n in names}, []
+    for n in names:
+        monkeypatch.setattr(layers, n, lambda *a, _f=own[n], **kw: (lambda got: (taken.append(got is not None), got)[1])(_f(*a, **kw)))
+    one = _peak(run)
+    for n in names:
+        monkeypatch.setattr(layers, n, lambda *a, **kw: None)
+    steps = _peak(run)
+    assert one <= steps + (B * T * cfg.d_model * 2 + 16 * 512 if taken[0] else 0), (one, steps, taken)
+    if (B, T) == (2, 16384):
+        for n in names:
+            monkeypatch.setattr(layers, n, own[n])
+        monkeypatch.setattr(layers, "WORKSPACE_LIMIT", 1 << 20)
+        assert _peak(run) <= steps
