@@ -396,3 +396,20 @@ def test_layer_calls_hold_no_more_memory_than_the_steps(kch, monkeypatch, kind, 
             monkeypatch.setattr(layers, n, own[n])
         monkeypatch.setattr(layers, "WORKSPACE_LIMIT", 1 << 20)
         assert _peak(run) <= steps
+
+
+def test_bench_line_has_the_products():
+    """The bench line's ``roofline`` is that of the products of a pass: five layers have three (KDA: projection, gate, output) or
+    three (CSA, HCA: input, queries, output) each, whichever way the layers are issued."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.join(root, "bench.py"), "--batch", "1", "--seq-len", "512", "--steps", "2", "--warmup", "3",
+                        "--no-decode", "--no-cpu-baseline"], capture_output=True, text=True, timeout=300, check=True)
+    roof = json.loads(r.stdout.strip().splitlines()[-1])["roofline"]
+    assert roof["launches"] == 2 * 15 and roof["achieved"] > 0 and sum(s["launches"] for s in roof["shapes"]) == roof["launches"]
+    # 131072 tokens of the default workload have 131072 / 512 times these
+    per_token = sum(2.0 * n * k for n, k in [(6288, 2048), (2048, 128), (2048, 2048)] * 3)
+    assert roof["flops_per_step"] > 512 * per_token
