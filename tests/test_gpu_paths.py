@@ -413,3 +413,43 @@ def test_bench_line_has_the_products():
     # 131072 tokens of the default workload have 131072 / 512 times these
     per_token = sum(2.0 * n * k for n, k in [(6288, 2048), (2048, 128), (2048, 2048)] * 3)
     assert roof["flops_per_step"] > 512 * per_token
+
+
+@pytest.mark.parametrize("T", [64, 131])
+@pytest.mark.parametrize("change", [
+    dict(csa_nh=17, hca_nh=17), dict(csa_nh=16, hca_nh=16), dict(csa_c=64, hca_c=64), dict(csa_c=12, hca_c=20, csa_nh=1), dict(csa_cI=32),
+    dict(csa_topk=0), dict(csa_topk=200), dict(csa_sliding_window=0, hca_sliding_window=0), dict(d_model=264), dict(d_model=2304),
+    dict(d_model=512, dtype="fp32"), dict(head_dim_k=64, head_dim_v=64), dict(kda_chunk_size=16), dict(kda_decay_scale=0.0), dict(scale=16.5)],
+    ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
+def test_the_rules_of_the_one_call_layers_are_those_of_the_steps(kch, monkeypatch, change, T):
+    """Which key type, which form of the queries, of the norm and of the gate a layer takes is decided once in Python and once in the
+    library: on both sides of each of those lines the one call gives the bits of the steps."""
+    from kch_b200 import layers
+    change = dict(change)
+    dtype = torch.float32 if change.pop("dtype", "") == "fp32" else torch.bfloat16
+    scale = change.pop("scale", 1.0)
+    geo = dict(d_model=256, n_heads_qk=1, n_heads_v=2, head_dim_k=128, head_dim_v=128, csa_nh=2, csa_c=128, csa_dc=64, csa_nIh=2, csa_cI=64,
+               csa_m=4, csa_topk=16, csa_sliding_window=16, hca_m2=16, hca_nh=2, hca_c=128, hca_dc=64, hca_sliding_window=16)
+    cfg = kch.HybridConfig(**{**geo, **change})
+    model = kch.HybridKCHAttention(cfg, 5)
+    model.load_state_dict(syn.hybrid_params(7, cfg, 5, dtype=dtype, random_sink=True), strict=True)
+    model = model.to(dtype).to(DEV).eval()
+    x = syn.hidden_states(8, 2, T, cfg.d_model, dtype).to(DEV)
+    c, h = model.layers[3], model.layers[4]
+
+    def run():
+        y, S, lbs = model.forward_functional(x, None, [None] * 3)
+        ws = [getattr(c, n).weight for n in ("W_aKV", "W_bKV", "W_aZ", "W_bZ")]
+        a = kch.naive_csa(x, *ws, c.Ba, c.Bb, c.W_DQ.weight, c.W_UQ.weight, c.W_IUQ.weight, c.W_w.weight, c.W_KV_idx.weight, c.W_Z_idx.weight,
+                          c.B_idx, m=cfg.csa_m, topk=cfg.csa_topk, nh=cfg.csa_nh, nIh=cfg.csa_nIh, c=cfg.csa_c, c_I=cfg.csa_cI, dc=cfg.csa_dc,
+                          scale=scale, sliding_window=cfg.csa_sliding_window, use_ste=False, normalize_qk=True)
+        b = kch.naive_hca(x, h.W_KV.weight, h.W_Z.weight, h.B_pos, h.W_DQ.weight, h.W_UQ.weight, m2=cfg.hca_m2, nh=cfg.hca_nh, c=cfg.hca_c,
+                          dc=cfg.hca_dc, scale=scale, sliding_window=cfg.hca_sliding_window, sink_logits=h.sink)
+        return [y, S, *lbs, a, b]
+    with torch.no_grad():
+        one = run()
+        for name in ("csa_layer", "hca_layer", "kda_layer"):
+            monkeypatch.setattr(layers, name, lambda *a, **kw: None)
+        steps = run()
+    for got, want in zip(one, steps):
+        assert torch.equal(got, want), float((got.double() - want.double()).abs().max())
