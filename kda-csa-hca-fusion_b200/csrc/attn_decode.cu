@@ -679,7 +679,7 @@ extern "C" int kch_attend_decode_splits(int B) {
   // One wave of CTAs (three fit on an SM beside their tile rings): each warp then streams a few tiles through its
   // ring instead of paying the query set-up and a partial-result round trip for a single tile.
   // (KCH_DECODE_SPLITS=n overrides, for comparison.)
-  int s = forced > 0 ? forced : (3 * 148) / B;
+  int s = forced > 0 ? forced : (3 * KCH_SMS) / B;
   return s < 1 ? 1 : (s > AD_MAX_SPLITS ? AD_MAX_SPLITS : s);
 }
 
@@ -746,7 +746,7 @@ extern "C" int kch_attend_decode(const kch_attend_decode_args* p, void* stream) 
   // The merge is started early only where the CTAs before it leave it room: three of them fill an SM, and a grid that fills
   // more than nine SMs in ten leaves the early CTAs to crowd on the few others (HCA, 3000 rows a sequence, early / not: 10
   // sequences x 32 CTAs 18.9 / 20.7 us, 12 x 32 19.5 / 20.7, 32 x 13 26.5 / 22.9, 16 x 27 27.1 / 20.7).
-  if ((int64_t)S * p->B <= 3 * 148 * 9 / 10)
+  if ((int64_t)S * p->B <= 3 * KCH_SMS * 9 / 10)
     KCH_CUDA_OK(kch_launch_chained(attn_decode_combine_kernel, dim3(p->nh, p->B), dim3(AD_THREADS), 0, s, 1, a, S));
   else
     attn_decode_combine_kernel<<<dim3(p->nh, p->B), AD_THREADS, 0, s>>>(a, S);

@@ -427,7 +427,7 @@ static double am_gather_us(double queries, double entries) {
   return 10. + 1e-3 * entries * (ns > 48. ? ns : 48.);
 }
 static double am_mask_us(double queries, int nh, double topk, double last, double mean) {
-  const double rounds = queries / (nh <= 8 ? 16 : 8) / (2 * 148), chain = 11. * last, chip = (nh <= 8 ? 4.05e-3 : 8.1e-3) * queries * mean;
+  const double rounds = queries / (nh <= 8 ? 16 : 8) / (2 * KCH_SMS), chain = 11. * last, chip = (nh <= 8 ? 4.05e-3 : 8.1e-3) * queries * mean;
   return 10. + 1e-3 * (6.5 * topk * (rounds > 1. ? rounds : 1.) + (chip > chain ? chip : chain));
 }
 

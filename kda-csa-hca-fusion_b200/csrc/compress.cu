@@ -279,7 +279,7 @@ static int launch_compress(const void* Ca, const void* Za, const void* Cb, const
   //   many short blocks: m = 16: 66 / 104 at 131072; m = 8: 14 / 25 at 16384; m = 4: 61 / 242.
   const int cgroups = (c + 31) / 32;
   const int64_t ctas = (int64_t)B * nblk * cgroups, length = (int64_t)m * c / (32 * cgroups);
-  const bool subsets = ctas <= 0x7FFFFFFF && m >= CR_SUBS && (ctas <= 8 * 148 || (m >= 64 && length >= (overlap ? 100 : 50)));
+  const bool subsets = ctas <= 0x7FFFFFFF && m >= CR_SUBS && (ctas <= 8 * KCH_SMS || (m >= 64 && length >= (overlap ? 100 : 50)));
   dim3 grid((unsigned)(subsets ? ctas : ceil_div64(total, 128))), block(subsets ? 32 * CR_SUBS : 128);
 #define GO(T, TB, OV)                                                                           \
   do {                                                                                          \

@@ -39,7 +39,7 @@ __device__ __forceinline__ void cvt8(uint4& raw, float (&o)[8]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) { o[2 * k] = __uint_as_float(w[k] << 16); o[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
 }
-// 8 consecutive parameters; `vec`: they start on a 16-byte boundary (one or two 16-byte loads instead of eight narrow ones)
+// 8 consecutive values that start on a 16-byte boundary: one or two 16-byte loads
 template <typename TW>
 __device__ __forceinline__ void ld8p(const TW* p, float (&o)[8]) {
   if constexpr (sizeof(TW) == 2) {
@@ -52,6 +52,7 @@ __device__ __forceinline__ void ld8p(const TW* p, float (&o)[8]) {
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
   }
 }
+// ... and where only the caller knows whether they do (`vec`; eight narrow loads otherwise)
 template <typename TW>
 __device__ __forceinline__ void ld8p(const TW* p, float (&o)[8], bool vec) {
   if (vec) { ld8p(p, o); return; }

@@ -191,7 +191,7 @@ int kch_decode_indexer_logits_tc5(const void* q, int q_dtype, int64_t q_ld, cons
   // A CTA's set-up (query terms, tensor memory) is worth eight tiles of keys when there are enough of them to fill the chip
   // (two CTAs per SM); a small batch is spread thinner instead: 8 sequences of 4000 blocks took 11.3 us in 32 CTAs.
   int rows = IXD_ROWS;
-  while (rows > IXD_TILE && (int64_t)B * ((cap + rows - 1) / rows) < 2 * 148) rows >>= 1;
+  while (rows > IXD_TILE && (int64_t)B * ((cap + rows - 1) / rows) < 2 * KCH_SMS) rows >>= 1;
   dim3 grid((unsigned)((cap + rows - 1) / rows), (unsigned)B);
   KCH_CUDA_OK(kch_launch_chained(decode_indexer_tc5_kernel, grid, dim3(IXD_THREADS), smem, s, 1, kmap, q, q_dtype, q_ld, norms, w,
                                  w_dtype, w_ld, logits, cap, n_ld, HI, normalize, scale, m, ctr, rows, status));

@@ -7,6 +7,8 @@
 
 #include "../../include/kch_b200.h"
 
+#define KCH_SMS 148            // of the chip that these kernels are for: the unit of the dispatch rules that were measured on it
+
 // ---- error reporting -----------------------------------------------------------------
 void kch_set_error(const char* fmt, ...);
 void kch_note_launch(int n);   // host-side count of kernels launched by this library

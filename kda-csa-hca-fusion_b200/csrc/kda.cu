@@ -224,7 +224,7 @@ kda_decode_step_kernel(const T* q, const T* k, const T* v, const T* g, const T* 
 // Steps of up to two heads an SM: one row a thread, and the form that projects the gate itself.  Beyond that the 32 KB of weights
 // that every CTA reads cost as much as the launch that they save (64 sequences, 16 heads, whole step: 356 us with the launch, 360
 // without; 8 sequences: 199 and 185).
-static bool kds_few(int B, int HV) { return (int64_t)HV * B <= 2 * 148; }
+static bool kds_few(int B, int HV) { return (int64_t)HV * B <= 2 * KCH_SMS; }
 
 template <typename T, bool GATE>
 static int launch_kda_step(const T* q, const T* k, const T* v, const T* g, const T* beta, const float* S0, T* o, float* S_out, int B, int H,
@@ -1045,7 +1045,7 @@ static int kda_chunk_impl(const void* q, const void* k, const void* v, const voi
   cudaStream_t s = kch_stream(stream);
   // value columns of a CTA of the scan: 8, or 4 where twice the CTAs still get an SM each (beyond that two of them would share
   // one and read every operand row twice as often)
-  const int VS = (int64_t)((V + 3) / 4) * HV * B <= 148 ? 4 : 8;
+  const int VS = (int64_t)((V + 3) / 4) * HV * B <= KCH_SMS ? 4 : 8;
   // four elements a load: q, k, g (1), v (2)
   const int es = dtype == KCH_BF16 ? 2 : 4;
   const int vec = ((K % 4) == 0 && (ld_qk % 4) == 0 && (ld_g % 4) == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)g) % (4 * es)) == 0 ? 1 : 0) |

@@ -720,7 +720,7 @@ static int km_split(int B, int T, int HV) {
   if (seg_env == 0 || !kch_kda_scan_tc5_enabled()) return 0;
   const int NT = (T + KM_C - 1) / KM_C;
   const int64_t heads = (int64_t)B * HV;
-  if (heads > 148) return 0;
+  if (heads > KCH_SMS) return 0;
   const bool pays = NT >= 20 && 5 * (int64_t)NT >= 7 * heads && heads <= 40 && (heads <= 24 || NT <= (heads <= 28 ? 128 : 63));
   return pays || seg_env == 1 ? kch_kda_scan_segments((int)heads, NT) : 0;
 }

@@ -13,21 +13,19 @@
 // units); entries above the diagonal may overflow but are never read.  Down to -2 PT_GMAX, where the gate never grows, the
 // channels beyond are centred half way (EK and QG times 2^-c, Y times 2^c, w times 2^c again): the operator's own gates,
 // -softplus(N(0, 1)), decay a chunk by 2^-74 on average and past 2^-96 in some channel of one chunk in 40, and one CTA on the
-// other path holds up a whole wave (64 heads, 32 chunks, both stages: 262 us on that path, 240 now).  The centre is taken out of a channel's
-// prefix and total, outside the loop over elements, and whether the gate grows is asked in such chunks only: a chunk of the
-// model's gate pays for neither (240 us; 246 with both in its loops and an image loop for each).  Beyond that the CTA runs the mma.sync path,
-// which re-centres the exponents per 16 x 16 block.  Each product is hi*hi + lo*hi + hi*lo of two-term bf16 splits
-// with fp32 accumulation in tensor memory, as everywhere in the KDA kernels.
+// other path holds up a whole wave (64 heads, 32 chunks, both stages: 262 us on that path, 240 now).  The centre is taken out
+// of a channel's prefix and total, outside the loop over elements, and whether the gate grows is asked in such chunks only: a
+// chunk of the model's gate pays for neither (240 us; 246 with both in its loops and an image loop for each).  Beyond that the
+// CTA runs the mma.sync path, which re-centres the exponents per 16 x 16 block.  Each product is hi*hi + lo*hi + hi*lo of
+// two-term bf16 splits with fp32 accumulation in tensor memory, as everywhere in the KDA kernels.
 //
 // Data movement: g, k, q are read once by the threads that turn them into operand images (registers -> swizzled
-// shared-memory tiles, the QG / KG images also straight to the chunk record); V arrives
-// through a tensor map (cp.async.bulk.tensor, 128-byte swizzle) while the triangular solve runs; w leaves through shared memory as bulk
-// copies; u^T and Aqk are written from the tensor-memory epilogues.  EK serves twice: K-major as the row operand of
-// the first product, MN-major (the same bytes) as the A operand of the second.
+// shared-memory tiles, the QG / KG images also straight to the chunk record); V arrives through a tensor map
+// (cp.async.bulk.tensor, 128-byte swizzle) while the triangular solve runs; w leaves through shared memory as bulk copies; u^T
+// and Aqk are written from the tensor-memory epilogues.  EK serves twice: K-major as the row operand of the first product,
+// MN-major (the same bytes) as the A operand of the second.
 #pragma once
 #include <cudaTypedefs.h>
-
-#include <type_traits>
 
 #include "tc5_utils.cuh"
 

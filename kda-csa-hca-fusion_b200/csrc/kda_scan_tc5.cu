@@ -99,8 +99,8 @@ __device__ __forceinline__ void t5_stn(uint32_t taddr, const uint32_t* r) {
 }
 
 // SEG: segments of a sequence side by side (see the host part).  A kernel of its own: with the choices of a segment made at run
-// time, the chain of a whole sequence took 1.5 us more before its first chunk and 1 % of both stages (64 heads: 2 chunks 29.8 us, 31.6
-// with them; 128 chunks 842, 850).
+// time, the chain of a whole sequence took 1.5 us more before its first chunk and 1 % of both stages (64 heads: 2 chunks
+// 29.8 us, 31.6 with them; 128 chunks 842, 850).
 template <bool SEG>
 __global__ void __launch_bounds__(T5_THREADS, 1) kda_scan_tc5_kernel(T5Args a) {
   extern __shared__ uint8_t t5_raw[];
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256) kda_join_kernel(float* starts, const floa
 int kch_kda_scan_segments(int BH, int NT) {
   int best = 0;
   float best_us = 0.f;
-  for (int P = 3; BH > 0 && (int64_t)BH * (1 + 2 * (P - 2)) <= 148 && P <= NT; ++P) {
+  for (int P = 3; BH > 0 && (int64_t)BH * (1 + 2 * (P - 2)) <= KCH_SMS && P <= NT; ++P) {
     const int per = (NT + P - 1) / P;
     if ((NT + per - 1) / per != P) continue;         // the last segment would be empty
     const float us = (1.75f + 2.25f) * per + 2.f * P;

@@ -1,7 +1,8 @@
 // Whole layers in one call: the launches of a KDA, CSA or HCA layer over several tokens, issued from here one after the
 // other.  Every launch is one of the library's own entry points with the arguments that the Python wrappers give it; what
 // goes away is the host work between them (tensor objects, views, allocations and a ctypes call each: 15 to 20 us a launch,
-// which is more than most of these kernels take below ~4000 tokens).  Intermediate results lie in one caller workspace.
+// which is more than most of these kernels take below ~4000 tokens).  Intermediate results lie in one caller workspace, over one
+// another where one is dead before the next is written.
 #include <math.h>
 #include <string.h>
 
