@@ -976,7 +976,7 @@ struct IxSmem {
 };
 
 // c[t,h]: eight lanes a (query, head), 16 bytes a lane: four of them a warp instead of one after the other (2 x 10007 queries, 4
-// heads: 9.4 us one after the other).  The 32 pairs of squares are added by halves, pair p to pair p + 16 first, whatever lane holds them: the
+// heads took 9.4 us so; 131072 queries take 25).  The 32 pairs of squares are added by halves, pair p to pair p + 16 first, whatever lane holds them: the
 // lanes deal their four pairs out on the way.
 __global__ void __launch_bounds__(256) indexer_coef_kernel(const bf16* __restrict__ q, int64_t q_ld, const float* __restrict__ w,
                                                            float* __restrict__ coef, int64_t rows, int HI, float scale, int normalize) {
