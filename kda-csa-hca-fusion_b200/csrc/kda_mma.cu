@@ -710,10 +710,10 @@ bool kch_kda_mma_supported(int K, int V, int chunk_size, float g_clamp_min, int 
 //    1 head:   12 chunks 51 / 57  16: 61 / 62  [  20: 70 / 66    64: 190 / 99    512: 1203 / 273
 //    8 heads:  12 chunks 52 / 58  16: 61 / 62  [  20: 74 / 70    64: 203 / 136   512: 1293 / 591
 //   16 heads:  16 chunks 66 / 67  20: 88 / 92  [  24: 105 / 102  64: 236 / 176   512: 1408 / 1017
-//   24 heads:  24 chunks 119 / 122  28: 138 / 137 [ 40: 182 / 171  64: 259 / 240  512: 1528 / 1493
+//   24 heads:  24 chunks 119 / 122  28: 138 / 137 [ 32: 155 / 152  64: 259 / 240  512: 1528 / 1493
 //   28 heads:  28 chunks 147 / 148 [ 40: 193 / 183  64: 273 / 262  128: 471 / 458 ] 200: 675 / 674  512: 1590 / 1650
-//   32 heads:  40 chunks 204 / 201 [ 48: 241 / 230  63: 304 / 282 ] 64: 294 / 287  128: 484 / 521  300: 1025 / 1158
-//   40 heads:  48 chunks 262 / 259 [ 56: 309 / 301  63: 343 / 331 ] 64: 339 / 335  128: 577 / 609  300: 1221 / 1353
+//   32 heads:  32 chunks 166 / 165 [ 40: 204 / 201  63: 304 / 282 ] 64: 294 / 287  128: 484 / 521  300: 1025 / 1158
+//   40 heads:  40 chunks 225 / 228 [ 48: 262 / 259  63: 343 / 331 ] 64: 339 / 335  128: 577 / 609  300: 1221 / 1353
 //   49 heads:  56 chunks 340 / 338  63: 377 / 369  80: 454 / 457  128: 671 / 699: no segments
 static int km_split(int B, int T, int HV) {
   static const int seg_env = [] { const char* e = getenv("KCH_KDA_SPLIT"); return e ? atoi(e) : -1; }();
@@ -721,7 +721,7 @@ static int km_split(int B, int T, int HV) {
   const int NT = (T + KM_C - 1) / KM_C;
   const int64_t heads = (int64_t)B * HV;
   if (heads > KCH_SMS) return 0;
-  const bool pays = NT >= 20 && 5 * (int64_t)NT >= 7 * heads && heads <= 40 && (heads <= 24 || NT <= (heads <= 28 ? 128 : 63));
+  const bool pays = NT >= 20 && 5 * (int64_t)NT >= 4 * heads + 56 && heads <= 40 && (heads <= 24 || NT <= (heads <= 28 ? 128 : 63));
   return pays || seg_env == 1 ? kch_kda_scan_segments((int)heads, NT) : 0;
 }
 
