@@ -231,23 +231,31 @@ class _FusedWeights:
 _every_module = torch.nn.modules.module      # hooks registered for all modules live there
 
 
-def _as_written(module, *methods):
-    """Does calling ``module`` run its class's code and nothing else?  Not where it is watched (by hooks of its own or for all
-    modules) or where its ``forward``, or one of ``methods``, was put on the instance."""
+_written = {}       # (class, method): as this file has it, see the end of the file
+
+
+def _own(module, cls, *methods):
+    """Are these methods of ``module`` the ones that this file gives ``cls``, replaced neither on the instance nor on a class?"""
+    return all(name not in module.__dict__ and getattr(type(module), name) is _written[cls, name] for name in methods)
+
+
+def _unwatched(module):
+    """Neither hooks of its own nor hooks for all modules see a call of ``module``."""
     return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
                 or _every_module._global_forward_hooks or _every_module._global_forward_pre_hooks
-                or _every_module._global_backward_hooks or _every_module._global_backward_pre_hooks
-                or "forward" in module.__dict__ or any(name in module.__dict__ for name in methods))
+                or _every_module._global_backward_hooks or _every_module._global_backward_pre_hooks)
 
 
 def _plain_norm(norm):
     """A LayerNorm of the stack that nobody watches or replaces: its arithmetic may move into the layer's call."""
-    return type(norm) is _Fp32LayerNorm and _as_written(norm)
+    return type(norm) is _Fp32LayerNorm and _unwatched(norm) and _own(norm, _Fp32LayerNorm, "forward")
 
 
 def _plain_layer(layer):
     """A layer of the stack that nobody watches or replaces: it may be called with the keywords of its own class."""
-    return type(layer) in (KDAHybridLayer, CSAHybridLayer, HCAHybridLayer) and _as_written(layer, "forward_functional")
+    cls = type(layer)
+    return (cls in (KDAHybridLayer, CSAHybridLayer, HCAHybridLayer) and _unwatched(layer)
+            and (_own(layer, cls, "forward", "forward_functional") if cls is KDAHybridLayer else _own(layer, cls, "forward")))
 
 
 def _at_rest(w):
@@ -359,7 +367,7 @@ class KDAHybridLayer(nn.Module):
         B, T, _ = x.shape
         HV, V = cfg.n_heads_v, cfg.head_dim_v
         # a program's own `project` is what runs, with the arguments that it always had
-        own = "project" not in self.__dict__ and type(self).project is KDAHybridLayer.project
+        own = _own(self, KDAHybridLayer, "project")
         if T >= 2 and own and _single(self.tp) and not lookback_in_place and (norm is None or _plain_norm(norm)):
             lb = conv_lookback if conv_lookback is None or conv_lookback.shape[0] == B else None
             got = layers.kda_layer(x, cfg, self._fused.get(self.q_proj.weight, self.k_proj.weight, self.v_proj.weight,
@@ -476,7 +484,7 @@ class CSAHybridLayer(nn.Module):
             x, norm = norm(x), None
         if _rows_mode(self.tp):
             return _forward_by_rows(self, x, residual), None
-        if _single(self.tp) and "core" not in self.__dict__ and type(self).core is CSAHybridLayer.core:
+        if _single(self.tp) and _own(self, CSAHybridLayer, "core"):
             cfg = self.cfg
             got = layers.csa_layer(x, None, self.Ba, self.Bb, self.B_idx, self.sink, m=cfg.csa_m, topk=cfg.csa_topk, nh=cfg.csa_nh,
                                    nIh=cfg.csa_nIh, c=cfg.csa_c, c_I=cfg.csa_cI, dc=cfg.csa_dc, scale=1.0,
@@ -524,7 +532,7 @@ class HCAHybridLayer(nn.Module):
             x, norm = norm(x), None
         if _rows_mode(self.tp):
             return _forward_by_rows(self, x, residual), None
-        if _single(self.tp) and "core" not in self.__dict__ and type(self).core is HCAHybridLayer.core:
+        if _single(self.tp) and _own(self, HCAHybridLayer, "core"):
             cfg = self.cfg
             got = layers.hca_layer(x, None, self.B_pos, self.sink, m2=cfg.hca_m2, nh=cfg.hca_nh, c=cfg.hca_c, dc=cfg.hca_dc,
                                    scale=1.0, sliding_window=cfg.hca_sliding_window, W=self.fused_weight(), Wq=self.W_UQ.weight,
@@ -813,7 +821,7 @@ class HybridDecoding(nn.Module):
         """The first tokens of a session through a CSA / HCA layer: pre-norm, operator, output projection and residual in one
         call, whose projections and compressed rows fill the cache.  None where that call does not apply."""
         if (not _single(layer.tp) or not _plain_norm(norm) or type(layer) not in (CSAHybridLayer, HCAHybridLayer)
-                or "core" in layer.__dict__):
+                or not _own(layer, type(layer), "core")):
             return None
         cache = self._cache(i, layer, x)
         if cache.n_tokens_seen > 0:
@@ -1010,3 +1018,8 @@ class HybridDecoding(nn.Module):
         if T > 0 and not in_place:
             model._kda_state = model._stacked(states, final)
         return x
+
+
+for _cls, _names in ((_Fp32LayerNorm, ("forward",)), (KDAHybridLayer, ("forward", "forward_functional", "project")),
+                     (CSAHybridLayer, ("forward", "core")), (HCAHybridLayer, ("forward", "core"))):
+    _written.update({(_cls, _name): getattr(_cls, _name) for _name in _names})

@@ -453,3 +453,47 @@ def test_the_rules_of_the_one_call_layers_are_those_of_the_steps(kch, monkeypatc
         steps = run()
     for got, want in zip(one, steps):
         assert torch.equal(got, want), float((got.double() - want.double()).abs().max())
+
+
+@pytest.mark.parametrize("what", ["kda.forward_functional", "kda.project", "csa.forward", "csa.core", "hca.forward", "hca.core", "norm.forward"])
+@pytest.mark.parametrize("path", ["stack", "served"])
+def test_methods_replaced_on_the_class_run(kch, monkeypatch, what, path):
+    """The same for a method that a program replaces on the class, with the arguments that it had before the layers' own keywords."""
+    if path == "served" and what in ("csa.forward", "hca.forward"):
+        pytest.skip("a served session calls the operators of these layers")
+    model, x = _small(kch)
+    run = (lambda: model(x)) if path == "stack" else (lambda: _served(kch, model, x))
+    want = run()
+    model.reset_state()
+    kind, name = what.split(".")
+    cls = type(model.norms[0] if kind == "norm" else model.layers[{"kda": 0, "csa": 3, "hca": 4}[kind]])
+    own, calls = getattr(cls, name), []
+    if name == "core":
+        def method(self, x, *, return_projections=False, q_rows=None):
+            calls.append(x.shape[1])
+            return own(self, x, return_projections=return_projections, q_rows=q_rows)
+    elif name == "project":
+        def method(self, x, conv_lookback, lookback_in_place=False, norm=None, raw_gate=False):
+            calls.append(x.shape[1])
+            return own(self, x, conv_lookback, lookback_in_place, norm, raw_gate)
+    elif name == "forward_functional":
+        def method(self, x, state, lookback, *, residual=None, state_out=None, lookback_in_place=False, norm=None):
+            calls.append(x.shape[1])
+            return own(self, x, state, lookback, residual=residual, state_out=state_out, lookback_in_place=lookback_in_place, norm=norm)
+    elif kind == "norm":
+        def method(self, x):
+            calls.append(x.shape[1])
+            return own(self, x)
+    else:
+        def method(self, x, state=None, residual=None):
+            calls.append(x.shape[1])
+            return own(self, x, state, residual)
+    monkeypatch.setattr(cls, name, method)
+    got = run()
+    assert torch.equal(got, want)
+    per = {"kda": 3, "csa": 1, "hca": 1, "norm": 5}[kind]
+    lengths = [70] if path == "stack" else [60] if name == "core" else [60, 9, 1]      # (a later chunk does not call `core`)
+    if kind == "norm":                                     # fp32: LayerNorm and conv are two kernels, so all five norms run
+        assert sorted(calls) == sorted(lengths * per)
+    else:
+        assert calls == [n for n in lengths for _ in range(per)]
